@@ -315,6 +315,43 @@ int axi_fd_transform_f64(double* out, int ld_out, const double* in, int ld_in,
                          const double* Er_inv_w, const double* EzinvT, const double* inv_eig,
                          const double* Er, const double* EzT, double* work, int nr, int nz,
                          void* stream);
+/* ---------------------------------------------------------------------
+ * FP64 products on the tcgen05 tensor cores by integer slicing: each operand
+ * row is scaled by a power of two and written as nine signed 7-bit digits;
+ * products of digit planes are exact in the FP32 accumulators and summed as
+ * integers, with one rounding to FP64. A row or column that holds a value
+ * which is not finite gives NaN.
+ *
+ * The transform of axi_fd_transform_f64 with its bases sliced once:
+ * axi_sliced_transform_plan writes a plan of axi_sliced_transform_bytes into
+ * device memory (the four bases, its scratch and tables; synchronises the
+ * stream; the bases may be freed afterwards, inv_eig may not);
+ * axi_sliced_transform_run applies it (eight launches, no host round trip;
+ * `out` may alias `in`; calls on one plan share its scratch, so overlapping
+ * calls race). axi_sliced_transform_status reads the error word of its
+ * bounded waits (0: none ran out).
+ * ------------------------------------------------------------------ */
+int64_t axi_sliced_transform_bytes(int nr, int nz);
+int axi_sliced_transform_plan(void* plan, const double* Er_inv_w, const double* EzinvT,
+                              const double* inv_eig, const double* Er, const double* EzT, int nr,
+                              int nz, void* stream);
+int axi_sliced_transform_run(const void* plan, double* out, int ld_out, const double* in,
+                             int ld_in, int nr, int nz, void* stream);
+int axi_sliced_transform_status(const void* plan, int nr, int nz, int* error, void* stream);
+/* C (M, N) = A (M, K) * B (N, K)^T, optionally .* S (M, N), all row-major
+ * double, both operands sliced by this call. work: device scratch of
+ * axi_sliced_gemm_work_bytes. Synchronises the stream. */
+int64_t axi_sliced_gemm_work_bytes(int M, int N, int K);
+int axi_sliced_gemm_f64(double* C, const double* A, const double* B, const double* S, int M, int N,
+                        int K, void* work, void* stream);
+/* One sliced left operand (rows, K), element (i, k) at
+ * src[i * row_stride + k * k_stride]: dst takes axi_sliced_operand_bytes.
+ * Synchronises the stream. */
+int64_t axi_sliced_operand_bytes(int rows, int K);
+int axi_slice_operand_f64(void* dst, const double* src, int64_t row_stride, int64_t k_stride,
+                          int rows, int K, void* stream);
+/* Bytes of the sliced (nr, nz) field that a case of the double engine keeps. */
+int64_t axi_sliced_field_bytes(int nr, int nz);
 /* FP32 GEMM on the tcgen05 tensor cores with 3xTF32 split products (FP32
  * accuracy): C (M, N) = A (M, K) * B (N, K)^T, all row-major float, K a
  * multiple of 4. work: device scratch of axi_tf32x3_gemm_work_bytes(M, N, K)

@@ -59,6 +59,15 @@ def _signatures():
         "axi_fd_transform_static_max_cells": (I64, []),
         "axi_fd_transform_static_f64": (I, [P, I, P, I, P, P, P, P, P, I, I, P]),
         "axi_dgemm_f64": (I, [P, I, P, I, P, I, P, I, I, I, P]),
+        "axi_sliced_transform_bytes": (I64, [I, I]),
+        "axi_sliced_transform_plan": (I, [P, P, P, P, P, P, I, I, P]),
+        "axi_sliced_transform_run": (I, [P, P, I, P, I, I, I, P]),
+        "axi_sliced_transform_status": (I, [P, I, I, P, P]),
+        "axi_sliced_gemm_work_bytes": (I64, [I, I, I]),
+        "axi_sliced_gemm_f64": (I, [P, P, P, P, I, I, I, P, P]),
+        "axi_sliced_operand_bytes": (I64, [I, I]),
+        "axi_slice_operand_f64": (I, [P, P, I64, I64, I, I, P]),
+        "axi_sliced_field_bytes": (I64, [I, I]),
         "axi_tf32x3_gemm_work_bytes": (I64, [I, I, I]),
         "axi_tc_transform_plan": (I, [P, I, P, P, P]),
         "axi_tc_transform_run": (I, [P, P, P]),
