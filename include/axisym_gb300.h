@@ -539,6 +539,10 @@ typedef struct axi_case {
    * differences of neighbouring psi values keep the refined solve's
    * accuracy instead of the float rounding of psi. Start at zero. */
   void* psi_lo;
+  /* AXI_PLAN_SLICED: E_z^-1, E_r^-1 diag(r), E_z, E_r as sliced left operands
+   * (axi_slice_operand_f64) and a scratch of axi_sliced_field_bytes(nr, nz). */
+  const void* sliced_basis[4];
+  void* sliced_field;
 } axi_case;
 
 /* Launch choices of a plan that change the scheduling of the work, never its
@@ -578,6 +582,7 @@ typedef struct axi_plan_info {
   int32_t n_tc_tiles[4];   /* tensor-core tiles per spectral stage */
   int32_t n_dct_items;     /* row groups of the z transforms (AXI_PLAN_DCT_Z) */
   axi_tuning tune;         /* launch choices (zero: defaults) */
+  int32_t n_slice_items[2]; /* row groups sliced before the z / r products (AXI_PLAN_SLICED) */
 } axi_plan_info;
 
 /* AXI_PLAN_DCT_Z: the z-direction products run as orthonormal DCT-II /
@@ -595,7 +600,10 @@ typedef struct axi_plan_info {
  * the velocity kernels read back as psi + psi_lo. The solve error then
  * shrinks with the step-to-step change of psi instead of with psi itself; the
  * first solve of a case is the plain solve. Needs psi_lo. */
-enum { AXI_PLAN_TENSOR_CORES = 1, AXI_PLAN_DCT_Z = 2, AXI_PLAN_REFINE = 4 };
+/* AXI_PLAN_SLICED (double fields, neither of the flags above): the four
+ * products on the tensor cores by integer slicing, on the bases that
+ * sliced_basis holds. */
+enum { AXI_PLAN_TENSOR_CORES = 1, AXI_PLAN_DCT_Z = 2, AXI_PLAN_REFINE = 4, AXI_PLAN_SLICED = 8 };
 
 /* Host only: validates the cases, assigns each its first tile
  * (cases[k].stencil_tile0) and fills `info` (sizes of the plan). flags:

@@ -11,7 +11,8 @@
 // Launches per step, each covering every case of the plan:
 //   kill_reset   one block per case: sine tapers, free stream of this step,
 //                counters cleared, float copies of the step scalars
-//   transform    four grouped dense products (the spectral Poisson solve)
+//   transform    the spectral Poisson solve (float: two DCTs and two tensor-core
+//                products, or four products; double: four sliced products)
 //   vel_max      persistent, per tile: max(|u_z| + |u_r|) into the case
 //   step_dt      one thread per case: dt and the dt-dependent constants
 //   penalise     per tile: velocity + Brinkman + omega + curl(u_pen - u)
@@ -36,6 +37,7 @@
 #include "axi_common.cuh"
 #include "dct.cuh"
 #include "dct64.cuh"
+#include "sliced_gemm.cuh"
 #include "tc_gemm.cuh"
 #include "tma.cuh"
 
@@ -1534,6 +1536,9 @@ struct PlanView {
   const axi_dct::DctJob* dct_jobs;  // forward jobs, then inverse jobs (n_cases each)
   const int4* dct_items;
   const axi_dct64::Job* dct64_jobs;  // double engine: forward, then inverse jobs
+  const axi_sl::SliceJob* slice_jobs;  // AXI_PLAN_SLICED: four per case
+  const axi_sl::GemmJob* sliced_jobs;
+  const int4* slice_items[4];
   int* err;
 };
 
@@ -1542,6 +1547,7 @@ inline size_t align128(size_t x) { return (x + 127) & ~size_t(127); }
 
 struct PlanOffsets {
   size_t stencil, gemm, maps, jobs, tc_tiles[4], dct_jobs, dct_items, err, total;
+  size_t slice_jobs, sliced_jobs, slice_items[4];
 };
 
 // Plan buffer: cases | stencil tiles | SIMT GEMM tiles | stencil tensor maps
@@ -1574,6 +1580,19 @@ inline PlanOffsets plan_offsets(const axi_plan_info* info) {
   } else {
     o.dct_jobs = o.dct_items = 0;
   }
+  if (info->flags & AXI_PLAN_SLICED) {
+    o.slice_jobs = align16(end);
+    o.sliced_jobs = align16(o.slice_jobs + (size_t)4 * info->n_cases * sizeof(axi_sl::SliceJob));
+    end = o.sliced_jobs + (size_t)4 * info->n_cases * sizeof(axi_sl::GemmJob);
+    for (int st = 0; st < 4; ++st) {
+      o.slice_items[st] = align16(end);
+      o.tc_tiles[st] = o.slice_items[st] + (size_t)info->n_slice_items[st % 2] * sizeof(int4);
+      end = o.tc_tiles[st] + (size_t)info->n_tc_tiles[st] * sizeof(int4);
+    }
+  } else {
+    o.slice_jobs = o.sliced_jobs = 0;
+    for (int st = 0; st < 4; ++st) o.slice_items[st] = 0;
+  }
   o.err = align16(end);
   end = o.err + 16;
   o.total = align16(end);
@@ -1589,9 +1608,17 @@ inline PlanView plan_view(const void* plan_dev, const axi_plan_info* info) {
   v.gemm = reinterpret_cast<const int4*>(base + o.gemm);
   v.maps = reinterpret_cast<const CUtensorMap*>(base + o.maps);
   const bool tc = (info->flags & AXI_PLAN_TENSOR_CORES) != 0;
+  const bool sliced = (info->flags & AXI_PLAN_SLICED) != 0;
   v.jobs = tc ? reinterpret_cast<const axi_tc::TcJob*>(base + o.jobs) : nullptr;
   for (int st = 0; st < 4; ++st)
-    v.tc_tiles[st] = tc ? reinterpret_cast<const int4*>(base + o.tc_tiles[st]) : nullptr;
+    v.tc_tiles[st] =
+        (tc || sliced) ? reinterpret_cast<const int4*>(base + o.tc_tiles[st]) : nullptr;
+  v.slice_jobs =
+      sliced ? reinterpret_cast<const axi_sl::SliceJob*>(base + o.slice_jobs) : nullptr;
+  v.sliced_jobs =
+      sliced ? reinterpret_cast<const axi_sl::GemmJob*>(base + o.sliced_jobs) : nullptr;
+  for (int st = 0; st < 4; ++st)
+    v.slice_items[st] = sliced ? reinterpret_cast<const int4*>(base + o.slice_items[st]) : nullptr;
   const bool dct = (info->flags & AXI_PLAN_DCT_Z) != 0;
   const bool dbl = info->elem_bytes == 8;
   v.dct_jobs =
@@ -1857,6 +1884,13 @@ struct StencilGrid {
   }
 };
 
+// One of the four products of the double engine on sliced operands: its field
+// operand sliced, then the product.
+int run_sliced(const axi_plan_info* info, const PlanView& v, int st, cudaStream_t s) {
+  AXI_TRY(axi_sl::launch_slice(v.slice_jobs, v.slice_items[st], info->n_slice_items[st % 2], s));
+  return axi_sl::launch_gemm(v.sliced_jobs, v.tc_tiles[st], info->n_tc_tiles[st], v.err, s);
+}
+
 template <typename T>
 int run_phase(int phase, const axi_plan_info* info, const PlanView& v, cudaStream_t s) {
   const int nt = info->n_stencil_tiles, ng = info->n_gemm_tiles;
@@ -1876,6 +1910,10 @@ int run_phase(int phase, const axi_plan_info* info, const PlanView& v, cudaStrea
                                 false, s, info->tune.prefetch_waves));
         AXI_TRY(axi_tc::launch(v.jobs, v.tc_tiles[3], info->n_tc_tiles[3], v.err, s,
                                info->tune.tc_ctas_percent));
+        break;
+      }
+      if (v.sliced_jobs) {
+        for (int st = 0; st < 4; ++st) AXI_TRY(run_sliced(info, v, st, s));
         break;
       }
       if (v.jobs) {
@@ -1933,7 +1971,9 @@ int run_phase(int phase, const axi_plan_info* info, const PlanView& v, cudaStrea
     case PH_TRANSFORM_PART0 + 2:
     case PH_TRANSFORM_PART0 + 3: {
       const int st = phase - PH_TRANSFORM_PART0;
-      if (v.dct_jobs && (st == 0 || st == 2)) {
+      if (v.sliced_jobs) {
+        AXI_TRY(run_sliced(info, v, st, s));
+      } else if (v.dct_jobs && (st == 0 || st == 2)) {
         AXI_TRY(axi_dct::launch(st == 0 ? v.dct_jobs : v.dct_jobs + info->n_cases, v.dct_items,
                                 info->n_dct_items, st == 0, s, info->tune.prefetch_waves));
       } else if (v.dct64_jobs && (st == 0 || st == 2)) {
@@ -2059,6 +2099,11 @@ extern "C" int axi_plan_init(axi_case* cases, int n_cases, int elem_bytes, int f
     axi::set_error("plan_init: refinement belongs to the float engine");
     return AXI_ERR_INVALID;
   }
+  const bool sliced = (flags & AXI_PLAN_SLICED) != 0;
+  if (sliced && (elem_bytes != 8 || tc || dct)) {
+    axi::set_error("plan_init: sliced products are the double engine's, without other plan flags");
+    return AXI_ERR_INVALID;
+  }
   const axi_tuning tune = info->tune;  // the caller's launch choices survive re-planning
   memset(info, 0, sizeof(*info));
   info->tune = tune;
@@ -2100,13 +2145,24 @@ extern "C" int axi_plan_init(axi_case* cases, int n_cases, int elem_bytes, int f
       }
       nd += dct64_items_of(k);
     }
+    if (sliced) {
+      for (int st = 0; st < 4; ++st) {
+        if (!k.sliced_basis[st] || !k.sliced_field) {
+          axi::set_error("plan_init: case %d lacks sliced operands", c);
+          return AXI_ERR_INVALID;
+        }
+        const int M = st % 2 == 0 ? k.nz : k.nr, N = st % 2 == 0 ? k.nr : k.nz;
+        info->n_tc_tiles[st] += axi_sl::gemm_tiles(M, N);
+        if (st < 2) info->n_slice_items[st] += axi_sl::slice_items(N, axi_sl::KIND_B);
+      }
+    }
   }
   info->n_cases = n_cases;
   info->n_stencil_tiles = nt;
   info->n_gemm_tiles = ng;
   info->elem_bytes = elem_bytes;
   info->flags = (tc ? AXI_PLAN_TENSOR_CORES : 0) | (dct ? AXI_PLAN_DCT_Z : 0) |
-                (refine ? AXI_PLAN_REFINE : 0);
+                (refine ? AXI_PLAN_REFINE : 0) | (sliced ? AXI_PLAN_SLICED : 0);
   info->n_dct_items = nd;
   info->bytes = (int64_t)plan_offsets(info).total;
   return AXI_OK;
@@ -2230,6 +2286,33 @@ extern "C" int axi_plan_upload(const axi_case* cases, const axi_plan_info* info,
     if (q != info->n_dct_items) {
       axi::set_error("plan_upload: cases changed since plan_init");
       return AXI_ERR_INVALID;
+    }
+  }
+  if (info->flags & AXI_PLAN_SLICED) {
+    axi_sl::SliceJob* sj = reinterpret_cast<axi_sl::SliceJob*>(&buf[po.slice_jobs]);
+    axi_sl::GemmJob* gj = reinterpret_cast<axi_sl::GemmJob*>(&buf[po.sliced_jobs]);
+    std::vector<int4> items[4], tiles[4];
+    for (int c = 0; c < n; ++c) {
+      const axi_case& k = cases[c];
+      axi_sl::spectral_jobs(k.nr, k.nz, static_cast<const double*>(k.omega), k.nz,
+                            static_cast<double*>(k.psi), k.nz, static_cast<double*>(k.gemm_work),
+                            k.sliced_field, k.sliced_basis,
+                            static_cast<const double*>(k.inv_eig), sj + 4 * c, gj + 4 * c);
+      for (int st = 0; st < 4; ++st) {
+        const int M = st % 2 == 0 ? k.nz : k.nr, N = st % 2 == 0 ? k.nr : k.nz;
+        axi_sl::append_slice_items(items[st], 4 * c + st, N, axi_sl::KIND_B);
+        axi_sl::append_gemm_tiles(tiles[st], 4 * c + st, M, N, M);
+      }
+    }
+    for (int st = 0; st < 4; ++st) {
+      if ((int)items[st].size() != info->n_slice_items[st % 2] ||
+          (int)tiles[st].size() != info->n_tc_tiles[st]) {
+        axi::set_error("plan_upload: cases changed since plan_init");
+        return AXI_ERR_INVALID;
+      }
+      axi_sl::order_tiles(tiles[st]);
+      memcpy(&buf[po.slice_items[st]], items[st].data(), items[st].size() * sizeof(int4));
+      memcpy(&buf[po.tc_tiles[st]], tiles[st].data(), tiles[st].size() * sizeof(int4));
     }
   }
   cudaStream_t s = axi::as_stream(stream);

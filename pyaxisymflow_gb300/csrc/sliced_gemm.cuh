@@ -17,16 +17,23 @@
 // share accumulator d. Over K = 512 the accumulators 0 .. 7 stay within
 // 8 * 512 * 2^12 = 2^24 (exact), accumulator 8 (weight 2^-68) rounds in its
 // last bit. The epilogue adds the accumulators as integers (96 bits, exact for
-// any K) and rounds to FP64 once. Against products in long double the result
-// is 1e-16 of the row and column scales, where an FP64 FMA chain is at
-// 2-6e-16 (K = 48 .. 384); with eight digits the spectral solve lost a digit
-// in the velocities near the axis, whose psi is a cancelling sum.
+// any K) and rounds to FP64 once.
+//
+// Error of the four-product spectral solve against long double on the same
+// bases, 48 x 96 to 256 x 512 cells, smooth and white right-hand sides:
+// psi 0.8-2.0e-16 (FP64 FMA products 1.1-20e-16),
+// u_z 3-24e-16 (5-25e-16), u_r 4-53e-16 (8-76e-16), smaller in every case.
+// With eight digits psi stayed at 3-9e-16 but u_z and u_r went to 1-6e-14 (psi
+// near the axis is a cancelling sum), so nine are used.
 //
 // Why: GB300 executes FP64 at about 1.2 TFLOP/s and FP16 tensor work at about
 // 2 PFLOP/s. 45 plane products cost 45 * 2 M N K FP16 operations, 1/40 of the
 // time of the FP64 pipe. Measured, a soft-sphere step on 1024 x 512 cells (four
 // products): 4169 us with FP64 FMA products, 1143 us with these; a step of the
-// drop-in loop on 384 x 201 cells: 1178 and 488 us.
+// drop-in loop on 384 x 201 cells: 1178 and 488 us; a double engine step of
+// eight cases of 256 x 128 to 1024 x 512: 3543 us with FP64 DCTs in z and FMA
+// products in r, 837 us with four of these; of one 512 x 256 case 299 us
+// (553 with four FMA products) and 193 us.
 //
 // Operands are laid out by the slicing kernel exactly as shared memory wants
 // them: per block of rows and per 16 K-elements one contiguous piece (A: 128

@@ -17,8 +17,8 @@ import numpy as np
 import torch
 
 from . import _native as N
-from .kernels.FastDiagonalisationStokesSolver import FastDiagonalisationStokesSolver
-from .kernels._spectral import tf32_split
+from .kernels.FastDiagonalisationStokesSolver import stokes_operators
+from .kernels._spectral import eig_sorted_desc, radial_coord, tf32_split
 from .kernels.smooth_Heaviside import smooth_Heaviside
 
 ST_T, ST_DT, ST_CD, ST_STEPS, ST_UMAX, ST_COUNT, ST_STATUS, ST_FORCE = range(8)
@@ -55,6 +55,7 @@ class AxiCase(ctypes.Structure):
         ("tc_basis", ctypes.c_void_p * 8), ("tc_work", ctypes.c_void_p * 4),
         ("dct_table", ctypes.c_void_p),
         ("psi_lo", ctypes.c_void_p),
+        ("sliced_basis", ctypes.c_void_p * 4), ("sliced_field", ctypes.c_void_p),
     ]
 
 
@@ -167,12 +168,13 @@ class AxiPlanInfo(ctypes.Structure):
                 ("n_gemm_tiles", ctypes.c_int32), ("elem_bytes", ctypes.c_int32),
                 ("bytes", ctypes.c_int64), ("flags", ctypes.c_int32),
                 ("n_tc_tiles", ctypes.c_int32 * 4), ("n_dct_items", ctypes.c_int32),
-                ("tune", AxiTuning)]
+                ("tune", AxiTuning), ("n_slice_items", ctypes.c_int32 * 2)]
 
 
 PLAN_TENSOR_CORES = 1
 PLAN_DCT_Z = 2
 PLAN_REFINE = 4
+PLAN_SLICED = 8
 
 
 def dct_ok(nz, precision="f32"):
@@ -199,29 +201,48 @@ def dct_table(nz, dtype=np.float32):
     return np.concatenate([tw.ravel(), rot.ravel(), c, 1.0 / c]).astype(dtype)
 
 
+def cosine_basis(n):
+    """The orthonormal DCT-II matrix: row k is eigenvector k of the Neumann z
+    operator (angles reduced as integers, so every entry is rounded once)."""
+    q = np.outer(np.arange(n, dtype=np.int64), 2 * np.arange(n, dtype=np.int64) + 1) % (4 * n)
+    c = np.cos(q * (np.pi / (2 * n))) * np.sqrt(2.0 / n)
+    c[0] = np.sqrt(1.0 / n)
+    return c
+
+
 class _Bases:
     """Spectral bases shared by all cases with the same (nr, nz, dx).
 
     With `dct`, the z eigenbasis is the orthonormal DCT-II basis (the Neumann
-    z operator of the solver is diagonal in it): the z products become
-    transforms, inv_eig is 1 / (lambda_r_i + lambda_z_k) in DCT order and only
-    the radial operands are kept for the tensor cores."""
+    z operator of the solver is diagonal in it) and inv_eig is
+    1 / (lambda_r_i + lambda_z_k) in DCT order: the float engine's z products
+    become transforms and only its radial operands are kept for the tensor
+    cores. The double engine keeps all four bases as sliced operands."""
 
     def __init__(self, nr, nz, dx, dtype, device, tensor_cores=False, dct=False):
-        solver = FastDiagonalisationStokesSolver(nr, nz, dx, device=device)
-        d = solver.engine.dev
-        self.t = {k: d[k].to(dtype).contiguous() for k in
-                  ("Er", "Er_inv_w", "EzinvT", "EzT", "inv_eig")}
-        self.tc = []
-        self.dct_table = None
+        op_r, op_z = stokes_operators(nr, nz, dx)
+        vals_r, vecs_r = eig_sorted_desc(op_r)
         if dct:
-            lam_z = (2.0 - 2.0 * np.cos(np.pi * np.arange(nz) / nz)) / (dx * dx)
-            inv = 1.0 / (solver.engine.eig_vals_r.reshape(nr, 1) + lam_z.reshape(1, nz))
-            self.t["inv_eig"] = torch.tensor(inv, dtype=dtype, device=device)
-            self.dct_table = torch.tensor(
-                dct_table(nz, np.float64 if dtype == torch.float64 else np.float32), device=device)
+            vals_z = (2.0 - 2.0 * np.cos(np.pi * np.arange(nz) / nz)) / (dx * dx)
+            EzT = cosine_basis(nz)
+            EzinvT = EzT.T
+        else:
+            vals_z, vecs_z = eig_sorted_desc(op_z)
+            EzT, EzinvT = vecs_z.T, np.linalg.inv(vecs_z).T
+        h = dict(Er=vecs_r,
+                 Er_inv_w=np.linalg.inv(vecs_r) * radial_coord(dx, nr).reshape(1, nr),
+                 EzinvT=EzinvT, EzT=EzT,
+                 inv_eig=1.0 / (vals_z.reshape(1, nz) + vals_r.reshape(nr, 1)))
+        self.t = {k: torch.tensor(np.ascontiguousarray(v), dtype=dtype, device=device)
+                  for k, v in h.items()}
+        self.tc = []
+        self.sliced = []
+        self.dct_table = None
+        if dtype == torch.float64:
+            self._slice(device)
+        elif dct:
+            self.dct_table = torch.tensor(dct_table(nz, np.float32), device=device)
         if tensor_cores:
-            h = solver.engine.host
             # operands of the K-major tensor-core form (C = A B^T per stage):
             # E_z^-1, E_r^-1 diag(r), E_z, E_r (the z ones unused with dct)
             for k, m in enumerate((h["EzinvT"].T, h["Er_inv_w"], h["EzT"].T, h["Er"])):
@@ -231,6 +252,18 @@ class _Bases:
                 hi, lo = tf32_split(np.ascontiguousarray(m))
                 self.tc.append(torch.tensor(hi, device=device))
                 self.tc.append(torch.tensor(lo, device=device))
+
+    def _slice(self, device):
+        """E_z^-1, E_r^-1 diag(r), E_z, E_r as operands of the sliced products."""
+        for name, transposed in (("EzinvT", True), ("Er_inv_w", False), ("EzT", True),
+                                 ("Er", False)):
+            m = self.t[name]
+            n = m.shape[0]
+            out = torch.empty(int(N.lib().axi_sliced_operand_bytes(n, n)), dtype=torch.uint8,
+                              device=device)
+            N.call("axi_slice_operand_f64", N.ptr(out), N.ptr(m), 1 if transposed else n,
+                   n if transposed else 1, n, n, N.stream_of(out))
+            self.sliced.append(out)
 
 
 class CaseState:
@@ -282,6 +315,9 @@ class CaseState:
         if ens.tensor_cores:
             t["tc_work"] = [torch.zeros(c.nr * c.nz, dtype=torch.float32, device=dev)
                             for _ in range(4)]
+        if dtype == torch.float64:
+            t["sliced_field"] = torch.empty(int(N.lib().axi_sliced_field_bytes(c.nr, c.nz)),
+                                            dtype=torch.uint8, device=dev)
         if ens.refine:
             # low part of psi: the refined solve keeps psi as psi + psi_lo
             t["psi_lo"] = torch.zeros((c.nr, c.nz), dtype=torch.float32, device=dev)
@@ -325,8 +361,12 @@ class CaseState:
                 s.tc_basis[q] = b.tc[q].data_ptr() if b.tc[q] is not None else None
             for q in range(4):
                 s.tc_work[q] = t["tc_work"][q].data_ptr()
-        if ens.dct:
+        if b.dct_table is not None:
             s.dct_table = b.dct_table.data_ptr()
+        if dtype == torch.float64:
+            for q in range(4):
+                s.sliced_basis[q] = b.sliced[q].data_ptr()
+            s.sliced_field = t["sliced_field"].data_ptr()
         if ens.refine:
             s.psi_lo = t["psi_lo"].data_ptr()
         s.state = st.data_ptr()
@@ -383,10 +423,10 @@ class RigidEnsemble:
             raise ValueError("tensor-core products are for the f32 engine")
         cases = list(cases)
         if dct is None:
-            # z products as DCTs when every case's nz allows it (faster than
-            # the dense z products: tensor-core ones in the float engine, SIMT
-            # FP64 ones in the double engine); the float engine's DCT feeds
-            # the tensor-core radial products only
+            # z products on the cosine basis when every case's nz allows it:
+            # transforms in the float engine (faster than its dense z products;
+            # they feed the tensor-core radial products only), dense sliced
+            # products in the double engine
             dct = ((tensor_cores or precision == "f64")
                    and all(dct_ok(c.nz, precision) for c in cases))
         if dct and precision == "f32" and not tensor_cores:
@@ -483,8 +523,11 @@ class RigidEnsemble:
             return
         lib = N.lib()
         esize = 8 if self.precision == "f64" else 4
-        flags = ((PLAN_TENSOR_CORES if self.tensor_cores else 0) | (PLAN_DCT_Z if self.dct else 0)
-                 | (PLAN_REFINE if self.refine else 0))
+        if self.precision == "f64":
+            flags = PLAN_SLICED
+        else:
+            flags = ((PLAN_TENSOR_CORES if self.tensor_cores else 0)
+                     | (PLAN_DCT_Z if self.dct else 0) | (PLAN_REFINE if self.refine else 0))
         stream = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
         for idx in split_by_cells(self.cases, self.plan_group_count(n)):
             structs = (AxiCase * len(idx))()

@@ -21,6 +21,7 @@ from dataclasses import dataclass, field
 import numpy as np
 import torch
 
+from . import _native as N
 from .engine import TILE_NR, TILE_NZ, RigidBodyCase, RigidEnsemble
 
 
@@ -131,6 +132,8 @@ class SimulationServer:
                 n += 2 * blk(cells * 4)                  # omega's TF32 operand pair
         if ens.refine:
             n += blk(cells * 4)                          # psi_lo
+        if es == 8:
+            n += blk(int(N.lib().axi_sliced_field_bytes(nr, nz)))
         tiles = -(-nr // TILE_NR) * -(-nz // TILE_NZ)
         n += (blk(3 * case.kill_width * 8) + blk(nr * 8) + blk(nz * 8) + 3 * blk(nr * es)
               + blk(nz * es) + blk((2 * tiles + 8) * 8))

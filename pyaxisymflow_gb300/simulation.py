@@ -296,12 +296,11 @@ class SoftSphereEngine:
         self.graph = None
 
     def _setup_dct(self):
-        """The spectral solve with the z products as FP64 DCT-II / DCT-III row
-        transforms (the Neumann z operator is diagonal in the cosine basis;
-        psi does not depend on which eigenbasis diagonalises it): E_z^-1 and
-        E_z become O(nz log nz) per row, the radial products stay dense. psi
-        differs from the dense eigenvector products by ~1e-12 of a solve."""
-        from .engine import dct_ok, dct_table
+        """The spectral solve on the exact cosine basis in z (the Neumann z
+        operator is diagonal in it; psi does not depend on which eigenbasis
+        diagonalises it). psi differs from the LAPACK eigenvector products by
+        ~1e-12 of a solve."""
+        from .engine import cosine_basis, dct_ok
         N, s, c = self._N, self.sim, self.case
         nr, nz, dx = c.nr, c.nz, c.dx
         if not dct_ok(nz, "f64"):
@@ -312,32 +311,21 @@ class SoftSphereEngine:
         lam_z = (2.0 - 2.0 * np.cos(np.pi * np.arange(nz) / nz)) / (dx * dx)
         self.inv_eig_dct = torch.tensor(1.0 / (eng.eig_vals_r.reshape(nr, 1)
                                                + lam_z.reshape(1, nz)), **f64)
-        self.dct_tab = torch.tensor(dct_table(nz, np.float64), **f64)
-        self.w1 = torch.zeros((nr, nz), **f64)
-        self.w2 = torch.zeros((nr, nz), **f64)
-        nb = int(N.lib().axi_dct64_plan_bytes(nr, nz))
-        self.plan_fwd = torch.zeros(nb, dtype=torch.uint8, device=self.device)
-        self.plan_inv = torch.zeros(nb, dtype=torch.uint8, device=self.device)
-        st = N.stream_of(self.w1)
-        N.call("axi_dct64_plan_f64", N.ptr(s.vorticity), N.ptr(self.w1), nr, nz,
-               N.ptr(self.dct_tab), 1, N.ptr(self.plan_fwd), st)
-        N.call("axi_dct64_plan_f64", N.ptr(self.w2), N.ptr(self.w1), nr, nz,
-               N.ptr(self.dct_tab), 0, N.ptr(self.plan_inv), st)
+        EzT = torch.tensor(cosine_basis(nz), **f64)
+        self.plan_dct = torch.empty(int(N.lib().axi_sliced_transform_bytes(nr, nz)),
+                                    dtype=torch.uint8, device=self.device)
+        d = eng.dev
+        N.call("axi_sliced_transform_plan", N.ptr(self.plan_dct), N.ptr(d["Er_inv_w"]),
+               N.ptr(EzT.T.contiguous()), N.ptr(self.inv_eig_dct), N.ptr(d["Er"]), N.ptr(EzT), nr,
+               nz, N.stream_of(EzT))
 
     def _solve(self, st):
         N, s, c = self._N, self.sim, self.case
         if not self.dct:
             s.solver.solve(s.psi, s.vorticity)
             return
-        p = N.ptr
-        nr, nz = c.nr, c.nz
-        d = s.solver.engine.dev
-        N.call("axi_dct64_run_f64", p(self.plan_fwd), nr, nz, 1, st)
-        N.call("axi_dgemm_f64", p(self.w2), nz, p(d["Er_inv_w"]), nr, p(self.w1), nz,
-               p(self.inv_eig_dct), nr, nz, nr, st)
-        N.call("axi_dct64_run_f64", p(self.plan_inv), nr, nz, 0, st)
-        N.call("axi_dgemm_f64", p(s.psi), nz, p(d["Er"]), nr, p(self.w1), nz, None, nr, nz,
-               nr, st)
+        N.call("axi_sliced_transform_run", N.ptr(self.plan_dct), N.ptr(s.psi), c.nz,
+               N.ptr(s.vorticity), c.nz, c.nr, c.nz, st)
 
     # the launch groups of one step, in order (timed one at a time by phase())
     PARTS = ("solve_velocity_dt", "advect_pin_mask", "extrapolate", "solid_stress",
@@ -403,12 +391,12 @@ class SoftSphereEngine:
         with torch.cuda.stream(s):
             self._part(k, ctypes.c_void_p(s.cuda_stream))
 
-    # kernel launches of one step: kill (2), solve (4 products), velocity,
+    # kernel launches of one step: kill (2), solve (4 slicings, 4 products), velocity,
     # dt, eta advection, pin, omega advection, mask, extrapolation (prepare,
     # collect, 8 multi-block sweeps of 3 launches, the single-block finisher,
     # fold, copy back), stress, stress mask, div tau + curl (2), tether,
     # penalise (2), diffusion (2), advance
-    LAUNCHES_PER_STEP = (2 + 4 + 1 + 1 + 1 + 1 + 1 + 1 + (2 + 3 * 8 + 3) + 1 + 1 + 2 + 1 + 2
+    LAUNCHES_PER_STEP = (2 + 8 + 1 + 1 + 1 + 1 + 1 + 1 + (2 + 3 * 8 + 3) + 1 + 1 + 2 + 1 + 2
                          + 2 + 1)
 
     def step(self, n=1, stream=None):
