@@ -3,7 +3,9 @@
 
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <initializer_list>
 #include <string>
 
@@ -84,6 +86,58 @@ template <> __device__ __forceinline__ float rn_mul(float a, float b) { return _
 template <> __device__ __forceinline__ float rn_add(float a, float b) { return __fadd_rn(a, b); }
 template <> __device__ __forceinline__ float rn_sub(float a, float b) { return __fsub_rn(a, b); }
 template <> __device__ __forceinline__ float rn_div(float a, float b) { return __fdiv_rn(a, b); }
+
+// Division by a divisor that serves several quotients: the same correctly
+// rounded quotients as the / operator, for 4 FP64 instructions each instead of
+// about 20 (FP64 issues at 1/64 of the FP32 rate on GB300, so the FP64 stencils
+// are bound by exactly these). With the reciprocal held as y_h + y_l
+// (y_h = RN(1 / b), y_l its remainder), q = RN(a y_h + RN(a y_l)) is within one
+// unit of the quotient (Brisebarre, Muller and Raina, "Accelerating correctly
+// rounded floating-point division when the divisor is known in advance", IEEE
+// TC 53, 2004), so r = a - q b is exact and RN(q + r y_h) is correctly rounded
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM JRD 34, 1990). Dividends and divisors outside the exponent
+// range where all of it stays normal take the plain division; a zero dividend
+// gives its signed zero.
+template <typename T>
+struct KnownDivisor {
+  T b;
+  KnownDivisor() = default;
+  __host__ __device__ __forceinline__ explicit KnownDivisor(T d) : b(d) {}
+  __device__ __forceinline__ T quotient(T a) const { return rn_div(a, b); }
+};
+
+template <>
+struct KnownDivisor<double> {
+  double b, yh, yl;
+  int ok;
+  KnownDivisor() = default;
+  __host__ __device__ __forceinline__ explicit KnownDivisor(double d) : b(d) {
+#ifdef __CUDA_ARCH__
+    const unsigned int e = ((unsigned int)__double2hiint(d) >> 20) & 0x7ffu;
+    yh = __drcp_rn(d);
+    yl = __dmul_rn(__fma_rn(-yh, d, 1.0), yh);
+#else
+    unsigned long long bits;
+    memcpy(&bits, &d, sizeof(bits));
+    const unsigned int e = (unsigned int)(bits >> 52) & 0x7ffu;
+    yh = 1.0 / d;
+    yl = std::fma(-yh, d, 1.0) * yh;
+#endif
+    ok = e - 623u <= 800u;
+  }
+  __device__ __forceinline__ double quotient(double a) const {
+    const unsigned int hi = (unsigned int)__double2hiint(a);
+    if (ok) {
+      if (((hi >> 20) & 0x7ffu) - 523u <= 1000u) {
+        const double q = __fma_rn(a, yh, __dmul_rn(a, yl));
+        return __fma_rn(__fma_rn(-q, b, a), yh, q);
+      }
+      if (((hi << 1) | (unsigned int)__double2loint(a)) == 0) return __dmul_rn(a, yh);
+    }
+    return __ddiv_rn(a, b);
+  }
+};
 
 // Host-side product of two scalars (kept separate so no contraction applies).
 template <typename T> inline T rn_host_mul(T a, T b) { return a * b; }

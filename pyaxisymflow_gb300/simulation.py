@@ -392,12 +392,10 @@ class SoftSphereEngine:
             self._part(k, ctypes.c_void_p(s.cuda_stream))
 
     # kernel launches of one step: kill (2), solve (4 slicings, 4 products), velocity,
-    # dt, eta advection, pin, omega advection, mask, extrapolation (prepare,
-    # collect, 8 multi-block sweeps of 3 launches, the single-block finisher,
-    # fold, copy back), stress, stress mask, div tau + curl (2), tether,
-    # penalise (2), diffusion (2), advance
-    LAUNCHES_PER_STEP = (2 + 8 + 1 + 1 + 1 + 1 + 1 + 1 + (2 + 3 * 8 + 3) + 1 + 1 + 2 + 1 + 2
-                         + 2 + 1)
+    # dt, eta advection, pin, omega advection, mask, extrapolation (prepare, 8
+    # sweeps, finish), stress, stress mask, div tau + curl (2), tether, penalise
+    # (2), diffusion (2), advance
+    LAUNCHES_PER_STEP = 2 + 8 + 1 + 1 + 1 + 1 + 1 + 1 + 10 + 1 + 1 + 2 + 1 + 2 + 2 + 1
 
     def step(self, n=1, stream=None):
         """Advance n steps (asynchronous on `stream`, default torch's current)."""
