@@ -691,6 +691,10 @@ int axi_soft_extrapolate_eta_f64(const uint8_t* inside_solid, const double* ball
 /* sigma_ij *= chi (:236-238). */
 int axi_soft_stress_mask_f64(double* s11, double* s12, double* s22, const double* chi,
                              int64_t n, void* stream);
+/* axi_solid_sigma_f64 and then sigma *= chi, in one pass. */
+int axi_soft_stress_f64(double* s11, double* s12, double* s22, double G, double dx,
+                        const double* e1, const double* e2, double* e1z, double* e1r, double* e2z,
+                        double* e2r, const double* chi, int nr, int nz, void* stream);
 /* axi_update_vorticity_from_solid_stress_f64 with dt from the state (:239-241). */
 int axi_soft_update_vorticity_from_solid_stress_f64(double* vort, double* tau_z, double* tau_r,
                                                     const double* t11, const double* t12,

@@ -93,6 +93,7 @@ def _signatures():
         "axi_soft_mask_f64": (I, [P, P, P, I64, D, P]),
         "axi_soft_extrapolate_eta_f64": (
             I, [P, P, P, P, P, P, P, P, P, D, I, I, P, P, I, P, P, P]),
+        "axi_soft_stress_f64": (I, [P, P, P, D, D, P, P, P, P, P, P, P, I, I, P]),
         "axi_soft_stress_mask_f64": (I, [P, P, P, P, I64, P]),
         "axi_soft_update_vorticity_from_solid_stress_f64": (
             I, [P, P, P, P, P, P, P, I, I, D, P, P]),

@@ -139,6 +139,32 @@ struct KnownDivisor<double> {
   }
 };
 
+// Bit tests that need no FP64 instruction.
+__device__ __forceinline__ bool is_pos_zero(double x) { return __double_as_longlong(x) == 0; }
+__device__ __forceinline__ bool is_zero_bits(double x) { return (__double_as_longlong(x) << 1) == 0; }
+__device__ __forceinline__ int exponent_bits(double x) {
+  return (__double2hiint(x) >> 20) & 0x7ff;
+}
+// x with its sign flipped where `flip` (the compiler negates with an FP64 add)
+__device__ __forceinline__ double flip_sign(double x, bool flip) {
+  return __hiloint2double(__double2hiint(x) ^ (flip ? (int)0x80000000 : 0), __double2loint(x));
+}
+__device__ __forceinline__ float flip_sign(float x, bool flip) { return flip ? -x : x; }
+
+// Outside its blend band the smoothed Heaviside (kernels/smooth_Heaviside.py:10-14)
+// of a finite phi, from a finite old value, is exactly 1 or 0: the blend's
+// bracket is finite there and is multiplied by zero. True: `h` holds it (no
+// FP64 instruction); false: the caller evaluates the expression. w > 0, normal.
+__device__ __forceinline__ bool heaviside_outside(double h_old, double phi, double w, double& h) {
+  const long long a = __double_as_longlong(phi) & 0x7fffffffffffffffll;
+  if (exponent_bits(h_old) == 0x7ff || a < __double_as_longlong(w) ||
+      (int)(a >> 52) - exponent_bits(w) > 1000 || (a >> 52) > 1023 + 900 ||
+      (unsigned int)(exponent_bits(w) - 1) >= 0x7feu || __double_as_longlong(w) < 0)
+    return false;
+  h = __double_as_longlong(phi) >= 0 ? 1.0 : 0.0;
+  return true;
+}
+
 // Host-side product of two scalars (kept separate so no contraction applies).
 template <typename T> inline T rn_host_mul(T a, T b) { return a * b; }
 

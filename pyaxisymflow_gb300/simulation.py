@@ -362,10 +362,9 @@ class SoftSphereEngine:
                    p(self.flags[1]), float(c.extrap_zone), nr, nz, p(s.z), p(s.z),
                    self.max_sweeps, p(self.lsq_work), p(self.state), st)
         elif k == 3:
-            N.call("axi_solid_sigma_f64", p(s.s11), p(s.s12), p(s.s22), c.G, dx, p(s.eta1),
-                   p(s.eta2), p(s.e1z), p(s.e1r), p(s.e2z), p(s.e2r), nr, nz, st)
-            N.call("axi_soft_stress_mask_f64", p(s.s11), p(s.s12), p(s.s22),
-                   p(s.ball_char_func), n, st)
+            N.call("axi_soft_stress_f64", p(s.s11), p(s.s12), p(s.s22), c.G, dx, p(s.eta1),
+                   p(s.eta2), p(s.e1z), p(s.e1r), p(s.e2z), p(s.e2r), p(s.ball_char_func), nr, nz,
+                   st)
             N.call("axi_soft_update_vorticity_from_solid_stress_f64", p(w), p(s.tau_z),
                    p(s.tau_r), p(s.s11), p(s.s12), p(s.s22), p(s.R), nr, nz, dx, p(self.state),
                    st)
@@ -393,9 +392,9 @@ class SoftSphereEngine:
 
     # kernel launches of one step: kill (2), solve (4 slicings, 4 products), velocity,
     # dt, eta advection, pin, omega advection, mask, extrapolation (prepare, 8
-    # sweeps, finish), stress, stress mask, div tau + curl (2), tether, penalise
-    # (2), diffusion (2), advance
-    LAUNCHES_PER_STEP = 2 + 8 + 1 + 1 + 1 + 1 + 1 + 1 + 10 + 1 + 1 + 2 + 1 + 2 + 2 + 1
+    # sweeps, finish), stress, div tau + curl (2), tether, penalise (2), diffusion
+    # (2), advance
+    LAUNCHES_PER_STEP = 2 + 8 + 1 + 1 + 1 + 1 + 1 + 1 + 10 + 1 + 2 + 1 + 2 + 2 + 1
 
     def step(self, n=1, stream=None):
         """Advance n steps (asynchronous on `stream`, default torch's current)."""
