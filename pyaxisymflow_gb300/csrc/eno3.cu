@@ -20,90 +20,179 @@
 
 namespace {
 
-constexpr int BX = 32;
-constexpr int BY = 8;
+// Upwind selector u0 > -u1 (advection_flux.py:33). Doubles compare as integers
+// (sign and magnitude; zeros equal), which spares an FP64 instruction; NaN and
+// infinities take the comparison itself, out of line (inlined it would run for
+// every cell under a predicate, at full cost).
+__device__ __noinline__ bool upwind_plain(double u0, double u1) { return u0 > -u1; }
+__device__ __forceinline__ bool upwind(float u0, float u1) { return u0 > -u1; }
+__device__ __forceinline__ bool upwind(double u0, double u1) {
+  const long long b0 = __double_as_longlong(u0), b1 = __double_as_longlong(u1);
+  const long long m0 = b0 & 0x7fffffffffffffffll, m1 = b1 & 0x7fffffffffffffffll;
+  if (exponent_bits(u0) == 0x7ff || exponent_bits(u1) == 0x7ff) return upwind_plain(u0, u1);
+  return (b0 < 0 ? -m0 : m0) > (b1 < 0 ? m1 : -m1);
+}
 
-// Conservative face value of f*u between cells 0 and 1 (advection_flux.py:34-43).
+// Conservative face value of f*u between cells 0 and 1 (advection_flux.py:34-43):
+// the operands of the upwind side selected first, then evaluated once.
 template <typename T>
 __device__ __forceinline__ T face_cons(T fm1, T f0, T f1, T f2, T um1, T u0, T u1, T u2) {
   const T third = T(1) / T(3), five6 = T(5) / T(6), sixth = T(1) / T(6);
-  if (u0 > -u1) {
-    T a = rn_add(rn_mul(rn_mul(third, f1), u1), rn_mul(rn_mul(five6, f0), u0));
-    return rn_sub(a, rn_mul(rn_mul(sixth, fm1), um1));
-  }
-  T a = rn_add(rn_mul(rn_mul(third, f0), u0), rn_mul(rn_mul(five6, f1), u1));
-  return rn_sub(a, rn_mul(rn_mul(sixth, f2), u2));
+  const bool l = upwind(u0, u1);
+  const T a = rn_add(rn_mul(rn_mul(third, l ? f1 : f0), l ? u1 : u0),
+                     rn_mul(rn_mul(five6, l ? f0 : f1), l ? u0 : u1));
+  return rn_sub(a, rn_mul(rn_mul(sixth, l ? fm1 : f2), l ? um1 : u2));
 }
 
 // Non-conservative face value of f between cells 0 and 1 (advection_flux.py:193-199).
 template <typename T>
-__device__ __forceinline__ T face_noncons(T fm1, T f0, T f1, T f2, T u0, T u1) {
+__device__ __forceinline__ T face_noncons(T fm1, T f0, T f1, T f2, bool l) {
   const T third = T(1) / T(3), five6 = T(5) / T(6), sixth = T(1) / T(6);
-  if (u0 > -u1) return rn_sub(rn_add(rn_mul(third, f1), rn_mul(five6, f0)), rn_mul(sixth, fm1));
-  return rn_sub(rn_add(rn_mul(third, f0), rn_mul(five6, f1)), rn_mul(sixth, f2));
+  return rn_sub(rn_add(rn_mul(third, l ? f1 : f0), rn_mul(five6, l ? f0 : f1)),
+                rn_mul(sixth, l ? fm1 : f2));
 }
 
-// Value of a mirrored field at (row, col), row >= -2: rows below the axis are
-// parity * row (-1 - row).
+// A reference-map cell of a warp (all lanes call it): its new value. Out of
+// line, so that none of it runs ahead of the test for an all-zero warp.
 template <typename T>
-__device__ __forceinline__ T mir(const T* __restrict__ f, int row, int col, int nz, T parity) {
-  return row >= 0 ? f[(long long)row * nz + col] : parity * f[(long long)(-1 - row) * nz + col];
+__device__ __noinline__ T noncons_cell(T fm1, T f0, T f1, T f2, T gm2, T gm1, T g1, T g2, T v0, T v1,
+                                       T wm1, T w0, T w1, T a, bool inner) {
+  const T xf = face_noncons(fm1, f0, f1, f2, upwind(v0, v1));
+  const T xb = __shfl_up_sync(0xffffffffu, xf, 1);
+  const T yf = face_noncons(gm1, f0, g1, g2, upwind(w0, w1));
+  const T yb = face_noncons(gm2, gm1, f0, g1, upwind(wm1, w0));
+  T flux = T(0);
+  flux = rn_add(flux, rn_mul(rn_mul(a, xf), v0));
+  flux = rn_sub(flux, rn_mul(rn_mul(a, xb), v0));
+  flux = rn_add(flux, rn_mul(rn_mul(a, yf), w0));
+  flux = rn_sub(flux, rn_mul(rn_mul(a, yb), w0));
+  return rn_add(f0, inner ? flux : T(0));
 }
+
+// 0 for +0 only
+__device__ __forceinline__ unsigned int value_bits(float x) { return __float_as_uint(x); }
+__device__ __forceinline__ unsigned int value_bits(double x) {
+  return (unsigned int)__double2hiint(x) | (unsigned int)__double2loint(x);
+}
+__device__ __forceinline__ bool finite_bits(float x) {
+  return (__float_as_uint(x) & 0x7f800000u) != 0x7f800000u;
+}
+__device__ __forceinline__ bool finite_bits(double x) { return exponent_bits(x) != 0x7ff; }
 
 // One Euler step for NF fields sharing the velocity (u_z even, u_r odd).
-// src[k] holds the pre-step copy of field k, dst[k] receives the new values.
+// src[k] holds the pre-step copy of field k, dst[k] (a copy of it on entry)
+// receives the new values.
+//
+// Bound by FP64 issue in the double form. A z face serves its two cells: a
+// warp covers 31 cells of a row, lane l holding the face behind its cell and
+// passing it to lane l + 1 (lane 0 only forms a face). The conservative form
+// also walks up `strip` rows keeping the r face between them: 25 instructions
+// per cell where forming all four faces took 56. A warp whose reference-map
+// stencils are all +0 (outside the solid and its extrapolation band) leaves
+// them without any. Measured at 1024 x 512: omega 60 -> 43 us, both eta fields
+// 90 -> 18 us.
+constexpr int ENO_WARPS = 8;   // warps per block, one strip of rows each
+constexpr int ENO_COLS = 31;   // cells per warp
+
 template <typename T, int NF, bool CONS>
-__global__ void eno3_step_kernel(T* __restrict__ dst0, T* __restrict__ dst1,
-                                 const T* __restrict__ src0, const T* __restrict__ src1,
-                                 T par0, T par1, const T* __restrict__ uz,
-                                 const T* __restrict__ ur, int nr, int nz, T a,
-                                 const double* __restrict__ dt_dev, T dx) {
-  const int j = blockIdx.x * BX + threadIdx.x;
-  const int i = blockIdx.y * BY + threadIdx.y;
-  if (i >= nr || j >= nz) return;
+__global__ void __launch_bounds__(32 * ENO_WARPS)
+    eno3_step_kernel(T* __restrict__ dst0, T* __restrict__ dst1, const T* __restrict__ src0,
+                     const T* __restrict__ src1, bool odd0, bool odd1, const T* __restrict__ uz,
+                     const T* __restrict__ ur, int nr, int nz, T a,
+                     const double* __restrict__ dt_dev, T dx, int strip) {
+  __shared__ T s_a;
   // a device-resident time step (the soft-sphere loop): a = -(dt / dx)
-  if (dt_dev) a = -rn_div(static_cast<T>(dt_dev[0]), dx);
-  const long long c = (long long)i * nz + j;
-  const bool interior = (i < nr - 2) && (j >= 2) && (j < nz - 2);
+  if (threadIdx.x == 0 && threadIdx.y == 0)
+    s_a = dt_dev ? -rn_div(static_cast<T>(dt_dev[0]), dx) : a;
+  __syncthreads();
+  a = s_a;
+  const int lane = threadIdx.x;
+  const int j = blockIdx.x * ENO_COLS - 1 + lane;
+  const int first = (blockIdx.y * ENO_WARPS + threadIdx.y) * strip;
+  const int last = min(first + strip, nr);
+  const bool cell = lane > 0 && j < nz;
+  const bool inner_j = lane > 0 && j >= 2 && j <= nz - 3;
+  // Every load of a row is unconditional (columns and rows clamped into the
+  // grid, the clamped values unused), so that all are in flight at once.
+  auto col = [nz](int x) { return min(max(x, 0), nz - 1); };
+  const int cm2 = col(j - 2), cm1 = col(j - 1), c0 = col(j), c1 = col(j + 1), c2 = col(j + 2);
+  // rows i - 2 .. i + 2 at column j; below the axis mirrored
+  auto below2 = [=](int i) { return (long long)(i >= 2 ? i - 2 : 1 - i) * nz + c0; };
+  auto below1 = [=](int i) { return (long long)(i >= 1 ? i - 1 : -i) * nz + c0; };
+  T yb = T(0);  // conservative: r face below row i
+  if (CONS && first < last) {
+    const long long c = (long long)first * nz + c0, up = (long long)min(first + 1, nr - 1) * nz + c0;
+    yb = face_cons(flip_sign(src0[below2(first)], odd0 && first < 2),
+                   flip_sign(src0[below1(first)], odd0 && first < 1), src0[c], src0[up],
+                   flip_sign(ur[below2(first)], first < 2), flip_sign(ur[below1(first)], first < 1),
+                   ur[c], ur[up]);
+  }
+  for (int i = first; i < last; ++i) {
+    const long long row = (long long)i * nz;
+    const long long rm2 = below2(i), rm1 = below1(i);
+    const long long r1 = (long long)min(i + 1, nr - 1) * nz + c0;
+    const long long r2 = (long long)min(i + 2, nr - 1) * nz + c0;
+    const bool inner = inner_j && i <= nr - 3;
+    const T v0 = uz[row + c0], v1 = uz[row + c1];
+    const T w0 = ur[row + c0], w1 = ur[r1];
+    const T wm1 = flip_sign(ur[rm1], i < 1);
+    T vm1 = T(0), v2 = T(0), w2 = T(0);
+    if (CONS) {
+      vm1 = uz[row + cm1];
+      v2 = uz[row + c2];
+      w2 = ur[r2];
+    }
+    T fm2[NF], fm1[NF], f0[NF], f1[NF], f2[NF], gm2[NF], gm1[NF], g1[NF], g2[NF];
+    // every value of the stencils +0 (tested as integers: a comparison with zero
+    // would be an FP64 instruction per value)
+    unsigned int zero_bits = 0;
 #pragma unroll
-  for (int k = 0; k < NF; ++k) {
-    const T* __restrict__ src = k == 0 ? src0 : src1;
-    T* __restrict__ dst = k == 0 ? dst0 : dst1;
-    const T par = k == 0 ? par0 : par1;
-    T flux = T(0);
-    if (interior) {
-      // x direction (z axis): cells j-2 .. j+2 of row i
-      const T* row = src + (long long)i * nz;
-      const T* vrow = uz + (long long)i * nz;
-      const T fm2 = row[j - 2], fm1 = row[j - 1], f0 = row[j], f1 = row[j + 1], f2 = row[j + 2];
-      const T vm2 = vrow[j - 2], vm1 = vrow[j - 1], v0 = vrow[j], v1 = vrow[j + 1],
-              v2 = vrow[j + 2];
-      // y direction (r axis): rows i-2 .. i+2 of column j through the mirror
-      const T gm2 = mir(src, i - 2, j, nz, par), gm1 = mir(src, i - 1, j, nz, par);
-      const T g1 = src[c + nz], g2 = src[c + 2LL * nz];
-      const T wm2 = mir(ur, i - 2, j, nz, T(-1)), wm1 = mir(ur, i - 1, j, nz, T(-1));
-      const T w0 = ur[c], w1 = ur[c + nz], w2 = ur[c + 2LL * nz];
-      if (CONS) {
-        const T xf = face_cons(fm1, f0, f1, f2, vm1, v0, v1, v2);
-        const T xb = face_cons(fm2, fm1, f0, f1, vm2, vm1, v0, v1);
-        const T yf = face_cons(gm1, f0, g1, g2, wm1, w0, w1, w2);
-        const T yb = face_cons(gm2, gm1, f0, g1, wm2, wm1, w0, w1);
+    for (int k = 0; k < NF; ++k) {
+      const T* __restrict__ src = k == 0 ? src0 : src1;
+      fm1[k] = src[row + cm1];
+      f0[k] = src[row + c0];
+      f1[k] = src[row + c1];
+      f2[k] = src[row + c2];
+      gm1[k] = src[rm1];
+      g1[k] = src[r1];
+      g2[k] = src[r2];
+      if (!CONS) {
+        fm2[k] = src[row + cm2];
+        gm2[k] = src[rm2];
+        zero_bits |= value_bits(fm2[k]) | value_bits(fm1[k]) | value_bits(f0[k]) |
+                     value_bits(f1[k]) | value_bits(f2[k]) | value_bits(gm2[k]) |
+                     value_bits(gm1[k]) | value_bits(g1[k]) | value_bits(g2[k]);
+      }
+      const bool odd = k == 0 ? odd0 : odd1;
+      gm1[k] = flip_sign(gm1[k], i < 1 && odd);
+      if (!CONS) gm2[k] = flip_sign(gm2[k], i < 2 && odd);
+    }
+    // a warp whose cells are all +0 keeps them (with finite velocities)
+    const bool zero = !CONS && i >= 2 && zero_bits == 0 && finite_bits(v0) && finite_bits(w0) &&
+                      finite_bits(a);
+    if (!CONS && __all_sync(0xffffffffu, zero)) continue;
+#pragma unroll
+    for (int k = 0; k < NF; ++k) {
+      T* __restrict__ dst = k == 0 ? dst0 : dst1;
+      T out;
+      if constexpr (CONS) {
+        const T xf = face_cons(fm1[k], f0[k], f1[k], f2[k], vm1, v0, v1, v2);
+        const T xb = __shfl_up_sync(0xffffffffu, xf, 1);
+        const T yf = face_cons(gm1[k], f0[k], g1[k], g2[k], wm1, w0, w1, w2);
+        T flux = T(0);
         flux = rn_add(flux, rn_mul(a, xf));
         flux = rn_sub(flux, rn_mul(a, xb));
         flux = rn_add(flux, rn_mul(a, yf));
         flux = rn_sub(flux, rn_mul(a, yb));
+        yb = yf;
+        out = rn_add(f0[k], inner ? flux : T(0));
       } else {
-        const T xf = face_noncons(fm1, f0, f1, f2, v0, v1);
-        const T xb = face_noncons(fm2, fm1, f0, f1, vm1, v0);
-        const T yf = face_noncons(gm1, f0, g1, g2, w0, w1);
-        const T yb = face_noncons(gm2, gm1, f0, g1, wm1, w0);
-        flux = rn_add(flux, rn_mul(rn_mul(a, xf), v0));
-        flux = rn_sub(flux, rn_mul(rn_mul(a, xb), v0));
-        flux = rn_add(flux, rn_mul(rn_mul(a, yf), w0));
-        flux = rn_sub(flux, rn_mul(rn_mul(a, yb), w0));
+        out = noncons_cell(fm1[k], f0[k], f1[k], f2[k], gm2[k], gm1[k], g1[k], g2[k], v0, v1, wm1,
+                           w0, w1, a, inner);
       }
+      // ghost cells take a zero flux (which turns -0 into +0)
+      if (cell) dst[row + j] = out;
     }
-    dst[c] = rn_add(src[c], flux);
   }
 }
 
@@ -127,10 +216,17 @@ int eno3_launch(T* f0, T* f1, T par0, T par1, const T* uz, const T* ur, T* scrat
     if (cudaMemcpyAsync(s1, f1, bytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
       return axi::launch_status(what);
   }
-  dim3 grid(axi::ceil_div(nz, BX), axi::ceil_div(nr, BY));
-  eno3_step_kernel<T, NF, CONS><<<grid, dim3(BX, BY), 0, s>>>(f0, f1, scratch, s1, par0, par1,
-                                                              uz, ur, nr, nz, -dt_by_dx,
-                                                              dt_dev, dx);
+  // Strips as long as the GPU stays filled (24 warps per SM): a longer strip
+  // spares FP64 instructions but walks its rows one load latency after the
+  // other (strips of 8, filling it less: 41 us for omega, but 42 instead of 26
+  // for eta, most of which is zeros).
+  const int cols = axi::ceil_div(nz, ENO_COLS);
+  const long long per = (long long)nr * cols / (24LL * axi::sm_count());
+  const int most = CONS ? 4 : 1;
+  const int strip = per < 1 ? 1 : per > most ? most : (int)per;
+  dim3 grid(cols, axi::ceil_div(nr, ENO_WARPS * strip));
+  eno3_step_kernel<T, NF, CONS><<<grid, dim3(32, ENO_WARPS), 0, s>>>(
+      f0, f1, scratch, s1, par0 < T(0), par1 < T(0), uz, ur, nr, nz, -dt_by_dx, dt_dev, dx, strip);
   return axi::launch_status(what);
 }
 
