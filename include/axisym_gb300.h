@@ -317,7 +317,7 @@ int axi_fd_transform_f64(double* out, int ld_out, const double* in, int ld_in,
                          void* stream);
 /* ---------------------------------------------------------------------
  * FP64 products on the tcgen05 tensor cores by integer slicing: each operand
- * row is scaled by a power of two and written as nine signed 7-bit digits;
+ * row is scaled by a power of two and written as eight signed 8-bit digits;
  * products of digit planes are exact in the FP32 accumulators and summed as
  * integers, with one rounding to FP64. A row or column that holds a value
  * which is not finite gives NaN.
@@ -582,7 +582,9 @@ typedef struct axi_plan_info {
   int32_t n_tc_tiles[4];   /* tensor-core tiles per spectral stage */
   int32_t n_dct_items;     /* row groups of the z transforms (AXI_PLAN_DCT_Z) */
   axi_tuning tune;         /* launch choices (zero: defaults) */
-  int32_t n_slice_items[2]; /* row groups sliced before the z / r products (AXI_PLAN_SLICED) */
+  int32_t n_slice_items[4]; /* AXI_PLAN_SLICED: work items of each slicing */
+  int32_t sliced_form[4];   /* AXI_PLAN_SLICED: tile form of each product (internal) */
+  int32_t slice_groups[4];  /* AXI_PLAN_SLICED: row groups before sharing of K (internal) */
 } axi_plan_info;
 
 /* AXI_PLAN_DCT_Z: the z-direction products run as orthonormal DCT-II /

@@ -64,6 +64,40 @@ inline int check_ptrs(const char* what, std::initializer_list<const void*> ptrs,
 // Number of SMs on the current device (cached per device).
 int sm_count();
 
+// Launch with programmatic dependent launch (the kernel may start while its
+// predecessor on the stream runs; it waits with pdl_wait before it touches
+// what that one reads or writes) and, with cluster > 1, thread-block clusters.
+template <typename... P, typename... A>
+inline int launch_pdl(const char* what, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                      cudaStream_t s, int cluster, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = cluster;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  if (e != cudaSuccess) {
+    set_error("%s: CUDA launch failed: %s", what, cudaGetErrorString(e));
+    cudaGetLastError();
+    return AXI_ERR_CUDA;
+  }
+  return AXI_OK;
+}
+// Waits until the grids this one depends on are complete and their writes visible.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next grid of a launch_pdl chain start once every block got here.
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 }  // namespace axi
 
 #define AXI_TRY(expr)            \

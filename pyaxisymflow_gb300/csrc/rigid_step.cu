@@ -1586,7 +1586,7 @@ inline PlanOffsets plan_offsets(const axi_plan_info* info) {
     end = o.sliced_jobs + (size_t)4 * info->n_cases * sizeof(axi_sl::GemmJob);
     for (int st = 0; st < 4; ++st) {
       o.slice_items[st] = align16(end);
-      o.tc_tiles[st] = o.slice_items[st] + (size_t)info->n_slice_items[st % 2] * sizeof(int4);
+      o.tc_tiles[st] = o.slice_items[st] + (size_t)info->n_slice_items[st] * sizeof(int4);
       end = o.tc_tiles[st] + (size_t)info->n_tc_tiles[st] * sizeof(int4);
     }
   } else {
@@ -1887,8 +1887,9 @@ struct StencilGrid {
 // One of the four products of the double engine on sliced operands: its field
 // operand sliced, then the product.
 int run_sliced(const axi_plan_info* info, const PlanView& v, int st, cudaStream_t s) {
-  AXI_TRY(axi_sl::launch_slice(v.slice_jobs, v.slice_items[st], info->n_slice_items[st % 2], s));
-  return axi_sl::launch_gemm(v.sliced_jobs, v.tc_tiles[st], info->n_tc_tiles[st], v.err, s);
+  AXI_TRY(axi_sl::launch_slice(v.slice_jobs, v.slice_items[st], info->n_slice_items[st], s));
+  return axi_sl::launch_gemm(v.sliced_jobs, v.tc_tiles[st], info->n_tc_tiles[st],
+                             info->sliced_form[st], true, v.err, s);
 }
 
 template <typename T>
@@ -2152,9 +2153,28 @@ extern "C" int axi_plan_init(axi_case* cases, int n_cases, int elem_bytes, int f
           return AXI_ERR_INVALID;
         }
         const int M = st % 2 == 0 ? k.nz : k.nr, N = st % 2 == 0 ? k.nr : k.nz;
-        info->n_tc_tiles[st] += axi_sl::gemm_tiles(M, N);
-        if (st < 2) info->n_slice_items[st] += axi_sl::slice_items(N, axi_sl::KIND_B);
+        info->n_tc_tiles[st] += axi_sl::gemm_tiles(M, N, axi_sl::FORM_NARROW);
       }
+    }
+  }
+  for (int st = 0; sliced && st < 4; ++st) {
+    // one form per launch, from the tiles of all cases
+    const int form = axi_sl::choose_form(info->n_tc_tiles[st], axi::sm_count());
+    info->sliced_form[st] = form;
+    info->n_tc_tiles[st] = info->n_slice_items[st] = 0;
+    int groups = 0;
+    for (int c = 0; c < n_cases; ++c) {
+      const axi_case& k = cases[c];
+      const int M = st % 2 == 0 ? k.nz : k.nr, N = st % 2 == 0 ? k.nr : k.nz;
+      info->n_tc_tiles[st] += axi_sl::gemm_tiles(M, N, form);
+      groups += axi_sl::slice_groups(N, axi_sl::form_cols(form));
+    }
+    info->slice_groups[st] = groups;
+    for (int c = 0; c < n_cases; ++c) {
+      const axi_case& k = cases[c];
+      const int M = st % 2 == 0 ? k.nz : k.nr, N = st % 2 == 0 ? k.nr : k.nz;
+      info->n_slice_items[st] += axi_sl::slice_groups(N, axi_sl::form_cols(form)) *
+                                 axi_sl::slice_parts(groups, M, axi::sm_count());
     }
   }
   info->n_cases = n_cases;
@@ -2294,18 +2314,20 @@ extern "C" int axi_plan_upload(const axi_case* cases, const axi_plan_info* info,
     std::vector<int4> items[4], tiles[4];
     for (int c = 0; c < n; ++c) {
       const axi_case& k = cases[c];
-      axi_sl::spectral_jobs(k.nr, k.nz, static_cast<const double*>(k.omega), k.nz,
+      axi_sl::spectral_jobs(k.nr, k.nz, info->sliced_form, static_cast<const double*>(k.omega), k.nz,
                             static_cast<double*>(k.psi), k.nz, static_cast<double*>(k.gemm_work),
                             k.sliced_field, k.sliced_basis,
                             static_cast<const double*>(k.inv_eig), sj + 4 * c, gj + 4 * c);
       for (int st = 0; st < 4; ++st) {
         const int M = st % 2 == 0 ? k.nz : k.nr, N = st % 2 == 0 ? k.nr : k.nz;
-        axi_sl::append_slice_items(items[st], 4 * c + st, N, axi_sl::KIND_B);
-        axi_sl::append_gemm_tiles(tiles[st], 4 * c + st, M, N, M);
+        axi_sl::append_slice_items(
+            items[st], 4 * c + st, N, axi_sl::form_cols(info->sliced_form[st]),
+            axi_sl::slice_parts(info->slice_groups[st], M, axi::sm_count()));
+        axi_sl::append_gemm_tiles(tiles[st], 4 * c + st, M, N, M, info->sliced_form[st]);
       }
     }
     for (int st = 0; st < 4; ++st) {
-      if ((int)items[st].size() != info->n_slice_items[st % 2] ||
+      if ((int)items[st].size() != info->n_slice_items[st] ||
           (int)tiles[st].size() != info->n_tc_tiles[st]) {
         axi::set_error("plan_upload: cases changed since plan_init");
         return AXI_ERR_INVALID;

@@ -17,23 +17,20 @@ using axi_tma::mbar_wait;
 using axi_tma::smem_u32;
 
 // ---------------------------------------------------------------------------
-// Slicing. One block per 8 rows: the largest exponent of each row, then each
-// thread turns 8 consecutive K elements of one row into nine 16-byte pieces
-// (one per digit plane). Lanes 0 .. 7 of a warp hold the 8 rows of one core
-// matrix, so each plane store of a warp is four full 128-byte lines. All
-// arithmetic is on integers (FP64 instructions run at 1/64 of their rate).
+// Slicing. A block takes 8 rows (or a share of their K): the largest exponent of
+// each row, then each thread turns 8 consecutive K elements of one row into
+// eight 16-byte pieces (one per digit plane). Lanes 0 .. 7 of a warp hold the 8
+// rows of one core matrix, so each plane store of a warp is four full 128-byte
+// lines. All arithmetic is on integers (FP64 instructions run at 1/64 of their
+// rate).
 // ---------------------------------------------------------------------------
 constexpr int SL_THREADS = 256;
 
-// sum of 64 * 2^(7 j): makes every digit non-negative
-constexpr unsigned long long DIGIT_BIAS = [] {
-  unsigned long long b = 0;
-  for (int j = 0; j < DIGITS; ++j) b += 64ull << (BITS * j);
-  return b;
-}();
+// 128 in every byte: makes every digit non-negative
+constexpr unsigned long long DIGIT_BIAS = 0x8080808080808080ull;
 
-// x 2^62 / 2^(emax + 1 - bias) as a signed integer plus DIGIT_BIAS; emax: the
-// row's largest biased exponent (at least 1).
+// x 2^62 / 2^(emax + 1 - bias) as a signed integer plus DIGIT_BIAS, whose bytes
+// are the digits plus 128; emax: the row's largest biased exponent (at least 1).
 __device__ __forceinline__ unsigned long long biased_fixed(double x, int emax) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const int e = (int)(b >> 52) & 0x7ff;
@@ -64,7 +61,7 @@ __device__ __forceinline__ void load8(const double* p, long long ks, int n, doub
 
 template <bool VEC>
 __device__ __forceinline__ void slice_rows(const SliceJob& j, const double* src, long long rs,
-                                           int group, int* s_max) {
+                                           int group, int part, int parts, int* s_max) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r = lane & 7;
   const int row = group * 8 + r;
@@ -72,31 +69,37 @@ __device__ __forceinline__ void slice_rows(const SliceJob& j, const double* src,
   const bool live = row < j.rows;
   const double* p = src + (long long)row * rs;
   const long long ks = j.ks;
+  const int k_lane = (warp * 4 + (lane >> 3)) * 8;
   // pass 1: largest biased exponent of each row
   int em = 0;
-  for (int k = (warp * 4 + (lane >> 3)) * 8; k < K; k += SL_THREADS) {
-    double v[8];
-    load8<VEC>(p + k * ks, ks, live ? min(8, K - k) : 0, v);
+  if (j.have_exps) {
+    em = live ? j.exps[row] : 0;
+  } else {
+    for (int k = k_lane; k < K; k += SL_THREADS) {
+      double v[8];
+      load8<VEC>(p + k * ks, ks, live ? min(8, K - k) : 0, v);
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-      em = max(em, (int)((unsigned long long)__double_as_longlong(v[q]) >> 52) & 0x7ff);
+      for (int q = 0; q < 8; ++q)
+        em = max(em, (int)((unsigned long long)__double_as_longlong(v[q]) >> 52) & 0x7ff);
+    }
+    if (threadIdx.x < 8) s_max[threadIdx.x] = 0;
+    __syncthreads();
+    atomicMax(&s_max[r], em);
+    __syncthreads();
+    em = s_max[r];
+    if (part == 0 && warp == 0 && lane < 8) j.exps[row] = em;
   }
-  if (threadIdx.x < 8) s_max[threadIdx.x] = 1;
-  __syncthreads();
-  atomicMax(&s_max[r], em);
-  __syncthreads();
-  em = s_max[r];
   const bool finite = em != 0x7ff;
-  if (warp == 0 && lane < 8) j.exps[row] = finite ? em - 1022 : EXP_NONFINITE;
+  em = max(em, 1);
   // pass 2: the digits
-  const bool is_a = j.kind == KIND_A;
-  const int br = is_a ? BM : BN;                // rows per block of the layout
-  const int stage = is_a ? A_STAGE : B_STAGE;   // bytes per (row block, K step)
-  // A: planes of [2 K halves][16 row groups], B: [2 K halves][planes][4 row groups]
-  const int plane_stride = is_a ? BM * BK * 2 : BN / 8 * 128;
-  const int half_stride = is_a ? BM / 8 * 128 : DIGITS * BN / 8 * 128;
+  const int br = j.block;                       // rows per block of the layout
+  const bool is_a = br == BM;
+  const int stage = DIGITS * br * BK * 2;       // bytes per (row block, K step)
+  // A: planes of [2 K halves][row groups], B: [2 K halves][planes][row groups]
+  const int plane_stride = is_a ? BM * BK * 2 : br / 8 * 128;
+  const int half_stride = is_a ? BM / 8 * 128 : DIGITS * br / 8 * 128;
   uint8_t* dst = j.planes + (size_t)(row / br) * nk * stage + (row % br) / 8 * 128 + r * 16;
-  for (int k = (warp * 4 + (lane >> 3)) * 8; k < nk * BK; k += SL_THREADS) {
+  for (int k = part * SL_THREADS + k_lane; k < nk * BK; k += parts * SL_THREADS) {
     double v[8];
     load8<VEC>(p + k * ks, ks, live && finite ? min(8, K - k) : 0, v);
     unsigned long long f[8];
@@ -105,19 +108,19 @@ __device__ __forceinline__ void slice_rows(const SliceJob& j, const double* src,
     uint8_t* d = dst + (size_t)(k / BK) * stage + ((k / 8) & 1) * half_stride;
 #pragma unroll
     for (int i = 0; i < DIGITS; ++i) {
-      const int sh = BITS * (DIGITS - 1 - i);
+      // digit i is byte 7 - i
       uint32_t w[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        uint32_t u0 = (uint32_t)(f[2 * q] >> sh), u1 = (uint32_t)(f[2 * q + 1] >> sh);
-        if (i > 0) {
-          u0 &= 127u;
-          u1 &= 127u;
-        }
-        // half(1024 + u) has the bits 0x6400 + u; subtract 1024 + 64
-        const uint32_t h = 0x64006400u + u0 + (u1 << 16);
+        const uint32_t w0 = (uint32_t)(f[2 * q] >> (i < 4 ? 32 : 0));
+        const uint32_t w1 = (uint32_t)(f[2 * q + 1] >> (i < 4 ? 32 : 0));
+        const uint32_t byte = 3 - i % 4;
+        // half(1024 + u) has the bits 0x6400 + u; subtract 1024 + 128
+        const uint32_t h =
+            (__byte_perm(w0, w1, byte | byte << 4 | (byte + 4) << 8 | (byte + 4) << 12) &
+             0x00ff00ffu) | 0x64006400u;
         const __half2 x = __hsub2(*reinterpret_cast<const __half2*>(&h),
-                                  __half2half2(__ushort_as_half(0x6440)));
+                                  __half2half2(__ushort_as_half(0x6480)));
         w[q] = *reinterpret_cast<const uint32_t*>(&x);
       }
       *reinterpret_cast<uint4*>(d + i * plane_stride) = make_uint4(w[0], w[1], w[2], w[3]);
@@ -125,20 +128,31 @@ __device__ __forceinline__ void slice_rows(const SliceJob& j, const double* src,
   }
 }
 
+__device__ __forceinline__ int pad_rows_dev(int rows, int block) {
+  return (rows + block - 1) / block * block;
+}
+
+// items: job, group of 8 rows, share of K, shares
 __global__ void __launch_bounds__(SL_THREADS)
     slice_kernel(const SliceJob* __restrict__ jobs, const int4* __restrict__ items,
                  const double* src_override, long long rs_override) {
   __shared__ int s_max[8];
   const int4 it = items[blockIdx.x];
   const SliceJob& j = jobs[it.x];
+  axi::pdl_trigger();
+  axi::pdl_wait();
   const double* src = src_override ? src_override : j.src;
   const long long rs = src_override ? rs_override : j.rs;
   // 16-byte loads where every row starts on 16 bytes and K runs contiguously
   const bool vec = j.ks == 1 && (rs & 1) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+  // the next product's row exponents start at zero
+  for (int q = (it.y * it.w + it.z) * SL_THREADS + threadIdx.x; q < j.n_clear;
+       q += (pad_rows_dev(j.rows, j.block) / 8) * it.w * SL_THREADS)
+    j.clear[q] = 0;
   if (vec)
-    slice_rows<true>(j, src, rs, it.y, s_max);
+    slice_rows<true>(j, src, rs, it.y, it.z, it.w, s_max);
   else
-    slice_rows<false>(j, src, rs, it.y, s_max);
+    slice_rows<false>(j, src, rs, it.y, it.z, it.w, s_max);
 }
 
 // ---------------------------------------------------------------------------
@@ -210,22 +224,15 @@ __device__ __forceinline__ void tmem_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// The two accumulator sets overlap by two groups of 32 columns (2 x 288 of 512
-// columns): set 0 starts at column 0, set 1 at column 224. The columns shared
-// are groups 7, 8 of set 0 and groups 0, 1 of set 1.
-constexpr int SET1 = 512 - DIGITS * BN;
-constexpr int SHARED_GROUPS = (2 * DIGITS * BN - 512) / BN;
-static_assert(SHARED_GROUPS == 2 && SET1 % BN == 0, "accumulator sets");
-
-// Sum of the accumulators of one output element as hi 2^28 + lo: groups
-// 0 .. 4 go to hi, 5 .. 8 to lo (weights 2^(7 (8 - d)) relative to the last).
+// Sum of the accumulators of one output element as hi 2^32 + lo: groups
+// 0 .. 3 go to hi, 4 .. 7 to lo (weights 2^(8 (7 - d)) relative to the last).
 template <int G>
 __device__ __forceinline__ void add_group(uint32_t bits, long long& hi, long long& lo) {
   const int s = __float2int_rn(__uint_as_float(bits));
-  if constexpr (G <= 4)
-    hi += (long long)s * (1 << (BITS * (4 - G)));
+  if constexpr (G <= 3)
+    hi += (long long)s * (1 << (8 * (3 - G)));
   else
-    lo += (long long)s * (1 << (BITS * (8 - G)));
+    lo += (long long)s * (1 << (8 * (7 - G)));
 }
 
 template <int G>
@@ -234,32 +241,36 @@ __device__ __forceinline__ void add_groups8(uint32_t (&r)[8], long long* hi, lon
   for (int q = 0; q < 8; ++q) add_group<G>(r[q], hi[q], lo[q]);
 }
 
-// Groups FIRST .. FIRST + COUNT - 1 of this warp's 16 columns into hi, lo.
-template <int FIRST, int COUNT>
-__device__ __forceinline__ void drain_groups(uint32_t taddr, long long (&hi)[16],
-                                             long long (&lo)[16]) {
+// Groups FIRST .. FIRST + COUNT - 1 of this warp's BN / 2 columns into hi, lo.
+template <int BN, int FIRST, int COUNT>
+__device__ __forceinline__ void drain_groups(uint32_t taddr, long long (&hi)[BN / 2],
+                                             long long (&lo)[BN / 2]) {
   if constexpr (COUNT > 0) {
-    constexpr int N = COUNT >= 2 ? 2 : COUNT;  // up to 32 registers in flight
-    uint32_t r[N][2][8];
+    constexpr int H = BN / 16;                   // 8-column pieces
+    constexpr int MOST = 4 / H;                  // up to 32 registers in flight
+    constexpr int N = COUNT >= MOST ? MOST : COUNT;
+    uint32_t r[N][H][8];
 #pragma unroll
     for (int g = 0; g < N; ++g)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) tmem_ld8(taddr + (FIRST + g) * BN + 8 * h, r[g][h]);
+      for (int h = 0; h < H; ++h) tmem_ld8(taddr + (FIRST + g) * BN + 8 * h, r[g][h]);
     tmem_wait_ld();
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < H; ++h) {
       add_groups8<FIRST>(r[0][h], hi + 8 * h, lo + 8 * h);
       if constexpr (N > 1) add_groups8<FIRST + 1>(r[1][h], hi + 8 * h, lo + 8 * h);
+      if constexpr (N > 2) add_groups8<FIRST + 2>(r[2][h], hi + 8 * h, lo + 8 * h);
+      if constexpr (N > 3) add_groups8<FIRST + 3>(r[3][h], hi + 8 * h, lo + 8 * h);
     }
-    drain_groups<FIRST + N, COUNT - N>(taddr, hi, lo);
+    drain_groups<BN, FIRST + N, COUNT - N>(taddr, hi, lo);
   }
 }
 
-// (hi 2^28 + lo) 2^e rounded once to FP64, with integer instructions.
+// (hi 2^32 + lo) 2^e rounded once to FP64, with integer instructions.
 __device__ __forceinline__ double assemble(long long hi, long long lo, int e) {
   // 128-bit sum: (w1, w0)
-  unsigned long long w0 = (unsigned long long)hi << 28;
-  long long w1 = hi >> 36;
+  unsigned long long w0 = (unsigned long long)hi << 32;
+  long long w1 = hi >> 32;
   const unsigned long long lo_u = (unsigned long long)lo;
   w0 += lo_u;
   w1 += (lo >> 63) + (w0 < lo_u ? 1 : 0);
@@ -295,40 +306,100 @@ __device__ __forceinline__ double assemble(long long hi, long long lo, int e) {
   return sign ? -v : v;
 }
 
+// A may be read ahead of the predecessor's end; the successor may start early.
+enum { FLAG_A_READY = 1, FLAG_TRIGGER = 2 };
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// 16 bytes into the shared memory of block `rank` of the cluster, at the place
+// that `addr` has in this block
+__device__ __forceinline__ void store_remote(uint32_t addr, int rank, long long x, long long y) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  asm volatile("st.shared::cluster.v2.b64 [%0], {%1, %2};" ::"r"(r), "l"(x), "l"(y) : "memory");
+}
+
+// partial sums received from the other blocks of a split tile
+constexpr int exchange_bytes(int bn, int split) {
+  return split > 1 ? (split - 1) * BM * (bn / split) * 16 : 0;
+}
+constexpr int smem_bytes(int bn, int split) {
+  return NSTAGE * (A_STAGE + b_stage(bn)) + exchange_bytes(bn, split) + 128 + 256;
+}
+
 // Persistent, warp-specialised: warp 0 copies stages, warp 1 issues MMAs,
-// warps 2 .. 9 (two per TMEM lane quarter, 16 columns each) drain an
-// accumulator set while the MMAs fill the other. A unit of work is one tile
-// and up to 512 of its K; the integer sums run on over the units of a tile.
+// warps 2 .. 9 (two per TMEM lane quarter, BN / 2 columns each) drain one of
+// two accumulator sets while the MMAs fill the other. A unit of work is one
+// tile and up to 128 of its K; the integer sums run on over the units of a tile.
+//
+// Bound by shared memory: a step of 16 K with BN = 32 writes 40 KB and its MMAs
+// read 68 KB, 844 cycles at 128 bytes per cycle, where the MMAs themselves take
+// 576. (Sharing A's loads between the blocks of a cluster by multicast changed
+// nothing: 199.6 against 198.3 us for a 1024 x 512 solve.)
+//
+// SPLIT > 1: a cluster of SPLIT blocks per tile, each taking a share of its K;
+// then every block finishes BN / SPLIT of the columns, with the partial sums
+// that the others wrote into its shared memory.
+template <int BN, int SPLIT>
 __global__ void __launch_bounds__(THREADS, 1)
     sliced_gemm_kernel(const GemmJob* __restrict__ jobs, const int4* __restrict__ tiles,
-                       int n_tiles, int* __restrict__ err, double* c_override, int ldc_override) {
+                       int n_tiles, int flags, int* __restrict__ err, double* c_override,
+                       int ldc_override) {
+  constexpr int B_STAGE = b_stage(BN);
+  constexpr int STAGE_BYTES = A_STAGE + B_STAGE;
+  constexpr int COLS = BN / 2;  // columns per epilogue warp
+  constexpr int SET = DIGITS * BN;  // TMEM columns of an accumulator set
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) &
                                              ~static_cast<uintptr_t>(127));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + NSTAGE * STAGE_BYTES);
-  // full[NSTAGE], empty[NSTAGE], acc_full, acc_shared (drained), quiet
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NSTAGE + 3);
+  uint8_t* exchange = smem + NSTAGE * STAGE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(exchange + exchange_bytes(BN, SPLIT));
+  // full[NSTAGE], empty[NSTAGE], acc_full[2], acc_empty[2], quiet
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NSTAGE + 5);
   int* progress = reinterpret_cast<int*>(tmem_slot + 1);  // [0] loads issued, [1] consumed
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = SPLIT > 1 ? (int)cluster_rank() : 0;
+  // first tile of this block, its stride, and its share of a tile's K steps
+  const int tile0 = blockIdx.x / SPLIT, tile_step = gridDim.x / SPLIT;
+  auto k_begin = [rank](int nk) { return nk * rank / SPLIT; };
+  auto k_end = [rank](int nk) { return nk * (rank + 1) / SPLIT; };
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + NSTAGE);
   const uint32_t acc_full = smem_u32(bars + 2 * NSTAGE);
-  const uint32_t acc_shared = smem_u32(bars + 2 * NSTAGE + 1);
-  const uint32_t quiet = smem_u32(bars + 2 * NSTAGE + 2);
+  const uint32_t acc_empty = smem_u32(bars + 2 * NSTAGE + 2);
+  const uint32_t quiet = smem_u32(bars + 2 * NSTAGE + 4);
 
+  // The next kernel of the chain (slicing) may start early only where this one
+  // leaves half of the SMs free: its blocks do not fit beside these, and on few
+  // free SMs they would pile up (a 1024 x 512 solve: 174 -> 198 us).
+  if (flags & FLAG_TRIGGER) axi::pdl_trigger();
+  if (SPLIT > 1) cluster_arrive();  // (waited for before the first remote store)
   if (threadIdx.x == 0) {
     for (int s = 0; s < NSTAGE; ++s) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, 1);
     }
-    mbar_init(acc_full, 1);
-    mbar_init(acc_shared, EPI_WARPS);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(acc_full + 8 * b, 1);
+      mbar_init(acc_empty + 8 * b, EPI_WARPS);
+    }
     mbar_init(quiet, 1);
     progress[0] = 0;
     progress[1] = 0;
     axi_tma::fence_mbar_init();
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(tmem_slot), 512);
+    tmem_alloc(smem_u32(tmem_slot), 2 * SET);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -340,13 +411,25 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (lane == 0) {
       int g = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+      int ahead = 0;  // first steps of the first tile whose A is already on its way
+      if (flags & FLAG_A_READY) {
+        const int4 tr = tiles[tile0];
+        const uint8_t* a = jobs[tr.x].a + ((size_t)tr.y * tr.w + k_begin(tr.w)) * A_STAGE;
+        const int steps = k_end(tr.w) - k_begin(tr.w);
+        for (; ahead < steps && ahead < NSTAGE; ++ahead) {
+          mbar_expect_tx(full0 + 8 * ahead, STAGE_BYTES);
+          bulk_load(smem_u32(smem + ahead * STAGE_BYTES), a + (size_t)ahead * A_STAGE, A_STAGE,
+                    full0 + 8 * ahead);
+        }
+      }
+      axi::pdl_wait();
+      for (int t = tile0; t < n_tiles && ok; t += tile_step) {
         const int4 tr = tiles[t];  // job, row block of A, row block of B, K steps
         const GemmJob& job = jobs[tr.x];
         const int nk = tr.w;
         const uint8_t* a = job.a + (size_t)tr.y * nk * A_STAGE;
         const uint8_t* b = job.b + (size_t)tr.z * nk * B_STAGE;
-        for (int kb = 0; kb < nk; ++kb, ++g) {
+        for (int kb = k_begin(nk); kb < k_end(nk); ++kb, ++g) {
           const int s = g % NSTAGE, use = g / NSTAGE;
           if (use > 0 && !mbar_wait(empty0 + 8 * s, (use - 1) & 1, err, ERR_PRODUCER)) {
             ok = false;
@@ -354,28 +437,35 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
           const uint32_t st = smem_u32(smem + s * STAGE_BYTES);
           const uint32_t fb = full0 + 8 * s;
-          mbar_expect_tx(fb, STAGE_BYTES);
-          bulk_load(st, a + (size_t)kb * A_STAGE, A_STAGE, fb);
+          if (g >= ahead) {
+            mbar_expect_tx(fb, STAGE_BYTES);
+            bulk_load(st, a + (size_t)kb * A_STAGE, A_STAGE, fb);
+          }
           bulk_load(st + A_STAGE, b + (size_t)kb * B_STAGE, B_STAGE, fb);
         }
       }
-      progress[0] = g;
+      progress[0] = g > ahead ? g : ahead;
     }
     __syncwarp();
+    if (SPLIT > 1) {
+      cluster_wait();
+      cluster_arrive();
+      cluster_wait();
+    }
   } else if (warp == 1) {
     if (lane == 0) {
       int g = 0, u = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-        const int nk = tiles[t].w;
-        for (int k0 = 0; k0 < nk && ok; k0 += CHUNK, ++u) {
-          // the set before the last is drained, and of the last the shared columns
-          if (u > 0 && !mbar_wait(acc_shared, (u - 1) & 1, err, ERR_MMA)) {
+      for (int t = tile0; t < n_tiles && ok; t += tile_step) {
+        const int nk = k_end(tiles[t].w);
+        for (int k0 = k_begin(tiles[t].w); k0 < nk && ok; k0 += CHUNK, ++u) {
+          const int set = u & 1, use = u >> 1;
+          if (use > 0 && !mbar_wait(acc_empty + 8 * set, (use - 1) & 1, err, ERR_MMA)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t d = tmem + (u & 1) * SET1;
+          const uint32_t d = tmem + set * SET;
           const int k1 = min(nk, k0 + CHUNK);
           for (int kb = k0; kb < k1; ++kb, ++g) {
             const int s = g % NSTAGE, use = g / NSTAGE;
@@ -387,18 +477,14 @@ __global__ void __launch_bounds__(THREADS, 1)
             const uint32_t st = smem_u32(smem + s * STAGE_BYTES);
             const uint64_t a = operand_desc(st, BM / 8 * 128);
             const uint64_t b = operand_desc(st + A_STAGE, DIGITS * BN / 8 * 128);
-            // plane 0 of A against all nine planes of B, in two halves (N <= 256):
-            // it also starts every accumulator of the set
-            constexpr int H = DIGITS * BN / 2;
-            const uint32_t first = kb == k0 ? 0u : 1u;
-            umma_f16(d, a, b, idesc_f16(H), first);
-            umma_f16(d + H, a, b + (H / 8 * 128 >> 4), idesc_f16(H), first);
+            // plane 0 of A against all planes of B also starts every accumulator
 #pragma unroll
-            for (int i = 1; i < DIGITS; ++i)
-              umma_f16(d + i * BN, a + (i * BM * BK * 2 >> 4), b, idesc_f16((DIGITS - i) * BN), 1u);
+            for (int i = 0; i < DIGITS; ++i)
+              umma_f16(d + i * BN, a + (i * BM * BK * 2 >> 4), b, idesc_f16((DIGITS - i) * BN),
+                       i > 0 || kb > k0 ? 1u : 0u);
             umma_commit(empty0 + 8 * s);
           }
-          if (ok) umma_commit(acc_full);
+          if (ok) umma_commit(acc_full + 8 * set);
         }
       }
       progress[1] = g;
@@ -406,13 +492,19 @@ __global__ void __launch_bounds__(THREADS, 1)
       mbar_wait(quiet, 0, err, ERR_MMA);
     }
     __syncwarp();
+    if (SPLIT > 1) {
+      cluster_wait();
+      cluster_arrive();
+      cluster_wait();
+    }
   } else {
-    const int q = warp & 3;          // TMEM lane quarter
-    const int half = (warp - 2) >> 2;  // columns 16 half .. 16 half + 15
+    const int q = warp & 3;            // TMEM lane quarter
+    const int half = (warp - 2) >> 2;  // columns COLS half .. COLS half + COLS - 1
     const uint32_t lane_base = static_cast<uint32_t>(32 * q) << 16;
     int u = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+    axi::pdl_wait();
+    for (int t = tile0; t < n_tiles && ok; t += tile_step) {
       const int4 tr = tiles[t];
       const GemmJob& job = jobs[tr.x];
       const int M = job.M, N = job.N;
@@ -420,51 +512,83 @@ __global__ void __launch_bounds__(THREADS, 1)
       const long long ldc = c_override ? ldc_override : job.ldc;
       const double* const scale = job.scale;
       const int row = tr.y * BM + 32 * q + lane;
-      const int col0 = tr.z * BN + 16 * half;
-      const int ea = job.ea[row];
+      const int col0 = tr.z * BN + COLS * half;
+      const int ea_raw = job.ea[row];
+      const int ea = max(ea_raw, 1) - 1022;
       const int* eb = job.eb + col0;
-      const int nk = tr.w;
-      long long hi[16], lo[16];
+      int* const row_exps = job.row_exps;
+      int e_max = 0;
+      const int nk = k_end(tr.w);
+      long long hi[COLS], lo[COLS];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) hi[j] = lo[j] = 0;
-      for (int k0 = 0; k0 < nk; k0 += CHUNK, ++u) {
-        ok = __all_sync(0xffffffffu, mbar_wait(acc_full, u & 1, err, ERR_EPILOGUE));
+      for (int j = 0; j < COLS; ++j) hi[j] = lo[j] = 0;
+      for (int k0 = k_begin(tr.w); k0 < nk; k0 += CHUNK, ++u) {
+        const int set = u & 1;
+        ok = __all_sync(0xffffffffu,
+                        mbar_wait(acc_full + 8 * set, (u >> 1) & 1, err, ERR_EPILOGUE));
         if (!ok) break;
         tc_fence_after();
-        const uint32_t ta = tmem + lane_base + (u & 1) * SET1 + 16 * half;
-        // the columns that the next unit also uses come first
-        if (u & 1) {
-          drain_groups<0, SHARED_GROUPS>(ta, hi, lo);
-        } else {
-          drain_groups<DIGITS - SHARED_GROUPS, SHARED_GROUPS>(ta, hi, lo);
-        }
+        drain_groups<BN, 0, DIGITS>(tmem + lane_base + set * SET + COLS * half, hi, lo);
         tc_fence_before();
         __syncwarp();
         if (lane == 0)
-          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_shared) : "memory");
-        if (u & 1) {
-          drain_groups<SHARED_GROUPS, DIGITS - SHARED_GROUPS>(ta, hi, lo);
-        } else {
-          drain_groups<0, DIGITS - SHARED_GROUPS>(ta, hi, lo);
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty + 8 * set)
+                       : "memory");
+      }
+      int j0 = 0, j1 = COLS;  // columns that this warp finishes
+      if constexpr (SPLIT > 1) {
+        // columns PART r .. of the tile are finished by block r; this warp's
+        // columns belong to blocks half SPLIT / 2 ..
+        constexpr int PART = BN / SPLIT;
+        const uint32_t ex = smem_u32(exchange) + (32 * q + lane) * 16;
+        cluster_wait();  // every block of the cluster is running
+#pragma unroll
+        for (int j = 0; j < COLS; ++j) {
+          const int to = half * (SPLIT / 2) + j / PART;
+          const int slot = rank < to ? rank : rank - 1;  // by sender, without `to` itself
+          if (to != rank && ok)
+            store_remote(ex + (slot * PART + j % PART) * BM * 16, to, hi[j], lo[j]);
+        }
+        cluster_arrive();
+        cluster_wait();  // every partial sum has arrived
+        const int mine = rank - half * (SPLIT / 2);
+        j0 = j1 = 0;
+        if (ok && mine >= 0 && mine < SPLIT / 2) {
+          j0 = mine * PART;
+          j1 = j0 + PART;
+#pragma unroll
+          for (int j = 0; j < COLS; ++j) {
+            if (j < j0 || j >= j1) continue;
+#pragma unroll
+            for (int slot = 0; slot < SPLIT - 1; ++slot) {
+              const longlong2 v = *reinterpret_cast<const longlong2*>(
+                  exchange + ((slot * PART + j % PART) * BM + 32 * q + lane) * 16);
+              hi[j] += v.x;
+              lo[j] += v.y;
+            }
+          }
         }
       }
       if (!ok) break;
       if (row < M) {
         double* const cr = c + row * ldc + col0;
         const double* const sr = scale ? scale + (long long)row * N + col0 : nullptr;
-        const int n = min(16, N - col0);
-        const bool vec = n == 16 && (reinterpret_cast<uintptr_t>(cr) & 15) == 0;
+        const int n = min(COLS, N - col0);
+        const bool vec = n == COLS && (reinterpret_cast<uintptr_t>(cr) & 15) == 0;
 #pragma unroll
-        for (int j = 0; j < 16; j += 2) {
+        for (int j = 0; j < COLS; j += 2) {
+          if (SPLIT > 1 && (j < j0 || j >= j1)) continue;
           double v[2];
 #pragma unroll
           for (int w = 0; w < 2; ++w) {
-            const int e = eb[j + w];
-            // ea + eb - 12 - 7 * 8; a row or column that is not finite gives NaN
+            const int e_raw = eb[j + w];
+            const int e = max(e_raw, 1) - 1022;
+            // ea + eb - 12 - 8 * 7; a row or column that is not finite gives NaN
             v[w] = assemble(hi[j + w], lo[j + w], ea + e - 68);
-            if (ea == EXP_NONFINITE || e == EXP_NONFINITE)
+            if (ea_raw == 0x7ff || e_raw == 0x7ff)
               v[w] = __longlong_as_double(0x7ff8000000000000ll);
             if (sr && j + w < n) v[w] *= sr[j + w];
+            if (j + w < n) e_max = max(e_max, (__double2hiint(v[w]) >> 20) & 0x7ff);
           }
           if (vec) {
             *reinterpret_cast<double2*>(cr + j) = make_double2(v[0], v[1]);
@@ -473,6 +597,8 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (j + 1 < n) cr[j + 1] = v[1];
           }
         }
+        // what the next slicing needs, so that it reads its source once
+        if (row_exps && e_max > 0) atomicMax(row_exps + row, e_max);
       }
     }
   }
@@ -486,20 +612,22 @@ __global__ void __launch_bounds__(THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 1) tmem_dealloc(tmem, 512);
+  if (warp == 1) tmem_dealloc(tmem, 2 * SET);
 }
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 }  // namespace
 
-void append_slice_items(std::vector<int4>& items, int job, int rows, int kind) {
-  for (int g = 0; g < slice_items(rows, kind); ++g) items.push_back(make_int4(job, g, 0, 0));
+void append_slice_items(std::vector<int4>& items, int job, int rows, int block, int parts) {
+  for (int g = 0; g < slice_groups(rows, block); ++g)
+    for (int p = 0; p < parts; ++p) items.push_back(make_int4(job, g, p, parts));
 }
 
-void append_gemm_tiles(std::vector<int4>& tiles, int job, int M, int N, int K) {
+void append_gemm_tiles(std::vector<int4>& tiles, int job, int M, int N, int K, int form) {
+  const int cols = form_cols(form);
   for (int m = 0; m < (M + BM - 1) / BM; ++m)
-    for (int n = 0; n < (N + BN - 1) / BN; ++n) tiles.push_back(make_int4(job, m, n, k_steps(K)));
+    for (int n = 0; n < (N + cols - 1) / cols; ++n) tiles.push_back(make_int4(job, m, n, k_steps(K)));
 }
 
 void order_tiles(std::vector<int4>& tiles) {
@@ -510,53 +638,90 @@ void order_tiles(std::vector<int4>& tiles) {
 int launch_slice(const SliceJob* jobs_dev, const int4* items_dev, int n_items, cudaStream_t s,
                  const double* src, long long rs) {
   if (n_items <= 0) return AXI_OK;
-  slice_kernel<<<n_items, SL_THREADS, 0, s>>>(jobs_dev, items_dev, src, rs);
-  return axi::launch_status("slice");
+  return axi::launch_pdl("slice", slice_kernel, dim3(n_items), dim3(SL_THREADS), 0, s, 1, jobs_dev,
+                         items_dev, src, rs);
 }
 
-int launch_gemm(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, int* err_dev,
-                cudaStream_t s, double* c, int ldc) {
+template <int BN, int SPLIT>
+int launch_tiles(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, bool a_ready,
+                 int* err_dev, cudaStream_t s, double* c, int ldc) {
   static std::once_flag once;
   static cudaError_t attr_status = cudaSuccess;
   std::call_once(once, [] {
-    attr_status = cudaFuncSetAttribute(sliced_gemm_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    attr_status = cudaFuncSetAttribute(sliced_gemm_kernel<BN, SPLIT>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       smem_bytes(BN, SPLIT));
   });
   if (attr_status != cudaSuccess) {
-    axi::set_error("sliced GEMM: cannot reserve %d bytes of shared memory", SMEM_BYTES);
+    axi::set_error("sliced GEMM: cannot reserve %d bytes of shared memory",
+                   smem_bytes(BN, SPLIT));
     return AXI_ERR_CUDA;
   }
   if (n_tiles <= 0) return AXI_OK;
   const int sms = axi::sm_count();
-  sliced_gemm_kernel<<<n_tiles < sms ? n_tiles : sms, THREADS, SMEM_BYTES, s>>>(
-      jobs_dev, tiles_dev, n_tiles, err_dev, c, ldc);
-  return axi::launch_status("sliced_gemm");
+  // a split tile's blocks take one tile (the exchange is used once)
+  const int blocks = SPLIT > 1 ? SPLIT * n_tiles : n_tiles < sms ? n_tiles : sms;
+  return axi::launch_pdl("sliced_gemm", sliced_gemm_kernel<BN, SPLIT>, dim3(blocks), dim3(THREADS),
+                         smem_bytes(BN, SPLIT), s, SPLIT, jobs_dev, tiles_dev, n_tiles,
+                         (a_ready ? FLAG_A_READY : 0) | (2 * blocks <= sms ? FLAG_TRIGGER : 0),
+                         err_dev, c, ldc);
 }
+
+int launch_gemm(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, int form, bool a_ready,
+                int* err_dev, cudaStream_t s, double* c, int ldc) {
+  switch (form) {
+    case FORM_NARROW4:
+      return launch_tiles<16, 4>(jobs_dev, tiles_dev, n_tiles, a_ready, err_dev, s, c, ldc);
+    case FORM_NARROW2:
+      return launch_tiles<16, 2>(jobs_dev, tiles_dev, n_tiles, a_ready, err_dev, s, c, ldc);
+    case FORM_NARROW:
+      return launch_tiles<16, 1>(jobs_dev, tiles_dev, n_tiles, a_ready, err_dev, s, c, ldc);
+    default:
+      return launch_tiles<32, 1>(jobs_dev, tiles_dev, n_tiles, a_ready, err_dev, s, c, ldc);
+  }
+}
+
+namespace {
+// One planes buffer that the four stages use in turn (padding to 32 rows covers
+// every form), then the row exponents of each.
+size_t spectral_plane_bytes(int nr, int nz) {
+  return (std::max(plane_bytes(nr, nz, 32), plane_bytes(nz, nr, 32)) + 255) / 256 * 256;
+}
+}  // namespace
 
 size_t spectral_slice_bytes(int nr, int nz) {
-  return std::max(slice_bytes(nr, nz, KIND_B), slice_bytes(nz, nr, KIND_B));
+  return spectral_plane_bytes(nr, nz) +
+         (size_t)2 * (pad_rows(nr, 32) + pad_rows(nz, 32)) * sizeof(int);
 }
 
-void spectral_jobs(int nr, int nz, const double* in, long long ld_in, double* out, int ld_out,
-                   double* work, void* slices, const void* const basis[4], const double* inv_eig,
-                   SliceJob sl[4], GemmJob gm[4]) {
+void spectral_jobs(int nr, int nz, const int form[4], const double* in, long long ld_in,
+                   double* out, int ld_out, double* work, void* slices,
+                   const void* const basis[4], const double* inv_eig, SliceJob sl[4],
+                   GemmJob gm[4]) {
   double* x = work;
   double* y = work + (size_t)nr * nz;
-  sl[0] = slice_job(in, ld_in, 1, nr, nz, KIND_B, slices);
-  sl[1] = slice_job(x, nr, 1, nz, nr, KIND_B, slices);
-  sl[2] = slice_job(y, nz, 1, nr, nz, KIND_B, slices);
-  sl[3] = slice_job(x, nr, 1, nz, nr, KIND_B, slices);
+  int* exps = reinterpret_cast<int*>(static_cast<uint8_t*>(slices) + spectral_plane_bytes(nr, nz));
+  const double* src[4] = {in, x, y, x};
+  const long long rs[4] = {ld_in, nr, nz, nr};
   double* c[4] = {x, y, x, out};
   const int ldc[4] = {nr, nz, nr, ld_out};
   for (int st = 0; st < 4; ++st) {
     const int M = st % 2 == 0 ? nz : nr, N = st % 2 == 0 ? nr : nz, K = M;
+    sl[st] = slice_job(src[st], rs[st], 1, N, K, form_cols(form[st]), slices, exps);
+    sl[st].have_exps = st > 0;
+    exps += pad_rows(N, 32);
+    if (st < 3) {
+      sl[st].clear = exps;
+      sl[st].n_clear = pad_rows(M, 32);
+    }
     GemmJob& g = gm[st];
     g.a = static_cast<const uint8_t*>(basis[st]);
-    g.ea = reinterpret_cast<const int*>(g.a + plane_bytes(M, K, KIND_A));
+    g.ea = reinterpret_cast<const int*>(g.a + plane_bytes(M, K, BM));
     g.b = sl[st].planes;
     g.eb = sl[st].exps;
     g.c = c[st];
     g.scale = st == 1 ? inv_eig : nullptr;
+    g.row_exps = st < 3 ? exps : nullptr;
     g.M = M;
     g.N = N;
     g.ldc = ldc[st];
@@ -577,7 +742,7 @@ using namespace axi_sl;
 // [tiles x 4][error word][sliced bases x 4][sliced field][X, Y]
 struct TransformLayout {
   size_t sjobs, gjobs, items[4], tiles[4], err, basis[4], slices, work, total;
-  int n_items[4], n_tiles[4];
+  int n_items[4], n_tiles[4], form[4], parts[4];
 };
 
 TransformLayout transform_layout(int nr, int nz) {
@@ -587,15 +752,20 @@ TransformLayout transform_layout(int nr, int nz) {
   L.gjobs = o; o = align_up(o + 4 * sizeof(GemmJob), 256);
   for (int st = 0; st < 4; ++st) {
     const int M = st % 2 == 0 ? nz : nr, N = st % 2 == 0 ? nr : nz;
-    L.n_items[st] = slice_items(N, KIND_B);
-    L.n_tiles[st] = gemm_tiles(M, N);
-    L.items[st] = o; o = align_up(o + L.n_items[st] * sizeof(int4), 256);
-    L.tiles[st] = o; o = align_up(o + L.n_tiles[st] * sizeof(int4), 256);
+    L.form[st] = choose_form(gemm_tiles(M, N, FORM_NARROW), axi::sm_count());
+    const int groups = slice_groups(N, form_cols(L.form[st]));
+    L.parts[st] = slice_parts(groups, M, axi::sm_count());
+    L.n_items[st] = groups * L.parts[st];
+    L.n_tiles[st] = gemm_tiles(M, N, L.form[st]);
+    // room for any form, so that the size does not depend on the device
+    L.items[st] = o;
+    o = align_up(o + (size_t)slice_groups(N, 32) * ((M + 255) / 256) * sizeof(int4), 256);
+    L.tiles[st] = o; o = align_up(o + gemm_tiles(M, N, FORM_NARROW) * sizeof(int4), 256);
   }
   L.err = o; o = align_up(o + 16, 256);
   for (int st = 0; st < 4; ++st) {
     const int M = st % 2 == 0 ? nz : nr;
-    L.basis[st] = o; o = align_up(o + slice_bytes(M, M, KIND_A), 256);
+    L.basis[st] = o; o = align_up(o + slice_bytes(M, M, BM), 256);
   }
   L.slices = o; o = align_up(o + spectral_slice_bytes(nr, nz), 256);
   L.work = o; o = align_up(o + (size_t)2 * nr * nz * sizeof(double), 256);
@@ -606,7 +776,7 @@ TransformLayout transform_layout(int nr, int nz) {
 // Slices one matrix (blocking: the job record is copied from this stack).
 int slice_now(const SliceJob& j, cudaStream_t s) {
   std::vector<int4> items;
-  append_slice_items(items, 0, j.rows, j.kind);
+  append_slice_items(items, 0, j.rows, j.block, 1);
   const size_t off = align_up(sizeof(SliceJob), 256);
   char* d = nullptr;
   if (cudaMallocAsync(reinterpret_cast<void**>(&d), off + items.size() * sizeof(int4), s) !=
@@ -637,7 +807,7 @@ int check_shape(const char* what, int a, int b) {
 
 extern "C" int64_t axi_sliced_operand_bytes(int rows, int K) {
   if (rows <= 0 || K <= 0) return 0;
-  return (int64_t)align_up(slice_bytes(rows, K, KIND_A), 256);
+  return (int64_t)align_up(slice_bytes(rows, K, BM), 256);
 }
 
 extern "C" int axi_slice_operand_f64(void* dst, const double* src, int64_t row_stride,
@@ -646,7 +816,7 @@ extern "C" int axi_slice_operand_f64(void* dst, const double* src, int64_t row_s
   const char* what = "slice_operand";
   AXI_TRY(check_shape(what, rows, K));
   AXI_TRY(axi::check_ptrs(what, {dst, src}, {"dst", "src"}));
-  return slice_now(slice_job(src, row_stride, k_stride, rows, K, KIND_A, dst),
+  return slice_now(slice_job(src, row_stride, k_stride, rows, K, BM, dst, exps_of(dst, rows, K, BM)),
                    axi::as_stream(stream));
 }
 
@@ -678,12 +848,12 @@ extern "C" int axi_sliced_transform_plan(void* plan, const double* Er_inv_w, con
     const int M = st % 2 == 0 ? nz : nr;
     basis[st] = base + L.basis[st];
     const bool transposed = st % 2 == 0;
-    AXI_TRY(slice_now(slice_job(src[st], transposed ? 1 : M, transposed ? M : 1, M, M, KIND_A,
-                                base + L.basis[st]), s));
+    AXI_TRY(slice_now(slice_job(src[st], transposed ? 1 : M, transposed ? M : 1, M, M, BM,
+                                base + L.basis[st], exps_of(base + L.basis[st], M, M, BM)), s));
   }
   SliceJob sl[4];
   GemmJob gm[4];
-  spectral_jobs(nr, nz, nullptr, nz, nullptr, nz, reinterpret_cast<double*>(base + L.work),
+  spectral_jobs(nr, nz, L.form, nullptr, nz, nullptr, nz, reinterpret_cast<double*>(base + L.work),
                 base + L.slices, basis, inv_eig, sl, gm);
   std::vector<char> head(L.err + 16, 0);
   memcpy(&head[L.sjobs], sl, sizeof(sl));
@@ -691,8 +861,8 @@ extern "C" int axi_sliced_transform_plan(void* plan, const double* Er_inv_w, con
   for (int st = 0; st < 4; ++st) {
     const int M = st % 2 == 0 ? nz : nr, N = st % 2 == 0 ? nr : nz;
     std::vector<int4> items, tiles;
-    append_slice_items(items, st, N, KIND_B);
-    append_gemm_tiles(tiles, st, M, N, M);
+    append_slice_items(items, st, N, form_cols(L.form[st]), L.parts[st]);
+    append_gemm_tiles(tiles, st, M, N, M, L.form[st]);
     memcpy(&head[L.items[st]], items.data(), items.size() * sizeof(int4));
     memcpy(&head[L.tiles[st]], tiles.data(), tiles.size() * sizeof(int4));
   }
@@ -722,8 +892,8 @@ extern "C" int axi_sliced_transform_run(const void* plan, double* out, int ld_ou
   for (int st = 0; st < 4; ++st) {
     AXI_TRY(launch_slice(sj, reinterpret_cast<const int4*>(base + L.items[st]), L.n_items[st], s,
                          st == 0 ? in : nullptr, ld_in));
-    AXI_TRY(launch_gemm(gj, reinterpret_cast<const int4*>(base + L.tiles[st]), L.n_tiles[st], err,
-                        s, st == 3 ? out : nullptr, ld_out));
+    AXI_TRY(launch_gemm(gj, reinterpret_cast<const int4*>(base + L.tiles[st]), L.n_tiles[st],
+                        L.form[st], true, err, s, st == 3 ? out : nullptr, ld_out));
   }
   return AXI_OK;
 }
@@ -750,7 +920,7 @@ namespace {
 
 struct GemmLayout {
   size_t sjobs, gjob, items, tiles, err, a, b, total;
-  int n_items, n_tiles;
+  int n_items, n_tiles, form;
 };
 
 GemmLayout gemm_layout(int M, int N, int K) {
@@ -758,13 +928,14 @@ GemmLayout gemm_layout(int M, int N, int K) {
   size_t o = 0;
   L.sjobs = o; o = align_up(o + 2 * sizeof(SliceJob), 256);
   L.gjob = o; o = align_up(o + sizeof(GemmJob), 256);
-  L.n_items = slice_items(M, KIND_A) + slice_items(N, KIND_B);
-  L.n_tiles = gemm_tiles(M, N);
-  L.items = o; o = align_up(o + L.n_items * sizeof(int4), 256);
-  L.tiles = o; o = align_up(o + L.n_tiles * sizeof(int4), 256);
+  L.form = choose_form(gemm_tiles(M, N, FORM_NARROW), axi::sm_count());
+  L.n_items = slice_groups(M, BM) + slice_groups(N, form_cols(L.form));
+  L.n_tiles = gemm_tiles(M, N, L.form);
+  L.items = o; o = align_up(o + (size_t)(slice_groups(M, BM) + slice_groups(N, 32)) * sizeof(int4), 256);
+  L.tiles = o; o = align_up(o + gemm_tiles(M, N, FORM_NARROW) * sizeof(int4), 256);
   L.err = o; o = align_up(o + 16, 256);
-  L.a = o; o = align_up(o + slice_bytes(M, K, KIND_A), 256);
-  L.b = o; o = align_up(o + slice_bytes(N, K, KIND_B), 256);
+  L.a = o; o = align_up(o + slice_bytes(M, K, BM), 256);
+  L.b = o; o = align_up(o + slice_bytes(N, K, 32), 256);
   L.total = o;
   return L;
 }
@@ -786,15 +957,16 @@ extern "C" int axi_sliced_gemm_f64(double* C, const double* A, const double* B, 
   cudaStream_t s = axi::as_stream(stream);
   const GemmLayout L = gemm_layout(M, N, K);
   char* base = static_cast<char*>(work);
-  SliceJob sl[2] = {slice_job(A, K, 1, M, K, KIND_A, base + L.a),
-                    slice_job(B, K, 1, N, K, KIND_B, base + L.b)};
+  const int cols = form_cols(L.form);
+  SliceJob sl[2] = {slice_job(A, K, 1, M, K, BM, base + L.a, exps_of(base + L.a, M, K, BM)),
+                    slice_job(B, K, 1, N, K, cols, base + L.b, exps_of(base + L.b, N, K, cols))};
   GemmJob g;
   g.a = sl[0].planes; g.ea = sl[0].exps; g.b = sl[1].planes; g.eb = sl[1].exps;
-  g.c = C; g.scale = S; g.M = M; g.N = N; g.ldc = N; g.nk = k_steps(K);
+  g.c = C; g.scale = S; g.row_exps = nullptr; g.M = M; g.N = N; g.ldc = N; g.nk = k_steps(K);
   std::vector<int4> items, tiles;
-  append_slice_items(items, 0, M, KIND_A);
-  append_slice_items(items, 1, N, KIND_B);
-  append_gemm_tiles(tiles, 0, M, N, K);
+  append_slice_items(items, 0, M, BM, 1);
+  append_slice_items(items, 1, N, cols, 1);
+  append_gemm_tiles(tiles, 0, M, N, K, L.form);
   std::vector<char> head(L.err + 16, 0);
   memcpy(&head[L.sjobs], sl, sizeof(sl));
   memcpy(&head[L.gjob], &g, sizeof(g));
@@ -806,7 +978,8 @@ extern "C" int axi_sliced_gemm_f64(double* C, const double* A, const double* B, 
                        reinterpret_cast<const int4*>(base + L.items), L.n_items, s));
   int* err = reinterpret_cast<int*>(base + L.err);
   AXI_TRY(launch_gemm(reinterpret_cast<const GemmJob*>(base + L.gjob),
-                      reinterpret_cast<const int4*>(base + L.tiles), L.n_tiles, err, s));
+                      reinterpret_cast<const int4*>(base + L.tiles), L.n_tiles, L.form, false, err,
+                      s));
   int code = 0;
   if (cudaMemcpyAsync(&code, err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)

@@ -5,44 +5,52 @@
 // The method is the error-free slicing of Ozaki, Ogita, Oishi and Rump
 // ("Error-free transformations of matrix multiplication by using fast
 // routines of matrix multiplication", Numer. Algorithms 59, 2012): every row
-// of an operand is scaled by a power of two to |x| < 1 and written as nine
-// signed 7-bit digits,
+// of an operand is scaled by a power of two to |x| < 1 and written as eight
+// signed digits of radix 256,
 //
-//   x = sum_{i=0..8} d_i 2^(-6 - 7 i),  |d_i| <= 64      (62 bits below the row's
+//   x = sum_{i=0..7} d_i 2^(-6 - 8 i),  |d_i| <= 128     (62 bits below the row's
 //                                                          power of two)
 //
 // each digit plane stored as 16-bit floats (small integers, exact). A product
-// of two planes is a sum of integers of at most 2^12, so the FP32 accumulators
-// of the tensor cores hold it exactly; the planes i, j with i + j = d <= 8
-// share accumulator d. Over K = 512 the accumulators 0 .. 7 stay within
-// 8 * 512 * 2^12 = 2^24 (exact), accumulator 8 (weight 2^-68) rounds in its
-// last bit. The epilogue adds the accumulators as integers (96 bits, exact for
-// any K) and rounds to FP64 once.
+// of two planes is a sum of integers of at most 2^14, so the FP32 accumulators
+// of the tensor cores hold it exactly; the planes i, j with i + j = d <= 7
+// share accumulator d. Over K = 128 the accumulators stay within
+// 8 * 128 * 2^14 = 2^24, so all of them are exact; every 128 of K the epilogue
+// adds them to integer sums (96 bits, exact for any K), which it rounds to
+// FP64 once.
 //
 // Error of the four-product spectral solve against long double on the same
 // bases, 48 x 96 to 256 x 512 cells, smooth and white right-hand sides:
 // psi 0.8-2.0e-16 (FP64 FMA products 1.1-20e-16),
 // u_z 3-24e-16 (5-25e-16), u_r 4-53e-16 (8-76e-16), smaller in every case.
-// With eight digits psi stayed at 3-9e-16 but u_z and u_r went to 1-6e-14 (psi
-// near the axis is a cancelling sum), so nine are used.
+// With 55 bits below the row's power of two psi stayed at 3-9e-16 but u_z and
+// u_r went to 1-6e-14 (psi near the axis is a cancelling sum), so 62 are kept.
+// Nine digits of radix 128 give the same bits with 45 plane products instead
+// of 36 and accumulators that last for K = 512; the smaller digit count won
+// (shared-memory traffic per step, which bounds the main loop, 132 -> 108 KB).
 //
 // Why: GB300 executes FP64 at about 1.2 TFLOP/s and FP16 tensor work at about
-// 2 PFLOP/s. 45 plane products cost 45 * 2 M N K FP16 operations, 1/40 of the
+// 2 PFLOP/s. 36 plane products cost 36 * 2 M N K FP16 operations, 1/40 of the
 // time of the FP64 pipe. Measured, a soft-sphere step on 1024 x 512 cells (four
-// products): 4169 us with FP64 FMA products, 1143 us with these; a step of the
-// drop-in loop on 384 x 201 cells: 1178 and 488 us; a double engine step of
-// eight cases of 256 x 128 to 1024 x 512: 3543 us with FP64 DCTs in z and FMA
-// products in r, 837 us with four of these; of one 512 x 256 case 299 us
-// (553 with four FMA products) and 193 us.
+// products): 4169 us with FP64 FMA products, 1143 us with the first form of
+// these; a double engine step of eight cases of 256 x 128 to 1024 x 512: 3543 us
+// with FP64 DCTs in z and FMA products in r, 837 us with four of these. From
+// nine 7-bit digits and one tile form to the present (solve alone, us): 256 x
+// 128 80 -> 40, 512 x 256 109 -> 62, 1024 x 512 174 -> 154, 2048 x 1024 910 ->
+// 859.
 //
 // Operands are laid out by the slicing kernel exactly as shared memory wants
 // them: per block of rows and per 16 K-elements one contiguous piece (A: 128
-// rows, 36 KB; B: 32 rows, 9 KB) in the tensor core's unswizzled K-major
+// rows, 32 KB; B: 32 or 16 rows) in the tensor core's unswizzled K-major
 // layout (8-row x 16-byte core matrices), so a pipeline stage is two bulk
-// copies and every MMA is free of bank conflicts. B's nine planes follow each
-// other in its rows: one MMA of A's plane i against B's planes 0 .. 8 - i
-// (N = 32 (9 - i)) adds to the accumulators i .. 8, which are neighbouring
-// TMEM columns, so a K step of 16 takes 10 MMAs.
+// copies and every MMA is free of bank conflicts. B's eight planes follow each
+// other in its rows: one MMA of A's plane i against B's planes 0 .. 7 - i
+// (N = 32 (8 - i)) adds to the accumulators i .. 7, which are neighbouring
+// TMEM columns, so a K step of 16 takes 8 MMAs.
+//
+// Slicing and product kernels form a chain of programmatic dependent launches:
+// a kernel sets up its barriers and TMEM, reads its job and fills its stages
+// with A (constant) while its predecessor finishes.
 #pragma once
 
 #include <cuda.h>
@@ -54,38 +62,40 @@
 
 namespace axi_sl {
 
-constexpr int DIGITS = 9;
-constexpr int BITS = 7;
+constexpr int DIGITS = 8;
 constexpr int BM = 128;                              // rows of A per tile
-constexpr int BN = 32;                               // rows of B per tile
 constexpr int BK = 16;                               // K elements per stage
-constexpr int A_STAGE = DIGITS * BM * BK * 2;        // 36864 bytes
-constexpr int B_STAGE = DIGITS * BN * BK * 2;        // 9216 bytes
-constexpr int STAGE_BYTES = A_STAGE + B_STAGE;
+constexpr int A_STAGE = DIGITS * BM * BK * 2;        // 32768 bytes
 constexpr int NSTAGE = 5;
-constexpr int CHUNK = 512 / BK;                      // K steps whose sums stay exact
-constexpr int SMEM_BYTES = NSTAGE * STAGE_BYTES + 128 + 256;
+constexpr int CHUNK = 128 / BK;                      // K steps whose sums stay exact
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 32 * (2 + EPI_WARPS);
 
-enum { ERR_PRODUCER = 7, ERR_MMA = 8, ERR_EPILOGUE = 9, ERR_DRAIN = 10 };
-enum { KIND_A = 0, KIND_B = 1 };
-
-// exponent of a row that holds a value which is not finite: its products are NaN
-constexpr int EXP_NONFINITE = 1 << 20;
-
-inline int pad_rows(int rows, int kind) {
-  const int b = kind == KIND_A ? BM : BN;
-  return (rows + b - 1) / b * b;
+// Forms of a product launch: columns of C per tile (= rows of a block of B),
+// and blocks that share a tile's K (a cluster; their exact integer sums are
+// exchanged through distributed shared memory, so the split changes no bit).
+enum Form { FORM_WIDE = 0, FORM_NARROW = 1, FORM_NARROW2 = 2, FORM_NARROW4 = 3 };
+constexpr int form_cols(int form) { return form == FORM_WIDE ? 32 : 16; }
+constexpr int form_split(int form) {
+  return form == FORM_NARROW4 ? 4 : form == FORM_NARROW2 ? 2 : 1;
 }
+constexpr int b_stage(int bn) { return DIGITS * bn * BK * 2; }
+
+enum { ERR_PRODUCER = 7, ERR_MMA = 8, ERR_EPILOGUE = 9, ERR_DRAIN = 10 };
+
+// Sliced operands are laid out in blocks of `block` rows: BM for A, the tile
+// width for B.
+inline int pad_rows(int rows, int block) { return (rows + block - 1) / block * block; }
 inline int k_steps(int K) { return (K + BK - 1) / BK; }
 
-// Bytes of one sliced operand: the digit planes, then one exponent per row.
-inline size_t plane_bytes(int rows, int K, int kind) {
-  return (size_t)pad_rows(rows, kind) * k_steps(K) * BK * DIGITS * 2;
+// Bytes of one sliced operand: the digit planes, then one word per row, the
+// largest biased exponent of its values (0x7ff: a value is not finite, and the
+// row's products are NaN).
+inline size_t plane_bytes(int rows, int K, int block) {
+  return (size_t)pad_rows(rows, block) * k_steps(K) * BK * DIGITS * 2;
 }
-inline size_t slice_bytes(int rows, int K, int kind) {
-  return plane_bytes(rows, K, kind) + (size_t)pad_rows(rows, kind) * sizeof(int);
+inline size_t slice_bytes(int rows, int K, int block) {
+  return plane_bytes(rows, K, block) + (size_t)pad_rows(rows, block) * sizeof(int);
 }
 
 // One operand to slice: src[row * rs + k * ks].
@@ -93,10 +103,12 @@ struct SliceJob {
   const double* src;
   long long rs, ks;
   int rows, K;
-  int kind;
-  int pad;
+  int block;     // rows per block of the layout
+  int have_exps; // the product that wrote src also left its row exponents in exps
   uint8_t* planes;
   int* exps;
+  int* clear;    // words that the next product's epilogue accumulates into
+  int n_clear;
 };
 
 struct GemmJob {
@@ -106,33 +118,64 @@ struct GemmJob {
   const int* eb;
   double* c;
   const double* scale;  // elementwise factor, row-major (M, N), or null
+  int* row_exps;        // largest exponent of each row of C, accumulated (or null)
   int M, N, ldc;
   int nk;               // K steps
 };
 
-inline SliceJob slice_job(const double* src, long long rs, long long ks, int rows, int K, int kind,
-                          void* dst) {
+inline SliceJob slice_job(const double* src, long long rs, long long ks, int rows, int K, int block,
+                          void* planes, int* exps) {
   SliceJob j;
-  j.src = src; j.rs = rs; j.ks = ks; j.rows = rows; j.K = K; j.kind = kind; j.pad = 0;
-  j.planes = static_cast<uint8_t*>(dst);
-  j.exps = reinterpret_cast<int*>(j.planes + plane_bytes(rows, K, kind));
+  j.src = src; j.rs = rs; j.ks = ks; j.rows = rows; j.K = K; j.block = block;
+  j.have_exps = 0;
+  j.planes = static_cast<uint8_t*>(planes);
+  j.exps = exps;
+  j.clear = nullptr;
+  j.n_clear = 0;
   return j;
 }
+// The exponents behind the planes of an operand.
+inline int* exps_of(void* planes, int rows, int K, int block) {
+  return reinterpret_cast<int*>(static_cast<uint8_t*>(planes) + plane_bytes(rows, K, block));
+}
 
-// Items of the slicing kernel (8 rows each) and tiles of the product.
-inline int slice_items(int rows, int kind) { return pad_rows(rows, kind) / 8; }
-inline int gemm_tiles(int M, int N) { return ((M + BM - 1) / BM) * ((N + BN - 1) / BN); }
-void append_slice_items(std::vector<int4>& items, int job, int rows, int kind);
-void append_gemm_tiles(std::vector<int4>& tiles, int job, int M, int N, int K);
+// Items of the slicing kernel: 8 rows each, and a share of their K where the
+// row groups of a launch alone would leave SMs idle (a row's largest exponent
+// is then found by every share, unless the product before has left it).
+inline int slice_groups(int rows, int block) { return pad_rows(rows, block) / 8; }
+inline int slice_parts(int groups_of_launch, int K, int sms) {
+  const int want = (2 * sms + groups_of_launch - 1) / groups_of_launch;
+  const int most = (K + 255) / 256;
+  return want < 1 ? 1 : want < most ? want : most;
+}
+// Tiles of the product.
+inline int gemm_tiles(int M, int N, int form) {
+  const int cols = form_cols(form);
+  return ((M + BM - 1) / BM) * ((N + cols - 1) / cols);
+}
+// Form of a launch that has `narrow_tiles` tiles of 16 columns: the most blocks
+// that all run at once. Solves (four products and slicings, us) wide / narrow /
+// narrow, K in two / in four: 128 x 64 cells 56 / 40 / 38 / 33, 256 x 128 70 /
+// 53 / 47 / 40, 512 x 256 104 / 81 / 64 / 85, 768 x 384 130 / 109 / 140 / 187,
+// 1024 x 512 159 / 229 / 312 / 391.
+inline int choose_form(int narrow_tiles, int sms) {
+  return 4 * narrow_tiles <= sms   ? FORM_NARROW4
+         : 2 * narrow_tiles <= sms ? FORM_NARROW2
+         : narrow_tiles <= sms     ? FORM_NARROW
+                                   : FORM_WIDE;
+}
+void append_slice_items(std::vector<int4>& items, int job, int rows, int block, int parts);
+void append_gemm_tiles(std::vector<int4>& tiles, int job, int M, int N, int K, int form);
 // longest main loop first, stable
 void order_tiles(std::vector<int4>& tiles);
 
 // The first operand's source / the output may be given per call (overrides,
-// null: as in the job table; only for tables of one job).
+// null: as in the job table; only for tables of one job). a_ready: A is not written by kernels still
+// running, so it may be read ahead of the launch's dependencies.
 int launch_slice(const SliceJob* jobs_dev, const int4* items_dev, int n_items, cudaStream_t s,
                  const double* src = nullptr, long long rs = 0);
-int launch_gemm(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, int* err_dev,
-                cudaStream_t s, double* c = nullptr, int ldc = 0);
+int launch_gemm(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, int form, bool a_ready,
+                int* err_dev, cudaStream_t s, double* c = nullptr, int ldc = 0);
 
 // The four spectral products of one case on sliced operands (as C = A B^T):
 //   0  X (nz, nr)   = Ezinv * in^T                 in   (nr, nz), row stride ld_in
@@ -143,7 +186,7 @@ int launch_gemm(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, int
 // hand (spectral_slice_bytes). basis: Ezinv, Erinv_w, Ez, Er as sliced A
 // operands.
 size_t spectral_slice_bytes(int nr, int nz);
-void spectral_jobs(int nr, int nz, const double* in, long long ld_in, double* out, int ld_out,
+void spectral_jobs(int nr, int nz, const int form[4], const double* in, long long ld_in, double* out, int ld_out,
                    double* work, void* slices, const void* const basis[4], const double* inv_eig,
                    SliceJob sl[4], GemmJob gm[4]);
 
