@@ -421,6 +421,46 @@ __device__ __forceinline__ unsigned long long order_bits(T v) {
                         : (unsigned long long)__float_as_uint((float)v);
 }
 
+// Value tests on the bits (a comparison of doubles is an FP64 instruction).
+__device__ __forceinline__ bool nonzero_bits(double x) {
+  return ((__double2hiint(x) << 1) | __double2loint(x)) != 0;
+}
+__device__ __forceinline__ bool nonzero_bits(float x) { return __float_as_uint(x) << 1 != 0; }
+
+// Sum of a thread value over a warp, in double and in a fixed order. Most tiles
+// lie outside the body and sum zeros: a warp of zeros spends no FP64
+// instruction (each holds the scheduler's FP64 unit for 64 cycles).
+template <typename T>
+__device__ __forceinline__ double warp_sum(T v) {
+  double x = 0.0;
+  if (__any_sync(0xffffffffu, nonzero_bits(v))) {
+    x = (double)v;
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+  }
+  return x;
+}
+// Sum of the block's warp sums, by the lanes of warp 0 (all lanes get it).
+__device__ __forceinline__ double block_sum(const double* red) {
+  const int lane = threadIdx.x & 31;
+  double x = red[lane & (NT / 32 - 1)];
+  if (!__any_sync(0xffffffffu, nonzero_bits(x))) return 0.0;
+  for (int o = NT / 64; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+// Sum of a case's tile partials, by the lanes of warp 0 in a fixed order (all
+// lanes get it). One thread adding them one after the other held up the end of
+// the kernel: 64 cycles each, 256 of them on a 1024 x 512 case.
+__device__ __forceinline__ double partial_sum(const double* partials, unsigned int n) {
+  const int lane = threadIdx.x & 31;
+  double x = 0.0;
+  for (unsigned int q = lane; q < n; q += 32) {
+    const double v = ((const volatile double*)partials)[q];
+    if (nonzero_bits(v)) x += v;
+  }
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
 // dt = min(diffusive limit, CFL / max(|u_z| + |u_r|)) (flow_past_sphere.py:150-155)
 // from the maximum that vel_max left in the state block. Every block that
 // needs dt evaluates it from the same bits, so all get the same value.
@@ -567,11 +607,25 @@ __global__ void __launch_bounds__(NT) vel_max_kernel(const axi_case* __restrict_
 // drag integrand); the curl of the difference then updates omega of the
 // owned cells.
 // ---------------------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ void penalise_point(T uz, T ur, T lc, T ubody, T& pz, T& pr) {
-  const T inv = T(1) / (T(1) + lc);
-  pz = (uz + lc * ubody) * inv;
-  pr = ur * inv;
+// Double engine, one point of the body: penalised velocity, its difference from
+// the velocity and the drag / penalisation force integrand r chi (u_z - U_body)
+// (flow_past_sphere.py:173, compute_forces.py:14; the float engine adds it as
+// -r chi (U - u) / (1 + lam dt chi)). Out of line, so that its division is not
+// run ahead for the points outside the body.
+struct PenalisedPoint {
+  double pz, pr, dz, dr, drag;
+};
+__device__ __noinline__ PenalisedPoint penalise_point(double uz, double ur, double lamdt, double ch,
+                                                      double ubody, double r) {
+  const double lc = lamdt * ch;
+  const double inv = 1.0 / (1.0 + lc);
+  PenalisedPoint v;
+  v.pz = (uz + lc * ubody) * inv;
+  v.pr = ur * inv;
+  v.dz = v.pz - uz;
+  v.dr = v.pr - ur;
+  v.drag = r * ch * (v.pz - ubody);
+  return v;
 }
 
 constexpr int PN_SW = TX + 2, PN_SH = TY + 2;  // u_pen - u, halo 1
@@ -675,11 +729,16 @@ __global__ void __launch_bounds__(NT, penalise_min_blocks<T, PAIR>()) penalise_k
     const int gjm = j0 + qm;
     // u_pen - u at one point of the tile + halo 1 (p in [-1, TY], q in [-1, TX])
     auto point = [&](int p, int q, T uz, T ur, T ch, int gi, int gj) {
-      T pz, pr, dz, dr;
-      if constexpr (sizeof(T) == 8) {
-        penalise_point<T>(uz, ur, lamdt * ch, ubody, pz, pr);
-        dz = pz - uz;
-        dr = pr - ur;
+      T pz = uz, pr = ur, dz = T(0), dr = T(0);
+      // outside the body (chi 0: most points) the velocity stays
+      if (!nonzero_bits(ch)) {
+      } else if constexpr (sizeof(T) == 8) {
+        const PenalisedPoint v = penalise_point(uz, ur, lamdt, ch, ubody, rowf[1][p + 1]);
+        pz = v.pz;
+        pr = v.pr;
+        dz = v.dz;
+        dr = v.dr;
+        if (p >= 0 && p < TY && q >= 0 && q < TX) cd_part += v.drag;
       } else {
         // u_pen - u = lam dt chi (U - u) / (1 + lam dt chi), formed directly:
         // inside the body u is close to U, and the difference of the rounded
@@ -702,10 +761,6 @@ __global__ void __launch_bounds__(NT, penalise_min_blocks<T, PAIR>()) penalise_k
         const int c = gi * nz + gj;
         uzp[c] = pz;
         urp[c] = pr;
-        // drag / penalisation force integrand r chi (u_z - U_body)
-        // (flow_past_sphere.py:173, compute_forces.py:14); the float engine
-        // adds it above as -r chi (U - u) / (1 + lam dt chi)
-        if constexpr (sizeof(T) == 8) cd_part += rowf[1][p + 1] * ch * (pz - ubody);
       }
     };
     {
@@ -803,20 +858,25 @@ __global__ void __launch_bounds__(NT, penalise_min_blocks<T, PAIR>()) penalise_k
       }
     }
     // drag: thread sums in T, then warps, tiles and cases in double, fixed order
-    double x = cd_part;
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if ((threadIdx.x & 31) == 0) red[it & 1][threadIdx.x >> 5] = (double)x;
+    const double x = warp_sum(cd_part);
+    if ((threadIdx.x & 31) == 0) red[it & 1][threadIdx.x >> 5] = x;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
       const unsigned int ntiles = dev_tiles_of(k);
-      double sum = 0.0;
-      for (int q = 0; q < NT / 32; ++q) sum += red[it & 1][q];
-      k.partials[tr.w] = sum;
-      __threadfence();
-      if (atomicAdd(counter(k, 1), 1u) == ntiles - 1) {
+      const double sum = block_sum(red[it & 1]);
+      unsigned int arrived = 0;
+      if (threadIdx.x == 0) {
+        k.partials[tr.w] = sum;
         __threadfence();
-        double tot = 0.0;
-        for (unsigned int q = 0; q < ntiles; ++q) tot += ((volatile double*)k.partials)[q];
+        arrived = atomicAdd(counter(k, 1), 1u);
+      }
+      arrived = __shfl_sync(0xffffffffu, arrived, 0);
+      double tot = 0.0;
+      if (arrived == ntiles - 1) {
+        __threadfence();
+        tot = partial_sum(k.partials, ntiles);
+      }
+      if (threadIdx.x == 0 && arrived == ntiles - 1) {
         const double dt = k.state[AXI_ST_DT];
         if (!(tot == tot) || !(fabs(tot) <= 1.7976931348623157e308))
           atomicOr(reinterpret_cast<unsigned int*>(&k.state[AXI_ST_STATUS]),
@@ -855,15 +915,27 @@ __device__ __forceinline__ T face_flux_g(T gm1, T g0, T g1, T g2, T u0, T u1) {
   return u0 > -u1 ? a : b;
 }
 
+// u0 > -u1 of doubles on the integer pipe (sign and magnitude, zeros equal);
+// infinities and NaN by the comparison itself, out of line.
+__device__ __noinline__ bool upwind_plain(double u0, double u1) { return u0 > -u1; }
+__device__ __forceinline__ bool upwind(double u0, double u1) {
+  const long long b0 = __double_as_longlong(u0), b1 = __double_as_longlong(u1);
+  const long long m0 = b0 & 0x7fffffffffffffffll, m1 = b1 & 0x7fffffffffffffffll;
+  if (exponent_bits(u0) == 0x7ff || exponent_bits(u1) == 0x7ff) return upwind_plain(u0, u1);
+  return (b0 < 0 ? -m0 : m0) > (b1 < 0 ? m1 : -m1);
+}
+
 template <typename T>
 __device__ __forceinline__ T face_flux(T fm1, T f0, T f1, T f2, T um1, T u0, T u1, T u2) {
   const T third = T(1) / T(3), five6 = T(5) / T(6), sixth = T(1) / T(6);
   if constexpr (sizeof(T) == 4) {
     return face_flux_g(fm1 * um1, f0 * u0, f1 * u1, f2 * u2, u0, u1);
   } else {
-    // the reference's products and order (bit-exact with the FP64 oracle)
-    if (u0 > -u1) return third * f1 * u1 + five6 * f0 * u0 - sixth * fm1 * um1;
-    return third * f0 * u0 + five6 * f1 * u1 - sixth * f2 * u2;
+    // the reference's products and order (bit-exact with the FP64 oracle), the
+    // operands of the upwind side selected first
+    const bool l = upwind(u0, u1);
+    return third * (l ? f1 : f0) * (l ? u1 : u0) + five6 * (l ? f0 : f1) * (l ? u0 : u1) -
+           sixth * (l ? fm1 : f2) * (l ? um1 : u2);
   }
 }
 
@@ -1046,7 +1118,7 @@ __device__ __forceinline__ T advect_point(const T* sw, const T* sz, const T* sr,
 // FP32: 4 resident blocks per SM (up to 64 registers; at 5 blocks the
 // pairwise flux divergence spilled and ran 5 % slower)
 template <typename T>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 1) advect_diffuse_kernel(const axi_case* __restrict__ cases,
+__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 2) advect_diffuse_kernel(const axi_case* __restrict__ cases,
                                                             const int4* __restrict__ tiles,
                                                             int n_tiles,
                                                             const CUtensorMap* __restrict__ maps,
@@ -1055,6 +1127,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 1) advect_diffuse_ker
   __shared__ __align__(8) uint64_t bars[AD_NBUF];
   __shared__ double red[2][NT / 32];
   __shared__ T rowf[3][AD_SH];  // 1 / (2 dx r), 1 / r^2, r of rows i0 - 1 .. i0 + TY
+  // double engine: z faces left of the two warps' columns, per row
+  __shared__ T face0[sizeof(T) == 8 ? 2 * AD_AH : 1];
   AdRing<T> ring{reinterpret_cast<T*>(align_smem(ad_raw)), axi_tma::smem_u32(bars)};
   T* wa = ring.base + AdRing<T>::BYTES / sizeof(T);
   constexpr int which[3] = {MAP_W, MAP_UZ, MAP_UR};
@@ -1177,6 +1251,14 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 1) advect_diffuse_ker
       const bool jin = gjm < nz, jflux = gjm >= 2 && gjm < nz - 2;
       const int p0 = -2 + AD_RA * grp;
       int c = ad_box(p0, qm);
+      // z-direction face fluxes: lane l passes the face behind its column to
+      // lane l + 1; those before columns 0 and 32 are formed first
+      if (threadIdx.x < 2 * AD_AH) {
+        const int e = ad_box(-2 + (int)threadIdx.x / 2, (threadIdx.x & 1) * 32);
+        face0[threadIdx.x] = face_flux(sw[e - 2], sw[e - 1], sw[e], sw[e + 1], sz[e - 2],
+                                       sz[e - 1], sz[e], sz[e + 1]);
+      }
+      __syncthreads();
       // r-direction face fluxes: yb of row p is yf of row p - 1
       T fm2 = sw[c - 2 * L], fm1 = sw[c - L], f0 = sw[c], f1 = sw[c + L];
       T um2 = sr[c - 2 * L], um1 = sr[c - L], u0 = sr[c], u1 = sr[c + L];
@@ -1186,16 +1268,16 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 1) advect_diffuse_ker
         const int pr = p0 + m, gi = i0 + pr;
         const T f2 = sw[c + 2 * L], u2 = sr[c + 2 * L];
         const T yf = face_flux(fm1, f0, f1, f2, um1, u0, u1, u2);
+        const T xf = face_flux(sw[c - 1], f0, sw[c + 1], sw[c + 2], sz[c - 1], sz[c], sz[c + 1],
+                               sz[c + 2]);
+        T xb = __shfl_up_sync(0xffffffffu, xf, 1);
+        if (lane == 0) xb = face0[2 * (pr + 2) + (warp & 1)];
         T val = T(0);
         if (jin && gi >= 0 && gi < nr) {
           T flux = T(0);
           // pystencils ghost layers: no flux in the last two rows and the
           // first and last two columns
           if (jflux && gi < nr - 2) {
-            const T xf = face_flux(sw[c - 1], f0, sw[c + 1], sw[c + 2], sz[c - 1], sz[c],
-                                   sz[c + 1], sz[c + 2]);
-            const T xb = face_flux(sw[c - 2], sw[c - 1], f0, sw[c + 1], sz[c - 2], sz[c - 1],
-                                   sz[c], sz[c + 1]);
             flux = a * xf;
             flux = flux - a * xb;
             flux = flux + a * yf;
@@ -1357,29 +1439,32 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 1) advect_diffuse_ker
       }
     }
     if (sediment) {
-      double x = cd_part;
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      if ((threadIdx.x & 31) == 0) red[it & 1][threadIdx.x >> 5] = (double)x;
+      const double x = warp_sum(cd_part);
+      if ((threadIdx.x & 31) == 0) red[it & 1][threadIdx.x >> 5] = x;
     }
     // end of tile: the boxes and wa / tp may be reused from here on
     __syncthreads();
-    if (threadIdx.x != 0) continue;
+    if (threadIdx.x >= 32) continue;
     if (!sediment) {
-      if (tr.w == 0) {
+      if (threadIdx.x == 0 && tr.w == 0) {
         k.state[AXI_ST_T] += k.state[AXI_ST_DT];
         k.state[AXI_ST_STEPS] += 1.0;
       }
       continue;
     }
     const unsigned int ntiles = dev_tiles_of(k);
-    double sum = 0.0;
-    for (int q = 0; q < NT / 32; ++q) sum += red[it & 1][q];
-    k.partials[ntiles + tr.w] = sum;
+    const double sum = block_sum(red[it & 1]);
+    unsigned int arrived = 0;
+    if (threadIdx.x == 0) {
+      k.partials[ntiles + tr.w] = sum;
+      __threadfence();
+      arrived = atomicAdd(counter(k, 1), 1u);
+    }
+    arrived = __shfl_sync(0xffffffffu, arrived, 0);
+    if (arrived != 2 * ntiles - 1) continue;
     __threadfence();
-    if (atomicAdd(counter(k, 1), 1u) != 2 * ntiles - 1) continue;
-    __threadfence();
-    double tot = 0.0;
-    for (unsigned int q = 0; q < ntiles; ++q) tot += ((volatile double*)k.partials)[ntiles + q];
+    const double tot = partial_sum(k.partials + ntiles, ntiles);
+    if (threadIdx.x != 0) continue;
     const double cd = k.cd_scale * tot;
     const double dt = k.state[AXI_ST_DT];
     // body ODE, falling_rigid_sphere.py:176-181 (FP64)
