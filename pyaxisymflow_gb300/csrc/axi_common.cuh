@@ -68,21 +68,26 @@ int sm_count();
 // predecessor on the stream runs; it waits with pdl_wait before it touches
 // what that one reads or writes) and, with cluster > 1, thread-block clusters.
 template <typename... P, typename... A>
-inline int launch_pdl(const char* what, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
-                      cudaStream_t s, int cluster, A... args) {
+inline int launch_chain(bool pdl, const char* what, void (*kernel)(P...), dim3 grid, dim3 block,
+                        size_t smem, cudaStream_t s, int cluster, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = cluster;
-  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  cfg.numAttrs = 0;
+  if (pdl) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[cfg.numAttrs].val.clusterDim.x = cluster;
+    at[cfg.numAttrs].val.clusterDim.y = at[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
   if (e != cudaSuccess) {
     set_error("%s: CUDA launch failed: %s", what, cudaGetErrorString(e));
@@ -93,7 +98,7 @@ inline int launch_pdl(const char* what, void (*kernel)(P...), dim3 grid, dim3 bl
 }
 // Waits until the grids this one depends on are complete and their writes visible.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Lets the next grid of a launch_pdl chain start once every block got here.
+// Lets the next grid of a chain start once every block got here.
 __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

@@ -161,6 +161,7 @@ __global__ void __launch_bounds__(THREADS) dct_rows_kernel(const DctJob* __restr
   float2* a = dsm;
   float2* b = dsm + ELEMS;
   __shared__ DctJob sjob;
+  axi::pdl_trigger();
   const int4 it = items[blockIdx.x];
   if (threadIdx.x == 0) sjob = jobs[it.x];
   if (threadIdx.x == 32 && blockIdx.x + ahead < n_items) {
@@ -193,6 +194,7 @@ __global__ void __launch_bounds__(THREADS) dct_rows_kernel(const DctJob* __restr
   if (threadIdx.x == 0) sjob.twiddle = tws;
   for (int m = threadIdx.x; m < n_tw; m += blockDim.x)
     tws[padded ? reg_tw_index(m) : m] = __ldg(gtw + m);
+  axi::pdl_wait();  // the rows (and the output) belong to the kernel before until here
   __syncthreads();
   const DctJob& job = sjob;
   const int N = job.N, half = N / 2;
@@ -732,7 +734,7 @@ bool plan_radices(int N, int* radix, int* nstages) {
 }
 
 int launch(const DctJob* jobs_dev, const int4* items_dev, int n_items, bool forward,
-           cudaStream_t s, int prefetch_waves) {
+           cudaStream_t s, int prefetch_waves, bool pdl) {
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
   std::call_once(once, [] {
@@ -755,9 +757,9 @@ int launch(const DctJob* jobs_dev, const int4* items_dev, int n_items, bool forw
   // prefetch distance: `prefetch_waves` resident waves ahead (n_items: none)
   const int wave = per_sm * axi::sm_count();
   const int ahead = prefetch_waves < 0 ? n_items : wave * (prefetch_waves > 0 ? prefetch_waves : 1);
-  dct_rows_kernel<<<n_items, THREADS, SMEM_BYTES, s>>>(jobs_dev, items_dev, n_items, ahead,
-                                                       forward ? 1 : 0);
-  return axi::launch_status("dct_rows");
+  return axi::launch_chain(pdl, "dct_rows", dct_rows_kernel, dim3(n_items), dim3(THREADS),
+                           SMEM_BYTES, s, 1, jobs_dev, items_dev, n_items, ahead,
+                           forward ? 1 : 0);
 }
 
 }  // namespace axi_dct

@@ -157,6 +157,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) kill_reset_kernel(const axi_case* __restrict__ cases,
                                                          unsigned int* __restrict__ vm_done) {
   const axi_case& k = cases[blockIdx.y];
+  axi::pdl_trigger();
+  axi::pdl_wait();
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *vm_done = 0u;  // vel_max arrivals
   T* w = F<T>(k.omega);
   const int nr = k.nr, nz = k.nz, wd = k.kill_width;
@@ -516,8 +518,10 @@ __global__ void __launch_bounds__(NT) vel_max_kernel(const axi_case* __restrict_
   VmRing<T> ring{reinterpret_cast<T*>(align_smem(vm_raw)), axi_tma::smem_u32(bars)};
   constexpr int which[1] = {MAP_PSI};
   int issued = 0;
+  axi::pdl_trigger();
+  if (threadIdx.x == 0) ring.init();
+  axi::pdl_wait();
   if (threadIdx.x == 0) {
-    ring.init();
     issued = ring_prologue<VmRing<T>, VM_NBUF, 1>(ring, maps, tiles, n_tiles, which, -2);
   }
   __syncthreads();
@@ -659,8 +663,10 @@ __global__ void __launch_bounds__(NT, penalise_min_blocks<T, PAIR>()) penalise_k
   constexpr int which3[3] = {MAP_PSI, MAP_CHI, MAP_PSI_LO};
   const int(&which)[NB] = *reinterpret_cast<const int(*)[NB]>(&which3);
   int issued = 0;
+  axi::pdl_trigger();
+  if (threadIdx.x == 0) ring.init();
+  axi::pdl_wait();
   if (threadIdx.x == 0) {
-    ring.init();
     issued = ring_prologue<Ring, PN_NBUF, NB>(ring, maps, tiles, n_tiles, which, -2);
   }
   __syncthreads();
@@ -1133,8 +1139,10 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 2) advect_diffuse_ker
   T* wa = ring.base + AdRing<T>::BYTES / sizeof(T);
   constexpr int which[3] = {MAP_W, MAP_UZ, MAP_UR};
   int issued = 0;
+  axi::pdl_trigger();
+  if (threadIdx.x == 0) ring.init();
+  axi::pdl_wait();
   if (threadIdx.x == 0) {
-    ring.init();
     issued = ring_prologue<AdRing<T>, AD_NBUF, 3>(ring, maps, tiles, n_tiles, which, -AD_H);
   }
   __syncthreads();
@@ -1969,6 +1977,19 @@ struct StencilGrid {
   }
 };
 
+// The launches of a float step with DCTs chain as programmatic dependent
+// launches (each sets up its barriers, TMEM, job and twiddle table while its
+// predecessor drains) where a plan is small. Without / with, us per step: one
+// 256 x 128 case 65.9 / 62.8, five cases of 256 x 128 to 1024 x 512 (544 tiles)
+// 150.8 / 142.9; but 64 cases (2 x 4496 tiles) 748 / 758, the dense products of
+// 500 x 252 101 / 106 and eight cases of the double engine 723 / 728: there the
+// blocks that wait take room from others, or start on SMs with cold caches.
+constexpr int CHAIN_TILES = 1024;
+inline bool chained(const axi_plan_info* info) {
+  return info->elem_bytes == 4 && (info->flags & AXI_PLAN_DCT_Z) &&
+         info->n_stencil_tiles <= CHAIN_TILES;
+}
+
 // One of the four products of the double engine on sliced operands: its field
 // operand sliced, then the product.
 int run_sliced(const axi_plan_info* info, const PlanView& v, int st, cudaStream_t s) {
@@ -1980,22 +2001,23 @@ int run_sliced(const axi_plan_info* info, const PlanView& v, int st, cudaStream_
 template <typename T>
 int run_phase(int phase, const axi_plan_info* info, const PlanView& v, cudaStream_t s) {
   const int nt = info->n_stencil_tiles, ng = info->n_gemm_tiles;
+  const bool pdl = chained(info);
   switch (phase) {
     case PH_KILL:
-      kill_reset_kernel<T><<<dim3(KILL_BLOCKS, info->n_cases), 256, 0, s>>>(
-          v.cases, reinterpret_cast<unsigned int*>(v.err + 1));
-      break;
+      return axi::launch_chain(pdl, "kill_reset", kill_reset_kernel<T>,
+                               dim3(KILL_BLOCKS, info->n_cases), dim3(256), 0, s, 1, v.cases,
+                               reinterpret_cast<unsigned int*>(v.err + 1));
     case PH_TRANSFORM:
       if (v.dct_jobs) {
         // z transform, radial product, inverse z transform, radial product
         AXI_TRY(axi_dct::launch(v.dct_jobs, v.dct_items, info->n_dct_items, true, s,
-                                info->tune.prefetch_waves));
+                                info->tune.prefetch_waves, pdl));
         AXI_TRY(axi_tc::launch(v.jobs, v.tc_tiles[1], info->n_tc_tiles[1], v.err, s,
-                               info->tune.tc_ctas_percent));
+                               info->tune.tc_ctas_percent, pdl));
         AXI_TRY(axi_dct::launch(v.dct_jobs + info->n_cases, v.dct_items, info->n_dct_items,
-                                false, s, info->tune.prefetch_waves));
+                                false, s, info->tune.prefetch_waves, pdl));
         AXI_TRY(axi_tc::launch(v.jobs, v.tc_tiles[3], info->n_tc_tiles[3], v.err, s,
-                               info->tune.tc_ctas_percent));
+                               info->tune.tc_ctas_percent, pdl));
         break;
       }
       if (v.sliced_jobs) {
@@ -2005,7 +2027,7 @@ int run_phase(int phase, const axi_plan_info* info, const PlanView& v, cudaStrea
       if (v.jobs) {
         for (int st = 0; st < 4; ++st)
           AXI_TRY(axi_tc::launch(v.jobs, v.tc_tiles[st], info->n_tc_tiles[st], v.err, s,
-                                 info->tune.tc_ctas_percent));
+                                 info->tune.tc_ctas_percent, pdl));
         break;
       }
       if (v.dct64_jobs) {
@@ -2024,34 +2046,32 @@ int run_phase(int phase, const axi_plan_info* info, const PlanView& v, cudaStrea
       break;
     case PH_VEL_MAX:
       AXI_TRY(stencil_attrs<T>());
-      vel_max_kernel<T><<<StencilGrid<T>::get(info, PH_VEL_MAX, nt), NT, vel_max_smem<T>(), s>>>(
-          v.cases, v.stencil, nt, v.maps, v.err, info->n_cases,
-          reinterpret_cast<unsigned int*>(v.err + 1));
-      break;
+      return axi::launch_chain(pdl, "vel_max", vel_max_kernel<T>,
+                               dim3(StencilGrid<T>::get(info, PH_VEL_MAX, nt)), dim3(NT),
+                               vel_max_smem<T>(), s, 1, v.cases, v.stencil, nt, v.maps, v.err,
+                               info->n_cases, reinterpret_cast<unsigned int*>(v.err + 1));
     case PH_PENALISE:
       AXI_TRY(stencil_attrs<T>());
       if constexpr (sizeof(T) == 4) {
         if (info->flags & AXI_PLAN_REFINE) {
           // psi read as psi + psi_lo
-          penalise_kernel<T, true>
-              <<<StencilGrid<T>::get(info, PH_PENALISE, nt, true), NT, penalise_smem<T, true>(),
-                 s>>>(v.cases, v.stencil, nt, v.maps, v.err,
-                      StencilGrid<T>::ahead(info, PH_PENALISE, nt, true));
-          break;
+          return axi::launch_chain(pdl, "penalise", penalise_kernel<T, true>,
+                                   dim3(StencilGrid<T>::get(info, PH_PENALISE, nt, true)),
+                                   dim3(NT), penalise_smem<T, true>(), s, 1, v.cases, v.stencil,
+                                   nt, v.maps, v.err,
+                                   StencilGrid<T>::ahead(info, PH_PENALISE, nt, true));
         }
       }
-      penalise_kernel<T, false>
-          <<<StencilGrid<T>::get(info, PH_PENALISE, nt), NT, penalise_smem<T, false>(), s>>>(
-              v.cases, v.stencil, nt, v.maps, v.err,
-              StencilGrid<T>::ahead(info, PH_PENALISE, nt));
-      break;
+      return axi::launch_chain(pdl, "penalise", penalise_kernel<T, false>,
+                               dim3(StencilGrid<T>::get(info, PH_PENALISE, nt)), dim3(NT),
+                               penalise_smem<T, false>(), s, 1, v.cases, v.stencil, nt, v.maps,
+                               v.err, StencilGrid<T>::ahead(info, PH_PENALISE, nt));
     case PH_ADVECT_DIFFUSE:
       AXI_TRY(stencil_attrs<T>());
-      advect_diffuse_kernel<T>
-          <<<StencilGrid<T>::get(info, PH_ADVECT_DIFFUSE, nt), NT, advect_diffuse_smem<T>(), s>>>(
-              v.cases, v.stencil, nt, v.maps, v.err,
-              StencilGrid<T>::ahead(info, PH_ADVECT_DIFFUSE, nt));
-      break;
+      return axi::launch_chain(pdl, "advect_diffuse", advect_diffuse_kernel<T>,
+                               dim3(StencilGrid<T>::get(info, PH_ADVECT_DIFFUSE, nt)), dim3(NT),
+                               advect_diffuse_smem<T>(), s, 1, v.cases, v.stencil, nt, v.maps,
+                               v.err, StencilGrid<T>::ahead(info, PH_ADVECT_DIFFUSE, nt));
     case PH_TRANSFORM_PART0:
     case PH_TRANSFORM_PART0 + 1:
     case PH_TRANSFORM_PART0 + 2:

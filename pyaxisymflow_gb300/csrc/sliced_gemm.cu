@@ -638,7 +638,7 @@ void order_tiles(std::vector<int4>& tiles) {
 int launch_slice(const SliceJob* jobs_dev, const int4* items_dev, int n_items, cudaStream_t s,
                  const double* src, long long rs) {
   if (n_items <= 0) return AXI_OK;
-  return axi::launch_pdl("slice", slice_kernel, dim3(n_items), dim3(SL_THREADS), 0, s, 1, jobs_dev,
+  return axi::launch_chain(true, "slice", slice_kernel, dim3(n_items), dim3(SL_THREADS), 0, s, 1, jobs_dev,
                          items_dev, src, rs);
 }
 
@@ -661,7 +661,7 @@ int launch_tiles(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, bo
   const int sms = axi::sm_count();
   // a split tile's blocks take one tile (the exchange is used once)
   const int blocks = SPLIT > 1 ? SPLIT * n_tiles : n_tiles < sms ? n_tiles : sms;
-  return axi::launch_pdl("sliced_gemm", sliced_gemm_kernel<BN, SPLIT>, dim3(blocks), dim3(THREADS),
+  return axi::launch_chain(true, "sliced_gemm", sliced_gemm_kernel<BN, SPLIT>, dim3(blocks), dim3(THREADS),
                          smem_bytes(BN, SPLIT), s, SPLIT, jobs_dev, tiles_dev, n_tiles,
                          (a_ready ? FLAG_A_READY : 0) | (2 * blocks <= sms ? FLAG_TRIGGER : 0),
                          err_dev, c, ldc);

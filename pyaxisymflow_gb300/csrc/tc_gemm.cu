@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   const uint32_t accf0 = smem_u32(bars + 2 * NSTAGE), acce0 = smem_u32(bars + 2 * NSTAGE + 2);
   const uint32_t quiet = smem_u32(bars + 2 * NSTAGE + 4);
 
+  axi::pdl_trigger();
   if (threadIdx.x == 0) {
     for (int s = 0; s < NSTAGE; ++s) {
       mbar_init(full0 + 8 * s, 1);
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   if (warp == 0) {
     if (lane == 0) {
       // ---- TMA producer: one continuous ring over all tiles of this CTA ----
+      axi::pdl_wait();
       int g = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
@@ -235,6 +237,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;
     constexpr int CHUNKS = BN / 32 / 2;  // 32-column chunks per warp
+    axi::pdl_wait();
     float* stg = stage_out + (warp - 2) * 32 * 33;
     int it = 0;
     for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++it) {
@@ -415,7 +418,7 @@ void order_tiles_by_k(int4* tiles, int n, const TcJob* jobs, bool sort) {
 }
 
 int launch(const TcJob* jobs_dev, const int4* tiles_dev, int n_tiles, int* err_dev,
-           cudaStream_t s, int ctas_percent) {
+           cudaStream_t s, int ctas_percent, bool pdl) {
   static std::once_flag once;
   static cudaError_t attr_status = cudaSuccess;
   std::call_once(once, [] {
@@ -430,8 +433,8 @@ int launch(const TcJob* jobs_dev, const int4* tiles_dev, int n_tiles, int* err_d
   int ctas = axi::sm_count();
   if (ctas_percent > 0 && ctas_percent < 100) ctas = ctas * ctas_percent / 100 > 0 ? ctas * ctas_percent / 100 : 1;
   const int grid = n_tiles < ctas ? n_tiles : ctas;
-  tf32x3_gemm_kernel<<<grid, THREADS, SMEM_BYTES, s>>>(jobs_dev, tiles_dev, n_tiles, err_dev);
-  return axi::launch_status("tf32x3_gemm");
+  return axi::launch_chain(pdl, "tf32x3_gemm", tf32x3_gemm_kernel, dim3(grid), dim3(THREADS),
+                           SMEM_BYTES, s, 1, jobs_dev, tiles_dev, n_tiles, err_dev);
 }
 
 }  // namespace axi_tc

@@ -113,7 +113,8 @@ void order_tiles_by_k(int4* tiles, int n, const TcJob* jobs, bool sort = true);
 
 // Host: launch the grouped kernel over `n_tiles` (job, m0, n0, k-blocks) tiles
 // with `ctas_percent` of the SMs as persistent CTAs (0: all of them).
+// `pdl`: as a programmatic dependent launch.
 int launch(const TcJob* jobs_dev, const int4* tiles_dev, int n_tiles, int* err_dev,
-           cudaStream_t s, int ctas_percent = 0);
+           cudaStream_t s, int ctas_percent = 0, bool pdl = false);
 
 }  // namespace axi_tc
