@@ -9,7 +9,7 @@
 // a run of steps can be captured in a CUDA graph.
 //
 // Launches per step, each covering every case of the plan:
-//   kill_reset   one block per case: sine tapers, free stream of this step,
+//   kill_reset   four blocks per case: sine tapers, free stream of this step,
 //                counters cleared, float copies of the step scalars
 //   transform    the spectral Poisson solve (float: two DCTs and two tensor-core
 //                products, or four products; double: four sliced products)
@@ -167,27 +167,43 @@ __global__ void __launch_bounds__(256) kill_reset_kernel(const axi_case* __restr
   const double* cz0 = k.kill_coef;
   const double* cz1 = k.kill_coef + wd;
   const double* cr = k.kill_coef + 2 * wd;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    *reinterpret_cast<unsigned long long*>(&k.state[AXI_ST_UMAX]) = 0ull;
-    counter(k, 0)[0] = 0u;
-    counter(k, 1)[0] = 0u;
-    const double t = k.state[AXI_ST_T];
-    double prefac = 1.0;
-    if (k.t_ramp > 0.0 && t < k.t_ramp) prefac = sin(0.5 * kPi * t / k.t_ramp);
-    k.state[AXI_ST_UFREE] = k.U0 * prefac;
+  // the case's scalars, one to a lane of the last block's last warp: their
+  // divisions and conversions (64 cycles of a scheduler each, whatever the
+  // active lanes) issue once for all of them
+  const int lane = threadIdx.x - 224;
+  if (blockIdx.x == KILL_BLOCKS - 1 && lane >= 0 && lane < 8) {
+    if (lane == 7) {
+      *reinterpret_cast<unsigned long long*>(&k.state[AXI_ST_UMAX]) = 0ull;
+      counter(k, 0)[0] = 0u;
+      counter(k, 1)[0] = 0u;
+    }
+    double v = 0.0, d = 1.0;
+    int hi = -1, lo = -1;
+    switch (lane) {
+      case 0: v = k.state[AXI_ST_ZCM]; d = k.dx; hi = SF_S_HI; lo = SF_S_LO; break;
+      case 1: v = k.r_body; d = k.dx; hi = SF_R_HI; lo = SF_R_LO; break;
+      case 2: v = k.blend_w; d = k.dx; hi = SF_W; break;
+      case 3: v = k.inv_2dx; hi = SF_INV2DX; break;
+      case 4: v = k.inv_dx2; hi = SF_INVDX2; break;
+      case 5:  // the body velocity as a float pair
+        v = (k.flags & AXI_CASE_SEDIMENTING) ? k.state[AXI_ST_UBODY] : k.U_body;
+        hi = SF_UBODY; lo = SF_UBODY_LO;
+        break;
+      case 6: {
+        const double t = k.state[AXI_ST_T];
+        v = k.U0;
+        if (k.t_ramp > 0.0 && t < k.t_ramp) v = k.U0 * sin(0.5 * kPi * t / k.t_ramp);
+        k.state[AXI_ST_UFREE] = v;
+        hi = SF_UFREE;
+        break;
+      }
+    }
+    v = v / d;
+    const float h = (float)v;
+    const float l = (float)(v - (double)h);
     float* f = fslots(k);
-    f[SF_UFREE] = (float)(k.U0 * prefac);
-    const double ub = (k.flags & AXI_CASE_SEDIMENTING) ? k.state[AXI_ST_UBODY] : k.U_body;
-    f[SF_UBODY] = (float)ub;
-    f[SF_UBODY_LO] = (float)(ub - (double)(float)ub);  // the body velocity as a float pair
-    f[SF_INV2DX] = (float)k.inv_2dx;
-    f[SF_INVDX2] = (float)k.inv_dx2;
-    const double sc = k.state[AXI_ST_ZCM] / k.dx, rc = k.r_body / k.dx;
-    f[SF_S_HI] = (float)sc;
-    f[SF_S_LO] = (float)(sc - (double)(float)sc);
-    f[SF_R_HI] = (float)rc;
-    f[SF_R_LO] = (float)(rc - (double)(float)rc);
-    f[SF_W] = (float)(k.blend_w / k.dx);
+    if (hi >= 0) f[hi] = h;
+    if (lo >= 0) f[lo] = l;
   }
   const int band = (nr - wd) * nz;  // first outer row
   // output pointers in registers (a store through a pointer read from the
