@@ -382,8 +382,8 @@ typedef struct axi_tc_transform {
 
 typedef struct axi_tc_plan_info {
   int32_t n;             /* transforms in the plan */
-  int32_t n_tiles[4];    /* 128 x 128 output tiles per product stage */
-  int32_t reserved;
+  int32_t n_tiles[4];    /* output tiles per product stage */
+  uint8_t tile_cols[4];  /* their columns (internal) */
   int64_t bytes;         /* device bytes of the plan */
 } axi_tc_plan_info;
 
@@ -583,7 +583,7 @@ typedef struct axi_plan_info {
   int32_t n_dct_items;     /* row groups of the z transforms (AXI_PLAN_DCT_Z) */
   axi_tuning tune;         /* launch choices (zero: defaults) */
   int32_t n_slice_items[4]; /* AXI_PLAN_SLICED: work items of each slicing */
-  int32_t sliced_form[4];   /* AXI_PLAN_SLICED: tile form of each product (internal) */
+  int32_t tile_form[4];    /* tile form of each stage's products (internal) */
   int32_t slice_groups[4];  /* AXI_PLAN_SLICED: row groups before sharing of K (internal) */
 } axi_plan_info;
 

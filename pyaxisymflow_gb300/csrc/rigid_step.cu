@@ -1749,25 +1749,26 @@ inline PlanView plan_view(const void* plan_dev, const axi_plan_info* info) {
 // kernels/FastDiagonalisationStokesSolver.py:137-156.
 // With `dct`, stages 0 and 2 run as z transforms (build_dct_jobs) and stage 1
 // writes its scaled result plain for the inverse transform.
-int build_tc_jobs(const axi_case& k, axi_tc::TcJob job[4], bool dct, bool refine) {
+int build_tc_jobs(const axi_case& k, axi_tc::TcJob job[4], bool dct, bool refine,
+                  const int32_t bn[4]) {
   const int nr = k.nr, nz = k.nz;
   const float* const* b = reinterpret_cast<const float* const*>(k.tc_basis);
   float* const* w = reinterpret_cast<float* const*>(k.tc_work);
   memset(job, 0, 4 * sizeof(axi_tc::TcJob));
   if (dct) {
-    AXI_TRY(axi_tc::encode_operand(&job[1].a_hi, b[2], nr, nr, nr));
-    AXI_TRY(axi_tc::encode_operand(&job[1].a_lo, b[3], nr, nr, nr));
-    AXI_TRY(axi_tc::encode_operand(&job[1].b_hi, w[0], nz, nr, nr));
-    AXI_TRY(axi_tc::encode_operand(&job[1].b_lo, w[1], nz, nr, nr));
+    AXI_TRY(axi_tc::encode_operand(&job[1].a_hi, b[2], nr, nr, nr, axi_tc::BM));
+    AXI_TRY(axi_tc::encode_operand(&job[1].a_lo, b[3], nr, nr, nr, axi_tc::BM));
+    AXI_TRY(axi_tc::encode_operand(&job[1].b_hi, w[0], nz, nr, nr, bn[1]));
+    AXI_TRY(axi_tc::encode_operand(&job[1].b_lo, w[1], nz, nr, nr, bn[1]));
     // the inverse spectrum is applied by the inverse transform as it reads
     // the rows (the same float product), keeping this epilogue a plain store
     job[1].c = w[2];
     job[1].M = nr; job[1].N = nz; job[1].K = nr; job[1].ldc = nz;
     job[1].mode = axi_tc::MODE_PLAIN;
-    AXI_TRY(axi_tc::encode_operand(&job[3].a_hi, b[6], nr, nr, nr));
-    AXI_TRY(axi_tc::encode_operand(&job[3].a_lo, b[7], nr, nr, nr));
-    AXI_TRY(axi_tc::encode_operand(&job[3].b_hi, w[0], nz, nr, nr));
-    AXI_TRY(axi_tc::encode_operand(&job[3].b_lo, w[1], nz, nr, nr));
+    AXI_TRY(axi_tc::encode_operand(&job[3].a_hi, b[6], nr, nr, nr, axi_tc::BM));
+    AXI_TRY(axi_tc::encode_operand(&job[3].a_lo, b[7], nr, nr, nr, axi_tc::BM));
+    AXI_TRY(axi_tc::encode_operand(&job[3].b_hi, w[0], nz, nr, nr, bn[3]));
+    AXI_TRY(axi_tc::encode_operand(&job[3].b_lo, w[1], nz, nr, nr, bn[3]));
     job[3].c = static_cast<float*>(k.psi); job[3].M = nr; job[3].N = nz;
     job[3].K = nr; job[3].ldc = nz; job[3].mode = axi_tc::MODE_PLAIN;
     if (refine) {
@@ -1785,32 +1786,32 @@ int build_tc_jobs(const axi_case& k, axi_tc::TcJob job[4], bool dct, bool refine
     return AXI_OK;
   }
   // stage 0
-  AXI_TRY(axi_tc::encode_operand(&job[0].a_hi, b[0], nz, nz, nz));
-  AXI_TRY(axi_tc::encode_operand(&job[0].a_lo, b[1], nz, nz, nz));
-  AXI_TRY(axi_tc::encode_operand(&job[0].b_hi, static_cast<const float*>(k.omega_hi), nr, nz, nz));
-  AXI_TRY(axi_tc::encode_operand(&job[0].b_lo, static_cast<const float*>(k.omega_lo), nr, nz, nz));
+  AXI_TRY(axi_tc::encode_operand(&job[0].a_hi, b[0], nz, nz, nz, axi_tc::BM));
+  AXI_TRY(axi_tc::encode_operand(&job[0].a_lo, b[1], nz, nz, nz, axi_tc::BM));
+  AXI_TRY(axi_tc::encode_operand(&job[0].b_hi, static_cast<const float*>(k.omega_hi), nr, nz, nz, bn[0]));
+  AXI_TRY(axi_tc::encode_operand(&job[0].b_lo, static_cast<const float*>(k.omega_lo), nr, nz, nz, bn[0]));
   job[0].c = w[0]; job[0].c_lo = w[1]; job[0].M = nz; job[0].N = nr; job[0].K = nz;
   job[0].ldc = nr; job[0].mode = axi_tc::MODE_SPLIT;
   // stage 1
-  AXI_TRY(axi_tc::encode_operand(&job[1].a_hi, b[2], nr, nr, nr));
-  AXI_TRY(axi_tc::encode_operand(&job[1].a_lo, b[3], nr, nr, nr));
-  AXI_TRY(axi_tc::encode_operand(&job[1].b_hi, w[0], nz, nr, nr));
-  AXI_TRY(axi_tc::encode_operand(&job[1].b_lo, w[1], nz, nr, nr));
+  AXI_TRY(axi_tc::encode_operand(&job[1].a_hi, b[2], nr, nr, nr, axi_tc::BM));
+  AXI_TRY(axi_tc::encode_operand(&job[1].a_lo, b[3], nr, nr, nr, axi_tc::BM));
+  AXI_TRY(axi_tc::encode_operand(&job[1].b_hi, w[0], nz, nr, nr, bn[1]));
+  AXI_TRY(axi_tc::encode_operand(&job[1].b_lo, w[1], nz, nr, nr, bn[1]));
   job[1].c = w[2]; job[1].c_lo = w[3]; job[1].scale = static_cast<const float*>(k.inv_eig);
   job[1].M = nr; job[1].N = nz; job[1].K = nr; job[1].ldc = nz;
   job[1].mode = axi_tc::MODE_SCALE_SPLIT;
   // stage 2
-  AXI_TRY(axi_tc::encode_operand(&job[2].a_hi, b[4], nz, nz, nz));
-  AXI_TRY(axi_tc::encode_operand(&job[2].a_lo, b[5], nz, nz, nz));
-  AXI_TRY(axi_tc::encode_operand(&job[2].b_hi, w[2], nr, nz, nz));
-  AXI_TRY(axi_tc::encode_operand(&job[2].b_lo, w[3], nr, nz, nz));
+  AXI_TRY(axi_tc::encode_operand(&job[2].a_hi, b[4], nz, nz, nz, axi_tc::BM));
+  AXI_TRY(axi_tc::encode_operand(&job[2].a_lo, b[5], nz, nz, nz, axi_tc::BM));
+  AXI_TRY(axi_tc::encode_operand(&job[2].b_hi, w[2], nr, nz, nz, bn[2]));
+  AXI_TRY(axi_tc::encode_operand(&job[2].b_lo, w[3], nr, nz, nz, bn[2]));
   job[2].c = w[0]; job[2].c_lo = w[1]; job[2].M = nz; job[2].N = nr; job[2].K = nz;
   job[2].ldc = nr; job[2].mode = axi_tc::MODE_SPLIT;
   // stage 3
-  AXI_TRY(axi_tc::encode_operand(&job[3].a_hi, b[6], nr, nr, nr));
-  AXI_TRY(axi_tc::encode_operand(&job[3].a_lo, b[7], nr, nr, nr));
-  AXI_TRY(axi_tc::encode_operand(&job[3].b_hi, w[0], nz, nr, nr));
-  AXI_TRY(axi_tc::encode_operand(&job[3].b_lo, w[1], nz, nr, nr));
+  AXI_TRY(axi_tc::encode_operand(&job[3].a_hi, b[6], nr, nr, nr, axi_tc::BM));
+  AXI_TRY(axi_tc::encode_operand(&job[3].a_lo, b[7], nr, nr, nr, axi_tc::BM));
+  AXI_TRY(axi_tc::encode_operand(&job[3].b_hi, w[0], nz, nr, nr, bn[3]));
+  AXI_TRY(axi_tc::encode_operand(&job[3].b_lo, w[1], nz, nr, nr, bn[3]));
   job[3].c = static_cast<float*>(k.psi); job[3].c_lo = nullptr; job[3].M = nr; job[3].N = nz;
   job[3].K = nr; job[3].ldc = nz; job[3].mode = axi_tc::MODE_PLAIN;
   if (!axi_tc::encode_output(&job[3])) {
@@ -1899,10 +1900,10 @@ inline int dct64_items_of(const axi_case& k) {
   return (k.nr + r - 1) / r;
 }
 
-inline int tc_tiles_of(const axi_case& k, int stage) {
+inline int tc_tiles_of(const axi_case& k, int stage, int cols) {
   const int M = (stage % 2 == 0) ? k.nz : k.nr;
   const int N = (stage % 2 == 0) ? k.nr : k.nz;
-  return ((M + axi_tc::BM - 1) / axi_tc::BM) * ((N + axi_tc::BN - 1) / axi_tc::BN);
+  return axi_tc::tile_count(M, N, cols);
 }
 
 enum { PH_KILL = 0, PH_TRANSFORM = 1, PH_VEL_MAX = 2, PH_PENALISE = 3, PH_ADVECT_DIFFUSE = 4,
@@ -2011,7 +2012,7 @@ inline bool chained(const axi_plan_info* info) {
 int run_sliced(const axi_plan_info* info, const PlanView& v, int st, cudaStream_t s) {
   AXI_TRY(axi_sl::launch_slice(v.slice_jobs, v.slice_items[st], info->n_slice_items[st], s));
   return axi_sl::launch_gemm(v.sliced_jobs, v.tc_tiles[st], info->n_tc_tiles[st],
-                             info->sliced_form[st], true, v.err, s);
+                             info->tile_form[st], true, v.err, s);
 }
 
 template <typename T>
@@ -2028,11 +2029,13 @@ int run_phase(int phase, const axi_plan_info* info, const PlanView& v, cudaStrea
         // z transform, radial product, inverse z transform, radial product
         AXI_TRY(axi_dct::launch(v.dct_jobs, v.dct_items, info->n_dct_items, true, s,
                                 info->tune.prefetch_waves, pdl));
-        AXI_TRY(axi_tc::launch(v.jobs, v.tc_tiles[1], info->n_tc_tiles[1], v.err, s,
+        AXI_TRY(axi_tc::launch(v.jobs, v.tc_tiles[1], info->n_tc_tiles[1],
+                               info->tile_form[1], v.err, s,
                                info->tune.tc_ctas_percent, pdl));
         AXI_TRY(axi_dct::launch(v.dct_jobs + info->n_cases, v.dct_items, info->n_dct_items,
                                 false, s, info->tune.prefetch_waves, pdl));
-        AXI_TRY(axi_tc::launch(v.jobs, v.tc_tiles[3], info->n_tc_tiles[3], v.err, s,
+        AXI_TRY(axi_tc::launch(v.jobs, v.tc_tiles[3], info->n_tc_tiles[3],
+                               info->tile_form[3], v.err, s,
                                info->tune.tc_ctas_percent, pdl));
         break;
       }
@@ -2042,7 +2045,8 @@ int run_phase(int phase, const axi_plan_info* info, const PlanView& v, cudaStrea
       }
       if (v.jobs) {
         for (int st = 0; st < 4; ++st)
-          AXI_TRY(axi_tc::launch(v.jobs, v.tc_tiles[st], info->n_tc_tiles[st], v.err, s,
+          AXI_TRY(axi_tc::launch(v.jobs, v.tc_tiles[st], info->n_tc_tiles[st],
+                               info->tile_form[st], v.err, s,
                                  info->tune.tc_ctas_percent, pdl));
         break;
       }
@@ -2102,7 +2106,8 @@ int run_phase(int phase, const axi_plan_info* info, const PlanView& v, cudaStrea
         AXI_TRY(axi_dct64::launch(st == 0 ? v.dct64_jobs : v.dct64_jobs + info->n_cases,
                                   v.dct_items, info->n_dct_items, st == 0, s));
       } else if (v.jobs) {
-        AXI_TRY(axi_tc::launch(v.jobs, v.tc_tiles[st], info->n_tc_tiles[st], v.err, s,
+        AXI_TRY(axi_tc::launch(v.jobs, v.tc_tiles[st], info->n_tc_tiles[st],
+                               info->tile_form[st], v.err, s,
                                  info->tune.tc_ctas_percent));
       } else if (st == 0) {
         grouped_gemm_kernel<T, 0><<<ng, gemm_threads<T>(), 0, s>>>(v.cases, v.gemm);
@@ -2254,8 +2259,6 @@ extern "C" int axi_plan_init(axi_case* cases, int n_cases, int elem_bytes, int f
                        c, k.nz);
         return AXI_ERR_INVALID;
       }
-      for (int st = 0; st < 4; ++st)
-        if (!(dct && (st == 0 || st == 2))) info->n_tc_tiles[st] += tc_tiles_of(k, st);
       if (dct) nd += dct_items_of(k);
     } else if (dct) {
       // double engine: DCT z transforms around the SIMT radial products
@@ -2278,10 +2281,19 @@ extern "C" int axi_plan_init(axi_case* cases, int n_cases, int elem_bytes, int f
       }
     }
   }
+  for (int st = 0; tc && st < 4; ++st) {
+    // one tile width per launch, from the tiles of all cases
+    if (dct && (st == 0 || st == 2)) continue;
+    int tiles64 = 0;
+    for (int c = 0; c < n_cases; ++c) tiles64 += tc_tiles_of(cases[c], st, 64);
+    const int cols = axi_tc::choose_cols(tiles64, axi::sm_count());
+    info->tile_form[st] = cols;
+    for (int c = 0; c < n_cases; ++c) info->n_tc_tiles[st] += tc_tiles_of(cases[c], st, cols);
+  }
   for (int st = 0; sliced && st < 4; ++st) {
     // one form per launch, from the tiles of all cases
     const int form = axi_sl::choose_form(info->n_tc_tiles[st], axi::sm_count());
-    info->sliced_form[st] = form;
+    info->tile_form[st] = form;
     info->n_tc_tiles[st] = info->n_slice_items[st] = 0;
     int groups = 0;
     for (int c = 0; c < n_cases; ++c) {
@@ -2362,7 +2374,8 @@ extern "C" int axi_plan_upload(const axi_case* cases, const axi_plan_info* info,
     axi_tc::TcJob* jobs = reinterpret_cast<axi_tc::TcJob*>(&buf[o.jobs]);
     const bool dct = (info->flags & AXI_PLAN_DCT_Z) != 0;
     const bool refine = (info->flags & AXI_PLAN_REFINE) != 0;
-    for (int c = 0; c < n; ++c) AXI_TRY(build_tc_jobs(cases[c], jobs + 4 * c, dct, refine));
+    for (int c = 0; c < n; ++c) AXI_TRY(build_tc_jobs(cases[c], jobs + 4 * c, dct, refine,
+                                                  info->tile_form));
     if (dct) {
       axi_dct::DctJob* dj = reinterpret_cast<axi_dct::DctJob*>(&buf[o.dct_jobs]);
       int4* di = reinterpret_cast<int4*>(&buf[o.dct_items]);
@@ -2403,7 +2416,7 @@ extern "C" int axi_plan_upload(const axi_case* cases, const axi_plan_info* info,
         const int M = (st % 2 == 0) ? k.nz : k.nr;
         const int N = (st % 2 == 0) ? k.nr : k.nz;
         for (int m0 = 0; m0 < M; m0 += axi_tc::BM)
-          for (int n0 = 0; n0 < N; n0 += axi_tc::BN) tt[qq++] = make_int4(4 * c + st, m0, n0, 0);
+          for (int n0 = 0; n0 < N; n0 += info->tile_form[st]) tt[qq++] = make_int4(4 * c + st, m0, n0, 0);
       }
       if (qq != info->n_tc_tiles[st]) {
         axi::set_error("plan_upload: cases changed since plan_init");
@@ -2435,16 +2448,16 @@ extern "C" int axi_plan_upload(const axi_case* cases, const axi_plan_info* info,
     std::vector<int4> items[4], tiles[4];
     for (int c = 0; c < n; ++c) {
       const axi_case& k = cases[c];
-      axi_sl::spectral_jobs(k.nr, k.nz, info->sliced_form, static_cast<const double*>(k.omega), k.nz,
+      axi_sl::spectral_jobs(k.nr, k.nz, info->tile_form, static_cast<const double*>(k.omega), k.nz,
                             static_cast<double*>(k.psi), k.nz, static_cast<double*>(k.gemm_work),
                             k.sliced_field, k.sliced_basis,
                             static_cast<const double*>(k.inv_eig), sj + 4 * c, gj + 4 * c);
       for (int st = 0; st < 4; ++st) {
         const int M = st % 2 == 0 ? k.nz : k.nr, N = st % 2 == 0 ? k.nr : k.nz;
         axi_sl::append_slice_items(
-            items[st], 4 * c + st, N, axi_sl::form_cols(info->sliced_form[st]),
+            items[st], 4 * c + st, N, axi_sl::form_cols(info->tile_form[st]),
             axi_sl::slice_parts(info->slice_groups[st], M, axi::sm_count()));
-        axi_sl::append_gemm_tiles(tiles[st], 4 * c + st, M, N, M, info->sliced_form[st]);
+        axi_sl::append_gemm_tiles(tiles[st], 4 * c + st, M, N, M, info->tile_form[st]);
       }
     }
     for (int st = 0; st < 4; ++st) {

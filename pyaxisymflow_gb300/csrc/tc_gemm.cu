@@ -69,7 +69,7 @@ __device__ __forceinline__ uint64_t sw_desc(uint32_t saddr) {
   return d;
 }
 
-// Instruction descriptor: D = F32, A = B = TF32, both K-major, M = 128, N = 128.
+// Instruction descriptor: D = F32, A = B = TF32, both K-major, M x N.
 __host__ __device__ constexpr uint32_t idesc_tf32(int m, int n) {
   return (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
          (static_cast<uint32_t>(m >> 4) << 24);
@@ -108,11 +108,13 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 
 // Persistent, warp-specialised kernel (one CTA per SM, tiles strided over the
 // grid): warp 0 issues TMA, warp 1 issues MMAs into one of two TMEM
-// accumulators (2 x 128 columns), warps 2-9 drain the other accumulator, so
+// accumulators (2 x BN columns), warps 2-9 drain the other accumulator, so
 // the epilogue of a tile overlaps the main loop of the next one.
+template <int BN>
 __global__ void __launch_bounds__(THREADS, 1)
     tf32x3_gemm_kernel(const TcJob* __restrict__ jobs, const int4* __restrict__ tiles,
                        int n_tiles, int* __restrict__ err) {
+  constexpr int NSTAGE = stages(BN), STAGE_BYTES = stage_bytes(BN), B_BYTES = b_bytes(BN);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -180,10 +182,10 @@ __global__ void __launch_bounds__(THREADS, 1)
           const uint32_t fb = full0 + 8 * s;
           mbar_expect_tx(fb, STAGE_BYTES);
           const int kx = kb * BKF;
-          tma_load_2d(st + 0 * TILE_BYTES, &job.a_hi, kx, tr.y, fb);
-          tma_load_2d(st + 1 * TILE_BYTES, &job.a_lo, kx, tr.y, fb);
-          tma_load_2d(st + 2 * TILE_BYTES, &job.b_hi, kx, tr.z, fb);
-          tma_load_2d(st + 3 * TILE_BYTES, &job.b_lo, kx, tr.z, fb);
+          tma_load_2d(st, &job.a_hi, kx, tr.y, fb);
+          tma_load_2d(st + A_BYTES, &job.a_lo, kx, tr.y, fb);
+          tma_load_2d(st + 2 * A_BYTES, &job.b_hi, kx, tr.z, fb);
+          tma_load_2d(st + 2 * A_BYTES + B_BYTES, &job.b_lo, kx, tr.z, fb);
         }
       }
       progress[0] = g;
@@ -213,8 +215,9 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
           tc_fence_after();
           const uint32_t st = smem_u32(smem + s * STAGE_BYTES);
-          const uint64_t ah = sw_desc(st), al = sw_desc(st + TILE_BYTES);
-          const uint64_t bh = sw_desc(st + 2 * TILE_BYTES), bl = sw_desc(st + 3 * TILE_BYTES);
+          const uint64_t ah = sw_desc(st), al = sw_desc(st + A_BYTES);
+          const uint64_t bh = sw_desc(st + 2 * A_BYTES);
+          const uint64_t bl = sw_desc(st + 2 * A_BYTES + B_BYTES);
 #pragma unroll
           for (int kk = 0; kk < BKF / 8; ++kk) {
             const uint64_t o = static_cast<uint64_t>(kk * 32) >> 4;  // 8 TF32 = 32 bytes
@@ -254,21 +257,27 @@ __global__ void __launch_bounds__(THREADS, 1)
       const bool tma_out = job.c_tma != 0;
       const CUtensorMap* const cmap = &job.c_map;
       const int buf = it & 1;
-      const bool ok = mbar_wait(accf0 + 8 * buf, (it >> 1) & 1, err, ERR_EPILOGUE);
-      // all lanes leave together; a failure elsewhere in the grid surfaces at
-      // the next wait (the error word is read there) and on the host
-      if (!__all_sync(0xffffffffu, ok)) break;
-      tc_fence_after();
       const int row0 = tr.y + 32 * q;
       const bool scaled = mode == MODE_SCALE_SPLIT || mode == MODE_SCALE;
       const bool split = mode == MODE_SPLIT || mode == MODE_SCALE_SPLIT;
       const bool pair = mode == MODE_PAIR_ADD;
+      // the accumulator; all lanes leave together, a failure elsewhere in the
+      // grid surfaces at the next wait (the error word is read there) and on
+      // the host
+      auto acc_ready = [&]() {
+        const bool ok = mbar_wait(accf0 + 8 * buf, (it >> 1) & 1, err, ERR_EPILOGUE);
+        if (!__all_sync(0xffffffffu, ok)) return false;
+        tc_fence_after();
+        return true;
+      };
+      bool ok = true;
 #pragma unroll 1
       for (int cc = half * CHUNKS; cc < (half + 1) * CHUNKS; ++cc) {
         const int col = tr.z + cc * 32 + lane;
         // the elementwise factors of this 32 x 32 block are fetched before the
-        // accumulator is read, all 32 loads in flight at once (one load per
-        // row in the store loop left the epilogue waiting on L2 latency)
+        // accumulator is waited for and read, all 32 loads in flight at once
+        // (one load per row in the store loop left the epilogue waiting on L2
+        // latency)
         float sv[32];
         if (scaled) {
 #pragma unroll
@@ -288,6 +297,10 @@ __global__ void __launch_bounds__(THREADS, 1)
             ph[rr] = in ? c[idx] : 0.0f;
             pl[rr] = in ? c_lo[idx] : 0.0f;
           }
+        }
+        if (cc == half * CHUNKS && !acc_ready()) {
+          ok = false;
+          break;
         }
         uint32_t r[32];
         tmem_ld32(tmem + buf * BN + (static_cast<uint32_t>(32 * q) << 16) + cc * 32, r);
@@ -339,6 +352,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
         __syncwarp();
       }
+      if (!ok) break;
       tc_fence_before();
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acce0 + 8 * buf)
@@ -368,7 +382,8 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 }  // namespace
 
-int encode_operand(CUtensorMap* map, const float* base, int rows, int K, int ld) {
+int encode_operand(CUtensorMap* map, const float* base, int rows, int K, int ld,
+                   int box_rows) {
   auto fn = encode_fn();
   if (!fn) {
     axi::set_error("tensor core GEMM: cuTensorMapEncodeTiled unavailable");
@@ -380,7 +395,7 @@ int encode_operand(CUtensorMap* map, const float* base, int rows, int K, int ld)
   }
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 4};
-  const cuuint32_t box[2] = {BKF, BM};
+  const cuuint32_t box[2] = {BKF, static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides,
                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -417,24 +432,39 @@ void order_tiles_by_k(int4* tiles, int n, const TcJob* jobs, bool sort) {
                    [jobs](const int4& a, const int4& b) { return jobs[a.x].K > jobs[b.x].K; });
 }
 
-int launch(const TcJob* jobs_dev, const int4* tiles_dev, int n_tiles, int* err_dev,
-           cudaStream_t s, int ctas_percent, bool pdl) {
+namespace {
+
+template <int BN>
+int launch_cols(const TcJob* jobs_dev, const int4* tiles_dev, int n_tiles, int* err_dev,
+                cudaStream_t s, int ctas, bool pdl) {
   static std::once_flag once;
   static cudaError_t attr_status = cudaSuccess;
   std::call_once(once, [] {
-    attr_status = cudaFuncSetAttribute(tf32x3_gemm_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    attr_status = cudaFuncSetAttribute(tf32x3_gemm_kernel<BN>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(BN));
   });
   if (attr_status != cudaSuccess) {
-    axi::set_error("tensor core GEMM: cannot reserve %d bytes of shared memory", SMEM_BYTES);
+    axi::set_error("tensor core GEMM: cannot reserve %d bytes of shared memory", smem_bytes(BN));
     return AXI_ERR_CUDA;
   }
+  return axi::launch_chain(pdl, "tf32x3_gemm", tf32x3_gemm_kernel<BN>,
+                           dim3(n_tiles < ctas ? n_tiles : ctas), dim3(THREADS), smem_bytes(BN), s,
+                           1, jobs_dev, tiles_dev, n_tiles, err_dev);
+}
+
+}  // namespace
+
+int launch(const TcJob* jobs_dev, const int4* tiles_dev, int n_tiles, int cols, int* err_dev,
+           cudaStream_t s, int ctas_percent, bool pdl) {
   if (n_tiles <= 0) return AXI_OK;
   int ctas = axi::sm_count();
   if (ctas_percent > 0 && ctas_percent < 100) ctas = ctas * ctas_percent / 100 > 0 ? ctas * ctas_percent / 100 : 1;
-  const int grid = n_tiles < ctas ? n_tiles : ctas;
-  return axi::launch_chain(pdl, "tf32x3_gemm", tf32x3_gemm_kernel, dim3(grid), dim3(THREADS),
-                           SMEM_BYTES, s, 1, jobs_dev, tiles_dev, n_tiles, err_dev);
+  switch (cols) {
+    case 64: return launch_cols<64>(jobs_dev, tiles_dev, n_tiles, err_dev, s, ctas, pdl);
+    case 128: return launch_cols<128>(jobs_dev, tiles_dev, n_tiles, err_dev, s, ctas, pdl);
+  }
+  axi::set_error("tensor core GEMM: no tiles of %d columns", cols);
+  return AXI_ERR_INVALID;
 }
 
 }  // namespace axi_tc
@@ -512,7 +542,7 @@ TestLayout test_layout(int M, int N, int K) {
   L.b_hi = o; o = align_up(o + (size_t)N * K * 4, 256);
   L.b_lo = o; o = align_up(o + (size_t)N * K * 4, 256);
   L.job = o; o = align_up(o + sizeof(axi_tc::TcJob), 256);
-  const size_t nt = (size_t)((M + axi_tc::BM - 1) / axi_tc::BM) * ((N + axi_tc::BN - 1) / axi_tc::BN);
+  const size_t nt = axi_tc::tile_count(M, N, 64);
   L.tiles = o; o = align_up(o + nt * sizeof(int4), 256);
   L.err = o; o = align_up(o + 16, 256);
   L.total = o;
@@ -544,12 +574,13 @@ extern "C" int axi_tf32x3_gemm(float* C, const float* A, const float* B, int M, 
   split_kernel<<<axi::ceil_div((long long)M * K, 256), 256, 0, s>>>(A, ahi, alo, (long long)M * K);
   split_kernel<<<axi::ceil_div((long long)N * K, 256), 256, 0, s>>>(B, bhi, blo, (long long)N * K);
   AXI_TRY(axi::launch_status(what));
+  const int bn = axi_tc::choose_cols(axi_tc::tile_count(M, N, 64), axi::sm_count());
   axi_tc::TcJob job;
   memset(&job, 0, sizeof(job));
-  AXI_TRY(axi_tc::encode_operand(&job.a_hi, ahi, M, K, K));
-  AXI_TRY(axi_tc::encode_operand(&job.a_lo, alo, M, K, K));
-  AXI_TRY(axi_tc::encode_operand(&job.b_hi, bhi, N, K, K));
-  AXI_TRY(axi_tc::encode_operand(&job.b_lo, blo, N, K, K));
+  AXI_TRY(axi_tc::encode_operand(&job.a_hi, ahi, M, K, K, axi_tc::BM));
+  AXI_TRY(axi_tc::encode_operand(&job.a_lo, alo, M, K, K, axi_tc::BM));
+  AXI_TRY(axi_tc::encode_operand(&job.b_hi, bhi, N, K, K, bn));
+  AXI_TRY(axi_tc::encode_operand(&job.b_lo, blo, N, K, K, bn));
   job.c = C;
   job.c_lo = nullptr;
   job.scale = nullptr;
@@ -561,7 +592,7 @@ extern "C" int axi_tf32x3_gemm(float* C, const float* A, const float* B, int M, 
   axi_tc::encode_output(&job);  // TMA stores where the output allows them
   std::string tiles;
   for (int m0 = 0; m0 < M; m0 += axi_tc::BM)
-    for (int n0 = 0; n0 < N; n0 += axi_tc::BN) {
+    for (int n0 = 0; n0 < N; n0 += bn) {
       int4 t = make_int4(0, m0, n0, (K + axi_tc::BKF - 1) / axi_tc::BKF);
       tiles.append(reinterpret_cast<const char*>(&t), sizeof(t));
     }
@@ -572,7 +603,7 @@ extern "C" int axi_tf32x3_gemm(float* C, const float* A, const float* B, int M, 
       cudaMemsetAsync(w + L.err, 0, 16, s) != cudaSuccess)
     return axi::launch_status(what);
   AXI_TRY(axi_tc::launch(reinterpret_cast<const axi_tc::TcJob*>(w + L.job),
-                         reinterpret_cast<const int4*>(w + L.tiles), n_tiles,
+                         reinterpret_cast<const int4*>(w + L.tiles), n_tiles, bn,
                          reinterpret_cast<int*>(w + L.err), s));
   int err = 0;
   if (cudaMemcpyAsync(&err, w + L.err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||

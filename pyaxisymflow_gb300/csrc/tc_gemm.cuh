@@ -7,17 +7,18 @@
 // hi*hi + hi*lo + lo*hi in FP32 in tensor memory, which restores close to
 // FP32 accuracy (the dropped lo*lo term is near FP32 rounding).
 //
-// Persistent CTAs (one per SM) walk a list of 128 x 128 output tiles:
-//   warp 0, one thread   TMA producer: cp.async.bulk.tensor tiles (128 rows x
-//                        32 floats, 128-byte swizzle) of A_hi, A_lo, B_hi, B_lo
-//                        into a 3-stage shared-memory ring (mbarrier complete_tx),
-//                        continuous across tiles
+// Persistent CTAs (one per SM) walk a list of 128 x BN output tiles (BN = 128
+// or 64):
+//   warp 0, one thread   TMA producer: cp.async.bulk.tensor tiles (128 or BN rows
+//                        x 32 floats, 128-byte swizzle) of A_hi, A_lo, B_hi, B_lo
+//                        into a 3- or 4-stage shared-memory ring (mbarrier
+//                        complete_tx), continuous across tiles
 //   warp 1, one thread   MMA issuer: 3 x 4 tcgen05.mma.kind::tf32 per stage into
-//                        one of two 128-lane x 128-column FP32 accumulators in
+//                        one of two 128-lane x BN-column FP32 accumulators in
 //                        TMEM; tcgen05.commit releases stages and accumulators
 //   warps 2-9            epilogue: tcgen05.ld (warp w reads TMEM lanes
-//                        32 (w % 4) .., warps 2-5 columns 0-63, warps 6-9
-//                        columns 64-127); plain outputs go out as one TMA store
+//                        32 (w % 4) .., warps 2-5 the first half of the columns,
+//                        warps 6-9 the second); plain outputs go out as one TMA store
 //                        per 32 x 32 block (128-byte swizzled shared-memory
 //                        box), the split and scaled forms through a per-warp
 //                        shared-memory transpose and row-contiguous stores; it
@@ -37,26 +38,42 @@
 namespace axi_tc {
 
 constexpr int BM = 128;
-constexpr int BN = 128;
-// 128 x 128 tiles, 32 K floats (128-byte rows, 128-byte swizzle) per stage,
-// 3 stages. Measured alternatives, both slower on the spectral products:
-// 16-float stages with a 6-deep ring (64-byte swizzle; twice the barrier and
-// copy count per FLOP: 8 tiles of K = 512 per CTA take 107 us against 92 us,
-// so the main loop pays a fixed cost per stage rather than waiting on the
-// ring) and 128 x 256 tiles with two 96 KB stages (the ring too shallow to
-// cover the operand loads).
+// Tiles of 128 x BN, 32 K floats (128-byte rows, 128-byte swizzle) per stage.
+// BN is 128 where a launch has tiles for every SM and 64 where it has not
+// (choose_cols): a narrow tile's stage takes less time, and its result,
+// summed in the same order, is the same. Measured alternatives to the stage,
+// both slower on the spectral products: 16-float stages with a 6-deep ring
+// (64-byte swizzle; twice the barrier and copy count per FLOP: 8 tiles of
+// K = 512 per CTA take 107 us against 92 us, so the main loop pays a fixed
+// cost per stage rather than waiting on the ring) and 128 x 256 tiles with two
+// 96 KB stages (the ring too shallow to cover the operand loads).
 constexpr int BKF = 32;                         // K floats per stage
 constexpr int ROW_BYTES = BKF * 4;              // swizzle span of a tile row
-constexpr int NSTAGE = 3;
-constexpr int TILE_BYTES = BM * BKF * 4;        // 16 KB per operand tile
-constexpr int STAGE_BYTES = 4 * TILE_BYTES;     // A_hi, A_lo, B_hi, B_lo
 constexpr int EPI_WARPS = 8;                    // two per TMEM lane quarter
 constexpr int THREADS = 32 * (2 + EPI_WARPS);   // TMA warp, MMA warp, 8 epilogue warps
 // epilogue staging: a 32 x 33-float transpose per warp, or (TMA stores) a
 // 32 x 32-float 128-byte-swizzled box per warp at 4 KB strides
 constexpr int EPI_STAGE_BYTES = EPI_WARPS * 32 * 33 * 4;
 static_assert(EPI_WARPS * 4096 <= EPI_STAGE_BYTES, "TMA store boxes fit the staging region");
-constexpr int SMEM_BYTES = NSTAGE * STAGE_BYTES + 1024 + EPI_STAGE_BYTES + 256;
+constexpr int A_BYTES = BM * ROW_BYTES;         // 16 KB per A operand tile
+constexpr int b_bytes(int bn) { return bn * ROW_BYTES; }
+constexpr int stage_bytes(int bn) { return 2 * (A_BYTES + b_bytes(bn)); }  // A_hi, A_lo, B_hi, B_lo
+constexpr int stages(int bn) { return bn == 64 ? 4 : 3; }
+constexpr int smem_bytes(int bn) {
+  return stages(bn) * stage_bytes(bn) + 1024 + EPI_STAGE_BYTES + 256;
+}
+static_assert(smem_bytes(128) <= 227 * 1024 && smem_bytes(64) <= 227 * 1024,
+              "shared memory of a block");
+
+inline int tile_count(int M, int N, int bn) { return ((M + BM - 1) / BM) * ((N + bn - 1) / bn); }
+// Tile columns of a launch, from its tile count at 64 columns: 64 where those
+// tiles run at once, 128 otherwise (twice the operand loads per product: 64
+// cases' radial products go from 77 / 119 to 125 / 148 us). 128 / 64 columns,
+// us per launch: K = 500, 500 x 252, 8 / 16 tiles: 20.5 / 15.0; K = 128,
+// 128 x 256 pair, 2 / 4 tiles: 11.7 / 8.4; five cases, 68 / 136 tiles: 18.0 /
+// 14.8. 32 columns leave half of the epilogue idle and load A once more per
+// tile: 18.5 and 11.0 us on the first two.
+inline int choose_cols(int tiles64, int sms) { return tiles64 <= sms ? 64 : 128; }
 
 // MODE_PAIR_ADD: the output is the float pair (c, c_lo) holding c + c_lo;
 // the product is added to it and the pair renormalised (c the rounded sum,
@@ -95,8 +112,9 @@ __device__ __forceinline__ void tf32_split(float x, float& hi, float& lo) {
 }
 
 // Host: encode a 2-D K-major FP32 operand (rows x K, row stride ld floats)
-// for 128-row x BKF-float boxes with the ROW_BYTES swizzle. Returns AXI status.
-int encode_operand(CUtensorMap* map, const float* base, int rows, int K, int ld);
+// for box_rows x BKF-float boxes (BM for A, the tile columns for B) with the
+// ROW_BYTES swizzle. Returns AXI status.
+int encode_operand(CUtensorMap* map, const float* base, int rows, int K, int ld, int box_rows);
 
 // Host: encode the output of a MODE_PLAIN job (rows x cols, row stride ld
 // floats) for 32 x 32-float TMA stores with the 128-byte swizzle; sets
@@ -112,9 +130,9 @@ bool encode_output(TcJob* job);
 void order_tiles_by_k(int4* tiles, int n, const TcJob* jobs, bool sort = true);
 
 // Host: launch the grouped kernel over `n_tiles` (job, m0, n0, k-blocks) tiles
-// with `ctas_percent` of the SMs as persistent CTAs (0: all of them).
+// of `cols` columns (those that the jobs' B operands are encoded for) with `ctas_percent` of the SMs as persistent CTAs (0: all of them).
 // `pdl`: as a programmatic dependent launch.
-int launch(const TcJob* jobs_dev, const int4* tiles_dev, int n_tiles, int* err_dev,
+int launch(const TcJob* jobs_dev, const int4* tiles_dev, int n_tiles, int cols, int* err_dev,
            cudaStream_t s, int ctas_percent = 0, bool pdl = false);
 
 }  // namespace axi_tc

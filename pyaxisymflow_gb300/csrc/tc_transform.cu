@@ -80,10 +80,16 @@ struct PlanLayout {
   size_t jobs, tiles[4], err, total;
 };
 
-int stage_tiles(const axi_tc_transform& t, int st) {
+int stage_tiles(const axi_tc_transform& t, int st, int cols) {
   const int M = (st % 2 == 0) ? t.nz : t.nr;
   const int N = (st % 2 == 0) ? t.nr : t.nz;
-  return ((M + axi_tc::BM - 1) / axi_tc::BM) * ((N + axi_tc::BN - 1) / axi_tc::BN);
+  return axi_tc::tile_count(M, N, cols);
+}
+
+int stage_cols(const axi_tc_transform* t, int n, int st) {
+  int tiles64 = 0;
+  for (int q = 0; q < n; ++q) tiles64 += stage_tiles(t[q], st, 64);
+  return axi_tc::choose_cols(tiles64, axi::sm_count());
 }
 
 PlanLayout layout(const axi_tc_transform* t, int n) {
@@ -94,7 +100,7 @@ PlanLayout layout(const axi_tc_transform* t, int n) {
   for (int st = 0; st < 4; ++st) {
     int tiles = 0;
     if (t)
-      for (int q = 0; q < n; ++q) tiles += stage_tiles(t[q], st);
+      for (int q = 0; q < n; ++q) tiles += stage_tiles(t[q], st, stage_cols(t, n, st));
     L.tiles[st] = o;
     o = align_up(o + (size_t)tiles * sizeof(int4), 16);
   }
@@ -121,7 +127,8 @@ extern "C" int axi_tc_transform_plan(const axi_tc_transform* t, int n, void* pla
   info->bytes = (int64_t)L.total;
   for (int st = 0; st < 4; ++st) {
     info->n_tiles[st] = 0;
-    for (int q = 0; q < n; ++q) info->n_tiles[st] += stage_tiles(t[q], st);
+    info->tile_cols[st] = stage_cols(t, n, st);
+    for (int q = 0; q < n; ++q) info->n_tiles[st] += stage_tiles(t[q], st, info->tile_cols[st]);
   }
   if (!plan_dev) return AXI_OK;  // size query
   std::string buf(L.total, '\0');
@@ -141,28 +148,28 @@ extern "C" int axi_tc_transform_plan(const axi_tc_transform* t, int n, void* pla
     AXI_TRY(axi::check_ptr(what, k.out, "out"));
     axi_tc::TcJob* j = jobs + 4 * q;
     memset(j, 0, 4 * sizeof(axi_tc::TcJob));
-    AXI_TRY(axi_tc::encode_operand(&j[0].a_hi, k.basis[0], nz, nz, nz));
-    AXI_TRY(axi_tc::encode_operand(&j[0].a_lo, k.basis[1], nz, nz, nz));
-    AXI_TRY(axi_tc::encode_operand(&j[0].b_hi, k.in_hi, nr, nz, nz));
-    AXI_TRY(axi_tc::encode_operand(&j[0].b_lo, k.in_lo, nr, nz, nz));
+    AXI_TRY(axi_tc::encode_operand(&j[0].a_hi, k.basis[0], nz, nz, nz, axi_tc::BM));
+    AXI_TRY(axi_tc::encode_operand(&j[0].a_lo, k.basis[1], nz, nz, nz, axi_tc::BM));
+    AXI_TRY(axi_tc::encode_operand(&j[0].b_hi, k.in_hi, nr, nz, nz, info->tile_cols[0]));
+    AXI_TRY(axi_tc::encode_operand(&j[0].b_lo, k.in_lo, nr, nz, nz, info->tile_cols[0]));
     j[0].c = k.work[0]; j[0].c_lo = k.work[1]; j[0].M = nz; j[0].N = nr; j[0].K = nz;
     j[0].ldc = nr; j[0].mode = axi_tc::MODE_SPLIT;
-    AXI_TRY(axi_tc::encode_operand(&j[1].a_hi, k.basis[2], nr, nr, nr));
-    AXI_TRY(axi_tc::encode_operand(&j[1].a_lo, k.basis[3], nr, nr, nr));
-    AXI_TRY(axi_tc::encode_operand(&j[1].b_hi, k.work[0], nz, nr, nr));
-    AXI_TRY(axi_tc::encode_operand(&j[1].b_lo, k.work[1], nz, nr, nr));
+    AXI_TRY(axi_tc::encode_operand(&j[1].a_hi, k.basis[2], nr, nr, nr, axi_tc::BM));
+    AXI_TRY(axi_tc::encode_operand(&j[1].a_lo, k.basis[3], nr, nr, nr, axi_tc::BM));
+    AXI_TRY(axi_tc::encode_operand(&j[1].b_hi, k.work[0], nz, nr, nr, info->tile_cols[1]));
+    AXI_TRY(axi_tc::encode_operand(&j[1].b_lo, k.work[1], nz, nr, nr, info->tile_cols[1]));
     j[1].c = k.work[2]; j[1].c_lo = k.work[3]; j[1].scale = k.inv_eig; j[1].M = nr;
     j[1].N = nz; j[1].K = nr; j[1].ldc = nz; j[1].mode = axi_tc::MODE_SCALE_SPLIT;
-    AXI_TRY(axi_tc::encode_operand(&j[2].a_hi, k.basis[4], nz, nz, nz));
-    AXI_TRY(axi_tc::encode_operand(&j[2].a_lo, k.basis[5], nz, nz, nz));
-    AXI_TRY(axi_tc::encode_operand(&j[2].b_hi, k.work[2], nr, nz, nz));
-    AXI_TRY(axi_tc::encode_operand(&j[2].b_lo, k.work[3], nr, nz, nz));
+    AXI_TRY(axi_tc::encode_operand(&j[2].a_hi, k.basis[4], nz, nz, nz, axi_tc::BM));
+    AXI_TRY(axi_tc::encode_operand(&j[2].a_lo, k.basis[5], nz, nz, nz, axi_tc::BM));
+    AXI_TRY(axi_tc::encode_operand(&j[2].b_hi, k.work[2], nr, nz, nz, info->tile_cols[2]));
+    AXI_TRY(axi_tc::encode_operand(&j[2].b_lo, k.work[3], nr, nz, nz, info->tile_cols[2]));
     j[2].c = k.work[0]; j[2].c_lo = k.work[1]; j[2].M = nz; j[2].N = nr; j[2].K = nz;
     j[2].ldc = nr; j[2].mode = axi_tc::MODE_SPLIT;
-    AXI_TRY(axi_tc::encode_operand(&j[3].a_hi, k.basis[6], nr, nr, nr));
-    AXI_TRY(axi_tc::encode_operand(&j[3].a_lo, k.basis[7], nr, nr, nr));
-    AXI_TRY(axi_tc::encode_operand(&j[3].b_hi, k.work[0], nz, nr, nr));
-    AXI_TRY(axi_tc::encode_operand(&j[3].b_lo, k.work[1], nz, nr, nr));
+    AXI_TRY(axi_tc::encode_operand(&j[3].a_hi, k.basis[6], nr, nr, nr, axi_tc::BM));
+    AXI_TRY(axi_tc::encode_operand(&j[3].a_lo, k.basis[7], nr, nr, nr, axi_tc::BM));
+    AXI_TRY(axi_tc::encode_operand(&j[3].b_hi, k.work[0], nz, nr, nr, info->tile_cols[3]));
+    AXI_TRY(axi_tc::encode_operand(&j[3].b_lo, k.work[1], nz, nr, nr, info->tile_cols[3]));
     j[3].c = k.out; j[3].M = nr; j[3].N = nz; j[3].K = nr; j[3].ldc = nz;
     j[3].mode = axi_tc::MODE_PLAIN;
   }
@@ -180,7 +187,7 @@ extern "C" int axi_tc_transform_plan(const axi_tc_transform* t, int n, void* pla
       const int M = (st % 2 == 0) ? t[q].nz : t[q].nr;
       const int N = (st % 2 == 0) ? t[q].nr : t[q].nz;
       for (int m0 = 0; m0 < M; m0 += axi_tc::BM)
-        for (int n0 = 0; n0 < N; n0 += axi_tc::BN) tt[qq++] = make_int4(4 * q + st, m0, n0, 0);
+        for (int n0 = 0; n0 < N; n0 += info->tile_cols[st]) tt[qq++] = make_int4(4 * q + st, m0, n0, 0);
     }
     axi_tc::order_tiles_by_k(tt, qq, jobs);
   }
@@ -210,7 +217,7 @@ extern "C" int axi_tc_transform_run(const axi_tc_plan_info* info, const void* pl
   cudaStream_t s = axi::as_stream(stream);
   for (int st = 0; st < 4; ++st)
     AXI_TRY(axi_tc::launch(jobs, reinterpret_cast<const int4*>(base + toff[st]),
-                           info->n_tiles[st], err, s));
+                           info->n_tiles[st], info->tile_cols[st], err, s));
   return AXI_OK;
 }
 

@@ -169,7 +169,7 @@ class AxiPlanInfo(ctypes.Structure):
                 ("bytes", ctypes.c_int64), ("flags", ctypes.c_int32),
                 ("n_tc_tiles", ctypes.c_int32 * 4), ("n_dct_items", ctypes.c_int32),
                 ("tune", AxiTuning), ("n_slice_items", ctypes.c_int32 * 4),
-                ("sliced_form", ctypes.c_int32 * 4), ("slice_groups", ctypes.c_int32 * 4)]
+                ("tile_form", ctypes.c_int32 * 4), ("slice_groups", ctypes.c_int32 * 4)]
 
 
 PLAN_TENSOR_CORES = 1

@@ -94,7 +94,7 @@ class AxiTcTransform(ctypes.Structure):
 class AxiTcPlanInfo(ctypes.Structure):
     """Mirror of ``axi_tc_plan_info`` in include/axisym_gb300.h."""
     _fields_ = [("n", ctypes.c_int32), ("n_tiles", ctypes.c_int32 * 4),
-                ("reserved", ctypes.c_int32), ("bytes", ctypes.c_int64)]
+                ("tile_cols", ctypes.c_uint8 * 4), ("bytes", ctypes.c_int64)]
 
 
 class FastDiagonalisationEngine:

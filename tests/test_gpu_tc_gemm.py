@@ -32,3 +32,17 @@ def test_tf32x3_gemm_matches_fp64(M, N, K):
     err = ((C - ref32).norm() / ref32.norm()).item()
     assert err < 1e-5, err
     assert ((C - ref).norm() / ref.norm()).item() < 1e-5
+
+
+# one tile of 64 columns, ragged; the last counts of 64-column tiles that run
+# at once and the first of 128-column ones on 152 SMs (8 x 19, 9 x 17)
+@pytest.mark.parametrize("M,N,K", [(100, 61, 36), (1000, 1210, 68), (1130, 1070, 100)])
+def test_tf32x3_gemm_tile_forms(M, N, K):
+    g = torch.Generator(device="cpu").manual_seed(M + N + K)
+    A = torch.randn((M, K), generator=g, dtype=torch.float32)
+    B = torch.randn((N, K), generator=g, dtype=torch.float32)
+    C = tc_gemm(A.cuda(), B.cuda()).double().cpu()
+    # an operand keeps 23 bits as hi + lo (2^-23 relative), the dropped lo lo
+    # term 2^-22; K / 8 x 3 additions into a float
+    bound = (A.abs().double() @ B.abs().double().T) * (2.0 ** -21 + (3 * K / 8 + 8) * 2.0 ** -23)
+    assert ((C - A.double() @ B.double().T).abs() <= bound).all()
