@@ -269,6 +269,16 @@ int axi_advect_particles_prepare_f64(double* z_particles, double* r_particles,
                                      double* vort_particles, const double* vorticity,
                                      const double* u_z, const double* u_r, int nr, int nz,
                                      double dt, void* stream);
+/* The whole remeshing step (kernels/advect_particle.py:5-68): the particles
+ * move as above, their vorticity is interpolated onto the mesh rows above the
+ * axis, and they go back to z_mesh, r_mesh (2 nr, nz). A particle that moved a
+ * cell or more leaves vorticity and the moved particles as they are;
+ * axi_p2m_status(work, 2 nr, nz) reports it. `work`: axi_p2m_mp4_work_bytes(
+ * 2 nr, nz) bytes of device scratch. */
+int axi_advect_particles_f64(double* z_particles, double* r_particles, double* vort_particles,
+                             double* vorticity, const double* z_mesh, const double* r_mesh,
+                             const double* u_z, const double* u_r, int nr, int nz, double dx,
+                             double dt, int periodic, void* work, void* stream);
 /* ---------------------------------------------------------------------
  * Level-set reinitialisation: the signed distance to the zero contour of phi
  * (nr, nz, spacing dx) within `narrow`, the role of

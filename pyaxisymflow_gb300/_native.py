@@ -52,6 +52,7 @@ def _signatures():
         "axi_level_set_work_bytes": (I64, [I, I]),
         "axi_level_set_distance_f64": (I, [P, P, I, I, D, D, P, P, P]),
         "axi_advect_particles_prepare_f64": (I, [P, P, P, P, P, P, I, I, D, P]),
+        "axi_advect_particles_f64": (I, [P, P, P, P, P, P, P, P, I, I, D, D, I, P, P]),
         "axi_extrapolate_lsq_first_order_f64": (I, [P, P, P, P, P, P, I, I, I, P, P, P]),
         "axi_extrapolate_eta_with_least_squares_f64": (
             I, [P, P, P, P, P, P, P, P, P, D, I, I, P, P, I, P, P, P]),

@@ -23,6 +23,16 @@ def _scratch(n0, n1, device):
     return _work[key]
 
 
+def _check(work, n0, n1, out):
+    """Raises when the last interpolation met a particle a cell or more from
+    its mesh point (synchronises the stream of `out`)."""
+    flag = N._c.c_int(0)
+    N.call("axi_p2m_status", N.ptr(work), n0, n1, N._c.byref(flag), N.stream_of(out))
+    if flag.value:
+        raise ValueError("particles_to_mesh: a particle moved a cell or more from its mesh "
+                         "point (|u| dt must stay below dx along each axis)")
+
+
 def _p2m(px, py, vin, out, delta_x, delta_y, periodic, check):
     N.require(px, py, vin, out, shape=out.shape, dtype=torch.float64,
               names=("particle_positions_x", "particle_positions_y",
@@ -32,11 +42,7 @@ def _p2m(px, py, vin, out, delta_x, delta_y, periodic, check):
     N.call("axi_particles_to_mesh_2d_mp4_f64", N.ptr(px), N.ptr(py), N.ptr(vin), N.ptr(out), n0,
            n1, float(delta_x), float(delta_y), int(periodic), N.ptr(work), N.stream_of(out))
     if check:
-        flag = N._c.c_int(0)
-        N.call("axi_p2m_status", N.ptr(work), n0, n1, N._c.byref(flag), N.stream_of(out))
-        if flag.value:
-            raise ValueError("particles_to_mesh: a particle moved a cell or more from its mesh "
-                             "point (|u| dt must stay below dx along each axis)")
+        _check(work, n0, n1, out)
 
 
 def particles_to_mesh_2D_mp4(particle_positions_x, particle_positions_y,

@@ -47,20 +47,18 @@ P2MLayout p2m_layout(int n0, int n1) {
 }
 
 // MP4 (core/src/particle_kernels/MP4.hpp): |x| <= 1 and 1 < |x| <= 2 branches,
-// evaluated in the reference's operation order without contraction.
+// evaluated in the reference's operation order without contraction (0.5 t is
+// exact, so 2.5 - 0.5 t is one fused instruction with the same rounding).
 __device__ __forceinline__ double mp4_inner(double t) {
   return __dadd_rn(1.0, __dmul_rn(__dmul_rn(t, t), __dadd_rn(-2.5, __dmul_rn(1.5, t))));
 }
 __device__ __forceinline__ double mp4_outer(double t) {
   return __dadd_rn(2.0,
-                   __dmul_rn(t, __dadd_rn(-4.0, __dmul_rn(t, __dsub_rn(2.5, __dmul_rn(0.5, t))))));
+                   __dmul_rn(t, __dadd_rn(-4.0, __dmul_rn(t, __fma_rn(-0.5, t, 2.5)))));
 }
 
-// Anchor h (mesh index nearest above the particle on the cell-centred mesh)
-// and the four stencil weights along one axis
-// (particles_to_mesh_2D.hpp:60-118; slot k has offset k - 2, the outer slots
-// 0 and 3 use the outer branch, core/src/particle_kernels/KernelWrapper.hpp:31-47).
-__device__ __forceinline__ int mp4_stencil(double pos, double w[4]) {
+// The weights as written in the reference, for positions of any size.
+__device__ __noinline__ int mp4_stencil_any(double pos, double w[4]) {
   const double fl = floor(pos);
   const int h = (pos >= __dadd_rn(fl, 0.5) ? 1 : 0) + (int)fl;
   const double base = __dadd_rn((double)h, 0.5);
@@ -72,20 +70,71 @@ __device__ __forceinline__ int mp4_stencil(double pos, double w[4]) {
   return h;
 }
 
+// 1.5 * 2^51: a double near it counts halves in its low word
+constexpr double HALVES = 3377699720527872.0;
+
+// floor(pos + 0.5) of |pos| < 2^30 from one rounded-down addition
+__device__ __forceinline__ int mp4_round(double pos) {
+  const int halves = __double2loint(__dadd_rd(pos, HALVES));  // floor(2 pos)
+  return (halves + 1) >> 1;
+}
+
+// Anchor h (mesh index nearest above the particle on the cell-centred mesh)
+// and the four stencil weights along one axis
+// (particles_to_mesh_2D.hpp:60-118; slot k has offset k - 2, the outer slots
+// 0 and 3 use the outer branch, core/src/particle_kernels/KernelWrapper.hpp:31-47).
+// FP64 issue bounds it, so the fast form counts instructions: from position 1
+// up to 2^30 the distance d to the centre h + 0.5 is a multiple of the
+// position's unit and at most 1, hence exact, as are 2 - d, 1 - d and 1 + d:
+// the same four distances that the reference rounds (6 instructions for anchor
+// and distances instead of about 14).
+__device__ __forceinline__ int mp4_stencil(double pos, double w[4]) {
+  if ((unsigned int)__double2hiint(pos) - 0x3ff00000u >= (30u << 20)) return mp4_stencil_any(pos, w);
+  const int h = mp4_round(pos);
+  const double centre =
+      __dsub_rn(__longlong_as_double(__double_as_longlong(HALVES) + (2 * h + 1)), HALVES);
+  const double d = __dsub_rn(centre, pos);
+  w[0] = mp4_outer(__dsub_rn(2.0, d));
+  w[1] = mp4_inner(__dsub_rn(1.0, d));
+  w[2] = mp4_inner(d);
+  w[3] = mp4_outer(__dadd_rn(1.0, d));
+  return h;
+}
+
+// the anchor alone
+__device__ __forceinline__ int mp4_anchor(double pos) {
+  if (exponent_bits(pos) < 1023 + 30) return mp4_round(pos);
+  const double fl = floor(pos);
+  return (pos >= __dadd_rn(fl, 0.5) ? 1 : 0) + (int)fl;
+}
+
+__device__ __forceinline__ bool displaced(int hx, int hy, int j, int i) {
+  return hx - i < 0 || hx - i > 1 || hy - j < 0 || hy - j > 1;
+}
+
+__device__ __forceinline__ void store_stencil(double px, double py, const KnownDivisor<double>& dx,
+                                              const KnownDivisor<double>& dy, int j, int i,
+                                              long long p, int2* __restrict__ H,
+                                              Weights4* __restrict__ WX, Weights4* __restrict__ WY,
+                                              int* __restrict__ flag) {
+  double wx[4], wy[4];
+  const int hx = mp4_stencil(dx.quotient(px), wx);
+  const int hy = mp4_stencil(dy.quotient(py), wy);
+  H[p] = make_int2(hx, hy);
+  WX[p] = Weights4{{wx[0], wx[1], wx[2], wx[3]}};
+  WY[p] = Weights4{{wy[0], wy[1], wy[2], wy[3]}};
+  if (displaced(hx, hy, j, i)) atomicOr(flag, 1);
+}
+
 __global__ void p2m_stencil_kernel(const double* __restrict__ px, const double* __restrict__ py,
-                                   int n0, int n1, double dx, double dy, int2* __restrict__ H,
+                                   int n0, int n1, KnownDivisor<double> dx,
+                                   KnownDivisor<double> dy, int2* __restrict__ H,
                                    Weights4* __restrict__ WX, Weights4* __restrict__ WY,
                                    int* __restrict__ flag) {
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= (long long)n0 * n1) return;
   const int j = (int)(p / n1), i = (int)(p % n1);
-  double wx[4], wy[4];
-  const int hx = mp4_stencil(__ddiv_rn(px[p], dx), wx);
-  const int hy = mp4_stencil(__ddiv_rn(py[p], dy), wy);
-  H[p] = make_int2(hx, hy);
-  WX[p] = Weights4{{wx[0], wx[1], wx[2], wx[3]}};
-  WY[p] = Weights4{{wy[0], wy[1], wy[2], wy[3]}};
-  if (hx - i < 0 || hx - i > 1 || hy - j < 0 || hy - j > 1) atomicOr(flag, 1);
+  store_stencil(px[p], py[p], dx, dy, j, i, p, H, WX, WY, flag);
 }
 
 // The up to five particle indices m - 2 .. m + 2 along one axis (wrapped when
@@ -109,12 +158,11 @@ __device__ __forceinline__ int candidates(int m, int n, bool periodic, int out[5
   return c;
 }
 
-__global__ void p2m_gather_kernel(const double* __restrict__ vin, const int2* __restrict__ H,
-                                  const Weights4* __restrict__ WX, const Weights4* __restrict__ WY,
-                                  double* __restrict__ out, int n0, int n1, int periodic) {
-  const int mi = blockIdx.x * blockDim.x + threadIdx.x;
-  const int mj = blockIdx.y;
-  if (mi >= n1 || mj >= n0) return;
+// The sum of mesh point (mj, mi).
+__device__ __forceinline__ double gather(const double* __restrict__ vin, const int2* __restrict__ H,
+                                         const Weights4* __restrict__ WX,
+                                         const Weights4* __restrict__ WY, int mj, int mi, int n0,
+                                         int n1, int periodic) {
   int rows[5], cols[5];
   const int nr = candidates(mj, n0, periodic != 0, rows);
   const int nc = candidates(mi, n1, periodic != 0, cols);
@@ -137,7 +185,16 @@ __global__ void p2m_gather_kernel(const double* __restrict__ vin, const int2* __
       acc = __dadd_rn(acc, __dmul_rn(w, vin[p]));
     }
   }
-  out[(long long)mj * n1 + mi] = acc;
+  return acc;
+}
+
+__global__ void p2m_gather_kernel(const double* __restrict__ vin, const int2* __restrict__ H,
+                                  const Weights4* __restrict__ WX, const Weights4* __restrict__ WY,
+                                  double* __restrict__ out, int n0, int n1, int periodic) {
+  const int mi = blockIdx.x * blockDim.x + threadIdx.x;
+  const int mj = blockIdx.y;
+  if (mi >= n1 || mj >= n0) return;
+  out[(long long)mj * n1 + mi] = gather(vin, H, WX, WY, mj, mi, n0, n1, periodic);
 }
 
 // Mesh-to-particle MP4 interpolation of two fields
@@ -157,13 +214,14 @@ __device__ __forceinline__ int wrap_index(int a, int n) {
 __global__ void m2p_mp4_kernel(const double* __restrict__ in_x, const double* __restrict__ in_y,
                                int n0, int n1, const double* __restrict__ px,
                                const double* __restrict__ py, double* __restrict__ out_x,
-                               double* __restrict__ out_y, long long n_particles, double dx,
-                               double dy, int periodic) {
+                               double* __restrict__ out_y, long long n_particles,
+                               KnownDivisor<double> dx, KnownDivisor<double> dy,
+                               int periodic) {
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n_particles) return;
   double wx[4], wy[4];
-  const int hx = mp4_stencil(__ddiv_rn(px[p], dx), wx);
-  const int hy = mp4_stencil(__ddiv_rn(py[p], dy), wy);
+  const int hx = mp4_stencil(dx.quotient(px[p]), wx);
+  const int hy = mp4_stencil(dy.quotient(py[p]), wy);
   int sx0 = -2, sx1 = 2, sy0 = -2, sy1 = 2;
   if (!periodic && (hx - 2 < 0 || hy - 2 < 0 || hx + 2 > n1 || hy + 2 > n0)) {
     sx0 = max(-2, -hx);
@@ -194,9 +252,25 @@ __global__ void m2p_mp4_kernel(const double* __restrict__ in_x, const double* __
   out_y[p] = acc_y;
 }
 
-// kernels/advect_particle.py:20-28 (and :53-61): particles on the mirrored
-// (2 nr, nz) domain move with the velocity (mirror rows: u_z even, u_r odd),
-// and carry the vorticity (mirror rows odd).
+// kernels/advect_particle.py:20-28 (and :53-61): particle (j, i) of the
+// mirrored (2 nr, nz) domain moves with the velocity (mirror rows: u_z even,
+// u_r odd), and carries the vorticity (mirror rows odd).
+__device__ __forceinline__ void move_particle(double* __restrict__ zp, double* __restrict__ rp,
+                                              double* __restrict__ vp,
+                                              const double* __restrict__ w,
+                                              const double* __restrict__ uz,
+                                              const double* __restrict__ ur, int j, int i, int nr,
+                                              int nz, double dt, double& z, double& r) {
+  const long long d = (long long)j * nz + i;
+  const bool mirror = j < nr;
+  const long long c = (long long)(mirror ? nr - 1 - j : j - nr) * nz + i;
+  z = __dadd_rn(zp[d], __dmul_rn(uz[c], dt));
+  r = __dadd_rn(rp[d], __dmul_rn(flip_sign(ur[c], mirror), dt));
+  zp[d] = z;
+  rp[d] = r;
+  vp[d] = flip_sign(w[c], mirror);
+}
+
 __global__ void particles_prepare_kernel(double* __restrict__ zp, double* __restrict__ rp,
                                          double* __restrict__ vp,
                                          const double* __restrict__ w,
@@ -206,18 +280,55 @@ __global__ void particles_prepare_kernel(double* __restrict__ zp, double* __rest
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y;  // row of the mirrored domain, 0 .. 2 nr - 1
   if (i >= nz || j >= 2 * nr) return;
-  const long long d = (long long)j * nz + i;
-  if (j >= nr) {
-    const long long c = (long long)(j - nr) * nz + i;
-    zp[d] = __dadd_rn(zp[d], __dmul_rn(uz[c], dt));
-    rp[d] = __dadd_rn(rp[d], __dmul_rn(ur[c], dt));
-    vp[d] = w[c];
-  } else {
-    const long long c = (long long)(nr - 1 - j) * nz + i;
-    zp[d] = __dadd_rn(zp[d], __dmul_rn(uz[c], dt));
-    rp[d] = __dadd_rn(rp[d], __dmul_rn(-ur[c], dt));
-    vp[d] = -w[c];
+  double z, r;
+  move_particle(zp, rp, vp, w, uz, ur, j, i, nr, nz, dt, z, r);
+}
+
+// The remeshing step as two kernels. Only the rows above the axis of the
+// interpolated vorticity are kept, so only the particles that reach those
+// (the upper rows and two rows beyond each end of them) get weights; the other
+// mirror particles only move and are checked for their displacement.
+// Bound by FP64 issue (64 cycles a warp instruction): 4 to move, 8 for the two
+// quotients, 52 for anchors and weights (88 before, and for every particle),
+// then 48 to 75 a kept mesh point, as its neighbours move alike or apart. At
+// 1024 x 512 cells a step takes 192 us (395 with weights and sums for the whole
+// mirrored domain), 160 of them in the two kernels; sums over lists of the
+// particles that reach a point, in place of the test in the loop, took 195.
+__global__ void advect_stencil_kernel(double* __restrict__ zp, double* __restrict__ rp,
+                                      double* __restrict__ vp, const double* __restrict__ w,
+                                      const double* __restrict__ uz, const double* __restrict__ ur,
+                                      int nr, int nz, double dt, KnownDivisor<double> dx,
+                                      int periodic, int2* __restrict__ H, Weights4* __restrict__ WX,
+                                      Weights4* __restrict__ WY, int* __restrict__ flag) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y;
+  if (i >= nz) return;
+  double z, r;
+  move_particle(zp, rp, vp, w, uz, ur, j, i, nr, nz, dt, z, r);
+  if (j >= nr - 2 || (periodic && j < 2)) {
+    store_stencil(z, r, dx, dx, j, i, (long long)j * nz + i, H, WX, WY, flag);
+  } else if (displaced(mp4_anchor(dx.quotient(z)), mp4_anchor(dx.quotient(r)), j, i)) {
+    atomicOr(flag, 1);
   }
+}
+
+// Vorticity above the axis from the particles, which go back to the mesh; when
+// a particle moved too far nothing is written, and the caller is told.
+__global__ void advect_gather_kernel(double* __restrict__ zp, double* __restrict__ rp,
+                                     const double* __restrict__ vp, double* __restrict__ w,
+                                     const double* __restrict__ Z, const double* __restrict__ R,
+                                     const int2* __restrict__ H, const Weights4* __restrict__ WX,
+                                     const Weights4* __restrict__ WY, int nr, int nz, int periodic,
+                                     const int* __restrict__ flag) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y;
+  if (i >= nz || *flag) return;
+  const long long lo = (long long)j * nz + i, up = (long long)(nr + j) * nz + i;
+  zp[lo] = Z[lo];
+  rp[lo] = R[lo];
+  zp[up] = Z[up];
+  rp[up] = R[up];
+  w[lo] = gather(vp, H, WX, WY, nr + j, i, 2 * nr, nz, periodic);
 }
 
 }  // namespace
@@ -252,8 +363,8 @@ extern "C" int axi_particles_to_mesh_2d_mp4_f64(const double* px, const double* 
   if (cudaMemsetAsync(flag, 0, sizeof(int), s) != cudaSuccess)
     return axi::launch_status("particles_to_mesh");
   const long long n = (long long)n0 * n1;
-  p2m_stencil_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(px, py, n0, n1, dx, dy, H, WX,
-                                                                  WY, flag);
+  p2m_stencil_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
+      px, py, n0, n1, KnownDivisor<double>(dx), KnownDivisor<double>(dy), H, WX, WY, flag);
   p2m_gather_kernel<<<dim3((n1 + 127) / 128, n0), 128, 0, s>>>(vin, H, WX, WY, out, n0, n1,
                                                                 periodic);
   return axi::launch_status("particles_to_mesh");
@@ -288,6 +399,40 @@ extern "C" int axi_advect_particles_prepare_f64(double* z_particles, double* r_p
   return axi::launch_status("advect_particles");
 }
 
+extern "C" int axi_advect_particles_f64(double* z_particles, double* r_particles,
+                                        double* vort_particles, double* vorticity,
+                                        const double* z_mesh, const double* r_mesh,
+                                        const double* u_z, const double* u_r, int nr, int nz,
+                                        double dx, double dt, int periodic, void* work,
+                                        void* stream) {
+  axi::clear_error();
+  const void* ptrs[] = {z_particles, r_particles, vort_particles, vorticity, z_mesh,
+                        r_mesh,      u_z,         u_r,            work};
+  for (const void* p : ptrs) AXI_TRY(axi::check_ptr("advect_particles", p, "field"));
+  if (nr < 3 || nr > 32767 || nz < 5 || !(dx > 0.0)) {
+    axi::set_error("advect_particles: grid %d x %d (mirrored: each side 5 .. 65535) or spacing "
+                   "invalid", nr, nz);
+    return AXI_ERR_INVALID;
+  }
+  const P2MLayout L = p2m_layout(2 * nr, nz);
+  char* wb = static_cast<char*>(work);
+  int2* H = reinterpret_cast<int2*>(wb + L.h);
+  Weights4* WX = reinterpret_cast<Weights4*>(wb + L.wx);
+  Weights4* WY = reinterpret_cast<Weights4*>(wb + L.wy);
+  int* flag = reinterpret_cast<int*>(wb + L.flag);
+  cudaStream_t s = axi::as_stream(stream);
+  if (cudaMemsetAsync(flag, 0, sizeof(int), s) != cudaSuccess)
+    return axi::launch_status("advect_particles");
+  const unsigned bx = (unsigned)((nz + 127) / 128);
+  advect_stencil_kernel<<<dim3(bx, 2 * nr), 128, 0, s>>>(
+      z_particles, r_particles, vort_particles, vorticity, u_z, u_r, nr, nz, dt,
+      KnownDivisor<double>(dx), periodic, H, WX, WY, flag);
+  advect_gather_kernel<<<dim3(bx, nr), 128, 0, s>>>(z_particles, r_particles, vort_particles,
+                                                    vorticity, z_mesh, r_mesh, H, WX, WY, nr, nz,
+                                                    periodic, flag);
+  return axi::launch_status("advect_particles");
+}
+
 extern "C" int axi_mesh_to_particles_2d_mp4_f64(const double* input_field_x,
                                                 const double* input_field_y, int n0, int n1,
                                                 const double* particle_positions_x,
@@ -308,6 +453,6 @@ extern "C" int axi_mesh_to_particles_2d_mp4_f64(const double* input_field_x,
   const long long n = (long long)p0 * p1;
   m2p_mp4_kernel<<<(unsigned)((n + 255) / 256), 256, 0, axi::as_stream(stream)>>>(
       input_field_x, input_field_y, n0, n1, particle_positions_x, particle_positions_y,
-      output_field_x, output_field_y, n, dx, dy, periodic);
+      output_field_x, output_field_y, n, KnownDivisor<double>(dx), KnownDivisor<double>(dy), periodic);
   return axi::launch_status("mesh_to_particles");
 }

@@ -75,6 +75,35 @@ def test_advect_vorticity_via_particles_matches_oracle_larger(nr, nz):
         np.testing.assert_array_equal(w.cpu().numpy(), w_ref)
 
 
+@pytest.mark.parametrize("nr,nz", [(3, 5), (4, 129), (65, 127)])
+def test_remeshing_edges_and_refusal(nr, nz):
+    """The fused step at its smallest grids and block edges, every field it
+    leaves, and what a particle that moved too far leaves (one mirror particle
+    alone: its own u, placed off the mesh)."""
+    from pyaxisymflow_gb300.kernels import advect_particle as ap
+    rng = np.random.default_rng(nr * nz)
+    dx = 0.3 / nz
+    Zd, Rd = np.meshgrid((np.arange(nz) + 0.5) * dx, (np.arange(2 * nr) + 0.5) * dx)
+    w0 = rng.standard_normal((nr, nz))
+    uz, ur = rng.uniform(-1, 1, (nr, nz)), rng.uniform(-1, 1, (nr, nz))
+    dt = 0.9 * dx
+    for ref_fn, fn in ((K.advect_vorticity_via_particles, ap.advect_vorticity_via_particles),
+                       (K.advect_vorticity_via_particles_periodic,
+                        ap.advect_vorticity_via_particles_periodic)):
+        w_ref, zp, rp, vp = w0.copy(), Zd.copy(), Rd.copy(), np.zeros_like(Zd)
+        ref_fn(zp, rp, vp, w_ref, Zd, Rd, nr, uz, ur, dx, dt)
+        w, zt, rt, vt, Zt, Rt = (cuda(a) for a in (w0, Zd, Rd, np.zeros_like(Zd), Zd, Rd))
+        fn(zt, rt, vt, w, Zt, Rt, nr, cuda(uz), cuda(ur), dx, dt)
+        for got, want in ((w, w_ref), (zt, Zd), (rt, Rd), (vt, vp)):
+            np.testing.assert_array_equal(got.cpu().numpy(), want)
+        zt[0, nz // 2] += 2 * dx
+        before = w.clone()
+        with pytest.raises(ValueError, match="cell or more"):
+            fn(zt, rt, vt, w, Zt, Rt, nr, cuda(0 * uz), cuda(0 * ur), dx, dt)
+        assert torch.equal(w, before)
+        assert float(zt[0, nz // 2] - Zt[0, nz // 2]) > dx and torch.equal(vt[nr:], before)
+
+
 @pytest.mark.parametrize("tag", ["a", "b", "c"])
 def test_mesh_to_particles_matches_reference_golden(golden, tag):
     """Mesh-to-particle MP4 (periodic and unbounded) on the device against
