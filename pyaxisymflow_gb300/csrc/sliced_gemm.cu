@@ -11,6 +11,7 @@
 namespace axi_sl {
 namespace {
 
+using axi_tma::elect_one;
 using axi_tma::mbar_expect_tx;
 using axi_tma::mbar_init;
 using axi_tma::mbar_wait;
@@ -343,10 +344,14 @@ constexpr int smem_bytes(int bn, int split) {
 // two accumulator sets while the MMAs fill the other. A unit of work is one
 // tile and up to 128 of its K; the integer sums run on over the units of a tile.
 //
-// Bound by shared memory: a step of 16 K with BN = 32 writes 40 KB and its MMAs
-// read 68 KB, 844 cycles at 128 bytes per cycle, where the MMAs themselves take
-// 576. (Sharing A's loads between the blocks of a cluster by multicast changed
-// nothing: 199.6 against 198.3 us for a 1024 x 512 solve.)
+// Bound by shared memory: an MMA of N columns takes the larger of N / 2 cycles
+// (the tensor rate) and 32 + N / 4 (its operands at 128 bytes per cycle), 660 a
+// step of 16 K with BN = 32, into which the copies of the next steps write
+// another 40 KB. The issuing thread took 844 a step until it ran under
+// elect.sync; the four products of 512 x 256 then went from 61.6 to 52.2 us and
+// those of eight cases from 418 to 380. (Sharing A's loads between the blocks
+// of a cluster by multicast changed nothing: 199.6 against 198.3 us for a
+// 1024 x 512 solve.)
 //
 // SPLIT > 1: a cluster of SPLIT blocks per tile, each taking a share of its K;
 // then every block finishes BN / SPLIT of the columns, with the partial sums
@@ -408,8 +413,9 @@ __global__ void __launch_bounds__(THREADS, 1)
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      int g = 0;
+    if (elect_one()) {
+      int g = 0, s = 0;
+      uint32_t lap = 1;  // parity of the phase that frees a stage
       bool ok = true;
       int ahead = 0;  // first steps of the first tile whose A is already on its way
       if (flags & FLAG_A_READY) {
@@ -430,8 +436,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         const uint8_t* a = job.a + (size_t)tr.y * nk * A_STAGE;
         const uint8_t* b = job.b + (size_t)tr.z * nk * B_STAGE;
         for (int kb = k_begin(nk); kb < k_end(nk); ++kb, ++g) {
-          const int s = g % NSTAGE, use = g / NSTAGE;
-          if (use > 0 && !mbar_wait(empty0 + 8 * s, (use - 1) & 1, err, ERR_PRODUCER)) {
+          if (g >= NSTAGE && !mbar_wait(empty0 + 8 * s, lap, err, ERR_PRODUCER)) {
             ok = false;
             break;
           }
@@ -442,6 +447,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             bulk_load(st, a + (size_t)kb * A_STAGE, A_STAGE, fb);
           }
           bulk_load(st + A_STAGE, b + (size_t)kb * B_STAGE, B_STAGE, fb);
+          if (++s == NSTAGE) s = 0, lap ^= 1;
         }
       }
       progress[0] = g > ahead ? g : ahead;
@@ -453,8 +459,11 @@ __global__ void __launch_bounds__(THREADS, 1)
       cluster_wait();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      int g = 0, u = 0;
+    if (elect_one()) {
+      const uint64_t a0 = operand_desc(smem_u32(smem), BM / 8 * 128);
+      const uint64_t b0 = operand_desc(smem_u32(smem) + A_STAGE, DIGITS * BN / 8 * 128);
+      int g = 0, u = 0, s = 0;
+      uint32_t lap = 0;
       bool ok = true;
       for (int t = tile0; t < n_tiles && ok; t += tile_step) {
         const int nk = k_end(tiles[t].w);
@@ -468,21 +477,20 @@ __global__ void __launch_bounds__(THREADS, 1)
           const uint32_t d = tmem + set * SET;
           const int k1 = min(nk, k0 + CHUNK);
           for (int kb = k0; kb < k1; ++kb, ++g) {
-            const int s = g % NSTAGE, use = g / NSTAGE;
-            if (!mbar_wait(full0 + 8 * s, use & 1, err, ERR_MMA)) {
+            if (!mbar_wait(full0 + 8 * s, lap, err, ERR_MMA)) {
               ok = false;
               break;
             }
             tc_fence_after();
-            const uint32_t st = smem_u32(smem + s * STAGE_BYTES);
-            const uint64_t a = operand_desc(st, BM / 8 * 128);
-            const uint64_t b = operand_desc(st + A_STAGE, DIGITS * BN / 8 * 128);
+            const uint64_t a = a0 + static_cast<uint32_t>(s * (STAGE_BYTES >> 4));
+            const uint64_t b = b0 + static_cast<uint32_t>(s * (STAGE_BYTES >> 4));
             // plane 0 of A against all planes of B also starts every accumulator
 #pragma unroll
             for (int i = 0; i < DIGITS; ++i)
               umma_f16(d + i * BN, a + (i * BM * BK * 2 >> 4), b, idesc_f16((DIGITS - i) * BN),
                        i > 0 || kb > k0 ? 1u : 0u);
             umma_commit(empty0 + 8 * s);
+            if (++s == NSTAGE) s = 0, lap ^= 1;
           }
           if (ok) umma_commit(acc_full + 8 * set);
         }

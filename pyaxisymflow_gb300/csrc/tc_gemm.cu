@@ -11,6 +11,7 @@
 namespace axi_tc {
 namespace {
 
+using axi_tma::elect_one;
 using axi_tma::globaltimer;
 using axi_tma::mbar_expect_tx;
 using axi_tma::mbar_init;
@@ -155,10 +156,11 @@ __global__ void __launch_bounds__(THREADS, 1)
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- TMA producer: one continuous ring over all tiles of this CTA ----
       axi::pdl_wait();
-      int g = 0;
+      int g = 0, s = 0;
+      uint32_t lap = 1;  // parity of the phase that frees a stage
       bool ok = true;
       for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
         const int4 tr = tiles[t];
@@ -173,8 +175,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           prefetch_tensormap(&nj.b_lo);
         }
         for (int kb = 0; kb < nk; ++kb, ++g) {
-          const int s = g % NSTAGE, use = g / NSTAGE;
-          if (use > 0 && !mbar_wait(empty0 + 8 * s, (use - 1) & 1, err, ERR_PRODUCER)) {
+          if (g >= NSTAGE && !mbar_wait(empty0 + 8 * s, lap, err, ERR_PRODUCER)) {
             ok = false;
             break;
           }
@@ -186,16 +187,21 @@ __global__ void __launch_bounds__(THREADS, 1)
           tma_load_2d(st + A_BYTES, &job.a_lo, kx, tr.y, fb);
           tma_load_2d(st + 2 * A_BYTES, &job.b_hi, kx, tr.z, fb);
           tma_load_2d(st + 2 * A_BYTES + B_BYTES, &job.b_lo, kx, tr.z, fb);
+          if (++s == NSTAGE) s = 0, lap ^= 1;
         }
       }
       progress[0] = g;
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---- MMA issuer ----
+    if (elect_one()) {
+      // ---- MMA issuer: its own instructions bound the main loop (the tensor
+      // pipe takes 48 or 64 cycles for an MMA of 64 or 128 columns), so
+      // descriptors and ring position are carried, not formed per stage ----
       constexpr uint32_t idesc = idesc_tf32(BM, BN);
-      int g = 0, it = 0;
+      const uint64_t desc0 = sw_desc(smem_u32(smem));
+      int g = 0, it = 0, s = 0;
+      uint32_t lap = 0;
       bool ok = true;
       // k-block count of the next tile, loaded one tile ahead (its latency
       // would otherwise sit between two tiles' MMAs)
@@ -208,16 +214,15 @@ __global__ void __launch_bounds__(THREADS, 1)
         tc_fence_after();
         const uint32_t d = tmem + buf * BN;
         for (int kb = 0; kb < nk; ++kb, ++g) {
-          const int s = g % NSTAGE, use = g / NSTAGE;
-          if (!mbar_wait(full0 + 8 * s, use & 1, err, ERR_MMA)) {
+          if (!mbar_wait(full0 + 8 * s, lap, err, ERR_MMA)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t st = smem_u32(smem + s * STAGE_BYTES);
-          const uint64_t ah = sw_desc(st), al = sw_desc(st + A_BYTES);
-          const uint64_t bh = sw_desc(st + 2 * A_BYTES);
-          const uint64_t bl = sw_desc(st + 2 * A_BYTES + B_BYTES);
+          const uint64_t ah = desc0 + static_cast<uint32_t>(s * (STAGE_BYTES >> 4));
+          const uint64_t al = ah + (A_BYTES >> 4);
+          const uint64_t bh = ah + (2 * A_BYTES >> 4);
+          const uint64_t bl = ah + ((2 * A_BYTES + B_BYTES) >> 4);
 #pragma unroll
           for (int kk = 0; kk < BKF / 8; ++kk) {
             const uint64_t o = static_cast<uint64_t>(kk * 32) >> 4;  // 8 TF32 = 32 bytes
@@ -226,6 +231,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             umma_tf32(d, al + o, bh + o, idesc, 1u);
           }
           umma_commit(empty0 + 8 * s);
+          if (++s == NSTAGE) s = 0, lap ^= 1;
         }
         if (ok) umma_commit(accf0 + 8 * buf);
       }

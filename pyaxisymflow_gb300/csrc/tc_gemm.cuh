@@ -43,10 +43,12 @@ constexpr int BM = 128;
 // (choose_cols): a narrow tile's stage takes less time, and its result,
 // summed in the same order, is the same. Measured alternatives to the stage,
 // both slower on the spectral products: 16-float stages with a 6-deep ring
-// (64-byte swizzle; twice the barrier and copy count per FLOP: 8 tiles of
-// K = 512 per CTA take 107 us against 92 us, so the main loop pays a fixed
-// cost per stage rather than waiting on the ring) and 128 x 256 tiles with two
-// 96 KB stages (the ring too shallow to cover the operand loads).
+// (64-byte swizzle; twice the barriers and copies per FLOP) and 128 x 256 tiles
+// with two 96 KB stages (the ring too shallow to cover the operand loads).
+// A stage takes 768 cycles at 128 columns (12 MMAs at the tensor rate) and 670
+// at 64 (the issuing thread; 576 for the MMAs, bound by the reads of A), 1044
+// for both before the issuer ran under elect.sync. Products of 512 x 256,
+// 768 x 384 and 1024 x 512 cases together 12.1 / 14.6 -> 9.3 / 12.0 us.
 constexpr int BKF = 32;                         // K floats per stage
 constexpr int ROW_BYTES = BKF * 4;              // swizzle span of a tile row
 constexpr int EPI_WARPS = 8;                    // two per TMEM lane quarter
