@@ -345,7 +345,7 @@ constexpr int smem_bytes(int bn, int split) {
 // tile and up to 128 of its K; the integer sums run on over the units of a tile.
 //
 // Bound by shared memory: an MMA of N columns takes the larger of N / 2 cycles
-// (the tensor rate) and 32 + N / 4 (its operands at 128 bytes per cycle), 660 a
+// (the tensor rate) and 32 + N / 4 (its operands at 128 bytes per cycle), 624 a
 // step of 16 K with BN = 32, into which the copies of the next steps write
 // another 40 KB. The issuing thread took 844 a step until it ran under
 // elect.sync; the four products of 512 x 256 then went from 61.6 to 52.2 us and
