@@ -16,11 +16,10 @@
 //   vel_max      persistent, per tile: max(|u_z| + |u_r|) into the case
 //   step_dt      one thread per case: dt and the dt-dependent constants
 //   penalise     per tile: velocity + Brinkman + omega + curl(u_pen - u)
-//                into the staging half of the work buffer, drag partials;
-//                the last tile of a case finalises the drag
+//                into the staging half of the work buffer, drag partials
 //   advect_diffuse per tile: ENO3 advection (axis mirror) and both RK2
 //                stages in shared memory (halo 4) from the staged omega
-//                into omega; advances the time
+//                into omega; forms the drag and advances the time
 //                (sedimenting cases: mask rebuild, drag, body ODE)
 // The stencil kernels receive their halo boxes by TMA.
 //
@@ -465,13 +464,15 @@ __device__ __forceinline__ double block_sum(const double* red) {
   for (int o = NT / 64; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   return x;
 }
-// Sum of a case's tile partials, by the lanes of warp 0 in a fixed order (all
-// lanes get it). One thread adding them one after the other held up the end of
+// Sum of those of a case's tile partials that are taken, by the lanes of a warp in
+// a fixed order (all lanes get it). One thread adding them one after the other held up the end of
 // the kernel: 64 cycles each, 256 of them on a 1024 x 512 case.
-__device__ __forceinline__ double partial_sum(const double* partials, unsigned int n) {
+template <typename Taken>
+__device__ __forceinline__ double partial_sum(const double* partials, unsigned int n, Taken taken) {
   const int lane = threadIdx.x & 31;
   double x = 0.0;
   for (unsigned int q = lane; q < n; q += 32) {
+    if (!taken((int)q)) continue;
     const double v = ((const volatile double*)partials)[q];
     if (nonzero_bits(v)) x += v;
   }
@@ -879,46 +880,14 @@ __global__ void __launch_bounds__(NT, penalise_min_blocks<T, PAIR>()) penalise_k
         zc = zn;
       }
     }
-    // drag: thread sums in T, then warps, tiles and cases in double, fixed order
+    // drag: thread sums in T, then warps and tiles in double, fixed order; the
+    // case's sum is formed by advect_diffuse (finish_drag)
     const double x = warp_sum(cd_part);
     if ((threadIdx.x & 31) == 0) red[it & 1][threadIdx.x >> 5] = x;
     __syncthreads();
     if (threadIdx.x < 32) {
-      const unsigned int ntiles = dev_tiles_of(k);
       const double sum = block_sum(red[it & 1]);
-      unsigned int arrived = 0;
-      if (threadIdx.x == 0) {
-        k.partials[tr.w] = sum;
-        __threadfence();
-        arrived = atomicAdd(counter(k, 1), 1u);
-      }
-      arrived = __shfl_sync(0xffffffffu, arrived, 0);
-      double tot = 0.0;
-      if (arrived == ntiles - 1) {
-        __threadfence();
-        tot = partial_sum(k.partials, ntiles);
-      }
-      if (threadIdx.x == 0 && arrived == ntiles - 1) {
-        const double dt = k.state[AXI_ST_DT];
-        if (!(tot == tot) || !(fabs(tot) <= 1.7976931348623157e308))
-          atomicOr(reinterpret_cast<unsigned int*>(&k.state[AXI_ST_STATUS]),
-                   1u << AXI_ERR_NONFINITE);
-        k.state[AXI_ST_FORCE] = tot;
-        if (k.flags & AXI_CASE_SEDIMENTING) {
-          // compute_forces.py:14-15 and falling_rigid_sphere.py:155
-          const double f_pen = k.rho_f * k.lam * tot;
-          const double f_un = (k.state[AXI_ST_DIFF] * k.part_vol) / dt;
-          k.state[AXI_ST_FTOTAL] = 2.0 * kPi * k.dx * k.dx * f_pen + f_un;
-        } else {
-          const double cd = k.cd_scale * tot;
-          const long long step = (long long)k.state[AXI_ST_STEPS];
-          if (k.history && step < k.history_len) {
-            k.history[2 * step] = dt;
-            k.history[2 * step + 1] = cd;
-          }
-          k.state[AXI_ST_CD] = cd;
-        }
-      }
+      if (threadIdx.x == 0) k.partials[tr.w] = sum;
     }
   }
   if (!ok && threadIdx.x == 0) ring.drain(it, issued, err);
@@ -1137,6 +1106,57 @@ __device__ __forceinline__ T advect_point(const T* sw, const T* sz, const T* sr,
   return f0 + flux;
 }
 
+// The penalisation force of a case from the tile sums that penalise left, by
+// one warp of the case's first tile while its boxes arrive. The kernel boundary
+// orders them: with an arrival count in penalise each of its blocks ended with
+// a fence and an atomic, two memory round trips in which it held its shared
+// memory.
+__device__ __forceinline__ void finish_drag(const axi_case& k) {
+  const double tot = partial_sum(k.partials, dev_tiles_of(k), [](int) { return true; });
+  if ((threadIdx.x & 31) != 0) return;
+  const double dt = k.state[AXI_ST_DT];
+  if (!(tot == tot) || !(fabs(tot) <= 1.7976931348623157e308))
+    atomicOr(reinterpret_cast<unsigned int*>(&k.state[AXI_ST_STATUS]), 1u << AXI_ERR_NONFINITE);
+  k.state[AXI_ST_FORCE] = tot;
+  if (k.flags & AXI_CASE_SEDIMENTING) {
+    // compute_forces.py:14-15 and falling_rigid_sphere.py:155
+    const double f_pen = k.rho_f * k.lam * tot;
+    const double f_un = (k.state[AXI_ST_DIFF] * k.part_vol) / dt;
+    k.state[AXI_ST_FTOTAL] = 2.0 * kPi * k.dx * k.dx * f_pen + f_un;
+  } else {
+    const double cd = k.cd_scale * tot;
+    const long long step = (long long)k.state[AXI_ST_STEPS];
+    if (k.history && step < k.history_len) {
+      k.history[2 * step] = dt;
+      k.history[2 * step + 1] = cd;
+    }
+    k.state[AXI_ST_CD] = cd;
+  }
+}
+
+// Float engine: whether the moving body's mask can be nonzero in a tile, from
+// the centre column, radius and blend width in cells that kill_reset left (the
+// same for every block of the step). A tile farther than R + 2 W from the body
+// centre (z_cm, 0) has mask 0 at every cell (phi < -w) and adds nothing to the
+// drag.
+__device__ __forceinline__ bool near_body(const axi_case& k, int i0, int j0) {
+  const float sc = scalar<float>(k, SF_S_HI);
+  const float zlo = (float)j0 + 0.5f, zhi = (float)(min(j0 + TX, k.nz) - 1) + 0.5f;
+  const float dz = sc < zlo ? zlo - sc : (sc > zhi ? sc - zhi : 0.0f);
+  const float rlo = (float)i0 + 0.5f;
+  const float reach = scalar<float>(k, SF_R_HI) + 2.0f * scalar<float>(k, SF_W) + 1.0f;
+  return dz * dz + rlo * rlo <= reach * reach;
+}
+// Tiles (numbered along z first) that take part in the closing drag sum: those
+// near the body and the first; in the double engine, whose mask reads the body
+// position that the sum moves, all of them.
+template <typename T>
+__device__ __forceinline__ bool sums_drag(const axi_case& k, int tile) {
+  if (sizeof(T) == 8 || tile == 0) return true;
+  const int per_row = (k.nz + TX - 1) / TX;
+  return near_body(k, tile / per_row * TY, tile % per_row * TX);
+}
+
 // FP32: 4 resident blocks per SM (up to 64 registers; at 5 blocks the
 // pairwise flux divergence spilled and ran 5 % slower)
 template <typename T>
@@ -1190,6 +1210,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 2) advect_diffuse_ker
       rowf[1][threadIdx.x] = rinv2[gi];
       rowf[2][threadIdx.x] = CF<T>(k.rw)[gi];
     }
+    if (tr.w == 0 && threadIdx.x >= NT - 32) finish_drag(k);
     if (!ring.wait_all(it, err)) {
       ok = false;
       break;
@@ -1377,6 +1398,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 2) advect_diffuse_ker
     // ---- RK2 stage 2 on the tile (rows 0..TY-1, columns 0..TX-1)
     const bool sediment = (k.flags & AXI_CASE_SEDIMENTING) != 0;
     T cd_part = T(0);
+    bool near;
     {
       // output pointers in registers (stores through pointers read from the
       // case record would force the record to be re-read after each store)
@@ -1384,10 +1406,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 2) advect_diffuse_ker
       float* const whi = static_cast<float*>(k.omega_hi);
       float* const wlo = static_cast<float*>(k.omega_lo);
       T* const chi = F<T>(k.chi);
-      // a tile farther than radius + 2 w from the body centre (z_cm, 0) has
-      // mask 0 at every cell (phi < -w) and adds nothing to the drag: the
-      // per-cell mask is skipped there (the same values)
-      bool near = sediment;
+      // where the mask is 0 at every cell it is not evaluated (the same values)
+      near = sediment;
       T zc = T(0), rbody = T(0), blendw = T(0), zcol = T(0);
       if constexpr (sizeof(T) == 8) {
         zc = scalar<T>(k, SF_ZCM);
@@ -1403,13 +1423,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 2) advect_diffuse_ker
           near = dz * dz + rlo * rlo <= reach * reach;
         }
       } else if (sediment) {
-        // in cells: centre column S, radius R, blend W
-        const float sc = scalar<T>(k, SF_S_HI);
-        const float zlo = (float)j0 + 0.5f, zhi = (float)(min(j0 + TX, nz) - 1) + 0.5f;
-        const float dz = sc < zlo ? zlo - sc : (sc > zhi ? sc - zhi : 0.0f);
-        const float rlo = (float)i0 + 0.5f;
-        const float reach = scalar<T>(k, SF_R_HI) + 2.0f * scalar<T>(k, SF_W) + 1.0f;
-        near = dz * dz + rlo * rlo <= reach * reach;
+        near = near_body(k, i0, j0);
       }
       const bool jin = gjm < nz, jint = gjm >= 1 && gjm < nz - 1;
       const int p0 = AD_RC * grp;
@@ -1462,7 +1476,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 2) advect_diffuse_ker
         c_ = n_;
       }
     }
-    if (sediment) {
+    const bool sums = sediment && (sizeof(T) == 8 || near || tr.w == 0);
+    if (sums) {
       const double x = warp_sum(cd_part);
       if ((threadIdx.x & 31) == 0) red[it & 1][threadIdx.x >> 5] = x;
     }
@@ -1476,6 +1491,9 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 2) advect_diffuse_ker
       }
       continue;
     }
+    // only the tiles that can hold a part of the sum arrive: the others end
+    // without a fence and an atomic
+    if (!sums) continue;
     const unsigned int ntiles = dev_tiles_of(k);
     const double sum = block_sum(red[it & 1]);
     unsigned int arrived = 0;
@@ -1485,14 +1503,18 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 2) advect_diffuse_ker
       arrived = atomicAdd(counter(k, 1), 1u);
     }
     arrived = __shfl_sync(0xffffffffu, arrived, 0);
-    if (arrived != 2 * ntiles - 1) continue;
+    unsigned int expected = 0;
+    for (unsigned int q = 0; q < ntiles; q += 32)
+      expected += __popc(__ballot_sync(0xffffffffu, q + lane < ntiles && sums_drag<T>(k, q + lane)));
+    if (arrived != expected - 1) continue;
     __threadfence();
-    const double tot = partial_sum(k.partials + ntiles, ntiles);
+    const double tot =
+        partial_sum(k.partials + ntiles, ntiles, [&](int q) { return sums_drag<T>(k, q); });
     if (threadIdx.x != 0) continue;
     const double cd = k.cd_scale * tot;
     const double dt = k.state[AXI_ST_DT];
     // body ODE, falling_rigid_sphere.py:176-181 (FP64)
-    const double ft = k.state[AXI_ST_FTOTAL];
+    const double ft = *(const volatile double*)&k.state[AXI_ST_FTOTAL];  // another block's
     const double u_old = k.state[AXI_ST_UBODY];
     const double acc = -k.grav / k.rho_s + ft / k.part_mass;
     k.state[AXI_ST_UBODY] = u_old + dt * (-k.grav + ft / k.part_mass);

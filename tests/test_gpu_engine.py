@@ -430,3 +430,41 @@ def test_engine_f32_drift_after_2000_steps_on_the_hardest_cases():
                 got = got + fb["psi_lo"].double()
             errs[n] = float(torch.linalg.norm(got - ref) / torch.linalg.norm(ref))
         assert errs["omega"] < 2e-5 and max(errs["psi"], errs["u_z"], errs["u_r"]) < 1e-5, errs
+
+
+@pytest.mark.parametrize("z_cm", [0.02, 1.0, 1.98, 3.0])
+def test_engine_f32_drag_sum_over_near_tiles(z_cm):
+    """The closing drag sum of a sedimenting float case takes the tiles near the
+    body and the first tile only, and the last of them closes the step: body
+    over the first tile, inside, over the last tile and outside the domain,
+    against the sum over every cell of the mask and velocity that the step
+    left. The factor between the two comes from the double engine, which sums
+    every tile."""
+    from pyaxisymflow_gb300.engine import (ST_CD, ST_STEPS, ST_T, ST_ZCM, RigidBodyCase,
+                                           RigidEnsemble)
+    nz, nr = 256, 100
+    w0 = 1e-2 * np.random.default_rng(3).standard_normal((nr, nz))
+    got = {}
+    for precision in ("f64", "f32"):
+        c = RigidBodyCase(nz=nz, nr=nr, dx=2.0 / nz, r_sphere=0.2, z_cm=z_cm, U0=0.0, ramp=False,
+                          sediment=True, rho_s=2.0)
+        e = RigidEnsemble([c], precision=precision, initial_vorticity=[w0])
+        e.step(3)
+        torch.cuda.synchronize()
+        # a body without a cell in the domain has no mass: its force is flagged,
+        # and the step still closes
+        assert (e.status()[0] == 0) == (z_cm < 2.5)
+        s = e.state[0].cpu().numpy()
+        r = (np.arange(nr) + 0.5)[:, None] * c.dx
+        t = r * e.fields[0]["chi"].double().cpu().numpy() * \
+            e.fields[0]["u_z"].double().cpu().numpy()
+        assert s[ST_STEPS] == 3 and s[ST_T] > 0 and s[ST_ZCM] != z_cm
+        if z_cm > 2.5:
+            continue
+        got[precision] = s[ST_CD], t.sum(), np.abs(t).sum()
+    if z_cm > 2.5:
+        return
+    cd, total, _ = got["f64"]
+    cd32, total32, abs32 = got["f32"]
+    # float products and thread sums of 8 cells: (8 + 3) 2^-24 of the terms
+    assert abs(cd32 - cd / total * total32) <= abs(cd / total) * abs32 * 11 * 2.0 ** -24
