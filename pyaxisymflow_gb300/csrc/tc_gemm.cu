@@ -107,6 +107,22 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// The pair of a tile into L2 (64 cases' second radial products 123 -> 118 us):
+// thread e of the epilogue takes half a row.
+template <int BN>
+__device__ __forceinline__ void prefetch_pair(const TcJob& job, int m0, int n0) {
+  const int e = threadIdx.x - 64;
+  const int row = m0 + (e >> 1), col = n0 + (e & 1) * (BN / 2);
+  if (row >= job.M || col >= job.N) return;
+  const float* h = job.c + (long long)row * job.ldc + col;
+  const float* l = job.c_lo + (long long)row * job.ldc + col;
+#pragma unroll
+  for (int q = 0; q < BN / 2 && col + q < job.N; q += 32) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(h + q));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(l + q));
+  }
+}
+
 // Persistent, warp-specialised kernel (one CTA per SM, tiles strided over the
 // grid): warp 0 issues TMA, warp 1 issues MMAs into one of two TMEM
 // accumulators (2 x BN columns), warps 2-9 drain the other accumulator, so
@@ -248,6 +264,10 @@ __global__ void __launch_bounds__(THREADS, 1)
     constexpr int CHUNKS = BN / 32 / 2;  // 32-column chunks per warp
     axi::pdl_wait();
     float* stg = stage_out + (warp - 2) * 32 * 33;
+    if (blockIdx.x < n_tiles) {
+      const int4 tr = tiles[blockIdx.x];
+      if (jobs[tr.x].mode == MODE_PAIR_ADD) prefetch_pair<BN>(jobs[tr.x], tr.y, tr.z);
+    }
     int it = 0;
     for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++it) {
       const int4 tr = tiles[t];
