@@ -414,48 +414,84 @@ struct DifPerm {
   }
 };
 
-// Sub-transform of length L at offset OFF of the register array v (size TOT);
-// tw: exp(-2 pi i m / NT), m < NT, in shared memory at reg_tw_index(m).
-template <int TOT, int L, int OFF, int NT, bool FWD>
-__device__ __forceinline__ void dif_rec(float2 (&v)[TOT], const float2* tw) {
+// exp(-2 pi i m / L), 0 <= m < L, at compile time, with the bits of the table
+// that the other passes read (engine.py dct_table: cosine and sine of the angle
+// rounded to double): the angle brought into the first octant as a fraction,
+// then the Taylor series in double (error below 1e-16), rounded once.
+struct Twiddle {
+  float c, s;
+};
+constexpr double series(double x, int first) {
+  double term = first ? x : 1.0, sum = term;
+  for (int k = first + 1; k < 24 && (term > 1e-30 || term < -1e-30); k += 2) {
+    term *= -x * x / (k * (k + 1));
+    sum += term;
+  }
+  return sum;
+}
+constexpr Twiddle twiddle(int m, int L) {
+  const int oct = 8 * m / L;                    // octant of the angle
+  const int q = (oct + 1) / 2;                  // nearest quarter turn
+  // within pi / 4 of it; the double nearest pi / 2 is 6.1e-17 short
+  const double x = 6.283185307179586 * (4 * m - q * L) / (4.0 * L) - q * 6.123233995736766e-17;
+  const double c = series(x, 0), s = series(x, 1);
+  switch (q & 3) {
+    case 0: return {(float)c, (float)-s};
+    case 1: return {(float)-s, (float)-c};
+    case 2: return {(float)-c, (float)s};
+    default: return {(float)s, (float)c};
+  }
+}
+// a times exp(-+ 2 pi i M / L). The fused forms are written out, so that the
+// rounding does not depend on how the compiler folds the constants.
+template <int M, int L, bool FWD>
+__device__ __forceinline__ float2 mul_twiddle(float2 a) {
+  if constexpr (M == 0) return a;
+  constexpr Twiddle w = twiddle(M, L);
+  constexpr float c = w.c, s = FWD ? w.s : -w.s;
+  const float re = __fmaf_rn(a.x, c, -__fmul_rn(a.y, s));
+  if constexpr (FWD && L % 3 == 0) return make_float2(re, __fmaf_rn(a.x, s, __fmul_rn(a.y, c)));
+  return make_float2(re, __fmaf_rn(a.y, c, __fmul_rn(a.x, s)));
+}
+
+// Sub-transform of length L at offset OFF of the register array v (size TOT).
+// Its twiddles are compile-time constants: read from the table in shared
+// memory they cost a load each and its latency (49 for 32 points).
+template <int TOT, int L, int OFF, bool FWD>
+__device__ __forceinline__ void dif_rec(float2 (&v)[TOT]);
+template <int TOT, int L, int OFF, bool FWD, int J>
+__device__ __forceinline__ void dif_butterflies(float2 (&v)[TOT]) {
+  constexpr int R = dif_radix(L);
+  constexpr int L1 = L / R;
+  if constexpr (J < L1) {
+    const float2 a0 = v[OFF + J], a1 = v[OFF + J + L1];
+    if constexpr (R == 2) {
+      v[OFF + J] = cadd(a0, a1);
+      v[OFF + J + L1] = mul_twiddle<J, L, FWD>(csub(a0, a1));
+    } else {
+      const float h = 0.86602540378443864676f;
+      const float2 a2 = v[OFF + J + 2 * L1];
+      const float2 t1 = cadd(a1, a2), t2 = csub(a1, a2);
+      const float2 m = make_float2(a0.x - 0.5f * t1.x, a0.y - 0.5f * t1.y);
+      const float2 r = FWD ? make_float2(h * t2.y, -h * t2.x) : make_float2(-h * t2.y, h * t2.x);
+      v[OFF + J] = cadd(a0, t1);
+      v[OFF + J + L1] = mul_twiddle<J, L, FWD>(cadd(m, r));
+      v[OFF + J + 2 * L1] = mul_twiddle<2 * J, L, FWD>(csub(m, r));
+    }
+    dif_butterflies<TOT, L, OFF, FWD, J + 1>(v);
+  }
+}
+template <int TOT, int L, int OFF, bool FWD>
+__device__ __forceinline__ void dif_rec(float2 (&v)[TOT]) {
   if constexpr (L > 1) {
     constexpr int R = dif_radix(L);
     constexpr int L1 = L / R;
-#pragma unroll
-    for (int j = 0; j < L1; ++j) {
-      float2 o[R];
-      if constexpr (R == 2) {
-        const float2 a0 = v[OFF + j], a1 = v[OFF + j + L1];
-        o[0] = cadd(a0, a1);
-        o[1] = csub(a0, a1);
-      } else {
-        const float h = 0.86602540378443864676f;
-        const float2 a0 = v[OFF + j], a1 = v[OFF + j + L1], a2 = v[OFF + j + 2 * L1];
-        const float2 t1 = cadd(a1, a2), t2 = csub(a1, a2);
-        const float2 m = make_float2(a0.x - 0.5f * t1.x, a0.y - 0.5f * t1.y);
-        const float2 r = FWD ? make_float2(h * t2.y, -h * t2.x) : make_float2(-h * t2.y, h * t2.x);
-        o[0] = cadd(a0, t1);
-        o[1] = cadd(m, r);
-        o[2] = csub(m, r);
-      }
-      v[OFF + j] = o[0];
-#pragma unroll
-      for (int q = 1; q < R; ++q) {
-        if (j == 0) {
-          v[OFF + j + q * L1] = o[q];
-        } else {
-          float2 w = tw[reg_tw_index(j * q * (NT / L))];
-          if (!FWD) w = conj2(w);
-          v[OFF + j + q * L1] = cmul(o[q], w);
-        }
-      }
-    }
-    dif_rec<TOT, L1, OFF, NT, FWD>(v, tw);
-    dif_rec<TOT, L1, OFF + L1, NT, FWD>(v, tw);
-    if constexpr (R == 3) dif_rec<TOT, L1, OFF + 2 * L1, NT, FWD>(v, tw);
+    dif_butterflies<TOT, L, OFF, FWD, 0>(v);
+    dif_rec<TOT, L1, OFF, FWD>(v);
+    dif_rec<TOT, L1, OFF + L1, FWD>(v);
+    if constexpr (R == 3) dif_rec<TOT, L1, OFF + 2 * L1, FWD>(v);
   }
 }
-
 // Four-step FFT of one complex row of length N = N1 x N2 held by one warp in
 // `buf` (N + N1 complex values): input in natural order, output in natural
 // order (in buf[0, N)). x[N2 n1 + n2] -> X[k1 + N1 k2]. With N1, N2 <= 32
@@ -468,13 +504,50 @@ __device__ __forceinline__ void warp_fft(float2* buf, const float2* tw, int lane
   static_assert(N1 <= 32 && N2 <= 32 && N1 * N2 == N, "four-step split");
   constexpr DifPerm<N1> perm1{};
   constexpr DifPerm<N2> perm2{};
+  if constexpr (N1 == N2 && N1 > 16) {
+    // Both passes by the same code. Each warp runs through it once per item,
+    // so the transform is bound by instruction fetch (the largest stall beside
+    // its loads), and half the code is fetched in less time. With the constant
+    // twiddles: the two transforms of 64 cases 146 / 99 -> 145 / 95 us alone; in
+    // steps whose groups overlap, 719 -> 711 us for 64 cases and 129 -> 121 us
+    // for five. (At 16 points a pass is short and the loop costs more.)
+    const float2* rd = buf + lane;
+    int rs = N2, ws = P;
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+      float2 v[N1];
+      if (lane < N1) {
+#pragma unroll
+        for (int n = 0; n < N1; ++n) v[n] = rd[n * rs];
+        dif_rec<N1, N1, 0, FWD>(v);
+      }
+      __syncwarp();
+      if (lane < N1) {
+        if (pass == 0) {
+#pragma unroll
+          for (int p = 1; p < N1; ++p) {
+            float2 w = tw[reg_tw_index(lane * perm1.v[p])];
+            if (!FWD) w = conj2(w);
+            v[p] = lane == 0 ? v[p] : cmul(v[p], w);
+          }
+        }
+#pragma unroll
+        for (int p = 0; p < N1; ++p) buf[lane + perm1.v[p] * ws] = v[p];
+      }
+      __syncwarp();
+      rd = buf + lane * P;
+      rs = 1;
+      ws = N1;
+    }
+    return;
+  }
   // pass 1: the length-N1 transform over n1 for n2 = lane
   const int n2 = lane;
   float2 v[N1];
   if (n2 < N2) {
 #pragma unroll
     for (int n1 = 0; n1 < N1; ++n1) v[n1] = buf[N2 * n1 + n2];
-    dif_rec<N1, N1, 0, N, FWD>(v, tw);
+    dif_rec<N1, N1, 0, FWD>(v);
   }
   __syncwarp();
   if (n2 < N2) {
@@ -494,7 +567,7 @@ __device__ __forceinline__ void warp_fft(float2* buf, const float2* tw, int lane
   if (k1 < N1) {
 #pragma unroll
     for (int m = 0; m < N2; ++m) o[m] = buf[k1 * P + m];
-    dif_rec<N2, N2, 0, N, FWD>(o, tw);
+    dif_rec<N2, N2, 0, FWD>(o);
   }
   __syncwarp();
   if (k1 < N1) {
