@@ -422,7 +422,12 @@ int axi_tc_split_f64(float* hi, float* lo, const double* x, int64_t n, void* str
 int axi_fd_residual_f64(double* res, const double* rhs, const double* psi,
                         const double* row_weight, const double* ar, const double* az, int nr,
                         int nz, double wrap0, double wrap1, void* stream);
-/* y += x and y = x (float -> double), n values. */
+/* The same residual as the TF32 pair of axi_tc_split_f64. */
+int axi_fd_residual_split_f64(float* hi, float* lo, const double* rhs, const double* psi,
+                              const double* row_weight, const double* ar, const double* az,
+                              int nr, int nz, double wrap0, double wrap1, void* stream);
+/* out = y + x, y += x and y = x (float -> double), n values. */
+int axi_sum_f32_to_f64(double* out, const double* y, const float* x, int64_t n, void* stream);
 int axi_add_f32_to_f64(double* y, const float* x, int64_t n, void* stream);
 int axi_widen_f32_to_f64(double* y, const float* x, int64_t n, void* stream);
 

@@ -76,6 +76,8 @@ def _signatures():
         "axi_tc_split_f32": (I, [P, P, P, I64, P]),
         "axi_tc_split_f64": (I, [P, P, P, I64, P]),
         "axi_fd_residual_f64": (I, [P, P, P, P, P, P, I, I, D, D, P]),
+        "axi_fd_residual_split_f64": (I, [P, P, P, P, P, P, P, I, I, D, D, P]),
+        "axi_sum_f32_to_f64": (I, [P, P, P, I64, P]),
         "axi_add_f32_to_f64": (I, [P, P, I64, P]),
         "axi_widen_f32_to_f64": (I, [P, P, I64, P]),
         "axi_tf32x3_gemm": (I, [P, P, P, I, I, I, P, P]),

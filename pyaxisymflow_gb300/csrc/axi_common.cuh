@@ -184,6 +184,16 @@ __device__ __forceinline__ bool is_zero_bits(double x) { return (__double_as_lon
 __device__ __forceinline__ int exponent_bits(double x) {
   return (__double2hiint(x) >> 20) & 0x7ff;
 }
+// (double)x without the FP64 pipe, which converts at the FP64 rate: a normal
+// float is the same number with its exponent rebiased.
+static __device__ __noinline__ double widen_plain(float x) { return (double)x; }
+__device__ __forceinline__ double widen(float x) {
+  const unsigned int b = __float_as_uint(x), e = (b >> 23) & 0xffu;
+  if (e - 1u < 254u)
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))),
+                            (int)(b << 29));
+  return (b << 1) == 0 ? __hiloint2double((int)b, 0) : widen_plain(x);
+}
 // x with its sign flipped where `flip` (the compiler negates with an FP64 add)
 __device__ __forceinline__ double flip_sign(double x, bool flip) {
   return __hiloint2double(__double2hiint(x) ^ (flip ? (int)0x80000000 : 0), __double2loint(x));

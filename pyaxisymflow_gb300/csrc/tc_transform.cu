@@ -10,8 +10,8 @@
 //   X (nz, nr) = Ez * Y^T               -> split
 //   out (nr, nz) = Er * X^T             -> plain FP32
 // A refinement step computes the residual rhs - L psi of the discrete
-// operator in FP64 (axi_fd_residual_f64), transforms it, and adds the
-// correction in FP64 (axi_add_f32_to_f64).
+// operator in FP64 (axi_fd_residual_split_f64), transforms it, and adds the
+// correction in FP64 (axi_sum_f32_to_f64).
 #include <cstring>
 #include <string>
 
@@ -27,15 +27,14 @@ __global__ void split_f32_kernel(const float* __restrict__ x, float* __restrict_
 
 // hi = nearest TF32 of fl32(x), lo = nearest TF32 of fl32(x - hi) (remainder
 // taken in double): the split of an FP64 value keeps about 23 significant bits.
+__device__ __forceinline__ void split_f64(double v, float& hi, float& lo) {
+  hi = axi_tc::tf32_round((float)v);
+  lo = axi_tc::tf32_round((float)(v - widen(hi)));
+}
 __global__ void split_f64_kernel(const double* __restrict__ x, float* __restrict__ hi,
                                  float* __restrict__ lo, long long n) {
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) {
-    const double v = x[k];
-    const float h = axi_tc::tf32_round((float)v);
-    hi[k] = h;
-    lo[k] = axi_tc::tf32_round((float)(v - (double)h));
-  }
+  if (k < n) split_f64(x[k], hi[k], lo[k]);
 }
 
 // The transform solves L psi = W rhs (W = diag(w) on rows, folded into its
@@ -44,34 +43,59 @@ __global__ void split_f64_kernel(const double* __restrict__ x, float* __restrict
 // three diagonals of each 1-D operator plus the two periodic wrap entries
 // A_z[0, nz-1] and A_z[nz-1, 0] (the FD matrices of
 // FastDiagonalisationStokesSolver.py:41-97 after the boundary edits).
-__global__ void residual_kernel(double* __restrict__ res, const double* __restrict__ rhs,
-                                const double* __restrict__ psi, const double* __restrict__ w,
-                                const double* __restrict__ ar, const double* __restrict__ zr,
-                                int nr, int nz, double wrap0, double wrap1) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+//
+// Written as the transform's operand pair (hi, lo) where `res` is null. Bound by
+// FP64 issue: 6 instructions for L psi, 5 for the quotient by the row's known
+// divisor and the difference, 3 for the split; 17 + 4 as two kernels that
+// divided in full and ran the wrap terms everywhere (2048 x 1024: 68 + 19 us).
+constexpr int RES_COLS = 4;  // columns per thread (the divisor is formed once per block)
+__device__ __noinline__ double add_wrap(double lp, double wrap, double psi) {
+  return lp + wrap * psi;
+}
+__global__ void __launch_bounds__(256)
+    residual_kernel(double* __restrict__ res, float* __restrict__ hi, float* __restrict__ lo,
+                    const double* __restrict__ rhs, const double* __restrict__ psi,
+                    const double* __restrict__ w, const double* __restrict__ ar,
+                    const double* __restrict__ zr, int nr, int nz, double wrap0, double wrap1) {
+  __shared__ KnownDivisor<double> row_weight;
   const int i = blockIdx.y;
-  if (i >= nr || j >= nz) return;
-  const long long c = (long long)i * nz + j;
+  if (w && threadIdx.x < 32) {
+    const KnownDivisor<double> d(w[i]);
+    if (threadIdx.x == 0) row_weight = d;
+  }
+  __syncthreads();
   // radial diagonals: ar[3 i + 0] (i, i-1), ar[3 i + 1] (i, i), ar[3 i + 2] (i, i+1)
-  double lp = ar[3 * i + 1] * psi[c];
-  if (i > 0) lp += ar[3 * i] * psi[c - nz];
-  if (i < nr - 1) lp += ar[3 * i + 2] * psi[c + nz];
-  lp += zr[3 * j + 1] * psi[c];
-  if (j > 0) lp += zr[3 * j] * psi[c - 1];
-  if (j < nz - 1) lp += zr[3 * j + 2] * psi[c + 1];
-  if (j == 0) lp += wrap0 * psi[c + nz - 1];
-  if (j == nz - 1) lp += wrap1 * psi[c - nz + 1];
-  res[c] = w ? rhs[c] - lp / w[i] : rhs[c] - lp;
+  const double as = ar[3 * i], ac = ar[3 * i + 1], an = ar[3 * i + 2];
+#pragma unroll
+  for (int q = 0; q < RES_COLS; ++q) {
+    const int j = (blockIdx.x * RES_COLS + q) * 256 + threadIdx.x;
+    if (j >= nz) break;
+    const long long c = (long long)i * nz + j;
+    double lp = ac * psi[c];
+    if (i > 0) lp += as * psi[c - nz];
+    if (i < nr - 1) lp += an * psi[c + nz];
+    lp += zr[3 * j + 1] * psi[c];
+    if (j > 0) lp += zr[3 * j] * psi[c - 1];
+    if (j < nz - 1) lp += zr[3 * j + 2] * psi[c + 1];
+    if (j == 0) lp = add_wrap(lp, wrap0, psi[c + nz - 1]);
+    if (j == nz - 1) lp = add_wrap(lp, wrap1, psi[c - nz + 1]);
+    const double v = rhs[c] - (w ? row_weight.quotient(lp) : lp);
+    if (res)
+      res[c] = v;
+    else
+      split_f64(v, hi[c], lo[c]);
+  }
 }
 
-__global__ void add_kernel(double* __restrict__ y, const float* __restrict__ x, long long n) {
+__global__ void add_kernel(double* out, const double* y, const float* __restrict__ x,
+                           long long n) {
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) y[k] += (double)x[k];
+  if (k < n) out[k] = y[k] + widen(x[k]);
 }
 
 __global__ void widen_kernel(double* __restrict__ y, const float* __restrict__ x, long long n) {
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) y[k] = (double)x[k];
+  if (k < n) y[k] = widen(x[k]);
 }
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -251,30 +275,56 @@ extern "C" int axi_tc_split_f64(float* hi, float* lo, const double* x, int64_t n
   return axi::launch_status("tc_split_f64");
 }
 
+namespace {
+
+int launch_residual(const char* what, double* res, float* hi, float* lo, const double* rhs,
+                    const double* psi, const double* row_weight, const double* ar,
+                    const double* az, int nr, int nz, double wrap0, double wrap1, void* stream) {
+  AXI_TRY(axi::check_grid(what, nr, nz, 1, 2));
+  if (nr > 65535) {
+    axi::set_error("%s: nr %d too large", what, nr);
+    return AXI_ERR_INVALID;
+  }
+  // row_weight may be null (no weight)
+  AXI_TRY(axi::check_ptrs(what, {rhs, psi, ar, az}, {"rhs", "psi", "op_r", "op_z"}));
+  dim3 grid(axi::ceil_div(nz, 256 * RES_COLS), nr);
+  residual_kernel<<<grid, 256, 0, axi::as_stream(stream)>>>(res, hi, lo, rhs, psi, row_weight, ar,
+                                                            az, nr, nz, wrap0, wrap1);
+  return axi::launch_status(what);
+}
+
+}  // namespace
+
 extern "C" int axi_fd_residual_f64(double* res, const double* rhs, const double* psi,
                                    const double* row_weight, const double* ar, const double* az,
                                    int nr, int nz, double wrap0, double wrap1, void* stream) {
   axi::clear_error();
-  AXI_TRY(axi::check_grid("fd_residual", nr, nz, 1, 2));
-  if (nr > 65535) {
-    axi::set_error("fd_residual: nr %d too large", nr);
-    return AXI_ERR_INVALID;
-  }
-  // row_weight may be null (no weight)
-  AXI_TRY(axi::check_ptrs("fd_residual", {res, rhs, psi, ar, az},
-                          {"residual", "rhs", "psi", "op_r", "op_z"}));
-  dim3 grid(axi::ceil_div(nz, 256), nr);
-  residual_kernel<<<grid, 256, 0, axi::as_stream(stream)>>>(res, rhs, psi, row_weight, ar, az, nr,
-                                                            nz, wrap0, wrap1);
-  return axi::launch_status("fd_residual");
+  AXI_TRY(axi::check_ptr("fd_residual", res, "residual"));
+  return launch_residual("fd_residual", res, nullptr, nullptr, rhs, psi, row_weight, ar, az, nr,
+                         nz, wrap0, wrap1, stream);
+}
+
+extern "C" int axi_fd_residual_split_f64(float* hi, float* lo, const double* rhs,
+                                         const double* psi, const double* row_weight,
+                                         const double* ar, const double* az, int nr, int nz,
+                                         double wrap0, double wrap1, void* stream) {
+  axi::clear_error();
+  AXI_TRY(axi::check_ptrs("fd_residual_split", {hi, lo}, {"hi", "lo"}));
+  return launch_residual("fd_residual_split", nullptr, hi, lo, rhs, psi, row_weight, ar, az, nr,
+                         nz, wrap0, wrap1, stream);
+}
+
+extern "C" int axi_sum_f32_to_f64(double* out, const double* y, const float* x, int64_t n,
+                                  void* stream) {
+  axi::clear_error();
+  if (n <= 0) return AXI_OK;
+  AXI_TRY(axi::check_ptrs("sum_f32_to_f64", {out, y, x}, {"out", "y", "x"}));
+  add_kernel<<<axi::ceil_div(n, 256), 256, 0, axi::as_stream(stream)>>>(out, y, x, n);
+  return axi::launch_status("sum_f32_to_f64");
 }
 
 extern "C" int axi_add_f32_to_f64(double* y, const float* x, int64_t n, void* stream) {
-  axi::clear_error();
-  if (n <= 0) return AXI_OK;
-  AXI_TRY(axi::check_ptrs("add_f32_to_f64", {y, x}, {"y", "x"}));
-  add_kernel<<<axi::ceil_div(n, 256), 256, 0, axi::as_stream(stream)>>>(y, x, n);
-  return axi::launch_status("add_f32_to_f64");
+  return axi_sum_f32_to_f64(y, y, x, n, stream);
 }
 
 extern "C" int axi_widen_f32_to_f64(double* y, const float* x, int64_t n, void* stream) {

@@ -165,7 +165,6 @@ class FastDiagonalisationEngine:
         self.tc_work = [torch.empty(nr * nz, **f32) for _ in range(4)]
         self.tc_out = torch.empty((nr, nz), **f32)
         self.tc_psi = torch.empty((nr, nz), **f64)
-        self.tc_res = torch.empty((nr, nz), **f64)
         self.weight = (torch.tensor(np.ascontiguousarray(row_weight), **f64)
                        if row_weight is not None else None)
         self.op_r = torch.tensor(tridiagonals(op_r), **f64) if op_r is not None else None
@@ -236,14 +235,17 @@ class FastDiagonalisationEngine:
             return
         if self.op_r is None:
             raise ValueError("refinement needs the discrete operator")
-        psi, res = self.tc_psi, self.tc_res
+        psi = self.tc_psi
         N.call("axi_widen_f32_to_f64", N.ptr(psi), N.ptr(self.tc_out), n, s)
         x64 = x if x.dtype == torch.float64 else x.double()
-        for _ in range(self.refine):
-            N.call("axi_fd_residual_f64", N.ptr(res), N.ptr(x64), N.ptr(psi),
+        # the last correction goes straight to a contiguous FP64 result
+        last = out if out.dtype == torch.float64 and out.is_contiguous() else psi
+        for q in range(self.refine):
+            N.call("axi_fd_residual_split_f64", N.ptr(hi), N.ptr(lo), N.ptr(x64), N.ptr(psi),
                    N.ptr(self.weight) if self.weight is not None else None, N.ptr(self.op_r),
                    N.ptr(self.op_z), nr, nz, self.wrap[0], self.wrap[1], s)
-            N.call("axi_tc_split_f64", N.ptr(hi), N.ptr(lo), N.ptr(res), n, s)
             self._tc_run(s)
-            N.call("axi_add_f32_to_f64", N.ptr(psi), N.ptr(self.tc_out), n, s)
-        out.copy_(psi)
+            N.call("axi_sum_f32_to_f64", N.ptr(last if q == self.refine - 1 else psi), N.ptr(psi),
+                   N.ptr(self.tc_out), n, s)
+        if last is not out:
+            out.copy_(psi)

@@ -87,3 +87,39 @@ def test_tensor_core_solve_float32_fields_and_potential():
     refd = w.copy()
     K.ImplicitEulerDiffusionStepper(dt, 1e-2, nr, nz, dx).step(refd, dt)
     assert rel_l2(x.cpu().numpy(), refd) < 1e-8
+
+
+@pytest.mark.parametrize("nr,nz,weight,wrap", [(2, 2, True, False), (3, 1025, True, True),
+                                               (5, 1024, False, True), (4, 260, True, False)])
+def test_residual_pair_at_block_edges(nr, nz, weight, wrap):
+    """The refinement residual as the TF32 pair: the sum of the pair against the
+    residual formed in FP64 on the host, at the edges of the blocks of 4 x 256
+    columns, with and without row weights and the periodic entries."""
+    from pyaxisymflow_gb300 import _native as N
+    rng = np.random.default_rng(nr * nz)
+    psi, rhs = rng.standard_normal((nr, nz)), rng.standard_normal((nr, nz))
+    ar, az = rng.standard_normal((nr, 3)), rng.standard_normal((nz, 3))
+    w = rng.uniform(0.3, 3.0, nr) if weight else np.ones(nr)
+    w0, w1 = (0.7, -1.3) if wrap else (0.0, 0.0)
+    below, above = np.zeros_like(psi), np.zeros_like(psi)
+    below[1:], above[:-1] = psi[:-1], psi[1:]
+    left, right = np.zeros_like(psi), np.zeros_like(psi)
+    left[:, 1:], right[:, :-1] = psi[:, :-1], psi[:, 1:]
+    wl, wr = np.zeros_like(psi), np.zeros_like(psi)
+    wl[:, 0], wr[:, -1] = w0 * psi[:, -1], w1 * psi[:, 0]
+    terms = [ar[:, :1] * below, ar[:, 1:2] * psi, ar[:, 2:] * above, az[None, :, 0] * left,
+             az[None, :, 1] * psi, az[None, :, 2] * right, wl, wr]
+    ref = rhs - sum(terms) / w[:, None]
+    size = np.abs(rhs) + sum(np.abs(t) for t in terms) / w[:, None]
+
+    def dev(a):
+        return torch.tensor(np.ascontiguousarray(a), device="cuda")
+
+    t = [dev(a) for a in (rhs, psi, w, ar, az)]
+    hi, lo = torch.empty(nr, nz, device="cuda"), torch.empty(nr, nz, device="cuda")
+    N.call("axi_fd_residual_split_f64", N.ptr(hi), N.ptr(lo), N.ptr(t[0]), N.ptr(t[1]),
+           N.ptr(t[2]) if weight else None, N.ptr(t[3]), N.ptr(t[4]), nr, nz, w0, w1,
+           N.stream_of(hi))
+    got = (hi.double() + lo.double()).cpu().numpy()
+    # 10 rounded FP64 operations, and a pair that keeps 23 bits of the value
+    assert (np.abs(got - ref) <= 10 * 2.0 ** -53 * size + 2.0 ** -23 * np.abs(ref)).all()
