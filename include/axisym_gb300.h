@@ -228,6 +228,26 @@ int axi_extrapolate_lsq_first_order_f64(int16_t* current_flag, const int16_t* ta
                                         const double* grid_y, int n0, int n1, int max_sweeps,
                                         void* work, int* sweeps_out, void* stream);
 /* ------------------------------------------------------------------
+ * Loop body of a rigid sphere at rest between the solve and the advection
+ * (examples/FlowPastSphere/flow_past_sphere.py:143-175), double.
+ *
+ * axi_sphere_speed_f64: u_z += add (the free stream), *umax (device) =
+ * max(|u_z| + |u_r|) over n cells, NaN if one is.
+ * axi_sphere_penalise_f64: the velocity is kept in old_u_z, old_u_r and
+ * penalised in place (kernels/brinkmann_penalize.py:11-16, body velocity 0);
+ * penal = curl(u - old) on the inner cells, vorticity += penal; *drag (device)
+ * = sum of R chi u_z in a fixed order. `partials`: device scratch of
+ * axi_sphere_penalise_partials(nr, nz) doubles.
+ * ------------------------------------------------------------------ */
+int axi_sphere_speed_f64(double* u_z, const double* u_r, double add, int64_t n, double* umax,
+                         void* stream);
+int64_t axi_sphere_penalise_partials(int nr, int nz);
+int axi_sphere_penalise_f64(double* vorticity, double* penal, double* u_z, double* u_r,
+                            double* old_u_z, double* old_u_r, const double* chi, const double* R,
+                            double lam, double dt, int nr, int nz, double dx, double* partials,
+                            double* drag, void* stream);
+
+/* ------------------------------------------------------------------
  * Particle remeshing (kernels/advect_particle.py:5-68)
  *
  * axi_particles_to_mesh_2d_mp4_f64 replaces the compiled

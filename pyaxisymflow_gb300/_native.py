@@ -45,6 +45,9 @@ def _signatures():
         "axi_last_error": (_c.c_char_p, []),
         "axi_reduction_scratch_doubles": (I64, [I64]),
         "axi_lsq_work_bytes": (I64, [I, I]),
+        "axi_sphere_speed_f64": (I, [P, P, D, I64, P, P]),
+        "axi_sphere_penalise_partials": (I64, [I, I]),
+        "axi_sphere_penalise_f64": (I, [P, P, P, P, P, P, P, P, D, D, I, I, D, P, P, P]),
         "axi_p2m_mp4_work_bytes": (I64, [I, I]),
         "axi_particles_to_mesh_2d_mp4_f64": (I, [P, P, P, P, I, I, D, D, I, P, P]),
         "axi_p2m_status": (I, [P, I, I, P, P]),

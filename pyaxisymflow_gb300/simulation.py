@@ -15,6 +15,7 @@ from dataclasses import dataclass
 import numpy as np
 import torch
 
+from . import _native as N
 from .kernels.advect_vorticity_via_eno3 import gen_advect_vorticity_via_eno3
 from .kernels.brinkmann_penalize import brinkmann_penalize
 from .kernels.compute_velocity_from_psi import compute_velocity_from_psi_unb
@@ -116,6 +117,8 @@ class RigidSphereSimulation:
         self.tmp = torch.zeros_like(self.psi)
         self.solver = FastDiagonalisationStokesSolver(c.nr, c.nz, c.dx, device=dev)
         self.advect = gen_advect_vorticity_via_eno3(c.dx, c.nr, c.nz)
+        self._umax, self._drag = torch.zeros(2, **f64)
+        self._partials = torch.zeros(int(N.lib().axi_sphere_penalise_partials(c.nr, c.nz)), **f64)
         self.t = 0.0
         self.it = 0
         self.dt = 0.0
@@ -132,18 +135,20 @@ class RigidSphereSimulation:
         prefac = 1.0
         if c.ramp and self.t < c.t_ramp:
             prefac = math.sin(0.5 * math.pi * self.t / c.t_ramp)
-        self.u_z += c.U0 * prefac
-        umax = float(torch.amax(torch.abs(self.u_z) + torch.abs(self.u_r)))
+        N.require(w, self.penal, self.u_z, self.u_r, self.u_z_upen, self.u_r_upen, self.char_func,
+                  self.R, shape=(c.nr, c.nz), dtype=torch.float64,
+                  names=("vorticity", "penal", "u_z", "u_r", "u_z_upen", "u_r_upen", "char_func",
+                         "R"))
+        s = N.stream_of(w)
+        N.call("axi_sphere_speed_f64", N.ptr(self.u_z), N.ptr(self.u_r), float(c.U0 * prefac),
+               c.nr * c.nz, N.ptr(self._umax), s)
+        umax = self._umax.item()
         dt = min(0.9 * dx ** 2 / 4 / c.nu, c.cfl * dx / (umax + EPS))
-        self.u_z_upen.copy_(self.u_z)
-        self.u_r_upen.copy_(self.u_r)
-        brinkmann_penalize(c.lam, dt, self.char_func, 0.0, 0.0, self.u_z_upen, self.u_r_upen,
-                           self.u_z, self.u_r)
-        compute_vorticity_from_velocity_unb(self.penal, self.u_z - self.u_z_upen,
-                                            self.u_r - self.u_r_upen, dx)
-        w += self.penal
-        self.Cd = (2 * 2 * math.pi * dx * dx * c.lam
-                   * float(torch.sum(self.R * self.char_func * self.u_z))
+        N.call("axi_sphere_penalise_f64", N.ptr(w), N.ptr(self.penal), N.ptr(self.u_z),
+               N.ptr(self.u_r), N.ptr(self.u_z_upen), N.ptr(self.u_r_upen), N.ptr(self.char_func),
+               N.ptr(self.R), float(c.lam), dt, c.nr, c.nz, float(dx), N.ptr(self._partials),
+               N.ptr(self._drag), s)
+        self.Cd = (2 * 2 * math.pi * dx * dx * c.lam * self._drag.item()
                    / (math.pi * c.r_sphere ** 2))
         self.advect(w, self.u_z, self.u_r, dt)
         diffusion_RK2_unb(w, self.tmp, self.R, c.nu, dt, dx)
@@ -271,7 +276,6 @@ class SoftSphereEngine:
     Extrapolation failures set bits of status() instead of raising."""
 
     def __init__(self, case, device="cuda", dct=False):
-        from . import _native as N
         from .core.extrapolate_using_least_squares import MAX_SWEEPS
         self._N = N
         self.max_sweeps = MAX_SWEEPS

@@ -63,3 +63,47 @@ def test_soft_sphere_loop_against_golden(golden):
         err = rel_l2(t.cpu().numpy(), g[f"soft/{f}_12"])
         assert err < 1e-12, (f, err)
     assert abs(s.t - float(g["soft/t_12"])) <= 1e-13 * float(g["soft/t_12"])
+
+
+@pytest.mark.parametrize("nr,nz", [(3, 3), (33, 31), (5, 1025)])
+def test_sphere_passes_match_the_array_operations(nr, nz):
+    """Free stream, maximum speed, penalisation, its vorticity and the drag sum of
+    the drop-in loop against the same operations on arrays, with a body over part
+    of the grid: the fields and the maximum bit for bit (one rounding per
+    operation on both sides), the sum within n unit roundings of its terms."""
+    from pyaxisymflow_gb300 import _native as N
+    rng = np.random.default_rng(nr * nz)
+    uz, ur, w, penal = (rng.standard_normal((nr, nz)) for _ in range(4))
+    R = np.repeat((np.arange(nr)[:, None] + 0.5) / nr, nz, 1)
+    chi = np.clip(rng.uniform(-2.0, 1.5, (nr, nz)), 0.0, 1.0)
+    chi[:, nz // 2:] = 0.0
+    lam, dt, dx, add = 1e4, 1e-3, 0.01, 0.25
+    dev = {k: torch.tensor(v, device="cuda") for k, v in
+           dict(uz=uz, ur=ur, w=w, penal=penal, R=R, chi=chi, oz=0 * uz, orr=0 * ur).items()}
+    out = torch.zeros(2, dtype=torch.float64, device="cuda")
+    parts = torch.empty(int(N.lib().axi_sphere_penalise_partials(nr, nz)), dtype=torch.float64,
+                        device="cuda")
+    s = N.stream_of(out)
+    N.call("axi_sphere_speed_f64", N.ptr(dev["uz"]), N.ptr(dev["ur"]), add, nr * nz,
+           N.ptr(out[:1]), s)
+    N.call("axi_sphere_penalise_f64", N.ptr(dev["w"]), N.ptr(dev["penal"]), N.ptr(dev["uz"]),
+           N.ptr(dev["ur"]), N.ptr(dev["oz"]), N.ptr(dev["orr"]), N.ptr(dev["chi"]),
+           N.ptr(dev["R"]), lam, dt, nr, nz, dx, N.ptr(parts), N.ptr(out[1:]), s)
+    uz = uz + add
+    umax = (np.abs(uz) + np.abs(ur)).max()
+    lc = lam * dt * chi
+    pz, pr = (uz + lc * 0.0) / (1 + lc), (ur + lc * 0.0) / (1 + lc)
+    dz, dr = pz - uz, pr - ur
+    penal[1:-1, 1:-1] = ((dr[1:-1, 2:] - dr[1:-1, :-2]) / (2 * dx)
+                         - (dz[2:, 1:-1] - dz[:-2, 1:-1]) / (2 * dx))
+    for k, ref in (("uz", pz), ("ur", pr), ("oz", uz), ("orr", ur), ("penal", penal),
+                   ("w", w + penal)):
+        np.testing.assert_array_equal(dev[k].cpu().numpy(), ref, err_msg=k)
+    got = out.cpu().numpy()
+    terms = R * chi * pz
+    assert got[0] == umax
+    assert abs(got[1] - terms.sum()) <= nr * nz * 2.0 ** -52 * np.abs(terms).sum()
+    dev["ur"][0, 0] = float("nan")
+    N.call("axi_sphere_speed_f64", N.ptr(dev["uz"]), N.ptr(dev["ur"]), add, nr * nz,
+           N.ptr(out[:1]), s)
+    assert np.isnan(out[0].item())
