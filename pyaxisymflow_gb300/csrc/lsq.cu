@@ -451,39 +451,45 @@ __global__ void __launch_bounds__(FS_THREADS)
   }
 }
 
-// After `sweeps` fused sweeps: flags back to 0 / 1, any further sweeps in this
-// CTA, and (state given: the soft loop) the outcome folded into its state
+// After `sweeps` fused sweeps: flags back to 0 / 1, any further sweeps in the
+// first block, and (state given: the soft loop) the outcome folded into its state
 // block (the status bit of a failure, sticky, and the largest sweep count
-// seen) and the filled cells of the upper half copied to eta1 and eta2.
+// seen) and the filled cells of the upper half copied to eta1 and eta2. A chain
+// of three loads a candidate: by one block it was 8 us of a 256 x 128 step (204 ->
+// 196 us).
+constexpr int FINISH_BLOCKS = 8;
 __global__ void __launch_bounds__(LSQ_THREADS)
     lsq_finish_kernel(int16_t* cf, const int16_t* tf, double* ex, double* ey, const double* gx,
                       const double* gy, int n0, int n1, int max_sweeps, LsqHeader* hdr,
                       const int* list, int4* front, int sweeps, double* state, double* eta1,
                       double* eta2) {
   const int ncand = hdr->n_candidates;
-  for (int q = threadIdx.x; q < ncand; q += LSQ_THREADS) {
-    const int k = list[q];
-    if (cf[k] > 1) cf[k] = 1;
-  }
   const int fail = hdr->fail;
   const bool more = fail == 0 && *sweep_count(hdr, sweeps - 1) != 0;
-  __syncthreads();
+  if (more && blockIdx.x > 0) return;
+  const int first = blockIdx.x * LSQ_THREADS + threadIdx.x;
+  const int step = more ? LSQ_THREADS : FINISH_BLOCKS * LSQ_THREADS;
+  const int half = n0 / 2 * n1;
+  auto copy_back = [&](int k) {
+    if (!state || k < half) return;
+    eta1[k - half] = ex[k];
+    eta2[k - half] = ey[k];
+  };
+  for (int q = first; q < ncand; q += step) {
+    const int k = list[q];
+    if (cf[k] > 1) cf[k] = 1;
+    if (!more) copy_back(k);
+  }
   if (more) {
+    __syncthreads();
     finish_sweeps(cf, tf, ex, ey, gx, gy, n0, n1, max_sweeps, hdr, list, front);
-  } else if (threadIdx.x == 0) {
+    __syncthreads();
+    for (int q = first; q < ncand; q += step) copy_back(list[q]);
+  } else if (first == 0) {
     hdr->status = fail & 0xff;
     hdr->done = 1;
   }
-  if (!state) return;
-  __syncthreads();
-  const int half = n0 / 2 * n1;
-  for (int q = threadIdx.x; q < ncand; q += LSQ_THREADS) {
-    const int k = list[q];
-    if (k < half) continue;
-    eta1[k - half] = ex[k];
-    eta2[k - half] = ey[k];
-  }
-  if (threadIdx.x != 0) return;
+  if (!state || first != 0) return;
   if (hdr->status != AXI_OK)
     atomicOr(reinterpret_cast<unsigned long long*>(state + AXI_SOFT_STATUS),
              1ull << hdr->status);
@@ -599,7 +605,7 @@ void issue_fused_sweeps(int16_t* cf, const int16_t* tf, double* ex, double* ey, 
   for (int k = 0; k < MB_SWEEPS; ++k)
     lsq_fused_sweep_kernel<<<blocks, FS_THREADS, 0, s>>>(cf, tf, ex, ey, gx, gy, n0, n1,
                                                          max_sweeps, hdr, list, k);
-  lsq_finish_kernel<<<1, LSQ_THREADS, 0, s>>>(cf, tf, ex, ey, gx, gy, n0, n1, max_sweeps, hdr,
+  lsq_finish_kernel<<<FINISH_BLOCKS, LSQ_THREADS, 0, s>>>(cf, tf, ex, ey, gx, gy, n0, n1, max_sweeps, hdr,
                                               list, front, MB_SWEEPS, state, eta1, eta2);
 }
 
