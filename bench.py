@@ -64,8 +64,8 @@ NCU_TRAFFIC = {
     ("ensemble64", "f32", "advect_diffuse"): 295.7e6,
 }
 # remeshing (2048 x 1024 cells, 4.19 M particles): FP64 instructions per
-# particle of the two kernels together (80 + 48) and their DRAM bytes per call
-FP64_INSTR_PER_PARTICLE = 128.0
+# particle of the two kernels together (68 + 48) and their DRAM bytes per call
+FP64_INSTR_PER_PARTICLE = 116.0
 FP64_PEAK_GINSTR = 625.0
 P2M_TRAFFIC = 673.2e6
 
@@ -553,7 +553,7 @@ def run_gb300(args, world, rank, local):
             ms64 = f0.elapsed_time(f1) / nf
             entry = {"value": cells * world / (ms64 / 1000.0), "ms_per_step": ms64,
                      "speedup_fp32_over_fp64": ms64 / ms_per_step,
-                     "z_transform": "FP64 DCT" if dct else "dense FP64 products"}
+                     "z_transform": "cosine basis" if dct else "eigenvectors"}
             if dct:
                 # per-phase device times of the FP64 step, and its stencil passes'
                 # algorithmic bytes (FP64 fields) over their time
@@ -652,9 +652,9 @@ def run_gb300(args, world, rank, local):
         "status_ok": bool(np.all(status == 0)),
     }
     # kill_reset, 4 spectral products (2 transforms + 2 products on the DCT
-    # path), vel_max (which also computes dt), penalise, advect_diffuse; per
-    # plan group
-    n_launch = (1 + 4 + 3) * n_plans
+    # path; in double each a slicing and a product), vel_max (which also
+    # computes dt), penalise, advect_diffuse; per plan group
+    n_launch = (1 + (8 if args.precision == "f64" else 4) + 3) * n_plans
     line["gpu_launches"] = n_launch * args.steps
     line["config"]["plan_groups"] = n_plans
     # ---- continuous-batching serving leg (config 5) ----------------------------
@@ -787,7 +787,7 @@ def run_poisson(args, world, rank, local):
                            "u_r": rel(ur32, ur64), "psi_without_refinement": rel(p0, psi64)},
         "e2e": {"value": cells / e2e_s, "unit": UNIT, "h2d_bytes_per_step": cells * 8,
                 "d2h_bytes_per_step": cells * 8},
-        "gpu_launches": args.steps * (2 + 4 + 4 + 3),
+        "gpu_launches": args.steps * (1 + 4 + 4 + 3),
         "clocks": clocks.summary(),
         "status_ok": s32.engine.tc_status() == 0,
     }
@@ -906,8 +906,8 @@ def run_soft(args, world, rank, local):
         "clocks": clocks.summary(),
         "status_ok": status == 0,
     }
-    # the same loop with the z products of the solve as FP64 DCTs (psi within
-    # ~1e-11 of the dense eigenvector products)
+    # the same loop with the exact cosine eigenvectors in z (psi within ~1e-11
+    # of the products with the computed ones)
     del eng
     torch.cuda.empty_cache()
     eng2 = SoftSphereEngine(case, device=dev, dct=True)
@@ -925,7 +925,7 @@ def run_soft(args, world, rank, local):
     ms2 = d0.elapsed_time(d1) / args.steps
     line["dct_variant"] = {"value": cells * world / (ms2 / 1e3), "ms_per_step": ms2,
                            "speedup_over_dense": ms / ms2, "status_ok": eng2.status() == 0,
-                           "z_transform": "FP64 DCT-II / DCT-III rows, dense radial products"}
+                           "z_transform": "cosine basis"}
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         line["cpu_baseline"] = soft_cpu_record(case, seconds=12.0)
     if rank == 0:
@@ -1090,9 +1090,9 @@ def run_remesh(args, world, rank, local):
                    "timing": "wall clock per call of the drop-in (it synchronises to check "
                              "particle displacement)"},
         # bit-exact with the reference's sequential FP64 sums, the two kernels
-        # are FP64-pipe bound: 80 FP64 instructions per particle (two IEEE
-        # divisions, eight MP4 weights) and 48 per mesh point (16 weight
-        # products, multiplies and adds), counted by ncu on this workload
+        # are FP64-pipe bound: 68 FP64 instructions per particle (two quotients
+        # by a known divisor, eight MP4 weights) and 48 per mesh point (16 weight
+        # products, multiplies and adds)
         "roofline": {"bound": "fp64", "kernel": "particles_to_mesh (stencil + gather)",
                      "achieved": FP64_INSTR_PER_PARTICLE * n_part / (p2m_ms / 1e3) / 1e9,
                      "peak": FP64_PEAK_GINSTR, "unit": "G FP64 instructions/s",
@@ -1103,7 +1103,7 @@ def run_remesh(args, world, rank, local):
                      "p2m_ms": p2m_ms,
                      "hbm_frac": alg / (p2m_ms / 1e3) / 1e9 / hbm,
                      "algorithmic_bytes": "32 B per particle"},
-        "gpu_launches": 3 * args.steps,
+        "gpu_launches": 2 * args.steps,
         "clocks": clocks.summary(),
     }
     if not args.no_cpu_baseline:
