@@ -95,7 +95,7 @@ __device__ __forceinline__ void store_split(const DctJob& job, int k, int i, flo
 template <int N>
 __device__ void dct_item_fixed(const DctJob& job, int row0, bool forward, float2* a, float2* b);
 template <int N>
-__device__ void dct_item_reg(const DctJob& job, int row0, bool forward, float2* dsm,
+__device__ void dct_item_reg(const DctJob& job, int row0, int rows, bool forward, float2* dsm,
                              const float2* tw);
 
 // Four consecutive outputs of row k (columns i .. i + 3, i a multiple of 4)
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(THREADS) dct_rows_kernel(const DctJob* __restr
     // an item are contiguous.
     const int4 nx = items[blockIdx.x + ahead];
     const DctJob& nj = jobs[nx.x];
-    const int nrows = min(rows_for(nj.N), nj.rows - nx.y);
+    const int nrows = min(nx.z, nj.rows - nx.y);
     const uint32_t bytes = (uint32_t)nrows * (uint32_t)nj.N * 4u;
     const long long off = (long long)nx.y * nj.N;
     prefetch_l2(nj.in + off, bytes);
@@ -200,15 +200,15 @@ __global__ void __launch_bounds__(THREADS) dct_rows_kernel(const DctJob* __restr
   const int N = job.N, half = N / 2;
   const int row0 = it.y;
   switch (N) {
-    case 256: dct_item_reg<256>(job, row0, forward != 0, dsm, tws); return;
-    case 512: dct_item_reg<512>(job, row0, forward != 0, dsm, tws); return;
-    case 768: dct_item_reg<768>(job, row0, forward != 0, dsm, tws); return;
-    case 1024: dct_item_reg<1024>(job, row0, forward != 0, dsm, tws); return;
+    case 256: dct_item_reg<256>(job, row0, it.z, forward != 0, dsm, tws); return;
+    case 512: dct_item_reg<512>(job, row0, it.z, forward != 0, dsm, tws); return;
+    case 768: dct_item_reg<768>(job, row0, it.z, forward != 0, dsm, tws); return;
+    case 1024: dct_item_reg<1024>(job, row0, it.z, forward != 0, dsm, tws); return;
     case 1536: dct_item_fixed<1536>(job, row0, forward != 0, a, b); return;
     case 2048: dct_item_fixed<2048>(job, row0, forward != 0, a, b); return;
     default: break;
   }
-  const int nrows = min(rows_per_item(N), job.rows - row0);
+  const int nrows = min(it.z, job.rows - row0);
   if (forward) {
     // v[n] = x[2n], v[N-1-n] = x[2n+1]
     for (int t = threadIdx.x; t < nrows * N; t += blockDim.x) {
@@ -659,9 +659,9 @@ __device__ __forceinline__ void residual_pair_to_buf(const DctJob& job, int ga, 
 
 // Work item of the register path: warp w transforms real rows 2w, 2w + 1 of
 // the item as one complex row in its own buffer; the block then stores the
-// results transposed (rows fastest).
+// results transposed (rows fastest, 2^gs groups of four rows to a column).
 template <int N>
-__device__ void dct_item_reg(const DctJob& job, int row0, bool forward, float2* dsm,
+__device__ void dct_item_reg(const DctJob& job, int row0, int rows, bool forward, float2* dsm,
                              const float2* tw) {
   constexpr int N1 = reg_n1(N);
   constexpr int W = reg_warps(N);
@@ -670,9 +670,11 @@ __device__ void dct_item_reg(const DctJob& job, int row0, bool forward, float2* 
   constexpr int RR = 2 * W;  // real rows of a full item
   static_assert(RR % 4 == 0, "float4 output groups");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nrows = min(2 * W, job.rows - row0);  // real rows of this item
+  const int nrows = min(rows, job.rows - row0);  // real rows of this item (at most 2 W)
   const int ra = 2 * warp, rb = ra + 1;
-  if (warp < W && forward && job.psi) {
+  if (ra >= nrows) {
+    // no rows for this warp
+  } else if (warp < W && forward && job.psi) {
     // refinement: the residual rows of the pair, four columns per lane and
     // float4 group at a time, straight into the warp buffer (Makhoul order)
     float2* buf = dsm + warp * BUF;
@@ -756,11 +758,12 @@ __device__ void dct_item_reg(const DctJob& job, int row0, bool forward, float2* 
   // transposed stores, four consecutive rows per thread as float4 (rows is a
   // multiple of 4 and items start at multiples of RR, so both the row count
   // of an item and the output offsets are multiples of 4)
-  constexpr int G = RR / 4;
+  const int gs = nrows > 8 ? 2 : nrows > 4 ? 1 : 0;
+  static_assert(RR <= 16, "groups of rows");
   if (forward) {
 #pragma unroll 4
-    for (int t = threadIdx.x; t < G * N; t += blockDim.x) {
-      const int k = t / G, g = t - k * G;
+    for (int t = threadIdx.x; t < N << gs; t += blockDim.x) {
+      const int k = t >> gs, g = t - (k << gs);
       const int r0 = 4 * g;
       if (r0 >= nrows) continue;
       const float2 cs = job.rot[k];
@@ -781,8 +784,8 @@ __device__ void dct_item_reg(const DctJob& job, int row0, bool forward, float2* 
   } else {
     const float inv_n = 1.0f / (float)N;
 #pragma unroll 4
-    for (int t = threadIdx.x; t < G * N; t += blockDim.x) {
-      const int j = t / G, g = t - j * G;
+    for (int t = threadIdx.x; t < N << gs; t += blockDim.x) {
+      const int j = t >> gs, g = t - (j << gs);
       const int r0 = 4 * g;
       if (r0 >= nrows) continue;
       const int src = (j & 1) ? N - 1 - (j >> 1) : (j >> 1);

@@ -92,11 +92,20 @@ __host__ __device__ inline int rows_for(int N) {
   return rows_per_item(N);
 }
 
+// Rows per work item where a launch's items are cut in `parts` (1, 2, 4 or 8):
+// at least 4, in fours, on the register path and 2 on the generic one. A row's
+// result does not depend on it.
+inline int rows_for(int N, int parts) {
+  const int r = rows_for(N), least = reg_n1(N) ? 4 : 2;
+  if (parts <= 1 || r <= least || N == 1536 || N == 2048) return r;
+  return r / parts > least ? r / parts : least;
+}
+
 // Host: Stockham radices of N (4s, then a 2, then 3s); false if N has
 // another factor or needs more than MAX_STAGES stages.
 bool plan_radices(int N, int* radix, int* nstages);
 
-// Host: launch over `n_items` work items (job, row0, -, -); forward = DCT-II
+// Host: launch over `n_items` work items (job, row0, rows, -); forward = DCT-II
 // (E_z^T x), else DCT-III (E_z y).
 // `prefetch_waves`: L2 prefetch distance in resident waves (0: one, -1: none).
 // `pdl`: as a programmatic dependent launch.

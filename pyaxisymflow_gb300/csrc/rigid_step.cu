@@ -1881,8 +1881,8 @@ int build_dct_jobs(const axi_case& k, axi_dct::DctJob* fwd, axi_dct::DctJob* inv
   return AXI_OK;
 }
 
-inline int dct_items_of(const axi_case& k) {
-  const int r = axi_dct::rows_for(k.nz);
+inline int dct_items_of(const axi_case& k, int parts) {
+  const int r = axi_dct::rows_for(k.nz, parts);
   return (k.nr + r - 1) / r;
 }
 
@@ -1915,6 +1915,21 @@ int build_dct64_jobs(const axi_case& k, axi_dct64::Job* fwd, axi_dct64::Job* inv
   inv->out = w1;
   inv->scale = t + (size_t)5 * k.nz;
   return AXI_OK;
+}
+
+// Parts to cut the transform items of a float plan in: as many as leave every
+// item a place of its own (two blocks per SM), since an item is a chain of
+// latencies, on the generic path one per row and thread. Step without / with, us:
+// 256 x 128 54.9 / 51.5, five cases of 256 x 128 to 1024 x 512 119 / 112,
+// 384 x 192 85.6 / 56.4, 648 x 324 + 288 x 144 + 216 x 108 112 / 82.6 (with
+// single rows on the generic path 57.0 and 89.3, with four 66.2 and 96.3).
+inline int dct_parts(const axi_case* cases, int n) {
+  for (int parts = 8; parts > 1; parts /= 2) {
+    long long items = 0;
+    for (int c = 0; c < n; ++c) items += dct_items_of(cases[c], parts);
+    if (items <= 2LL * axi::sm_count()) return parts;
+  }
+  return 1;
 }
 
 inline int dct64_items_of(const axi_case& k) {
@@ -2281,7 +2296,6 @@ extern "C" int axi_plan_init(axi_case* cases, int n_cases, int elem_bytes, int f
                        c, k.nz);
         return AXI_ERR_INVALID;
       }
-      if (dct) nd += dct_items_of(k);
     } else if (dct) {
       // double engine: DCT z transforms around the SIMT radial products
       int radix[axi_dct64::MAX_STAGES], ns;
@@ -2338,6 +2352,10 @@ extern "C" int axi_plan_init(axi_case* cases, int n_cases, int elem_bytes, int f
   info->elem_bytes = elem_bytes;
   info->flags = (tc ? AXI_PLAN_TENSOR_CORES : 0) | (dct ? AXI_PLAN_DCT_Z : 0) |
                 (refine ? AXI_PLAN_REFINE : 0) | (sliced ? AXI_PLAN_SLICED : 0);
+  if (tc && dct) {
+    const int parts = dct_parts(cases, n_cases);
+    for (int c = 0; c < n_cases; ++c) nd += dct_items_of(cases[c], parts);
+  }
   info->n_dct_items = nd;
   info->bytes = (int64_t)plan_offsets(info).total;
   return AXI_OK;
@@ -2412,6 +2430,7 @@ extern "C" int axi_plan_upload(const axi_case* cases, const axi_plan_info* info,
       // per pair of transforms on the 64-case ensemble), 1 plain case order,
       // 2 longest rows first
       const int order = info->tune.dct_item_order;
+      const int parts = dct_parts(cases, n);
       std::vector<int> by_case(n);
       for (int c = 0; c < n; ++c) by_case[c] = c;
       if (order == 2)
@@ -2421,8 +2440,8 @@ extern "C" int axi_plan_upload(const axi_case* cases, const axi_plan_info* info,
         for (int c : by_case) {
           if (order == 0 && (cases[c].nz == nz_min) != (pass == 1)) continue;
           if (order != 0 && pass == 1) continue;
-          const int rows = axi_dct::rows_for(cases[c].nz);
-          for (int r0 = 0; r0 < cases[c].nr; r0 += rows) di[q++] = make_int4(c, r0, 0, 0);
+          const int rows = axi_dct::rows_for(cases[c].nz, parts);
+          for (int r0 = 0; r0 < cases[c].nr; r0 += rows) di[q++] = make_int4(c, r0, rows, 0);
         }
       if (q != info->n_dct_items) {
         axi::set_error("plan_upload: cases changed since plan_init");

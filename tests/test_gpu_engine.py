@@ -468,3 +468,26 @@ def test_engine_f32_drag_sum_over_near_tiles(z_cm):
     cd32, total32, abs32 = got["f32"]
     # float products and thread sums of 8 cells: (8 + 3) 2^-24 of the terms
     assert abs(cd32 - cd / total * total32) <= abs(cd / total) * abs32 * 11 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("nz,nr", [(256, 84), (384, 92), (768, 196), (1024, 260), (972, 68)])
+def test_engine_transform_items_cut_or_whole(nz, nr):
+    """A float case alone (its transform items cut in parts) against the same case
+    among enough others that items stay whole, ragged last items on both: the
+    same bits."""
+    from pyaxisymflow_gb300.engine import RigidBodyCase, RigidEnsemble
+
+    def case(nz, nr):
+        return RigidBodyCase(nz=nz, nr=nr, dx=2.0 / nz, r_sphere=0.1, z_cm=0.5, ramp=False)
+
+    w0 = 1e-2 * np.random.default_rng(nz + nr).standard_normal((nr, nz))
+    alone = RigidEnsemble([case(nz, nr)], precision="f32", initial_vorticity=[w0])
+    others = [case(1024, 512)] * 10
+    mix = RigidEnsemble([case(nz, nr)] + others, precision="f32",
+                        initial_vorticity=[w0] + [np.zeros((512, 1024))] * 10)
+    mix.set_tuning({"plan_groups": 1})
+    alone.step(2)
+    mix.step(2)
+    torch.cuda.synchronize()
+    for f in ("omega", "psi", "psi_lo", "u_z", "u_r"):
+        assert torch.equal(alone.fields[0][f], mix.fields[0][f]), f
