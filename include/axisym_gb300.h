@@ -350,11 +350,14 @@ int axi_fd_transform_f64(double* out, int ld_out, const double* in, int ld_in,
  * row is scaled by a power of two and written as eight signed 8-bit digits;
  * products of digit planes are exact in the FP32 accumulators and summed as
  * integers, with one rounding to FP64. A row or column that holds a value
- * which is not finite gives NaN.
+ * which is not finite gives NaN. In the transform, the radial bases are scaled
+ * by powers of two against the size of the field's radial modes (or rows) and
+ * sliced on every call, so that its rows next to the axis are as accurate as
+ * with FP64 FMA products.
  *
  * The transform of axi_fd_transform_f64 with its bases sliced once:
  * axi_sliced_transform_plan writes a plan of axi_sliced_transform_bytes into
- * device memory (the four bases, its scratch and tables; synchronises the
+ * device memory (the four bases, its scratch and its tables; synchronises the
  * stream; the bases may be freed afterwards, inv_eig may not);
  * axi_sliced_transform_run applies it (eight launches, no host round trip;
  * `out` may alias `in`; calls on one plan share its scratch, so overlapping
@@ -574,8 +577,10 @@ typedef struct axi_case {
    * differences of neighbouring psi values keep the refined solve's
    * accuracy instead of the float rounding of psi. Start at zero. */
   void* psi_lo;
-  /* AXI_PLAN_SLICED: E_z^-1, E_r^-1 diag(r), E_z, E_r as sliced left operands
-   * (axi_slice_operand_f64) and a scratch of axi_sliced_field_bytes(nr, nz). */
+  /* AXI_PLAN_SLICED: E_z^-1 and E_z as sliced left operands
+   * (axi_slice_operand_f64) in [0] and [2] ([1] and [3] are not read: the radial
+   * bases are sliced in every step), and a scratch of
+   * axi_sliced_field_bytes(nr, nz). */
   const void* sliced_basis[4];
   void* sliced_field;
 } axi_case;

@@ -1713,7 +1713,8 @@ inline PlanOffsets plan_offsets(const axi_plan_info* info) {
   }
   if (info->flags & AXI_PLAN_SLICED) {
     o.slice_jobs = align16(end);
-    o.sliced_jobs = align16(o.slice_jobs + (size_t)4 * info->n_cases * sizeof(axi_sl::SliceJob));
+    o.sliced_jobs = align16(o.slice_jobs + (size_t)axi_sl::SLICE_JOBS * info->n_cases *
+                                             sizeof(axi_sl::SliceJob));
     end = o.sliced_jobs + (size_t)4 * info->n_cases * sizeof(axi_sl::GemmJob);
     for (int st = 0; st < 4; ++st) {
       o.slice_items[st] = align16(end);
@@ -2049,7 +2050,7 @@ inline bool chained(const axi_plan_info* info) {
 int run_sliced(const axi_plan_info* info, const PlanView& v, int st, cudaStream_t s) {
   AXI_TRY(axi_sl::launch_slice(v.slice_jobs, v.slice_items[st], info->n_slice_items[st], s));
   return axi_sl::launch_gemm(v.sliced_jobs, v.tc_tiles[st], info->n_tc_tiles[st],
-                             info->tile_form[st], true, v.err, s);
+                             info->tile_form[st], st % 2 == 0, v.err, s);
 }
 
 template <typename T>
@@ -2308,7 +2309,7 @@ extern "C" int axi_plan_init(axi_case* cases, int n_cases, int elem_bytes, int f
     }
     if (sliced) {
       for (int st = 0; st < 4; ++st) {
-        if (!k.sliced_basis[st] || !k.sliced_field) {
+        if ((st % 2 == 0 && !k.sliced_basis[st]) || !k.sliced_field) {
           axi::set_error("plan_init: case %d lacks sliced operands", c);
           return AXI_ERR_INVALID;
         }
@@ -2336,14 +2337,14 @@ extern "C" int axi_plan_init(axi_case* cases, int n_cases, int elem_bytes, int f
       const axi_case& k = cases[c];
       const int M = st % 2 == 0 ? k.nz : k.nr, N = st % 2 == 0 ? k.nr : k.nz;
       info->n_tc_tiles[st] += axi_sl::gemm_tiles(M, N, form);
-      groups += axi_sl::slice_groups(N, axi_sl::form_cols(form));
+      groups += axi_sl::stage_groups(k.nr, k.nz, st, form);
     }
     info->slice_groups[st] = groups;
     for (int c = 0; c < n_cases; ++c) {
       const axi_case& k = cases[c];
-      const int M = st % 2 == 0 ? k.nz : k.nr, N = st % 2 == 0 ? k.nr : k.nz;
-      info->n_slice_items[st] += axi_sl::slice_groups(N, axi_sl::form_cols(form)) *
-                                 axi_sl::slice_parts(groups, M, axi::sm_count());
+      const int K = st % 2 == 0 ? k.nz : k.nr;
+      info->n_slice_items[st] += axi_sl::stage_groups(k.nr, k.nz, st, form) *
+                                 axi_sl::slice_parts(groups, K, axi::sm_count());
     }
   }
   info->n_cases = n_cases;
@@ -2489,14 +2490,17 @@ extern "C" int axi_plan_upload(const axi_case* cases, const axi_plan_info* info,
     std::vector<int4> items[4], tiles[4];
     for (int c = 0; c < n; ++c) {
       const axi_case& k = cases[c];
+      const double* radial[2] = {static_cast<const double*>(k.Er_inv_w),
+                                 static_cast<const double*>(k.Er)};
       axi_sl::spectral_jobs(k.nr, k.nz, info->tile_form, static_cast<const double*>(k.omega), k.nz,
                             static_cast<double*>(k.psi), k.nz, static_cast<double*>(k.gemm_work),
-                            k.sliced_field, k.sliced_basis,
-                            static_cast<const double*>(k.inv_eig), sj + 4 * c, gj + 4 * c);
+                            k.sliced_field, k.sliced_basis, radial,
+                            static_cast<const double*>(k.inv_eig), sj + axi_sl::SLICE_JOBS * c,
+                            gj + 4 * c);
       for (int st = 0; st < 4; ++st) {
         const int M = st % 2 == 0 ? k.nz : k.nr, N = st % 2 == 0 ? k.nr : k.nz;
-        axi_sl::append_slice_items(
-            items[st], 4 * c + st, N, axi_sl::form_cols(info->tile_form[st]),
+        axi_sl::append_stage_items(
+            items[st], axi_sl::SLICE_JOBS * c, k.nr, k.nz, st, info->tile_form[st],
             axi_sl::slice_parts(info->slice_groups[st], M, axi::sm_count()));
         axi_sl::append_gemm_tiles(tiles[st], 4 * c + st, M, N, M, info->tile_form[st]);
       }

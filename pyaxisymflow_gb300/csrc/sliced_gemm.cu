@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "sliced_gemm.cuh"
 
@@ -30,16 +31,24 @@ constexpr int SL_THREADS = 256;
 // 128 in every byte: makes every digit non-negative
 constexpr unsigned long long DIGIT_BIAS = 0x8080808080808080ull;
 
-// x 2^62 / 2^(emax + 1 - bias) as a signed integer plus DIGIT_BIAS, whose bytes
-// are the digits plus 128; emax: the row's largest biased exponent (at least 1).
-__device__ __forceinline__ unsigned long long biased_fixed(double x, int emax) {
+// Biased exponent of x, as the row maxima count it: 0 for zeros and subnormal
+// numbers, NOT_FINITE for infinities and NaN.
+__device__ __forceinline__ int exponent_of(double x) {
+  const int e = (int)((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ff;
+  return e == 0x7ff ? NOT_FINITE : e;
+}
+
+// x 2^shift 2^62 / 2^(emax + 1 - bias) as a signed integer plus DIGIT_BIAS,
+// whose bytes are the digits plus 128; emax: the row's largest biased exponent
+// (at least 1), shifts included.
+__device__ __forceinline__ unsigned long long biased_fixed(double x, int emax, int shift) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const int e = (int)(b >> 52) & 0x7ff;
   unsigned long long m = b & 0xfffffffffffffull;
   if (e) m |= 1ull << 52;
-  const int s = emax - (e ? e : 1) - 9;  // right shift; at least -9
+  const int s = emax - (e ? e : 1) - shift - 9;  // right shift; at least -9 (m = 0: any)
   if (s <= 0)
-    m <<= -s;
+    m <<= min(-s, 9);
   else
     m = s > 54 ? 0ull : ((m >> (s - 1)) + 1) >> 1;  // rounded to nearest
   return (b >> 63) ? DIGIT_BIAS - m : DIGIT_BIAS + m;
@@ -60,7 +69,23 @@ __device__ __forceinline__ void load8(const double* p, long long ks, int n, doub
   }
 }
 
-template <bool VEC>
+// Powers of two that balance eight neighbouring K elements of a radial product
+// (spectral_jobs): the left operand's are multiplied by those of the field's
+// columns, the field's own divided by them.
+template <int BAL>
+__device__ __forceinline__ void load_shifts(const int* col_exps, int k, int K, int (&c)[8]) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) c[q] = 0;
+  if (BAL == 0 || k >= K) return;
+  const int4 a = *reinterpret_cast<const int4*>(col_exps + k);
+  const int4 b = *reinterpret_cast<const int4*>(col_exps + k + 4);
+  const int e[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+  for (int q = 0; q < 8; ++q) c[q] = BAL > 0 ? max(e[q], 1) : BALANCE_BIAS - max(e[q], 1);
+}
+
+// BAL: 0 as it is, 1 the left and -1 the right operand of a balanced product.
+template <bool VEC, int BAL>
 __device__ __forceinline__ void slice_rows(const SliceJob& j, const double* src, long long rs,
                                            int group, int part, int parts, int* s_max) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -78,10 +103,17 @@ __device__ __forceinline__ void slice_rows(const SliceJob& j, const double* src,
   } else {
     for (int k = k_lane; k < K; k += SL_THREADS) {
       double v[8];
+      int c[8];
       load8<VEC>(p + k * ks, ks, live ? min(8, K - k) : 0, v);
+      load_shifts<BAL>(j.col_exps, k, K, c);
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
-        em = max(em, (int)((unsigned long long)__double_as_longlong(v[q]) >> 52) & 0x7ff);
+      for (int q = 0; q < 8; ++q) {
+        const int e = exponent_of(v[q]);
+        if (BAL == 0)
+          em = max(em, e);
+        else if ((__double_as_longlong(v[q]) << 1) != 0)
+          em = max(em, e == NOT_FINITE ? e : max(e, 1) + c[q]);
+      }
     }
     if (threadIdx.x < 8) s_max[threadIdx.x] = 0;
     __syncthreads();
@@ -90,7 +122,7 @@ __device__ __forceinline__ void slice_rows(const SliceJob& j, const double* src,
     em = s_max[r];
     if (part == 0 && warp == 0 && lane < 8) j.exps[row] = em;
   }
-  const bool finite = em != 0x7ff;
+  const bool finite = em != NOT_FINITE;
   em = max(em, 1);
   // pass 2: the digits
   const int br = j.block;                       // rows per block of the layout
@@ -104,8 +136,10 @@ __device__ __forceinline__ void slice_rows(const SliceJob& j, const double* src,
     double v[8];
     load8<VEC>(p + k * ks, ks, live && finite ? min(8, K - k) : 0, v);
     unsigned long long f[8];
+    int c[8];
+    load_shifts<BAL>(j.col_exps, k, K, c);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) f[q] = biased_fixed(v[q], em);
+    for (int q = 0; q < 8; ++q) f[q] = biased_fixed(v[q], em, c[q]);
     uint8_t* d = dst + (size_t)(k / BK) * stage + ((k / 8) & 1) * half_stride;
 #pragma unroll
     for (int i = 0; i < DIGITS; ++i) {
@@ -150,10 +184,18 @@ __global__ void __launch_bounds__(SL_THREADS)
   for (int q = (it.y * it.w + it.z) * SL_THREADS + threadIdx.x; q < j.n_clear;
        q += (pad_rows_dev(j.rows, j.block) / 8) * it.w * SL_THREADS)
     j.clear[q] = 0;
-  if (vec)
-    slice_rows<true>(j, src, rs, it.y, it.z, it.w, s_max);
+  auto slice = [&](auto bal) {
+    if (vec)
+      slice_rows<true, bal()>(j, src, rs, it.y, it.z, it.w, s_max);
+    else
+      slice_rows<false, bal()>(j, src, rs, it.y, it.z, it.w, s_max);
+  };
+  if (j.balance == 0)
+    slice(std::integral_constant<int, 0>());
+  else if (j.balance > 0)
+    slice(std::integral_constant<int, 1>());
   else
-    slice_rows<false>(j, src, rs, it.y, it.z, it.w, s_max);
+    slice(std::integral_constant<int, -1>());
 }
 
 // ---------------------------------------------------------------------------
@@ -530,8 +572,10 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int ea_raw = job.ea[row];
       const int ea = max(ea_raw, 1) - 1022;
       const int* eb = job.eb + col0;
+      const int e_off = 68 + job.exp_bias;  // 12 + 8 * 7 of the digits' weights
       int* const row_exps = job.row_exps;
-      int e_max = 0;
+      int* const col_exps = job.col_exps;
+      int e_max = 0, e_col = 0;
       const int nk = k_end(tr.w);
       long long hi[COLS], lo[COLS];
 #pragma unroll
@@ -584,36 +628,42 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
       }
       if (!ok) break;
-      if (row < M) {
-        double* const cr = c + row * ldc + col0;
-        const double* const sr = scale ? scale + (long long)row * N + col0 : nullptr;
-        const int n = min(COLS, N - col0);
-        const bool vec = n == COLS && (reinterpret_cast<uintptr_t>(cr) & 15) == 0;
+      const bool row_in = row < M;
+      double* const cr = c + row * ldc + col0;
+      const double* const sr = scale ? scale + (long long)row * N + col0 : nullptr;
+      const int n = row_in ? min(COLS, N - col0) : 0;
+      const bool vec = n == COLS && (reinterpret_cast<uintptr_t>(cr) & 15) == 0;
 #pragma unroll
-        for (int j = 0; j < COLS; j += 2) {
-          if (SPLIT > 1 && (j < j0 || j >= j1)) continue;
-          double v[2];
+      for (int j = 0; j < COLS; j += 2) {
+        if (SPLIT > 1 && (j < j0 || j >= j1)) continue;
+        double v[2];
 #pragma unroll
-          for (int w = 0; w < 2; ++w) {
-            const int e_raw = eb[j + w];
-            const int e = max(e_raw, 1) - 1022;
-            // ea + eb - 12 - 8 * 7; a row or column that is not finite gives NaN
-            v[w] = assemble(hi[j + w], lo[j + w], ea + e - 68);
-            if (ea_raw == 0x7ff || e_raw == 0x7ff)
-              v[w] = __longlong_as_double(0x7ff8000000000000ll);
-            if (sr && j + w < n) v[w] *= sr[j + w];
-            if (j + w < n) e_max = max(e_max, (__double2hiint(v[w]) >> 20) & 0x7ff);
-          }
-          if (vec) {
-            *reinterpret_cast<double2*>(cr + j) = make_double2(v[0], v[1]);
-          } else {
-            if (j < n) cr[j] = v[0];
-            if (j + 1 < n) cr[j + 1] = v[1];
+        for (int w = 0; w < 2; ++w) {
+          const int e_raw = eb[j + w];
+          const int e = max(e_raw, 1) - 1022;
+          // a row or column that is not finite gives NaN
+          v[w] = assemble(hi[j + w], lo[j + w], ea + e - e_off);
+          if (ea_raw == NOT_FINITE || e_raw == NOT_FINITE)
+            v[w] = __longlong_as_double(0x7ff8000000000000ll);
+          if (sr && j + w < n) v[w] *= sr[j + w];
+          const int ev = j + w < n ? exponent_of(v[w]) : 0;
+          e_max = max(e_max, ev);
+          if (col_exps) {  // the largest of the column's finite values
+            const int most = __reduce_max_sync(0xffffffffu, ev == NOT_FINITE ? 0 : ev);
+            if (lane == j + w) e_col = most;
           }
         }
-        // what the next slicing needs, so that it reads its source once
-        if (row_exps && e_max > 0) atomicMax(row_exps + row, e_max);
+        if (vec) {
+          *reinterpret_cast<double2*>(cr + j) = make_double2(v[0], v[1]);
+        } else {
+          if (j < n) cr[j] = v[0];
+          if (j + 1 < n) cr[j + 1] = v[1];
+        }
       }
+      // what the next slicing needs: row maxima (so that it reads its source
+      // once) or column maxima
+      if (row_exps && e_max > 0) atomicMax(row_exps + row, e_max);
+      if (col_exps && e_col > 0 && col0 + lane < N) atomicMax(col_exps + col0 + lane, e_col);
     }
   }
   __syncthreads();
@@ -696,50 +746,74 @@ int launch_gemm(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, int
 }
 
 namespace {
-// One planes buffer that the four stages use in turn (padding to 32 rows covers
-// every form), then the row exponents of each.
+// The field's planes, which the four stages use in turn (padding to 32 rows
+// covers every form), those of the radial bases, which stages 1 and 3 do, then
+// the exponents: of each stage's field rows, of the columns of X (twice) and of
+// the radial bases' rows (twice).
 size_t spectral_plane_bytes(int nr, int nz) {
-  return (std::max(plane_bytes(nr, nz, 32), plane_bytes(nz, nr, 32)) + 255) / 256 * 256;
+  return align_up(std::max(plane_bytes(nr, nz, 32), plane_bytes(nz, nr, 32)), 256);
 }
+size_t radial_plane_bytes(int nr) { return align_up(plane_bytes(nr, nr, BM), 256); }
 }  // namespace
 
 size_t spectral_slice_bytes(int nr, int nz) {
-  return spectral_plane_bytes(nr, nz) +
-         (size_t)2 * (pad_rows(nr, 32) + pad_rows(nz, 32)) * sizeof(int);
+  return spectral_plane_bytes(nr, nz) + radial_plane_bytes(nr) +
+         (size_t)2 * (2 * pad_rows(nr, 32) + pad_rows(nz, 32) + pad_rows(nr, BM)) * sizeof(int);
 }
 
 void spectral_jobs(int nr, int nz, const int form[4], const double* in, long long ld_in,
                    double* out, int ld_out, double* work, void* slices,
-                   const void* const basis[4], const double* inv_eig, SliceJob sl[4],
-                   GemmJob gm[4]) {
+                   const void* const basis[4], const double* const radial[2],
+                   const double* inv_eig, SliceJob sl[SLICE_JOBS], GemmJob gm[4]) {
   double* x = work;
   double* y = work + (size_t)nr * nz;
-  int* exps = reinterpret_cast<int*>(static_cast<uint8_t*>(slices) + spectral_plane_bytes(nr, nz));
+  uint8_t* radial_planes = static_cast<uint8_t*>(slices) + spectral_plane_bytes(nr, nz);
+  int* exps = reinterpret_cast<int*>(radial_planes + radial_plane_bytes(nr));
+  auto take = [&exps](int n) {
+    int* p = exps;
+    exps += n;
+    return p;
+  };
+  int *rows[4], *cols[4] = {nullptr, nullptr, nullptr, nullptr};
+  for (int st = 0; st < 4; ++st) rows[st] = take(pad_rows(st % 2 == 0 ? nr : nz, 32));
+  for (int st = 0; st < 4; st += 2) cols[st] = take(pad_rows(nr, 32));
   const double* src[4] = {in, x, y, x};
   const long long rs[4] = {ld_in, nr, nz, nr};
   double* c[4] = {x, y, x, out};
   const int ldc[4] = {nr, nz, nr, ld_out};
   for (int st = 0; st < 4; ++st) {
-    const int M = st % 2 == 0 ? nz : nr, N = st % 2 == 0 ? nr : nz, K = M;
-    sl[st] = slice_job(src[st], rs[st], 1, N, K, form_cols(form[st]), slices, exps);
-    sl[st].have_exps = st > 0;
-    exps += pad_rows(N, 32);
-    if (st < 3) {
-      sl[st].clear = exps;
-      sl[st].n_clear = pad_rows(M, 32);
-    }
+    const bool along_r = st % 2 == 1;
+    const int M = along_r ? nr : nz, N = along_r ? nz : nr, K = M;
+    sl[st] = slice_job(src[st], rs[st], 1, N, K, form_cols(form[st]), slices, rows[st]);
     GemmJob& g = gm[st];
-    g.a = static_cast<const uint8_t*>(basis[st]);
-    g.ea = reinterpret_cast<const int*>(g.a + plane_bytes(M, K, BM));
     g.b = sl[st].planes;
     g.eb = sl[st].exps;
     g.c = c[st];
     g.scale = st == 1 ? inv_eig : nullptr;
-    g.row_exps = st < 3 ? exps : nullptr;
     g.M = M;
     g.N = N;
     g.ldc = ldc[st];
     g.nk = k_steps(K);
+    // X leaves its column maxima for the balanced product, Y its row maxima
+    g.col_exps = cols[st];
+    g.row_exps = st == 1 ? rows[2] : nullptr;
+    sl[st].have_exps = st == 2;
+    sl[st].clear = st == 1 ? rows[2] : cols[st];
+    sl[st].n_clear = sl[st].clear ? pad_rows(nr, 32) : 0;
+    if (along_r) {
+      SliceJob& a = sl[4 + st / 2];
+      a = slice_job(radial[st / 2], nr, 1, nr, nr, BM, radial_planes, take(pad_rows(nr, BM)));
+      a.balance = 1;
+      sl[st].balance = -1;
+      a.col_exps = sl[st].col_exps = cols[st - 1];
+      g.a = a.planes;
+      g.ea = a.exps;
+      g.exp_bias = BALANCE_BIAS;
+    } else {
+      g.a = static_cast<const uint8_t*>(basis[st]);
+      g.ea = reinterpret_cast<const int*>(g.a + plane_bytes(M, K, BM));
+      g.exp_bias = 0;
+    }
   }
 }
 
@@ -752,8 +826,8 @@ namespace {
 
 using namespace axi_sl;
 
-// Plan of the standalone transform: [SliceJob x 4][GemmJob x 4][slice items x 4]
-// [tiles x 4][error word][sliced bases x 4][sliced field][X, Y]
+// Plan of the standalone transform: [SliceJob x 6][GemmJob x 4][slice items x 4]
+// [tiles x 4][error word][sliced z bases, radial bases][sliced field][X, Y]
 struct TransformLayout {
   size_t sjobs, gjobs, items[4], tiles[4], err, basis[4], slices, work, total;
   int n_items[4], n_tiles[4], form[4], parts[4];
@@ -762,24 +836,25 @@ struct TransformLayout {
 TransformLayout transform_layout(int nr, int nz) {
   TransformLayout L;
   size_t o = 0;
-  L.sjobs = o; o = align_up(o + 4 * sizeof(SliceJob), 256);
+  L.sjobs = o; o = align_up(o + SLICE_JOBS * sizeof(SliceJob), 256);
   L.gjobs = o; o = align_up(o + 4 * sizeof(GemmJob), 256);
   for (int st = 0; st < 4; ++st) {
     const int M = st % 2 == 0 ? nz : nr, N = st % 2 == 0 ? nr : nz;
     L.form[st] = choose_form(gemm_tiles(M, N, FORM_NARROW), axi::sm_count());
-    const int groups = slice_groups(N, form_cols(L.form[st]));
+    const int groups = stage_groups(nr, nz, st, L.form[st]);
     L.parts[st] = slice_parts(groups, M, axi::sm_count());
     L.n_items[st] = groups * L.parts[st];
     L.n_tiles[st] = gemm_tiles(M, N, L.form[st]);
     // room for any form, so that the size does not depend on the device
     L.items[st] = o;
-    o = align_up(o + (size_t)slice_groups(N, 32) * ((M + 255) / 256) * sizeof(int4), 256);
+    o = align_up(o + (size_t)stage_groups(nr, nz, st, FORM_WIDE) * ((M + 255) / 256) * sizeof(int4),
+                 256);
     L.tiles[st] = o; o = align_up(o + gemm_tiles(M, N, FORM_NARROW) * sizeof(int4), 256);
   }
   L.err = o; o = align_up(o + 16, 256);
   for (int st = 0; st < 4; ++st) {
-    const int M = st % 2 == 0 ? nz : nr;
-    L.basis[st] = o; o = align_up(o + slice_bytes(M, M, BM), 256);
+    L.basis[st] = o;
+    o = align_up(o + (st % 2 == 0 ? slice_bytes(nz, nz, BM) : (size_t)nr * nr * sizeof(double)), 256);
   }
   L.slices = o; o = align_up(o + spectral_slice_bytes(nr, nz), 256);
   L.work = o; o = align_up(o + (size_t)2 * nr * nz * sizeof(double), 256);
@@ -855,27 +930,32 @@ extern "C" int axi_sliced_transform_plan(void* plan, const double* Er_inv_w, con
   cudaStream_t s = axi::as_stream(stream);
   const TransformLayout L = transform_layout(nr, nz);
   char* base = static_cast<char*>(plan);
-  // A operands: E_z^-1 and E_z are stored transposed
+  // E_z^-1 and E_z, stored transposed, sliced; copies of the radial bases
   const double* src[4] = {EzinvT, Er_inv_w, EzT, Er};
   const void* basis[4];
   for (int st = 0; st < 4; ++st) {
-    const int M = st % 2 == 0 ? nz : nr;
     basis[st] = base + L.basis[st];
-    const bool transposed = st % 2 == 0;
-    AXI_TRY(slice_now(slice_job(src[st], transposed ? 1 : M, transposed ? M : 1, M, M, BM,
-                                base + L.basis[st], exps_of(base + L.basis[st], M, M, BM)), s));
+    if (st % 2 == 0) {
+      AXI_TRY(slice_now(slice_job(src[st], 1, nz, nz, nz, BM, base + L.basis[st],
+                                  exps_of(base + L.basis[st], nz, nz, BM)), s));
+    } else if (cudaMemcpyAsync(base + L.basis[st], src[st], (size_t)nr * nr * sizeof(double),
+                               cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
+      return axi::launch_status(what);
+    }
   }
-  SliceJob sl[4];
+  const double* radial[2] = {static_cast<const double*>(basis[1]),
+                             static_cast<const double*>(basis[3])};
+  SliceJob sl[SLICE_JOBS];
   GemmJob gm[4];
   spectral_jobs(nr, nz, L.form, nullptr, nz, nullptr, nz, reinterpret_cast<double*>(base + L.work),
-                base + L.slices, basis, inv_eig, sl, gm);
+                base + L.slices, basis, radial, inv_eig, sl, gm);
   std::vector<char> head(L.err + 16, 0);
   memcpy(&head[L.sjobs], sl, sizeof(sl));
   memcpy(&head[L.gjobs], gm, sizeof(gm));
   for (int st = 0; st < 4; ++st) {
     const int M = st % 2 == 0 ? nz : nr, N = st % 2 == 0 ? nr : nz;
     std::vector<int4> items, tiles;
-    append_slice_items(items, st, N, form_cols(L.form[st]), L.parts[st]);
+    append_stage_items(items, 0, nr, nz, st, L.form[st], L.parts[st]);
     append_gemm_tiles(tiles, st, M, N, M, L.form[st]);
     memcpy(&head[L.items[st]], items.data(), items.size() * sizeof(int4));
     memcpy(&head[L.tiles[st]], tiles.data(), tiles.size() * sizeof(int4));
@@ -907,7 +987,7 @@ extern "C" int axi_sliced_transform_run(const void* plan, double* out, int ld_ou
     AXI_TRY(launch_slice(sj, reinterpret_cast<const int4*>(base + L.items[st]), L.n_items[st], s,
                          st == 0 ? in : nullptr, ld_in));
     AXI_TRY(launch_gemm(gj, reinterpret_cast<const int4*>(base + L.tiles[st]), L.n_tiles[st],
-                        L.form[st], true, err, s, st == 3 ? out : nullptr, ld_out));
+                        L.form[st], st % 2 == 0, err, s, st == 3 ? out : nullptr, ld_out));
   }
   return AXI_OK;
 }
@@ -976,7 +1056,8 @@ extern "C" int axi_sliced_gemm_f64(double* C, const double* A, const double* B, 
                     slice_job(B, K, 1, N, K, cols, base + L.b, exps_of(base + L.b, N, K, cols))};
   GemmJob g;
   g.a = sl[0].planes; g.ea = sl[0].exps; g.b = sl[1].planes; g.eb = sl[1].exps;
-  g.c = C; g.scale = S; g.row_exps = nullptr; g.M = M; g.N = N; g.ldc = N; g.nk = k_steps(K);
+  g.c = C; g.scale = S; g.row_exps = nullptr; g.col_exps = nullptr; g.exp_bias = 0;
+  g.M = M; g.N = N; g.ldc = N; g.nk = k_steps(K);
   std::vector<int4> items, tiles;
   append_slice_items(items, 0, M, BM, 1);
   append_slice_items(items, 1, N, cols, 1);

@@ -19,15 +19,25 @@
 // adds them to integer sums (96 bits, exact for any K), which it rounds to
 // FP64 once.
 //
-// Error of the four-product spectral solve against long double on the same
-// bases, 48 x 96 to 256 x 512 cells, smooth and white right-hand sides:
-// psi 0.8-2.0e-16 (FP64 FMA products 1.1-20e-16),
-// u_z 3-24e-16 (5-25e-16), u_r 4-53e-16 (8-76e-16), smaller in every case.
-// With 55 bits below the row's power of two psi stayed at 3-9e-16 but u_z and
-// u_r went to 1-6e-14 (psi near the axis is a cancelling sum), so 62 are kept.
-// Nine digits of radix 128 give the same bits with 45 plane products instead
-// of 36 and accumulators that last for K = 512; the smaller digit count won
-// (shared-memory traffic per step, which bounds the main loop, 132 -> 108 KB).
+// A digit string that starts at the row's largest value keeps 53 bits of the
+// elements within 2^9 of it and fewer of the smaller ones. Along z that is
+// enough (every row of a z basis is flat), along r it is not: the columns of E_r
+// grow with the mode where those of the field fall, so that the sums of the rows
+// next to the axis hung on elements cut short (relative errors of psi 1e-13 in
+// rows 1 to 3 and up to 1 in row 0). So a radial product is balanced: column m
+// of its left operand is multiplied by 2^c(m) and row m of the field divided by
+// it, 2^c(m) being the size of the field's largest value of index m in this
+// call. Both are exact; the left operand's rows then rank the terms of the sums as
+// they are. It costs the slicing of the radial bases in every call (a radial
+// slicing launch of eight cases 12.5 -> 22 us, their step 666 -> 714; steps of
+// one 512 x 256 case 119.5 -> 124.1, a soft sphere on 1024 x 512 453 -> 465).
+//
+// Error against long double on the same bases, 64 to 1024 radial rows (and 300, 65),
+// sources smooth at the axis, in a ring, white, within four cells of the axis,
+// and one cosine mode (FP64 FMA products in brackets): psi 0.6-8e-16
+// (1-51e-16), psi in rows 1 to 3 0.4-5e-16 (1-170e-16), in row 0, which the
+// operator decouples, 0.5e-16 to 2e-14 (3e-16 to 1e-13), the largest u_z
+// smaller or, where it is the rounding of psi at the outer wall, within 10 %.
 //
 // Why: GB300 executes FP64 at about 1.2 TFLOP/s and FP16 tensor work at about
 // 2 PFLOP/s. 36 plane products cost 36 * 2 M N K FP16 operations, 1/40 of the
@@ -81,6 +91,12 @@ constexpr int form_split(int form) {
 }
 constexpr int b_stage(int bn) { return DIGITS * bn * BK * 2; }
 
+// exponent word of a row that holds a value which is not finite (larger than
+// every biased exponent, shifted or not)
+constexpr int NOT_FINITE = 1 << 20;
+// balanced right operands carry their exponents this much higher
+constexpr int BALANCE_BIAS = 2048;
+
 enum { ERR_PRODUCER = 7, ERR_MMA = 8, ERR_EPILOGUE = 9, ERR_DRAIN = 10 };
 
 // Sliced operands are laid out in blocks of `block` rows: BM for A, the tile
@@ -89,8 +105,8 @@ inline int pad_rows(int rows, int block) { return (rows + block - 1) / block * b
 inline int k_steps(int K) { return (K + BK - 1) / BK; }
 
 // Bytes of one sliced operand: the digit planes, then one word per row, the
-// largest biased exponent of its values (0x7ff: a value is not finite, and the
-// row's products are NaN).
+// largest biased exponent of its values (NOT_FINITE: a value is not finite, and
+// the row's products are NaN).
 inline size_t plane_bytes(int rows, int K, int block) {
   return (size_t)pad_rows(rows, block) * k_steps(K) * BK * DIGITS * 2;
 }
@@ -109,6 +125,8 @@ struct SliceJob {
   int* exps;
   int* clear;    // words that the next product's epilogue accumulates into
   int n_clear;
+  int balance;   // 1 / -1: left / right operand of a balanced product, else 0
+  const int* col_exps;  // balanced: largest biased exponent of the field per K index
 };
 
 struct GemmJob {
@@ -119,8 +137,10 @@ struct GemmJob {
   double* c;
   const double* scale;  // elementwise factor, row-major (M, N), or null
   int* row_exps;        // largest exponent of each row of C, accumulated (or null)
+  int* col_exps;        // the same of each column, of its finite values (or null)
   int M, N, ldc;
   int nk;               // K steps
+  int exp_bias;         // of the operands' exponents together
 };
 
 inline SliceJob slice_job(const double* src, long long rs, long long ks, int rows, int K, int block,
@@ -132,6 +152,8 @@ inline SliceJob slice_job(const double* src, long long rs, long long ks, int row
   j.exps = exps;
   j.clear = nullptr;
   j.n_clear = 0;
+  j.balance = 0;
+  j.col_exps = nullptr;
   return j;
 }
 // The exponents behind the planes of an operand.
@@ -182,12 +204,28 @@ int launch_gemm(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, int
 //   1  Y (nr, nz)   = (Erinv_w * X^T) .* inv_eig
 //   2  X (nz, nr)   = Ez * Y^T
 //   3  out (nr, nz) = Er * X^T
-// work: X then Y (2 nr nz doubles); slices: the B operand of the stage at
-// hand (spectral_slice_bytes). basis: Ezinv, Erinv_w, Ez, Er as sliced A
-// operands.
+// work: X then Y (2 nr nz doubles); slices: the operands of the stage at hand
+// (spectral_slice_bytes). basis: Ezinv and Ez as sliced A operands (0, 2);
+// radial: Erinv_w and Er (nr, nr), row-major, which are balanced against the
+// field and sliced on every call, in the launch that slices the field.
+// sl: the field operands of the four stages, then the radial bases of stages 1
+// and 3.
+constexpr int SLICE_JOBS = 6;
 size_t spectral_slice_bytes(int nr, int nz);
-void spectral_jobs(int nr, int nz, const int form[4], const double* in, long long ld_in, double* out, int ld_out,
-                   double* work, void* slices, const void* const basis[4], const double* inv_eig,
-                   SliceJob sl[4], GemmJob gm[4]);
+void spectral_jobs(int nr, int nz, const int form[4], const double* in, long long ld_in,
+                   double* out, int ld_out, double* work, void* slices,
+                   const void* const basis[4], const double* const radial[2],
+                   const double* inv_eig, SliceJob sl[SLICE_JOBS], GemmJob gm[4]);
+// Row groups of 8 that the slicing launch of a stage covers, and its items.
+// `job0`: index of the case's first slicing job.
+inline int stage_groups(int nr, int nz, int st, int form) {
+  return st % 2 == 0 ? slice_groups(nr, form_cols(form))
+                     : slice_groups(nz, form_cols(form)) + slice_groups(nr, BM);
+}
+inline void append_stage_items(std::vector<int4>& items, int job0, int nr, int nz, int st, int form,
+                               int parts) {
+  append_slice_items(items, job0 + st, st % 2 == 0 ? nr : nz, form_cols(form), parts);
+  if (st % 2 == 1) append_slice_items(items, job0 + 4 + st / 2, nr, BM, parts);
+}
 
 }  // namespace axi_sl

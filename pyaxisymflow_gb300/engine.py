@@ -218,7 +218,8 @@ class _Bases:
     z operator of the solver is diagonal in it) and inv_eig is
     1 / (lambda_r_i + lambda_z_k) in DCT order: the float engine's z products
     become transforms and only its radial operands are kept for the tensor
-    cores. The double engine keeps all four bases as sliced operands."""
+    cores. The double engine keeps the z bases as sliced operands; the radial ones
+    are sliced in every step, balanced against the field."""
 
     def __init__(self, nr, nz, dx, dtype, device, tensor_cores=False, dct=False):
         op_r, op_z = stokes_operators(nr, nz, dx)
@@ -255,15 +256,13 @@ class _Bases:
                 self.tc.append(torch.tensor(lo, device=device))
 
     def _slice(self, device):
-        """E_z^-1, E_r^-1 diag(r), E_z, E_r as operands of the sliced products."""
-        for name, transposed in (("EzinvT", True), ("Er_inv_w", False), ("EzT", True),
-                                 ("Er", False)):
+        """E_z^-1 and E_z (stored transposed) as operands of the sliced products."""
+        for name in ("EzinvT", "EzT"):
             m = self.t[name]
             n = m.shape[0]
             out = torch.empty(int(N.lib().axi_sliced_operand_bytes(n, n)), dtype=torch.uint8,
                               device=device)
-            N.call("axi_slice_operand_f64", N.ptr(out), N.ptr(m), 1 if transposed else n,
-                   n if transposed else 1, n, n, N.stream_of(out))
+            N.call("axi_slice_operand_f64", N.ptr(out), N.ptr(m), 1, n, n, n, N.stream_of(out))
             self.sliced.append(out)
 
 
@@ -365,8 +364,7 @@ class CaseState:
         if b.dct_table is not None:
             s.dct_table = b.dct_table.data_ptr()
         if dtype == torch.float64:
-            for q in range(4):
-                s.sliced_basis[q] = b.sliced[q].data_ptr()
+            s.sliced_basis[0], s.sliced_basis[2] = (x.data_ptr() for x in b.sliced)
             s.sliced_field = t["sliced_field"].data_ptr()
         if ens.refine:
             s.psi_lo = t["psi_lo"].data_ptr()
