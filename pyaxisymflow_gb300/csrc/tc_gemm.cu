@@ -254,7 +254,9 @@ __global__ void __launch_bounds__(THREADS, 1)
       progress[1] = g;
       // every MMA of this CTA has completed once `quiet` fires
       umma_commit(quiet);
-      mbar_wait(quiet, 0, err, ERR_MMA);
+      // (also after a failure, whose code would end mbar_wait early: MMAs in
+      // flight must not outlive the block's shared and tensor memory)
+      if (!axi_tma::mbar_wait_drain(quiet, 0)) atomicCAS(err, 0, ERR_MMA);
     }
     __syncwarp();
   } else {
