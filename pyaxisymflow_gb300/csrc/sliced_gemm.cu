@@ -507,6 +507,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       int g = 0, u = 0, s = 0;
       uint32_t lap = 0;
       bool ok = true;
+      axi::pdl_wait();  // the time limit of the waits starts once the predecessor is done
       for (int t = tile0; t < n_tiles && ok; t += tile_step) {
         const int nk = k_end(tiles[t].w);
         for (int k0 = k_begin(tiles[t].w); k0 < nk && ok; k0 += CHUNK, ++u) {

@@ -219,6 +219,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       int g = 0, it = 0, s = 0;
       uint32_t lap = 0;
       bool ok = true;
+      axi::pdl_wait();  // the time limit of the waits starts once the predecessor is done
       // k-block count of the next tile, loaded one tile ahead (its latency
       // would otherwise sit between two tiles' MMAs)
       int nk_next = blockIdx.x < n_tiles ? tiles[blockIdx.x].w : 0;

@@ -23,3 +23,12 @@ def test_a_failed_block_waits_for_its_mmas(source):
     after = mma[mma.index("umma_commit(quiet)"):]
     assert "mbar_wait_drain(quiet" in after
     assert not re.search(r"\bmbar_wait\(quiet", after)
+
+
+@pytest.mark.parametrize("source", ["sliced_gemm.cu", "tc_gemm.cu"])
+@pytest.mark.parametrize("warp", [0, 1])
+def test_time_limits_start_after_the_predecessor(source, warp):
+    """A kernel of a chain may start while its predecessor runs; no wait with a
+    time limit starts before it has waited for that one."""
+    text = role(source, warp)
+    assert text.index("pdl_wait()") < re.search(r"\bmbar_wait\(", text).start()
