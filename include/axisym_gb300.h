@@ -361,8 +361,10 @@ int axi_fd_transform_f64(double* out, int ld_out, const double* in, int ld_in,
  * stream; the bases may be freed afterwards, inv_eig may not);
  * axi_sliced_transform_run applies it (eight launches, no host round trip;
  * `out` may alias `in`; calls on one plan share its scratch, so overlapping
- * calls race). axi_sliced_transform_status reads the error word of its
- * bounded waits (0: none ran out).
+ * calls race). A bounded wait that runs out leaves NaN in `out`;
+ * axi_sliced_transform_status reads the code (0: no wait ran out since the plan
+ * was written), at the first int of the plan for the last call, at the second
+ * for earlier ones. The next call starts afresh.
  * ------------------------------------------------------------------ */
 int64_t axi_sliced_transform_bytes(int nr, int nz);
 int axi_sliced_transform_plan(void* plan, const double* Er_inv_w, const double* EzinvT,

@@ -170,12 +170,17 @@ __device__ __forceinline__ int pad_rows_dev(int rows, int block) {
 // items: job, group of 8 rows, share of K, shares
 __global__ void __launch_bounds__(SL_THREADS)
     slice_kernel(const SliceJob* __restrict__ jobs, const int4* __restrict__ items,
-                 const double* src_override, long long rs_override) {
+                 const double* src_override, long long rs_override, int* err_begin) {
   __shared__ int s_max[8];
   const int4 it = items[blockIdx.x];
   const SliceJob& j = jobs[it.x];
   axi::pdl_trigger();
   axi::pdl_wait();
+  // a new run: an earlier one's failure goes to the record beside the word
+  if (err_begin && blockIdx.x == 0 && threadIdx.x == 0 && err_begin[0] != 0) {
+    err_begin[1] = err_begin[0];
+    err_begin[0] = 0;
+  }
   const double* src = src_override ? src_override : j.src;
   const long long rs = src_override ? rs_override : j.rs;
   // 16-byte loads where every row starts on 16 bytes and K runs contiguously
@@ -563,7 +568,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     int u = 0;
     bool ok = true;
     axi::pdl_wait();
-    for (int t = tile0; t < n_tiles && ok; t += tile_step) {
+    // (a failure ends the waiting, not the loop: the results of this tile and
+    // the later ones are written as NaN)
+    for (int t = tile0; t < n_tiles; t += tile_step) {
       const int4 tr = tiles[t];
       const GemmJob& job = jobs[tr.x];
       const int M = job.M, N = job.N;
@@ -583,7 +590,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       long long hi[COLS], lo[COLS];
 #pragma unroll
       for (int j = 0; j < COLS; ++j) hi[j] = lo[j] = 0;
-      for (int k0 = k_begin(tr.w); k0 < nk; k0 += CHUNK, ++u) {
+      for (int k0 = k_begin(tr.w); k0 < nk && ok; k0 += CHUNK, ++u) {
         const int set = u & 1;
         ok = __all_sync(0xffffffffu,
                         mbar_wait(acc_full + 8 * set, (u >> 1) & 1, err, ERR_EPILOGUE));
@@ -611,10 +618,11 @@ __global__ void __launch_bounds__(THREADS, 1)
             store_remote(ex + (slot * PART + j % PART) * BM * 16, to, hi[j], lo[j]);
         }
         cluster_arrive();
-        cluster_wait();  // every partial sum has arrived
+        cluster_wait();  // every partial sum has arrived, unless a block failed
+        ok = __all_sync(0xffffffffu, ok && *reinterpret_cast<volatile int*>(err) == 0);
         const int mine = rank - half * (SPLIT / 2);
         j0 = j1 = 0;
-        if (ok && mine >= 0 && mine < SPLIT / 2) {
+        if (mine >= 0 && mine < SPLIT / 2) {
           j0 = mine * PART;
           j1 = j0 + PART;
 #pragma unroll
@@ -630,7 +638,6 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
         }
       }
-      if (!ok) break;
       const bool row_in = row < M;
       double* const cr = c + row * ldc + col0;
       const double* const sr = scale ? scale + (long long)row * N + col0 : nullptr;
@@ -644,9 +651,9 @@ __global__ void __launch_bounds__(THREADS, 1)
         for (int w = 0; w < 2; ++w) {
           const int e_raw = eb[j + w];
           const int e = max(e_raw, 1) - 1022;
-          // a row or column that is not finite gives NaN
+          // a row or column that is not finite gives NaN, a failure everywhere
           v[w] = assemble(hi[j + w], lo[j + w], ea + e - e_off);
-          if (ea_raw == NOT_FINITE || e_raw == NOT_FINITE)
+          if (ea_raw == NOT_FINITE || e_raw == NOT_FINITE || !ok)
             v[w] = __longlong_as_double(0x7ff8000000000000ll);
           if (sr && j + w < n) v[w] *= sr[j + w];
           const int ev = j + w < n ? exponent_of(v[w]) : 0;
@@ -703,10 +710,10 @@ void order_tiles(std::vector<int4>& tiles) {
 }
 
 int launch_slice(const SliceJob* jobs_dev, const int4* items_dev, int n_items, cudaStream_t s,
-                 const double* src, long long rs) {
+                 const double* src, long long rs, int* err_begin) {
   if (n_items <= 0) return AXI_OK;
   return axi::launch_chain(true, "slice", slice_kernel, dim3(n_items), dim3(SL_THREADS), 0, s, 1, jobs_dev,
-                         items_dev, src, rs);
+                         items_dev, src, rs, err_begin);
 }
 
 template <int BN, int SPLIT>
@@ -829,16 +836,18 @@ namespace {
 
 using namespace axi_sl;
 
-// Plan of the standalone transform: [SliceJob x 6][GemmJob x 4][slice items x 4]
-// [tiles x 4][error word][sliced z bases, radial bases][sliced field][X, Y]
+// Plan of the standalone transform: [error word of the run, record of earlier
+// runs][SliceJob x 6][GemmJob x 4][slice items x 4][tiles x 4][sliced z bases,
+// radial bases][sliced field][X, Y]
 struct TransformLayout {
-  size_t sjobs, gjobs, items[4], tiles[4], err, basis[4], slices, work, total;
+  size_t err, sjobs, gjobs, items[4], tiles[4], basis[4], slices, work, total;
   int n_items[4], n_tiles[4], form[4], parts[4];
 };
 
 TransformLayout transform_layout(int nr, int nz) {
   TransformLayout L;
   size_t o = 0;
+  L.err = o; o = align_up(o + 16, 256);
   L.sjobs = o; o = align_up(o + SLICE_JOBS * sizeof(SliceJob), 256);
   L.gjobs = o; o = align_up(o + 4 * sizeof(GemmJob), 256);
   for (int st = 0; st < 4; ++st) {
@@ -854,7 +863,6 @@ TransformLayout transform_layout(int nr, int nz) {
                  256);
     L.tiles[st] = o; o = align_up(o + gemm_tiles(M, N, FORM_NARROW) * sizeof(int4), 256);
   }
-  L.err = o; o = align_up(o + 16, 256);
   for (int st = 0; st < 4; ++st) {
     L.basis[st] = o;
     o = align_up(o + (st % 2 == 0 ? slice_bytes(nz, nz, BM) : (size_t)nr * nr * sizeof(double)), 256);
@@ -952,7 +960,7 @@ extern "C" int axi_sliced_transform_plan(void* plan, const double* Er_inv_w, con
   GemmJob gm[4];
   spectral_jobs(nr, nz, L.form, nullptr, nz, nullptr, nz, reinterpret_cast<double*>(base + L.work),
                 base + L.slices, basis, radial, inv_eig, sl, gm);
-  std::vector<char> head(L.err + 16, 0);
+  std::vector<char> head(L.basis[0], 0);
   memcpy(&head[L.sjobs], sl, sizeof(sl));
   memcpy(&head[L.gjobs], gm, sizeof(gm));
   for (int st = 0; st < 4; ++st) {
@@ -988,7 +996,7 @@ extern "C" int axi_sliced_transform_run(const void* plan, double* out, int ld_ou
   int* err = reinterpret_cast<int*>(base + L.err);
   for (int st = 0; st < 4; ++st) {
     AXI_TRY(launch_slice(sj, reinterpret_cast<const int4*>(base + L.items[st]), L.n_items[st], s,
-                         st == 0 ? in : nullptr, ld_in));
+                         st == 0 ? in : nullptr, ld_in, st == 0 ? err : nullptr));
     AXI_TRY(launch_gemm(gj, reinterpret_cast<const int4*>(base + L.tiles[st]), L.n_tiles[st],
                         L.form[st], st % 2 == 0, err, s, st == 3 ? out : nullptr, ld_out));
   }
@@ -1002,11 +1010,12 @@ extern "C" int axi_sliced_transform_status(const void* plan, int nr, int nz, int
   AXI_TRY(check_shape(what, nr, nz));
   AXI_TRY(axi::check_ptrs(what, {plan, error}, {"plan", "error"}));
   cudaStream_t s = axi::as_stream(stream);
-  const char* base = static_cast<const char*>(plan);
-  if (cudaMemcpyAsync(error, base + transform_layout(nr, nz).err, sizeof(int),
-                      cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+  int words[2];
+  if (cudaMemcpyAsync(words, static_cast<const char*>(plan) + transform_layout(nr, nz).err,
+                      sizeof(words), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return axi::launch_status(what);
+  *error = words[0] ? words[0] : words[1];
   return AXI_OK;
 }
 

@@ -194,8 +194,11 @@ void order_tiles(std::vector<int4>& tiles);
 // The first operand's source / the output may be given per call (overrides,
 // null: as in the job table; only for tables of one job). a_ready: A is not written by kernels still
 // running, so it may be read ahead of the launch's dependencies.
+// A product whose bounded waits run out sets *err_dev and writes NaN; later waits
+// on a set word give up early. err_begin: two words, of which the first slicing
+// of a run clears [0] (the word of its products) after moving a code to [1].
 int launch_slice(const SliceJob* jobs_dev, const int4* items_dev, int n_items, cudaStream_t s,
-                 const double* src = nullptr, long long rs = 0);
+                 const double* src = nullptr, long long rs = 0, int* err_begin = nullptr);
 int launch_gemm(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, int form, bool a_ready,
                 int* err_dev, cudaStream_t s, double* c = nullptr, int ldc = 0);
 

@@ -97,6 +97,14 @@ class AxiTcPlanInfo(ctypes.Structure):
                 ("tile_cols", ctypes.c_uint8 * 4), ("bytes", ctypes.c_int64)]
 
 
+def sliced_status(plan, nr, nz):
+    """Error code of an axi_sliced_transform_plan (synchronises)."""
+    err = ctypes.c_int(0)
+    N.call("axi_sliced_transform_status", N.ptr(plan), nr, nz, ctypes.byref(err),
+           N.stream_of(plan))
+    return err.value
+
+
 class FastDiagonalisationEngine:
     """Device copy of one eigenbasis set and the transform that applies it.
 
@@ -191,11 +199,11 @@ class FastDiagonalisationEngine:
         N.call("axi_tc_transform_run", ctypes.byref(self.tc_info), N.ptr(self.tc_plan), s)
 
     def status(self):
-        """Error code of the FP64 products' bounded waits (0: none ran out)."""
-        err = ctypes.c_int(0)
-        N.call("axi_sliced_transform_status", N.ptr(self.plan), self.grid_size_r,
-               self.grid_size_z, ctypes.byref(err), N.stream_of(self.plan))
-        return err.value
+        """Error code of the products' bounded waits (0: none has run out; a
+        solve in which one did leaves NaN)."""
+        if self.precision == "f32":
+            return self.tc_status()
+        return sliced_status(self.plan, self.grid_size_r, self.grid_size_z)
 
     def tc_status(self):
         err = ctypes.c_int(0)

@@ -16,6 +16,7 @@ import numpy as np
 import torch
 
 from . import _native as N
+from .kernels._spectral import sliced_status
 from .kernels.advect_vorticity_via_eno3 import gen_advect_vorticity_via_eno3
 from .kernels.brinkmann_penalize import brinkmann_penalize
 from .kernels.compute_velocity_from_psi import compute_velocity_from_psi_unb
@@ -143,6 +144,9 @@ class RigidSphereSimulation:
         N.call("axi_sphere_speed_f64", N.ptr(self.u_z), N.ptr(self.u_r), float(c.U0 * prefac),
                c.nr * c.nz, N.ptr(self._umax), s)
         umax = self._umax.item()
+        if not math.isfinite(umax) and self.solver.engine.status():
+            raise RuntimeError("the spectral solve failed: a wait on the tensor-core pipeline "
+                               "ran out")
         dt = min(0.9 * dx ** 2 / 4 / c.nu, c.cfl * dx / (umax + EPS))
         N.call("axi_sphere_penalise_f64", N.ptr(w), N.ptr(self.penal), N.ptr(self.u_z),
                N.ptr(self.u_r), N.ptr(self.u_z_upen), N.ptr(self.u_r_upen), N.ptr(self.char_func),
@@ -435,8 +439,13 @@ class SoftSphereEngine:
         return int(self.state[SOFT_STEPS])
 
     def status(self):
-        """Sticky status bits (1 << AXI_ERR_*; 0 = healthy)."""
-        return int(self.state[SOFT_STATUS:SOFT_STATUS + 1].cpu().numpy().view(np.uint64)[0])
+        """Sticky status bits (1 << AXI_ERR_*; 0 = healthy); AXI_ERR_CUDA: a wait
+        in the products of a solve ran out."""
+        bits = int(self.state[SOFT_STATUS:SOFT_STATUS + 1].cpu().numpy().view(np.uint64)[0])
+        plan = self.plan_dct if self.dct else self.sim.solver.engine.plan
+        if sliced_status(plan, self.case.nr, self.case.nz):
+            bits |= 1 << self._N.AXI_ERR_CUDA
+        return bits
 
     # the fields, as SoftSphereSimulation names them
     def __getattr__(self, name):
