@@ -2050,7 +2050,7 @@ inline bool chained(const axi_plan_info* info) {
 int run_sliced(const axi_plan_info* info, const PlanView& v, int st, cudaStream_t s) {
   AXI_TRY(axi_sl::launch_slice(v.slice_jobs, v.slice_items[st], info->n_slice_items[st], s));
   return axi_sl::launch_gemm(v.sliced_jobs, v.tc_tiles[st], info->n_tc_tiles[st],
-                             info->tile_form[st], st % 2 == 0, v.err, s);
+                             info->tile_form[st], v.err, s);
 }
 
 template <typename T>

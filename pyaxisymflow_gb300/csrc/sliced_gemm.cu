@@ -167,11 +167,32 @@ __device__ __forceinline__ int pad_rows_dev(int rows, int block) {
   return (rows + block - 1) / block * block;
 }
 
-// items: job, group of 8 rows, share of K, shares
+// One item: a group of 8 rows, and share `part` of `parts` of its K.
+__device__ __forceinline__ void slice_item(const SliceJob& j, const double* src, long long rs,
+                                           int group, int part, int parts) {
+  __shared__ int s_max[8];
+  // 16-byte loads where every row starts on 16 bytes and K runs contiguously
+  const bool vec = j.ks == 1 && (rs & 1) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+  auto slice = [&](auto bal) {
+    if (vec)
+      slice_rows<true, bal()>(j, src, rs, group, part, parts, s_max);
+    else
+      slice_rows<false, bal()>(j, src, rs, group, part, parts, s_max);
+  };
+  if (j.balance == 0)
+    slice(std::integral_constant<int, 0>());
+  else if (j.balance > 0)
+    slice(std::integral_constant<int, 1>());
+  else
+    slice(std::integral_constant<int, -1>());
+}
+
+// items: job, group of 8 rows, share of K, shares. The tables are written and
+// synchronised when the plan is made, long before this launch, so that they may
+// be read ahead of its dependencies.
 __global__ void __launch_bounds__(SL_THREADS)
     slice_kernel(const SliceJob* __restrict__ jobs, const int4* __restrict__ items,
                  const double* src_override, long long rs_override, int* err_begin) {
-  __shared__ int s_max[8];
   const int4 it = items[blockIdx.x];
   const SliceJob& j = jobs[it.x];
   axi::pdl_trigger();
@@ -181,26 +202,17 @@ __global__ void __launch_bounds__(SL_THREADS)
     err_begin[1] = err_begin[0];
     err_begin[0] = 0;
   }
-  const double* src = src_override ? src_override : j.src;
-  const long long rs = src_override ? rs_override : j.rs;
-  // 16-byte loads where every row starts on 16 bytes and K runs contiguously
-  const bool vec = j.ks == 1 && (rs & 1) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
-  // the next product's row exponents start at zero
+  // what the next product's epilogue accumulates into starts at zero
   for (int q = (it.y * it.w + it.z) * SL_THREADS + threadIdx.x; q < j.n_clear;
        q += (pad_rows_dev(j.rows, j.block) / 8) * it.w * SL_THREADS)
     j.clear[q] = 0;
-  auto slice = [&](auto bal) {
-    if (vec)
-      slice_rows<true, bal()>(j, src, rs, it.y, it.z, it.w, s_max);
-    else
-      slice_rows<false, bal()>(j, src, rs, it.y, it.z, it.w, s_max);
-  };
-  if (j.balance == 0)
-    slice(std::integral_constant<int, 0>());
-  else if (j.balance > 0)
-    slice(std::integral_constant<int, 1>());
-  else
-    slice(std::integral_constant<int, -1>());
+  slice_item(j, src_override ? src_override : j.src, src_override ? rs_override : j.rs, it.y, it.z,
+             it.w);
+}
+
+// One matrix, a group of rows per block, without tables.
+__global__ void __launch_bounds__(SL_THREADS) slice_matrix_kernel(const SliceJob j) {
+  slice_item(j, j.src, j.rs, blockIdx.x, 0, 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -354,37 +366,7 @@ __device__ __forceinline__ double assemble(long long hi, long long lo, int e) {
   return sign ? -v : v;
 }
 
-// A may be read ahead of the predecessor's end; the successor may start early.
-enum { FLAG_A_READY = 1, FLAG_TRIGGER = 2 };
-
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_arrive() {
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() {
-  __syncwarp();
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// 16 bytes into the shared memory of block `rank` of the cluster, at the place
-// that `addr` has in this block
-__device__ __forceinline__ void store_remote(uint32_t addr, int rank, long long x, long long y) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  asm volatile("st.shared::cluster.v2.b64 [%0], {%1, %2};" ::"r"(r), "l"(x), "l"(y) : "memory");
-}
-
-// partial sums received from the other blocks of a split tile
-constexpr int exchange_bytes(int bn, int split) {
-  return split > 1 ? (split - 1) * BM * (bn / split) * 16 : 0;
-}
-constexpr int smem_bytes(int bn, int split) {
-  return NSTAGE * (A_STAGE + b_stage(bn)) + exchange_bytes(bn, split) + 128 + 256;
-}
+constexpr int smem_bytes(int bn) { return NSTAGE * (A_STAGE + b_stage(bn)) + 128 + 256; }
 
 // Persistent, warp-specialised: warp 0 copies stages, warp 1 issues MMAs,
 // warps 2 .. 9 (two per TMEM lane quarter, BN / 2 columns each) drain one of
@@ -395,18 +377,16 @@ constexpr int smem_bytes(int bn, int split) {
 // (the tensor rate) and 32 + N / 4 (its operands at 128 bytes per cycle), 624 a
 // step of 16 K with BN = 32, into which the copies of the next steps write
 // another 40 KB. The issuing thread took 844 a step until it ran under
-// elect.sync; the four products of 512 x 256 then went from 61.6 to 52.2 us and
-// those of eight cases from 418 to 380. (Sharing A's loads between the blocks
-// of a cluster by multicast changed nothing: 199.6 against 198.3 us for a
-// 1024 x 512 solve.)
+// elect.sync (the four products of 512 x 256 then went from 61.6 to 52.2 us, those
+// of eight cases from 418 to 380).
 //
-// SPLIT > 1: a cluster of SPLIT blocks per tile, each taking a share of its K;
-// then every block finishes BN / SPLIT of the columns, with the partial sums
-// that the others wrote into its shared memory.
-template <int BN, int SPLIT>
+// A block ends when no asynchronous operation of its own can still reach its
+// shared memory: its loads are consumed, its MMAs complete, and the releases of
+// its last stages have arrived.
+template <int BN>
 __global__ void __launch_bounds__(THREADS, 1)
     sliced_gemm_kernel(const GemmJob* __restrict__ jobs, const int4* __restrict__ tiles,
-                       int n_tiles, int flags, int* __restrict__ err, double* c_override,
+                       int n_tiles, int trigger, int* __restrict__ err, double* c_override,
                        int ldc_override) {
   constexpr int B_STAGE = b_stage(BN);
   constexpr int STAGE_BYTES = A_STAGE + B_STAGE;
@@ -415,17 +395,11 @@ __global__ void __launch_bounds__(THREADS, 1)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) &
                                              ~static_cast<uintptr_t>(127));
-  uint8_t* exchange = smem + NSTAGE * STAGE_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(exchange + exchange_bytes(BN, SPLIT));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + NSTAGE * STAGE_BYTES);
   // full[NSTAGE], empty[NSTAGE], acc_full[2], acc_empty[2], quiet
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NSTAGE + 5);
   int* progress = reinterpret_cast<int*>(tmem_slot + 1);  // [0] loads issued, [1] consumed
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = SPLIT > 1 ? (int)cluster_rank() : 0;
-  // first tile of this block, its stride, and its share of a tile's K steps
-  const int tile0 = blockIdx.x / SPLIT, tile_step = gridDim.x / SPLIT;
-  auto k_begin = [rank](int nk) { return nk * rank / SPLIT; };
-  auto k_end = [rank](int nk) { return nk * (rank + 1) / SPLIT; };
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + NSTAGE);
   const uint32_t acc_full = smem_u32(bars + 2 * NSTAGE);
   const uint32_t acc_empty = smem_u32(bars + 2 * NSTAGE + 2);
@@ -434,8 +408,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   // The next kernel of the chain (slicing) may start early only where this one
   // leaves half of the SMs free: its blocks do not fit beside these, and on few
   // free SMs they would pile up (a 1024 x 512 solve: 174 -> 198 us).
-  if (flags & FLAG_TRIGGER) axi::pdl_trigger();
-  if (SPLIT > 1) cluster_arrive();  // (waited for before the first remote store)
+  if (trigger) axi::pdl_trigger();
   if (threadIdx.x == 0) {
     for (int s = 0; s < NSTAGE; ++s) {
       mbar_init(full0 + 8 * s, 1);
@@ -464,47 +437,35 @@ __global__ void __launch_bounds__(THREADS, 1)
       int g = 0, s = 0;
       uint32_t lap = 1;  // parity of the phase that frees a stage
       bool ok = true;
-      int ahead = 0;  // first steps of the first tile whose A is already on its way
-      if (flags & FLAG_A_READY) {
-        const int4 tr = tiles[tile0];
-        const uint8_t* a = jobs[tr.x].a + ((size_t)tr.y * tr.w + k_begin(tr.w)) * A_STAGE;
-        const int steps = k_end(tr.w) - k_begin(tr.w);
-        for (; ahead < steps && ahead < NSTAGE; ++ahead) {
-          mbar_expect_tx(full0 + 8 * ahead, STAGE_BYTES);
-          bulk_load(smem_u32(smem + ahead * STAGE_BYTES), a + (size_t)ahead * A_STAGE, A_STAGE,
-                    full0 + 8 * ahead);
-        }
-      }
       axi::pdl_wait();
-      for (int t = tile0; t < n_tiles && ok; t += tile_step) {
+      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
         const int4 tr = tiles[t];  // job, row block of A, row block of B, K steps
         const GemmJob& job = jobs[tr.x];
         const int nk = tr.w;
         const uint8_t* a = job.a + (size_t)tr.y * nk * A_STAGE;
         const uint8_t* b = job.b + (size_t)tr.z * nk * B_STAGE;
-        for (int kb = k_begin(nk); kb < k_end(nk); ++kb, ++g) {
+        for (int kb = 0; kb < nk; ++kb, ++g) {
           if (g >= NSTAGE && !mbar_wait(empty0 + 8 * s, lap, err, ERR_PRODUCER)) {
             ok = false;
             break;
           }
           const uint32_t st = smem_u32(smem + s * STAGE_BYTES);
           const uint32_t fb = full0 + 8 * s;
-          if (g >= ahead) {
-            mbar_expect_tx(fb, STAGE_BYTES);
-            bulk_load(st, a + (size_t)kb * A_STAGE, A_STAGE, fb);
-          }
+          mbar_expect_tx(fb, STAGE_BYTES);
+          bulk_load(st, a + (size_t)kb * A_STAGE, A_STAGE, fb);
           bulk_load(st + A_STAGE, b + (size_t)kb * B_STAGE, B_STAGE, fb);
           if (++s == NSTAGE) s = 0, lap ^= 1;
         }
       }
-      progress[0] = g > ahead ? g : ahead;
+      progress[0] = g;
+      // releases of the last stages (commits arrive on their barriers by
+      // themselves, also after the block has gone)
+      for (int q = 0; q < NSTAGE && ok; ++q) {
+        if (g + q >= NSTAGE) ok = mbar_wait(empty0 + 8 * s, lap, err, ERR_PRODUCER);
+        if (++s == NSTAGE) s = 0, lap ^= 1;
+      }
     }
     __syncwarp();
-    if (SPLIT > 1) {
-      cluster_wait();
-      cluster_arrive();
-      cluster_wait();
-    }
   } else if (warp == 1) {
     if (elect_one()) {
       const uint64_t a0 = operand_desc(smem_u32(smem), BM / 8 * 128);
@@ -513,9 +474,9 @@ __global__ void __launch_bounds__(THREADS, 1)
       uint32_t lap = 0;
       bool ok = true;
       axi::pdl_wait();  // the time limit of the waits starts once the predecessor is done
-      for (int t = tile0; t < n_tiles && ok; t += tile_step) {
-        const int nk = k_end(tiles[t].w);
-        for (int k0 = k_begin(tiles[t].w); k0 < nk && ok; k0 += CHUNK, ++u) {
+      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+        const int nk = tiles[t].w;
+        for (int k0 = 0; k0 < nk && ok; k0 += CHUNK, ++u) {
           const int set = u & 1, use = u >> 1;
           if (use > 0 && !mbar_wait(acc_empty + 8 * set, (use - 1) & 1, err, ERR_MMA)) {
             ok = false;
@@ -556,11 +517,6 @@ __global__ void __launch_bounds__(THREADS, 1)
       if (!axi_tma::mbar_wait_drain(quiet, 0)) atomicCAS(err, 0, ERR_MMA);
     }
     __syncwarp();
-    if (SPLIT > 1) {
-      cluster_wait();
-      cluster_arrive();
-      cluster_wait();
-    }
   } else {
     const int q = warp & 3;            // TMEM lane quarter
     const int half = (warp - 2) >> 2;  // columns COLS half .. COLS half + COLS - 1
@@ -570,7 +526,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     axi::pdl_wait();
     // (a failure ends the waiting, not the loop: the results of this tile and
     // the later ones are written as NaN)
-    for (int t = tile0; t < n_tiles; t += tile_step) {
+    for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
       const int4 tr = tiles[t];
       const GemmJob& job = jobs[tr.x];
       const int M = job.M, N = job.N;
@@ -586,11 +542,11 @@ __global__ void __launch_bounds__(THREADS, 1)
       int* const row_exps = job.row_exps;
       int* const col_exps = job.col_exps;
       int e_max = 0, e_col = 0;
-      const int nk = k_end(tr.w);
+      const int nk = tr.w;
       long long hi[COLS], lo[COLS];
 #pragma unroll
       for (int j = 0; j < COLS; ++j) hi[j] = lo[j] = 0;
-      for (int k0 = k_begin(tr.w); k0 < nk && ok; k0 += CHUNK, ++u) {
+      for (int k0 = 0; k0 < nk && ok; k0 += CHUNK, ++u) {
         const int set = u & 1;
         ok = __all_sync(0xffffffffu,
                         mbar_wait(acc_full + 8 * set, (u >> 1) & 1, err, ERR_EPILOGUE));
@@ -603,41 +559,6 @@ __global__ void __launch_bounds__(THREADS, 1)
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty + 8 * set)
                        : "memory");
       }
-      int j0 = 0, j1 = COLS;  // columns that this warp finishes
-      if constexpr (SPLIT > 1) {
-        // columns PART r .. of the tile are finished by block r; this warp's
-        // columns belong to blocks half SPLIT / 2 ..
-        constexpr int PART = BN / SPLIT;
-        const uint32_t ex = smem_u32(exchange) + (32 * q + lane) * 16;
-        cluster_wait();  // every block of the cluster is running
-#pragma unroll
-        for (int j = 0; j < COLS; ++j) {
-          const int to = half * (SPLIT / 2) + j / PART;
-          const int slot = rank < to ? rank : rank - 1;  // by sender, without `to` itself
-          if (to != rank && ok)
-            store_remote(ex + (slot * PART + j % PART) * BM * 16, to, hi[j], lo[j]);
-        }
-        cluster_arrive();
-        cluster_wait();  // every partial sum has arrived, unless a block failed
-        ok = __all_sync(0xffffffffu, ok && *reinterpret_cast<volatile int*>(err) == 0);
-        const int mine = rank - half * (SPLIT / 2);
-        j0 = j1 = 0;
-        if (mine >= 0 && mine < SPLIT / 2) {
-          j0 = mine * PART;
-          j1 = j0 + PART;
-#pragma unroll
-          for (int j = 0; j < COLS; ++j) {
-            if (j < j0 || j >= j1) continue;
-#pragma unroll
-            for (int slot = 0; slot < SPLIT - 1; ++slot) {
-              const longlong2 v = *reinterpret_cast<const longlong2*>(
-                  exchange + ((slot * PART + j % PART) * BM + 32 * q + lane) * 16);
-              hi[j] += v.x;
-              lo[j] += v.y;
-            }
-          }
-        }
-      }
       const bool row_in = row < M;
       double* const cr = c + row * ldc + col0;
       const double* const sr = scale ? scale + (long long)row * N + col0 : nullptr;
@@ -645,7 +566,6 @@ __global__ void __launch_bounds__(THREADS, 1)
       const bool vec = n == COLS && (reinterpret_cast<uintptr_t>(cr) & 15) == 0;
 #pragma unroll
       for (int j = 0; j < COLS; j += 2) {
-        if (SPLIT > 1 && (j < j0 || j >= j1)) continue;
         double v[2];
 #pragma unroll
         for (int w = 0; w < 2; ++w) {
@@ -710,49 +630,37 @@ void order_tiles(std::vector<int4>& tiles) {
 }
 
 int launch_slice(const SliceJob* jobs_dev, const int4* items_dev, int n_items, cudaStream_t s,
-                 const double* src, long long rs, int* err_begin) {
+                 const double* src, long long rs, int* err_begin, bool chained) {
   if (n_items <= 0) return AXI_OK;
-  return axi::launch_chain(true, "slice", slice_kernel, dim3(n_items), dim3(SL_THREADS), 0, s, 1, jobs_dev,
+  return axi::launch_chain(chained, "slice", slice_kernel, dim3(n_items), dim3(SL_THREADS), 0, s, 1, jobs_dev,
                          items_dev, src, rs, err_begin);
 }
 
-template <int BN, int SPLIT>
-int launch_tiles(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, bool a_ready,
-                 int* err_dev, cudaStream_t s, double* c, int ldc) {
+template <int BN>
+int launch_tiles(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, int* err_dev,
+                 cudaStream_t s, double* c, int ldc) {
   static std::once_flag once;
   static cudaError_t attr_status = cudaSuccess;
   std::call_once(once, [] {
-    attr_status = cudaFuncSetAttribute(sliced_gemm_kernel<BN, SPLIT>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       smem_bytes(BN, SPLIT));
+    attr_status = cudaFuncSetAttribute(sliced_gemm_kernel<BN>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(BN));
   });
   if (attr_status != cudaSuccess) {
-    axi::set_error("sliced GEMM: cannot reserve %d bytes of shared memory",
-                   smem_bytes(BN, SPLIT));
+    axi::set_error("sliced GEMM: cannot reserve %d bytes of shared memory", smem_bytes(BN));
     return AXI_ERR_CUDA;
   }
   if (n_tiles <= 0) return AXI_OK;
   const int sms = axi::sm_count();
-  // a split tile's blocks take one tile (the exchange is used once)
-  const int blocks = SPLIT > 1 ? SPLIT * n_tiles : n_tiles < sms ? n_tiles : sms;
-  return axi::launch_chain(true, "sliced_gemm", sliced_gemm_kernel<BN, SPLIT>, dim3(blocks), dim3(THREADS),
-                         smem_bytes(BN, SPLIT), s, SPLIT, jobs_dev, tiles_dev, n_tiles,
-                         (a_ready ? FLAG_A_READY : 0) | (2 * blocks <= sms ? FLAG_TRIGGER : 0),
-                         err_dev, c, ldc);
+  const int blocks = n_tiles < sms ? n_tiles : sms;
+  return axi::launch_chain(true, "sliced_gemm", sliced_gemm_kernel<BN>, dim3(blocks),
+                           dim3(THREADS), smem_bytes(BN), s, 1, jobs_dev, tiles_dev, n_tiles,
+                           2 * blocks <= sms ? 1 : 0, err_dev, c, ldc);
 }
 
-int launch_gemm(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, int form, bool a_ready,
-                int* err_dev, cudaStream_t s, double* c, int ldc) {
-  switch (form) {
-    case FORM_NARROW4:
-      return launch_tiles<16, 4>(jobs_dev, tiles_dev, n_tiles, a_ready, err_dev, s, c, ldc);
-    case FORM_NARROW2:
-      return launch_tiles<16, 2>(jobs_dev, tiles_dev, n_tiles, a_ready, err_dev, s, c, ldc);
-    case FORM_NARROW:
-      return launch_tiles<16, 1>(jobs_dev, tiles_dev, n_tiles, a_ready, err_dev, s, c, ldc);
-    default:
-      return launch_tiles<32, 1>(jobs_dev, tiles_dev, n_tiles, a_ready, err_dev, s, c, ldc);
-  }
+int launch_gemm(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, int form, int* err_dev,
+                cudaStream_t s, double* c, int ldc) {
+  return form == FORM_NARROW ? launch_tiles<16>(jobs_dev, tiles_dev, n_tiles, err_dev, s, c, ldc)
+                             : launch_tiles<32>(jobs_dev, tiles_dev, n_tiles, err_dev, s, c, ldc);
 }
 
 namespace {
@@ -873,26 +781,11 @@ TransformLayout transform_layout(int nr, int nz) {
   return L;
 }
 
-// Slices one matrix (blocking: the job record is copied from this stack).
+// Slices one matrix and waits for it.
 int slice_now(const SliceJob& j, cudaStream_t s) {
-  std::vector<int4> items;
-  append_slice_items(items, 0, j.rows, j.block, 1);
-  const size_t off = align_up(sizeof(SliceJob), 256);
-  char* d = nullptr;
-  if (cudaMallocAsync(reinterpret_cast<void**>(&d), off + items.size() * sizeof(int4), s) !=
-      cudaSuccess)
-    return axi::launch_status("slice");
-  int st = AXI_OK;
-  if (cudaMemcpyAsync(d, &j, sizeof(j), cudaMemcpyHostToDevice, s) != cudaSuccess ||
-      cudaMemcpyAsync(d + off, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice,
-                      s) != cudaSuccess)
-    st = axi::launch_status("slice");
-  if (st == AXI_OK)
-    st = launch_slice(reinterpret_cast<const SliceJob*>(d), reinterpret_cast<const int4*>(d + off),
-                      (int)items.size(), s);
-  cudaFreeAsync(d, s);
-  if (cudaStreamSynchronize(s) != cudaSuccess && st == AXI_OK) st = axi::launch_status("slice");
-  return st;
+  slice_matrix_kernel<<<slice_groups(j.rows, j.block), SL_THREADS, 0, s>>>(j);
+  AXI_TRY(axi::launch_status("slice"));
+  return cudaStreamSynchronize(s) == cudaSuccess ? AXI_OK : axi::launch_status("slice");
 }
 
 int check_shape(const char* what, int a, int b) {
@@ -998,7 +891,7 @@ extern "C" int axi_sliced_transform_run(const void* plan, double* out, int ld_ou
     AXI_TRY(launch_slice(sj, reinterpret_cast<const int4*>(base + L.items[st]), L.n_items[st], s,
                          st == 0 ? in : nullptr, ld_in, st == 0 ? err : nullptr));
     AXI_TRY(launch_gemm(gj, reinterpret_cast<const int4*>(base + L.tiles[st]), L.n_tiles[st],
-                        L.form[st], st % 2 == 0, err, s, st == 3 ? out : nullptr, ld_out));
+                        L.form[st], err, s, st == 3 ? out : nullptr, ld_out));
   }
   return AXI_OK;
 }
@@ -1082,11 +975,11 @@ extern "C" int axi_sliced_gemm_f64(double* C, const double* A, const double* B, 
   if (cudaMemcpyAsync(work, head.data(), head.size(), cudaMemcpyHostToDevice, s) != cudaSuccess)
     return axi::launch_status(what);
   AXI_TRY(launch_slice(reinterpret_cast<const SliceJob*>(base + L.sjobs),
-                       reinterpret_cast<const int4*>(base + L.items), L.n_items, s));
+                       reinterpret_cast<const int4*>(base + L.items), L.n_items, s, nullptr, 0,
+                       nullptr, false));  // (its tables were copied just now)
   int* err = reinterpret_cast<int*>(base + L.err);
   AXI_TRY(launch_gemm(reinterpret_cast<const GemmJob*>(base + L.gjob),
-                      reinterpret_cast<const int4*>(base + L.tiles), L.n_tiles, L.form, false, err,
-                      s));
+                      reinterpret_cast<const int4*>(base + L.tiles), L.n_tiles, L.form, err, s));
   int code = 0;
   if (cudaMemcpyAsync(&code, err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)

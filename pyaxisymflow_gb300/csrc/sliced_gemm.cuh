@@ -59,8 +59,8 @@
 // TMEM columns, so a K step of 16 takes 8 MMAs.
 //
 // Slicing and product kernels form a chain of programmatic dependent launches:
-// a kernel sets up its barriers and TMEM, reads its job and fills its stages
-// with A (constant) while its predecessor finishes.
+// a kernel sets up its barriers and TMEM or reads its item while its predecessor
+// finishes.
 #pragma once
 
 #include <cuda.h>
@@ -81,14 +81,9 @@ constexpr int CHUNK = 128 / BK;                      // K steps whose sums stay 
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 32 * (2 + EPI_WARPS);
 
-// Forms of a product launch: columns of C per tile (= rows of a block of B),
-// and blocks that share a tile's K (a cluster; their exact integer sums are
-// exchanged through distributed shared memory, so the split changes no bit).
-enum Form { FORM_WIDE = 0, FORM_NARROW = 1, FORM_NARROW2 = 2, FORM_NARROW4 = 3 };
+// Forms of a product launch: columns of C per tile (= rows of a block of B).
+enum Form { FORM_WIDE = 0, FORM_NARROW = 1 };
 constexpr int form_cols(int form) { return form == FORM_WIDE ? 32 : 16; }
-constexpr int form_split(int form) {
-  return form == FORM_NARROW4 ? 4 : form == FORM_NARROW2 ? 2 : 1;
-}
 constexpr int b_stage(int bn) { return DIGITS * bn * BK * 2; }
 
 // exponent word of a row that holds a value which is not finite (larger than
@@ -175,16 +170,10 @@ inline int gemm_tiles(int M, int N, int form) {
   const int cols = form_cols(form);
   return ((M + BM - 1) / BM) * ((N + cols - 1) / cols);
 }
-// Form of a launch that has `narrow_tiles` tiles of 16 columns: the most blocks
-// that all run at once. Solves (four products and slicings, us) wide / narrow /
-// narrow, K in two / in four: 128 x 64 cells 56 / 40 / 38 / 33, 256 x 128 70 /
-// 53 / 47 / 40, 512 x 256 104 / 81 / 64 / 85, 768 x 384 130 / 109 / 140 / 187,
-// 1024 x 512 159 / 229 / 312 / 391.
+// Form of a launch that has `narrow_tiles` tiles of 16 columns: narrow where they
+// all run at once.
 inline int choose_form(int narrow_tiles, int sms) {
-  return 4 * narrow_tiles <= sms   ? FORM_NARROW4
-         : 2 * narrow_tiles <= sms ? FORM_NARROW2
-         : narrow_tiles <= sms     ? FORM_NARROW
-                                   : FORM_WIDE;
+  return narrow_tiles <= sms ? FORM_NARROW : FORM_WIDE;
 }
 void append_slice_items(std::vector<int4>& items, int job, int rows, int block, int parts);
 void append_gemm_tiles(std::vector<int4>& tiles, int job, int M, int N, int K, int form);
@@ -192,14 +181,16 @@ void append_gemm_tiles(std::vector<int4>& tiles, int job, int M, int N, int K, i
 void order_tiles(std::vector<int4>& tiles);
 
 // The first operand's source / the output may be given per call (overrides,
-// null: as in the job table; only for tables of one job). a_ready: A is not written by kernels still
-// running, so it may be read ahead of the launch's dependencies.
+// null: as in the job table; only for tables of one job). chained: as a
+// programmatic dependent launch, which reads its tables ahead of its
+// dependencies (not where the stream has only just copied them).
 // A product whose bounded waits run out sets *err_dev and writes NaN; later waits
 // on a set word give up early. err_begin: two words, of which the first slicing
 // of a run clears [0] (the word of its products) after moving a code to [1].
 int launch_slice(const SliceJob* jobs_dev, const int4* items_dev, int n_items, cudaStream_t s,
-                 const double* src = nullptr, long long rs = 0, int* err_begin = nullptr);
-int launch_gemm(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, int form, bool a_ready,
+                 const double* src = nullptr, long long rs = 0, int* err_begin = nullptr,
+                 bool chained = true);
+int launch_gemm(const GemmJob* jobs_dev, const int4* tiles_dev, int n_tiles, int form,
                 int* err_dev, cudaStream_t s, double* c = nullptr, int ldc = 0);
 
 // The four spectral products of one case on sliced operands (as C = A B^T):

@@ -207,6 +207,12 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
       }
       progress[0] = g;
+      // releases of the last stages (commits arrive on their barriers by
+      // themselves, also after the block has gone)
+      for (int q = 0; q < NSTAGE && ok; ++q) {
+        if (g + q >= NSTAGE) ok = mbar_wait(empty0 + 8 * s, lap, err, ERR_PRODUCER);
+        if (++s == NSTAGE) s = 0, lap ^= 1;
+      }
     }
     __syncwarp();
   } else if (warp == 1) {
