@@ -87,6 +87,60 @@ def ensemble_cases(workload, seed=4):
     return cases
 
 
+# characters of the line on stdout; readers that keep the end of a program's
+# output (3000 characters) must find the whole of it there
+LINE_CHARS = 2400
+LINE_KEYS = ("impl", "metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+             "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "config", "e2e",
+             "gpu_launches", "clocks", "status_ok", "roofline")
+
+
+def _rounded(x):
+    """Floats to seven significant digits."""
+    if isinstance(x, dict):
+        return {k: _rounded(v) for k, v in x.items()}
+    if isinstance(x, (list, tuple)):
+        return [_rounded(v) for v in x]
+    return float(f"{x:.7g}") if isinstance(x, float) else x
+
+
+def _scalars(x):
+    """The numbers, truth values and short texts of a record, without what is
+    nested deeper."""
+    if not isinstance(x, dict):
+        return x
+    return {k: v for k, v in x.items()
+            if not isinstance(v, (dict, list)) and len(str(v)) <= 60}
+
+
+def compact(line, limit=LINE_CHARS):
+    """The measurement and, while they fit, the records that explain it: whole,
+    else their scalars, else named in "omitted"."""
+    line = _rounded(line)
+    out = {k: line[k] for k in LINE_KEYS if k in line}
+    if len(json.dumps(out)) > limit // 2 and "roofline" in out:
+        out["roofline"] = _scalars(out["roofline"])
+    omitted = []
+    for k in line:
+        if k in out:
+            continue
+        for v in (line[k], _scalars(line[k])):
+            if len(json.dumps({**out, k: v, "omitted": omitted})) + 60 <= limit:
+                out[k] = v
+                break
+        else:
+            omitted.append(k)
+    if omitted:
+        out["omitted"] = omitted
+    return out
+
+
+def emit(line):
+    """One JSON line on stdout; the whole record on stderr."""
+    print(json.dumps(line), file=sys.stderr, flush=True)
+    print(json.dumps(compact(line)), flush=True)
+
+
 def peaks():
     path = os.path.join(HERE, "MEASURED_PEAKS.json")
     if os.path.exists(path):
@@ -378,7 +432,7 @@ def run_reference(args, world, rank):
                 "cpu_baseline": rec,
                 "e2e": {"value": rec["value"], "unit": UNIT, "h2d_bytes_per_step": 0,
                         "d2h_bytes_per_step": 0}}
-        print(json.dumps(line), flush=True)
+        emit(line)
         return
     cases = ensemble_cases(args.workload)
     cores = host_cores()
@@ -401,7 +455,7 @@ def run_reference(args, world, rank):
                          "sample": desc, "cpu_model": rec["cpu_model"]},
         "e2e": {"value": value, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
-    print(json.dumps(line), flush=True)
+    emit(line)
 
 
 def phase_times(ens, ids, rounds, stream):
@@ -671,7 +725,7 @@ def run_gb300(args, world, rank, local):
         except Exception as exc:  # noqa: BLE001
             line["cpu_baseline"] = {"error": f"{type(exc).__name__}: {exc}"[:500]}
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        emit(line)
 
 
 def vortex_rings(nr, nz, dx, seed=3, n=32):
@@ -792,7 +846,7 @@ def run_poisson(args, world, rank, local):
         "status_ok": s32.engine.tc_status() == 0,
     }
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        emit(line)
 
 
 def soft_case():
@@ -929,7 +983,7 @@ def run_soft(args, world, rank, local):
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         line["cpu_baseline"] = soft_cpu_record(case, seconds=12.0)
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        emit(line)
 
 
 def soft_cpu_record(case, seconds):
@@ -1027,7 +1081,7 @@ def run_serve(args, world, rank, local):
         "gpu_launches": 8 * leg["steps"],
     }
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        emit(line)
 
 
 def run_remesh(args, world, rank, local):
@@ -1125,7 +1179,7 @@ def run_remesh(args, world, rank, local):
                                 "kind": "port",
                                 "sample": f"{snz} x {snr} cells, {n} steps, numpy oracle, "
                                           f"{secs:.1f} s"}
-    print(json.dumps(line), flush=True)
+    emit(line)
 
 
 def main():
