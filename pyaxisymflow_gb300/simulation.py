@@ -320,11 +320,12 @@ class SoftSphereEngine:
         self.inv_eig_dct = torch.tensor(1.0 / (eng.eig_vals_r.reshape(nr, 1)
                                                + lam_z.reshape(1, nz)), **f64)
         EzT = torch.tensor(cosine_basis(nz), **f64)
+        EzinvT = EzT.T.contiguous()
         self.plan_dct = torch.empty(int(N.lib().axi_sliced_transform_bytes(nr, nz)),
                                     dtype=torch.uint8, device=self.device)
         d = eng.dev
         N.call("axi_sliced_transform_plan", N.ptr(self.plan_dct), N.ptr(d["Er_inv_w"]),
-               N.ptr(EzT.T.contiguous()), N.ptr(self.inv_eig_dct), N.ptr(d["Er"]), N.ptr(EzT), nr,
+               N.ptr(EzinvT), N.ptr(self.inv_eig_dct), N.ptr(d["Er"]), N.ptr(EzT), nr,
                nz, N.stream_of(EzT))
 
     def _solve(self, st):
