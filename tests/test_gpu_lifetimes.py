@@ -18,7 +18,8 @@ def watched(monkeypatch):
 
     def watch(t, *args):
         if isinstance(t, torch.Tensor):
-            taken.append(weakref.ref(t))
+            # (a view's memory is its base's)
+            taken.append(weakref.ref(t if t._base is None else t._base))
         return ptr(t, *args)
 
     def checked(name, *args):
