@@ -358,7 +358,9 @@ int axi_fd_transform_f64(double* out, int ld_out, const double* in, int ld_in,
  * The transform of axi_fd_transform_f64 with its bases sliced once:
  * axi_sliced_transform_plan writes a plan of axi_sliced_transform_bytes into
  * device memory (the four bases, its scratch and its tables; synchronises the
- * stream; the bases may be freed afterwards, inv_eig may not);
+ * stream; the bases may be freed afterwards, inv_eig may not; 32 nz^2 +
+ * 16 nr^2 bytes of bases, 16 a cell and 16 nr^2 of digit planes, 16 a cell of
+ * intermediates);
  * axi_sliced_transform_run applies it (eight launches, no host round trip;
  * `out` may alias `in`; calls on one plan share its scratch, so overlapping
  * calls race). A bounded wait that runs out leaves NaN in `out`;

@@ -13,9 +13,10 @@
 // the pre-sweep flag), so front cells are independent and run in parallel;
 // the arithmetic keeps the reference's order (no FMA) and gives the same bits.
 //
-// Layout: one multi-block pass collects the candidate cells (current ^
-// target) into a list; one CTA then runs all sweeps over that list, with an
-// iteration cap. Neighbours outside the array count as unknown; a window that
+// Layout: one multi-block pass collects the candidate cells (current ^ target)
+// into a list. Eight sweeps over that list are spread over the GPU (one launch
+// each on flags that the mirroring pass made, three on the caller's own); one
+// block runs any that are still needed, up to the cap. Neighbours outside the array count as unknown; a window that
 // leaves the array sets AXI_ERR_RANGE (the reference reads out of bounds).
 #include "axi_common.cuh"
 

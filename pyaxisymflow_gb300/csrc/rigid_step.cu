@@ -2034,11 +2034,15 @@ struct StencilGrid {
 
 // The launches of a float step with DCTs chain as programmatic dependent
 // launches (each sets up its barriers, TMEM, job and twiddle table while its
-// predecessor drains) where a plan is small. Without / with, us per step: one
-// 256 x 128 case 65.9 / 62.8, five cases of 256 x 128 to 1024 x 512 (544 tiles)
-// 150.8 / 142.9; but 64 cases (2 x 4496 tiles) 748 / 758, the dense products of
-// 500 x 252 101 / 106 and eight cases of the double engine 723 / 728: there the
-// blocks that wait take room from others, or start on SMs with cold caches.
+// predecessor drains) where a plan is small. Without / with, us per step. Steps
+// launched one by one: 256 x 128 67.0 / 46.1, 512 x 256 75.8 / 61.6, 768 x 384
+// 84.1 / 79.7, 1024 x 512 92.4 / 87.8. One step to a graph: 256 x 128 52.6 / 51.2,
+// five cases of 256 x 128 to 1024 x 512 (544 tiles) 116 / 111. Many steps to a
+// graph, which closes the gaps by itself: up to 450 tiles the early blocks only
+// take room (256 x 128 49.9 / 51.7, 768 x 384 67.7 / 77.5), 480 to 2048 tiles gain
+// (four of 1024 x 512 129 / 125), from 2300 on it is even or worse (12 of them,
+// 3072 tiles, 306 / 317; the two groups of 64 cases, 4496 tiles each, 748 / 758).
+// The dense products of 500 x 252 took 101 / 106.
 constexpr int CHAIN_TILES = 1024;
 inline bool chained(const axi_plan_info* info) {
   return info->elem_bytes == 4 && (info->flags & AXI_PLAN_DCT_Z) &&

@@ -377,8 +377,7 @@ constexpr int smem_bytes(int bn) { return NSTAGE * (A_STAGE + b_stage(bn)) + 128
 // (the tensor rate) and 32 + N / 4 (its operands at 128 bytes per cycle), 624 a
 // step of 16 K with BN = 32, into which the copies of the next steps write
 // another 40 KB. The issuing thread took 844 a step until it ran under
-// elect.sync (the four products of 512 x 256 then went from 61.6 to 52.2 us, those
-// of eight cases from 418 to 380).
+// elect.sync (those of eight cases then went from 418 to 380 us).
 //
 // A block ends when no asynchronous operation of its own can still reach its
 // shared memory: its loads are consumed, its MMAs complete, and the releases of
@@ -406,8 +405,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   const uint32_t quiet = smem_u32(bars + 2 * NSTAGE + 4);
 
   // The next kernel of the chain (slicing) may start early only where this one
-  // leaves half of the SMs free: its blocks do not fit beside these, and on few
-  // free SMs they would pile up (a 1024 x 512 solve: 174 -> 198 us).
+  // leaves half of the SMs free: its blocks do not fit beside these (registers),
+  // and on few free SMs they would pile up (a 1024 x 512 solve: 174 -> 198 us).
   if (trigger) axi::pdl_trigger();
   if (threadIdx.x == 0) {
     for (int s = 0; s < NSTAGE; ++s) {

@@ -29,8 +29,9 @@
 // it, 2^c(m) being the size of the field's largest value of index m in this
 // call. Both are exact; the left operand's rows then rank the terms of the sums as
 // they are. It costs the slicing of the radial bases in every call (a radial
-// slicing launch of eight cases 12.5 -> 22 us, their step 666 -> 714; steps of
-// one 512 x 256 case 119.5 -> 124.1, a soft sphere on 1024 x 512 453 -> 465).
+// slicing launch of eight cases of 256 x 128 to 1024 x 512: 12.5 -> 22 us, their
+// step 666 -> 714; the step of one 512 x 256 case 4.6 us, of a soft sphere on
+// 1024 x 512 cells 12).
 //
 // Error against long double on the same bases, 64 to 1024 radial rows (and 300, 65),
 // sources smooth at the axis, in a ring, white, within four cells of the axis,
@@ -40,14 +41,12 @@
 // smaller or, where it is the rounding of psi at the outer wall, within 10 %.
 //
 // Why: GB300 executes FP64 at about 1.2 TFLOP/s and FP16 tensor work at about
-// 2 PFLOP/s. 36 plane products cost 36 * 2 M N K FP16 operations, 1/40 of the
-// time of the FP64 pipe. Measured, a soft-sphere step on 1024 x 512 cells (four
-// products): 4169 us with FP64 FMA products, 1143 us with the first form of
-// these; a double engine step of eight cases of 256 x 128 to 1024 x 512: 3543 us
-// with FP64 DCTs in z and FMA products in r, 837 us with four of these. From
-// nine 7-bit digits and one tile form to the present (solve alone, us): 256 x
-// 128 80 -> 40, 512 x 256 109 -> 62, 1024 x 512 174 -> 154, 2048 x 1024 910 ->
-// 859.
+// 2 PFLOP/s; 36 plane products cost 36 * 2 M N K FP16 operations. A solve (four
+// products) takes, in us: 128 x 64 cells 41, 256 x 128 50, 512 x 256 68, 768 x 384
+// 85, 1024 x 512 142, 2048 x 1024 724 (36 TFLOP/s of FP64 products, 1.28 PFLOP/s
+// of FP16 ones). Steps with FP64 FMA products / with these: soft sphere on 1024 x
+// 512 cells 4171 / 460, double engine at 512 x 256 with FP64 DCTs in z 300 / 133,
+// with eigenvectors in z 553 / 134, at 2048 x 1024 (FP64 DCTs) 8062 / 1062.
 //
 // Operands are laid out by the slicing kernel exactly as shared memory wants
 // them: per block of rows and per 16 K-elements one contiguous piece (A: 128
@@ -171,7 +170,12 @@ inline int gemm_tiles(int M, int N, int form) {
   return ((M + BM - 1) / BM) * ((N + cols - 1) / cols);
 }
 // Form of a launch that has `narrow_tiles` tiles of 16 columns: narrow where they
-// all run at once.
+// all run at once. Steps of the double engine (all four launches in one form), us,
+// wide / narrow: 128 x 64 124 / 105, 256 x 128 133 / 111, eight of them 142 / 118,
+// 512 x 256 (64 tiles a launch) 156 / 130, 768 x 384 (144) 190 / 154, three of 512
+// x 256 (192) 201 / 203, 1024 x 512 (256) 251 / 271, 2048 x 1024 (1024) 1061 / 1174.
+// A mix of uneven cases just above the line would gain 4 % by narrow tiles (176
+// and 198 tiles: 202 / 194, 214 / 206).
 inline int choose_form(int narrow_tiles, int sms) {
   return narrow_tiles <= sms ? FORM_NARROW : FORM_WIDE;
 }

@@ -192,7 +192,7 @@ def dct_ok(nz, precision="f32"):
 
 def dct_table(nz, dtype=np.float32):
     """Tables of the z transform (layout of axi_case.dct_table), float for the
-    float engine, double for the double engine: exp(-2 pi i m / nz) as
+    float engine, double for the FP64 DCT entries: exp(-2 pi i m / nz) as
     (cos, sin), (cos, sin)(pi k / 2 nz), c_k, 1 / c_k."""
     m = np.arange(nz, dtype=np.float64)
     tw = np.stack([np.cos(2 * np.pi * m / nz), -np.sin(2 * np.pi * m / nz)], axis=1)
