@@ -746,6 +746,9 @@ using namespace axi_sl;
 // Plan of the standalone transform: [error word of the run, record of earlier
 // runs][SliceJob x 6][GemmJob x 4][slice items x 4][tiles x 4][sliced z bases,
 // radial bases][sliced field][X, Y]
+// It depends on the grid alone, so that a run finds the plan that was written,
+// whatever device is current: the forms and shares are those of a GB300.
+constexpr int PLAN_SMS = 152;
 struct TransformLayout {
   size_t err, sjobs, gjobs, items[4], tiles[4], basis[4], slices, work, total;
   int n_items[4], n_tiles[4], form[4], parts[4];
@@ -759,9 +762,9 @@ TransformLayout transform_layout(int nr, int nz) {
   L.gjobs = o; o = align_up(o + 4 * sizeof(GemmJob), 256);
   for (int st = 0; st < 4; ++st) {
     const int M = st % 2 == 0 ? nz : nr, N = st % 2 == 0 ? nr : nz;
-    L.form[st] = choose_form(gemm_tiles(M, N, FORM_NARROW), axi::sm_count());
+    L.form[st] = choose_form(gemm_tiles(M, N, FORM_NARROW), PLAN_SMS);
     const int groups = stage_groups(nr, nz, st, L.form[st]);
-    L.parts[st] = slice_parts(groups, M, axi::sm_count());
+    L.parts[st] = slice_parts(groups, M, PLAN_SMS);
     L.n_items[st] = groups * L.parts[st];
     L.n_tiles[st] = gemm_tiles(M, N, L.form[st]);
     // room for any form, so that the size does not depend on the device

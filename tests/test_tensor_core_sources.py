@@ -32,3 +32,20 @@ def test_time_limits_start_after_the_predecessor(source, warp):
     time limit starts before it has waited for that one."""
     text = role(source, warp)
     assert text.index("pdl_wait()") < re.search(r"\bmbar_wait\(", text).start()
+
+
+def test_standalone_plan_depends_on_the_grid_alone():
+    """The plan and the run of a transform form its layout each; neither asks the
+    device that happens to be current."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / "sliced_gemm.cu").read_text())
+    start = text.index("TransformLayout transform_layout(")
+    assert "sm_count" not in text[start:text.index("\n}\n", start)]
+
+
+@pytest.mark.parametrize("source", ["sliced_gemm.cu", "tc_gemm.cu"])
+def test_a_block_waits_for_the_releases_of_its_last_stages(source):
+    """Commits arrive on the stages' barriers by themselves; the copying warp waits
+    for the last ones before the block ends."""
+    text = role(source, 0)
+    tail = text[text.index("progress[0] = g"):]
+    assert re.search(r"g \+ q >= NSTAGE\) ok = mbar_wait\(empty0 \+ 8 \* s, lap", tail)
