@@ -121,7 +121,9 @@ def compact(line, limit=LINE_CHARS):
     if len(json.dumps(out)) > limit // 2 and "roofline" in out:
         out["roofline"] = _scalars(out["roofline"])
     omitted = []
-    for k in line:
+    # the comparisons before the autotuner's trials
+    first = [k for k in ("cpu_baseline", "plain_fp64", "serving") if k in line]
+    for k in first + sorted((k for k in line if k not in first), key=lambda k: k == "tuning"):
         if k in out:
             continue
         for v in (line[k], _scalars(line[k])):

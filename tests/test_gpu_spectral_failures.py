@@ -63,8 +63,8 @@ def test_sphere_loop_raises_on_a_failed_solve(monkeypatch):
 @pytest.mark.parametrize("nz,nr", [(128, 64), (512, 256), (1024, 512)])
 def test_engine_products_after_a_failure_are_right_or_nan(nz, nr):
     """With the plan's word set (it is not cleared there) waits may give up: psi
-    holds no value that is neither the product's nor NaN, for each of the tile
-    forms (K in four shares, two, wide tiles)."""
+    holds no value that is neither the product's nor NaN, with narrow tiles (two
+    sizes) and wide ones."""
     from pyaxisymflow_gb300.engine import RigidBodyCase, RigidEnsemble
     w0 = np.random.default_rng(nz).standard_normal((nr, nz))
     psi = []
