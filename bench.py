@@ -152,6 +152,15 @@ def peaks():
     return 6800.0, 1900.0, "fallback"
 
 
+def sliced_roofline(useful_tflops, bf16, src):
+    """Roofline of the FP64 products: each is 36 FP16 products of digit planes
+    (8 digits, the pairs whose weight reaches the result), and the FP16 dense
+    rate is the BF16 rate."""
+    return {"bound": "tensor", "achieved": 36 * useful_tflops, "peak": bf16, "unit": "TFLOP/s",
+            "useful_tflops": useful_tflops,
+            "peak_source": f"{src} bf16 (FP16 dense rate; 36 plane products each)"}
+
+
 class ClockSampler:
     """nvidia-smi clocks / throttle reasons sampled during the timed region."""
 
@@ -636,7 +645,8 @@ def run_gb300(args, world, rank, local):
         PHASE_FIELDS["advect_diffuse"] += 1   # the rebuilt mask
     if uses_refine:
         PHASE_FIELDS["penalise"] += 1         # psi_lo
-    zname = "z_transforms" if uses_dct else "z_products"
+    # the double engine's z transforms are products with the basis either way
+    zname = "z_transforms" if uses_dct and args.precision == "f32" else "z_products"
     kern_ms = {"kill": ph_ms["kill"], zname: part_ms[0] + part_ms[2],
                "r_products": part_ms[1] + part_ms[3], "vel_max": ph_ms["vel_max"],
                "penalise": ph_ms["penalise"], "advect_diffuse": ph_ms["advect_diffuse"]}
@@ -646,12 +656,11 @@ def run_gb300(args, world, rank, local):
         flops = sum(4.0 * (c.nr * c.nr * c.nz if dom == "r_products" else c.nz * c.nz * c.nr)
                     for c in cases)
         achieved = flops / (kern_ms[dom] / 1000.0) / 1e12
-        if args.precision == "f64" or not uses_tc:
-            roof = {"bound": "fp64" if args.precision == "f64" else "fp32",
-                    "achieved": achieved, "peak": 1.25 if args.precision == "f64" else 73.0,
-                    "unit": "TFLOP/s",
-                    "peak_source": "nominal GB300 FP64 (DFMA probe on this pool: 1.0)"
-                    if args.precision == "f64" else "nominal GB300 FP32"}
+        if args.precision == "f64":
+            roof = sliced_roofline(achieved, bf16, src)
+        elif not uses_tc:
+            roof = {"bound": "fp32", "achieved": achieved, "peak": 73.0, "unit": "TFLOP/s",
+                    "peak_source": "nominal GB300 FP32"}
         else:
             # 3xTF32: three tensor products per useful product; the TF32 dense
             # rate is half the BF16 rate
@@ -693,7 +702,9 @@ def run_gb300(args, world, rank, local):
         "roofline": roof,
         "phase_ms": ph_ms,
         "kernel_ms": kern_ms,
-        "transform": "z DCT + radial tensor-core products" if uses_dct
+        "transform": "FP64 products of digit planes on the tensor cores"
+                     if args.precision == "f64"
+                     else "z DCT + radial tensor-core products" if uses_dct
                      else ("tensor-core products" if uses_tc else "SIMT products"),
         "step_latency_ms": {"p50": float(np.percentile(step_ms, 50)),
                             "p99": float(np.percentile(step_ms, 99))},
@@ -907,13 +918,12 @@ def run_soft(args, world, rank, local):
     part_ms = {name: sum(pev[q][k][0].elapsed_time(pev[q][k][1]) for q in range(nph)) / nph
                for k, name in enumerate(eng.PARTS)}
     dom = max(part_ms, key=part_ms.get)
-    hbm, _, src = peaks()
+    hbm, bf16, src = peaks()
     if dom == "solve_velocity_dt":
         # the four FP64 products of the spectral solve: 2 n m k flops each
         flops = 4.0 * (case.nr * case.nz * case.nz + case.nr * case.nr * case.nz)
         achieved = flops / (part_ms[dom] / 1e3) / 1e12
-        roof = {"bound": "fp64", "achieved": achieved, "peak": 1.25, "unit": "TFLOP/s",
-                "peak_source": "nominal GB300 FP64 (dense products; no FP64 tensor path)"}
+        roof = sliced_roofline(achieved, bf16, src)
     else:
         # FP64 fields read + written per cell by the group (algorithmic)
         fields = {"advect_pin_mask": 23, "extrapolate": 12, "solid_stress": 17,
